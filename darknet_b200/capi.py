@@ -26,7 +26,7 @@ EXPORTS = (
     "xnor_b200_conv_forward_static", "xnor_b200_take_device_status",
     "xnor_b200_pack_input_pooled", "xnor_b200_conv_forward_pooled", "xnor_b200_float_conv_small", "xnor_b200_float_conv3_io", "xnor_b200_float_conv_map_weights_bytes",
     "xnor_b200_float_conv_map_prepare", "xnor_b200_float_conv_map", "xnor_b200_float_conv_map_yolo", "xnor_b200_float_conv_1x1_tc", "xnor_b200_yolo_activate", "xnor_b200_region_activate", "xnor_b200_conv_forward_io", "xnor_b200_conv_takes_masks", "xnor_b200_tap_major_weights",
-    "xnor_b200_yolo_detections", "xnor_b200_nms_sort", "xnor_b200_detection_rows",
+    "xnor_b200_yolo_detections", "xnor_b200_nms_sort", "xnor_b200_detection_rows", "xnor_b200_detect", "xnor_b200_rows_to_host",
     "xnor_b200_measure_popc_peak", "xnor_b200_measure_bmma_peak", "xnor_b200_measure_umma_i8_peak", "xnor_b200_measure_umma_mxf4_peak",
 )
 
@@ -143,6 +143,8 @@ def lib() -> C.CDLL:
     L.xnor_b200_yolo_detections.argtypes = [C.POINTER(YoloHead), ci, ci, ci, ci, ci, C.c_float, ci, ci, ci, C.POINTER(Detections), vp]
     L.xnor_b200_nms_sort.argtypes = [C.POINTER(Detections), ci, C.c_float, vp]
     L.xnor_b200_detection_rows.argtypes = [C.POINTER(Detections), ci, vp, ci, vp, vp]
+    L.xnor_b200_detect.argtypes = [C.POINTER(YoloHead), ci, ci, ci, ci, ci, ci, C.c_float, ci, ci, C.c_float, C.POINTER(Detections), vp, ci, vp, vp]
+    L.xnor_b200_rows_to_host.argtypes = [vp, ci, vp, ci, ci, vp, vp, vp]
     L.xnor_b200_conv_forward_static.argtypes = [dp, vp, vp, vp, vp, vp, vp, vp, vp]
     L.xnor_b200_take_device_status.argtypes = [C.POINTER(ci)]
     L.xnor_b200_measure_popc_peak.argtypes = [ci, C.POINTER(C.c_double), C.POINTER(C.c_double)]

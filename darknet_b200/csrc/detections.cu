@@ -12,129 +12,60 @@
 //                               the compact result a host copies back instead of the whole head tensors (Darknet pulls
 //                               batch * outputs floats per head and walks them on the CPU).
 //
-// All three run on the caller's stream, allocate nothing and synchronise nothing; counts live in device memory, so a head can
+//   xnor_b200_detect            the three in one launch.
+//
+// All run on the caller's stream, allocate nothing and synchronise nothing; counts live in device memory, so a head can
 // be appended behind another without the host knowing how many detections the first one found.
 #include "xnor_common.cuh"
+
+#include <cooperative_groups.h>
 
 namespace xnor
 {
 
-constexpr int DET_THREADS = 256;
-constexpr int DET_MAX_ANCHORS = 16;
+namespace cg = cooperative_groups;
 
-struct YoloParams
+constexpr int DET_CLUSTER = 8;            // CTAs per image
+constexpr int DET_THREADS = 512;
+constexpr int DET_WARPS = DET_THREADS / 32;
+constexpr int DET_ALL_WARPS = DET_CLUSTER * DET_WARPS;
+constexpr int DET_STEP = 4;               // candidates a thread looks at between two scans
+constexpr int DET_MAX_ANCHORS = 16;
+constexpr int DET_MAX_HEADS = 4;
+constexpr int DET_LIST_BYTES = 8;         // per candidate of one class: score, storage index, rank order
+constexpr int DET_SMEM_BUDGET = 192 * 1024;
+constexpr int DET_WARP_MAX = 64;          // candidates of one class that a warp suppresses by itself; more go to the whole CTA
+constexpr int DET_BLOCK = 128;            // ranks the CTA settles at a time
+
+struct YoloHeadParams
 {
 	const float * head;          // [batch][n][4 + 1 + classes][lh * lw], activated (xnor_b200_yolo_activate)
-	int batch, lw, lh, n, classes;
+	int lw, lh, n, new_coords;
 	float anchor_w[DET_MAX_ANCHORS], anchor_h[DET_MAX_ANCHORS];      // biases[2 * mask[a]], biases[2 * mask[a] + 1]
-	int netw, neth, img_w, img_h;
+};
+
+struct DetectParams
+{
+	// decode (n_heads > 0)
+	YoloHeadParams heads[DET_MAX_HEADS];
+	int n_heads, append;
+	int netw, neth, img_w, img_h, relative, letter;
 	float thresh;
-	int relative, letter, new_coords, append;
+	// the lists
 	float * boxes;               // [batch][max_dets][4]
 	float * objectness;          // [batch][max_dets]
 	float * probs;               // [batch][max_dets][classes]
 	int * count;                 // [batch]: detections found so far (may exceed max_dets: the surplus is not stored)
-	int max_dets;
+	int max_dets, classes;
+	// suppression
+	int nms;
+	float nms_thresh;
+	int lists;                   // per-class candidate lists that fit a CTA's shared memory (at most one per warp)
+	// compaction (rows != nullptr)
+	float * rows;                // [batch][max_rows][7]
+	int * row_count;             // [batch]: pairs found (may exceed max_rows: the surplus is not stored)
+	int max_rows;
 };
-
-// Exclusive prefix sum of one flag per thread over the CTA; returns this thread's offset, *total = number of set flags.
-__device__ __forceinline__ int block_scan_flags(bool flag, int * s_warp, int * total)
-{
-	const int lane = threadIdx.x & 31;
-	const int warp = threadIdx.x >> 5;
-	const unsigned ballot = __ballot_sync(0xffffffffu, flag);
-	const int in_warp = __popc(ballot & ((1u << lane) - 1u));
-	if (lane == 0) { s_warp[warp] = __popc(ballot); }
-	__syncthreads();
-	int before = 0, all = 0;
-	#pragma unroll
-	for (int w = 0; w < DET_THREADS / 32; ++w)
-	{
-		const int c = s_warp[w];
-		if (w < warp) { before += c; }
-		all += c;
-	}
-	__syncthreads();
-	*total = all;
-	return before + in_warp;
-}
-
-__global__ void __launch_bounds__(DET_THREADS)
-yolo_detections_kernel(const YoloParams p)
-{
-	__shared__ int s_warp[DET_THREADS / 32];
-	const int b = blockIdx.x;
-	const int cells = p.lw * p.lh;
-	const int entries = 4 + 1 + p.classes;
-	const float * pred = p.head + (size_t)b * p.n * entries * cells;
-	int base = p.append ? p.count[b] : 0;
-	__syncthreads();                                             // every thread has read the count before thread 0 rewrites it
-
-	// correct_yolo_boxes: the network-to-image mapping, in double as the reference computes it
-	int new_w = p.netw, new_h = p.neth;
-	if (p.letter)
-	{
-		if (((float)p.netw / p.img_w) < ((float)p.neth / p.img_h)) { new_w = p.netw; new_h = (p.img_h * p.netw) / p.img_w; }
-		else { new_h = p.neth; new_w = (p.img_w * p.neth) / p.img_h; }
-	}
-	const float deltaw = (float)(p.netw - new_w), deltah = (float)(p.neth - new_h);
-	const float ratiow = (float)new_w / p.netw, ratioh = (float)new_h / p.neth;
-
-	const int candidates = cells * p.n;
-	for (int q0 = 0; q0 < candidates; q0 += DET_THREADS)
-	{
-		const int q = q0 + threadIdx.x;                          // reference order: cell outer, anchor inner
-		const int i = q / p.n;
-		const int a = q - i * p.n;
-		float obj = 0.0f;
-		bool hit = false;
-		if (q < candidates)
-		{
-			obj = pred[(size_t)(a * entries + 4) * cells + i];
-			hit = obj > p.thresh;
-		}
-		int total;
-		const int slot = base + block_scan_flags(hit, s_warp, &total);
-		if (hit && slot < p.max_dets)
-		{
-			const int row = i / p.lw, col = i - row * p.lw;
-			const float * e = pred + (size_t)a * entries * cells + i;
-			float bx = ((float)col + e[0]) / (float)p.lw;
-			float by = ((float)row + e[(size_t)cells]) / (float)p.lh;
-			float bw, bh;
-			if (p.new_coords)
-			{
-				const float tw = e[(size_t)2 * cells], th = e[(size_t)3 * cells];
-				bw = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(tw, tw), 4.0f), p.anchor_w[a]), (float)p.netw);
-				bh = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(th, th), 4.0f), p.anchor_h[a]), (float)p.neth);
-			}
-			else
-			{
-				bw = __fdiv_rn(__fmul_rn(expf(e[(size_t)2 * cells]), p.anchor_w[a]), (float)p.netw);
-				bh = __fdiv_rn(__fmul_rn(expf(e[(size_t)3 * cells]), p.anchor_h[a]), (float)p.neth);
-			}
-			bx = (float)(((double)bx - (double)deltaw / 2. / p.netw) / (double)ratiow);
-			by = (float)(((double)by - (double)deltah / 2. / p.neth) / (double)ratioh);
-			bw = __fmul_rn(bw, __fdiv_rn(1.0f, ratiow));
-			bh = __fmul_rn(bh, __fdiv_rn(1.0f, ratioh));
-			if (!p.relative)
-			{
-				bx = __fmul_rn(bx, (float)p.img_w); bw = __fmul_rn(bw, (float)p.img_w);
-				by = __fmul_rn(by, (float)p.img_h); bh = __fmul_rn(bh, (float)p.img_h);
-			}
-			const size_t d = (size_t)b * p.max_dets + slot;
-			p.boxes[d * 4 + 0] = bx; p.boxes[d * 4 + 1] = by; p.boxes[d * 4 + 2] = bw; p.boxes[d * 4 + 3] = bh;
-			p.objectness[d] = obj;
-			for (int j = 0; j < p.classes; ++j)
-			{
-				const float prob = __fmul_rn(obj, e[(size_t)(5 + j) * cells]);
-				p.probs[d * p.classes + j] = (prob > p.thresh) ? prob : 0.0f;
-			}
-		}
-		base += total;
-	}
-	if (threadIdx.x == 0) { p.count[b] = base; }
-}
 
 // box_iou of src-lib/box.cpp:68-113, :310-344, operation for operation (no contraction into FMAs)
 __device__ __forceinline__ float overlap_1d(float x1, float w1, float x2, float w2)
@@ -156,75 +87,108 @@ __device__ __forceinline__ float box_iou_dev(const float4 a, const float4 b)
 	return __fdiv_rn(inter, uni);
 }
 
-struct NmsParams
+// Rank of candidate c by score, highest first; equal scores keep their storage order.
+__device__ __forceinline__ int score_rank(const float * s_score, int m, int c)
 {
-	const float * boxes;
-	float * probs;
-	const int * count;
-	int max_dets, classes;
-	float thresh;
-};
+	const float s = s_score[c];
+	int rank = 0;
+	#pragma unroll 4
+	for (int o = 0; o < m; ++o)
+	{
+		const float t = s_score[o];
+		rank += (t > s || (t == s && o < c)) ? 1 : 0;
+	}
+	return rank;
+}
 
-// One CTA per (class, image).  Shared: candidate index, score, sorted order, alive flag per stored detection.
-__global__ void __launch_bounds__(DET_THREADS)
-nms_sort_kernel(const NmsParams p)
+// Greedy suppression of one class's m <= DET_WARP_MAX candidates by one warp.  The boxes go to shared memory in rank order, lane l
+// decides about ranks l, l + 32, ...; its verdicts stay in a register, so a step is one shuffle, one broadcast read and the
+// overlaps (reading order, score and box per step from memory took 600 cycles a candidate, this takes about 150).
+__device__ __forceinline__ void suppress_warp(const DetectParams & p, int m, const float * s_score, const uint16_t * s_idx, uint16_t * s_order,
+		float4 * s_box, const float4 * boxes, float * probs, int k)
 {
-	extern __shared__ int s_nms[];
-	const int k = blockIdx.x;
-	const int b = blockIdx.y;
-	const int n = min(p.count[b], p.max_dets);
-	int * s_idx = s_nms;                                          // candidates of this class in storage order
-	float * s_score = reinterpret_cast<float *>(s_nms + p.max_dets);
-	int * s_order = s_nms + 2 * p.max_dets;                       // candidate (position in s_idx) at each rank
-	int * s_alive = s_nms + 3 * p.max_dets;
-	__shared__ int s_warp[DET_THREADS / 32];
-	__shared__ int s_m;
-	float * probs = p.probs + (size_t)b * p.max_dets * p.classes;
-	const float4 * boxes = reinterpret_cast<const float4 *>(p.boxes) + (size_t)b * p.max_dets;
-
-	// candidates: detections whose probability for this class is above zero, in storage order
-	int m = 0;
-	for (int d0 = 0; d0 < n; d0 += DET_THREADS)
+	const int lane = threadIdx.x & 31;
+	for (int c = lane; c < m; c += 32)
 	{
-		const int d = d0 + threadIdx.x;
-		const float s = (d < n) ? probs[(size_t)d * p.classes + k] : 0.0f;
-		int total;
-		const int slot = m + block_scan_flags(s > 0.0f, s_warp, &total);
-		if (s > 0.0f) { s_idx[slot] = d; s_score[slot] = s; }
-		m += total;
+		const int rank = score_rank(s_score, m, c);
+		s_order[rank] = s_idx[c];
+		s_box[rank] = __ldcg(boxes + s_idx[c]);
 	}
-	if (threadIdx.x == 0) { s_m = m; }
-	__syncthreads();
-	m = s_m;
-	if (m <= 1) { return; }
-	// rank by score, highest first; equal scores keep their storage order
-	for (int c = threadIdx.x; c < m; c += DET_THREADS)
-	{
-		const float s = s_score[c];
-		int rank = 0;
-		for (int o = 0; o < m; ++o)
-		{
-			const float t = s_score[o];
-			rank += (t > s || (t == s && o < c)) ? 1 : 0;
-		}
-		s_order[rank] = c;
-		s_alive[c] = 1;
-	}
-	__syncthreads();
-	// greedy suppression in rank order: a kept detection removes every later one that overlaps it too much
+	__syncwarp();
+	unsigned dead = 0;                                            // bit j: rank lane + 32 j is suppressed
 	for (int r = 0; r < m - 1; ++r)
 	{
-		const int ci = s_order[r];
-		if (s_alive[ci])                                          // uniform: every thread reads the same flag
+		const unsigned owner = __shfl_sync(0xffffffffu, dead, r & 31);
+		if ((owner >> (r >> 5)) & 1u) { continue; }
+		const float4 a = s_box[r];
+		for (int j = r >> 5; j * 32 < m; ++j)
 		{
-			const float4 a = boxes[s_idx[ci]];
-			for (int r2 = r + 1 + threadIdx.x; r2 < m; r2 += DET_THREADS)
+			const int r2 = j * 32 + lane;
+			if (r2 > r && r2 < m && box_iou_dev(a, s_box[r2]) > p.nms_thresh) { dead |= 1u << j; }
+		}
+	}
+	for (int j = 0; j * 32 < m; ++j)
+	{
+		if ((dead >> j) & 1u) { probs[(size_t)s_order[j * 32 + lane] * p.classes + k] = 0.0f; }
+	}
+}
+
+// The same for a crowded class, by the whole CTA, DET_BLOCK ranks at a time: every overlap inside the block at once as a bit
+// matrix, one warp walks the matrix in rank order (a step costs a shuffle), then the block's survivors are held against all later
+// ranks at once.  Step by step over the list, as a warp does it, 170 candidates took 45 us.
+__device__ __forceinline__ void suppress_cta(const DetectParams & p, int m, float * s_score, const uint16_t * s_idx, uint16_t * s_order,
+		const float4 * boxes, float * probs, int k)
+{
+	constexpr int WORDS = DET_BLOCK / 32;
+	static_assert(DET_BLOCK * WORDS == DET_THREADS, "one thread per word of the block's matrix");
+	__shared__ float4 s_box[DET_BLOCK];
+	__shared__ uint32_t s_hits[DET_BLOCK][WORDS + 1];
+	__shared__ uint32_t s_dead[WORDS];
+	const int tid = threadIdx.x;
+	for (int c = tid; c < m; c += DET_THREADS) { s_order[score_rank(s_score, m, c)] = (uint16_t)c; }
+	__syncthreads();
+	for (int r0 = 0; r0 < m; r0 += DET_BLOCK)
+	{
+		const int nb = min(DET_BLOCK, m - r0);
+		if (tid < nb) { s_box[tid] = boxes[s_idx[s_order[r0 + tid]]]; }
+		if (tid < WORDS) { s_dead[tid] = 0; }
+		__syncthreads();
+		const int r = tid / WORDS, w = tid % WORDS;
+		uint32_t hits = 0;
+		if (r < nb)
+		{
+			const float4 a = s_box[r];
+			for (int j = max(w * 32, r + 1); j < min(nb, w * 32 + 32); ++j)
 			{
-				const int cj = s_order[r2];
-				if (s_alive[cj] && box_iou_dev(a, boxes[s_idx[cj]]) > p.thresh)
+				if (box_iou_dev(a, s_box[j]) > p.nms_thresh) { hits |= 1u << (j & 31); }
+			}
+			if (s_score[s_order[r0 + r]] <= 0.0f && w == 0) { atomicOr(&s_dead[r >> 5], 1u << (r & 31)); }     // an earlier block's verdict
+		}
+		s_hits[r][w] = hits;
+		__syncthreads();
+		if (tid < 32)
+		{
+			uint32_t dead = (tid < WORDS) ? s_dead[tid] : 0;
+			for (int i = 0; i < nb; ++i)
+			{
+				const uint32_t word = __shfl_sync(0xffffffffu, dead, i >> 5);
+				if (((word >> (i & 31)) & 1u) == 0 && tid < WORDS) { dead |= s_hits[i][tid]; }
+			}
+			if (tid < WORDS) { s_dead[tid] = dead; }
+		}
+		__syncthreads();
+		if (tid < nb && ((s_dead[tid >> 5] >> (tid & 31)) & 1u)) { probs[(size_t)s_idx[s_order[r0 + tid]] * p.classes + k] = 0.0f; }
+		for (int q = r0 + DET_BLOCK + tid; q < m; q += DET_THREADS)
+		{
+			const int c = s_order[q];
+			if (s_score[c] <= 0.0f) { continue; }
+			const float4 z = boxes[s_idx[c]];
+			for (int i = 0; i < nb; ++i)
+			{
+				if (((s_dead[i >> 5] >> (i & 31)) & 1u) == 0 && box_iou_dev(s_box[i], z) > p.nms_thresh)
 				{
-					s_alive[cj] = 0;
-					probs[(size_t)s_idx[cj] * p.classes + k] = 0.0f;
+					s_score[c] = -1.0f;
+					break;
 				}
 			}
 		}
@@ -232,45 +196,263 @@ nms_sort_kernel(const NmsParams p)
 	}
 }
 
-struct RowsParams
+// One cluster of DET_CLUSTER CTAs per image runs decode, suppression and compaction back to back: a frame has some tens of
+// detections, so each step is a few microseconds of latency and the launches between them would cost as much again.  Work is
+// dealt to warps (a warp per detection, per class, per detection again), the scans that fix the order are short enough for every
+// CTA to do them all.  Values that another CTA of the cluster wrote are read past the L1 (__ldcg).
+// Measured at 416x416, 80 classes, one image: 237 us in four launches before (one CTA per image, a thread per detection walking the
+// classes at plane stride) at 174 detections and 843 rows, 48 us in one now; 14 us at 13 detections, 7 us at none.
+__global__ void __cluster_dims__(DET_CLUSTER, 1, 1) __launch_bounds__(DET_THREADS)
+detect_kernel(const __grid_constant__ DetectParams p)
 {
-	const float * boxes;
-	const float * objectness;
-	const float * probs;
-	const int * count;
-	int max_dets, classes;
-	float * rows;                // [batch][max_rows][7]
-	int * row_count;             // [batch]: pairs found (may exceed max_rows: the surplus is not stored)
-	int max_rows;
-};
+	extern __shared__ __align__(16) uint8_t det_smem[];
+	__shared__ __align__(16) int s_cnt[DET_STEP * DET_WARPS];
+	__shared__ int s_m[DET_WARPS];
+	cg::cluster_group cluster = cg::this_cluster();
+	const int rank = (int)cluster.block_rank();
+	const int b = blockIdx.y;
+	const int lane = threadIdx.x & 31;
+	const int warp = threadIdx.x >> 5;
+	const int all_warp = rank * DET_WARPS + warp;
+	float * probs = p.probs + (size_t)b * p.max_dets * p.classes;
+	const float4 * boxes = reinterpret_cast<const float4 *>(p.boxes) + (size_t)b * p.max_dets;
+	int found = (p.n_heads == 0 || p.append) ? p.count[b] : 0;
 
-__global__ void __launch_bounds__(DET_THREADS)
-detection_rows_kernel(const RowsParams p)
-{
-	__shared__ int s_warp[DET_THREADS / 32];
-	const int b = blockIdx.x;
-	const int n = min(p.count[b], p.max_dets);
-	const long long items = (long long)n * p.classes;
-	const float * probs = p.probs + (size_t)b * p.max_dets * p.classes;
-	int base = 0;
-	for (long long q0 = 0; q0 < items; q0 += DET_THREADS)
+	if (p.n_heads > 0)
 	{
-		const long long q = q0 + threadIdx.x;                     // (detection, class), detection-major
-		const float s = (q < items) ? probs[q] : 0.0f;
-		int total;
-		const int slot = base + block_scan_flags(s > 0.0f, s_warp, &total);
-		if (s > 0.0f && slot < p.max_rows)
+		int * s_hit = reinterpret_cast<int *>(det_smem);         // candidate number and head of each new detection
+		const int first = found;
+		for (int hd = 0; hd < p.n_heads; ++hd)
 		{
-			const int d = (int)(q / p.classes);
-			const int k = (int)(q - (long long)d * p.classes);
-			const size_t dd = (size_t)b * p.max_dets + d;
-			float * r = p.rows + ((size_t)b * p.max_rows + slot) * 7;
-			r[0] = p.boxes[dd * 4 + 0]; r[1] = p.boxes[dd * 4 + 1]; r[2] = p.boxes[dd * 4 + 2]; r[3] = p.boxes[dd * 4 + 3];
-			r[4] = p.objectness[dd]; r[5] = (float)k; r[6] = s;
+			const YoloHeadParams & h = p.heads[hd];
+			const int cells = h.lw * h.lh;
+			const int entries = 4 + 1 + p.classes;
+			const float * pred = h.head + (size_t)b * h.n * entries * cells;
+			const int candidates = cells * h.n;                  // reference order: cell outer, anchor inner
+			for (int q0 = 0; q0 < candidates; q0 += DET_STEP * DET_THREADS)
+			{
+				unsigned hits[DET_STEP];
+				#pragma unroll
+				for (int j = 0; j < DET_STEP; ++j)
+				{
+					const int q = q0 + j * DET_THREADS + threadIdx.x;
+					const int i = q / h.n;
+					const int a = q - i * h.n;
+					const float obj = (q < candidates) ? __ldg(pred + (size_t)(a * entries + 4) * cells + i) : 0.0f;
+					hits[j] = __ballot_sync(0xffffffffu, q < candidates && obj > p.thresh);
+				}
+				#pragma unroll
+				for (int j = 0; j < DET_STEP; ++j) { if (lane == 0) { s_cnt[j * DET_WARPS + warp] = __popc(hits[j]); } }
+				__syncthreads();
+				int total = 0, before[DET_STEP];
+				#pragma unroll
+				for (int j = 0; j < DET_STEP; ++j)
+				{
+					#pragma unroll
+					for (int w = 0; w < DET_WARPS; ++w)
+					{
+						if (w == warp) { before[j] = total; }
+						total += s_cnt[j * DET_WARPS + w];
+					}
+				}
+				#pragma unroll
+				for (int j = 0; j < DET_STEP; ++j)
+				{
+					if ((hits[j] >> lane) & 1u)
+					{
+						const int slot = found + before[j] + __popc(hits[j] & ((1u << lane) - 1u));
+						if (slot < p.max_dets) { s_hit[slot - first] = (hd << 28) | (q0 + j * DET_THREADS + (int)threadIdx.x); }
+					}
+				}
+				found += total;
+				__syncthreads();
+			}
 		}
-		base += total;
+		// correct_yolo_boxes: the network-to-image mapping, in double as the reference computes it
+		int new_w = p.netw, new_h = p.neth;
+		if (p.letter)
+		{
+			if (((float)p.netw / p.img_w) < ((float)p.neth / p.img_h)) { new_w = p.netw; new_h = (p.img_h * p.netw) / p.img_w; }
+			else { new_h = p.neth; new_w = (p.img_w * p.neth) / p.img_h; }
+		}
+		const float deltaw = (float)(p.netw - new_w), deltah = (float)(p.neth - new_h);
+		const float ratiow = (float)new_w / p.netw, ratioh = (float)new_h / p.neth;
+		const int stored = min(found, p.max_dets);
+		for (int slot = first + all_warp; slot < stored; slot += DET_ALL_WARPS)
+		{
+			const YoloHeadParams & h = p.heads[s_hit[slot - first] >> 28];
+			const int q = s_hit[slot - first] & 0x0fffffff;
+			const int cells = h.lw * h.lh;
+			const int entries = 4 + 1 + p.classes;
+			const int i = q / h.n;
+			const int a = q - i * h.n;
+			const float * e = h.head + ((size_t)b * h.n + a) * entries * cells + i;
+			const float v = (lane < entries) ? __ldg(e + (size_t)lane * cells) : 0.0f;
+			const float tx = __shfl_sync(0xffffffffu, v, 0), ty = __shfl_sync(0xffffffffu, v, 1);
+			const float tw = __shfl_sync(0xffffffffu, v, 2), th = __shfl_sync(0xffffffffu, v, 3);
+			const float obj = __shfl_sync(0xffffffffu, v, 4);
+			float * pr = probs + (size_t)slot * p.classes;
+			if (lane >= 5 && lane < entries)
+			{
+				const float prob = __fmul_rn(obj, v);
+				pr[lane - 5] = (prob > p.thresh) ? prob : 0.0f;
+			}
+			for (int j = lane + 32; j < entries; j += 32)
+			{
+				const float prob = __fmul_rn(obj, __ldg(e + (size_t)j * cells));
+				pr[j - 5] = (prob > p.thresh) ? prob : 0.0f;
+			}
+			const int row = i / h.lw, col = i - row * h.lw;
+			float bx = ((float)col + tx) / (float)h.lw;
+			float by = ((float)row + ty) / (float)h.lh;
+			float bw, bh;
+			if (h.new_coords)
+			{
+				bw = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(tw, tw), 4.0f), h.anchor_w[a]), (float)p.netw);
+				bh = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(th, th), 4.0f), h.anchor_h[a]), (float)p.neth);
+			}
+			else
+			{
+				bw = __fdiv_rn(__fmul_rn(expf(tw), h.anchor_w[a]), (float)p.netw);
+				bh = __fdiv_rn(__fmul_rn(expf(th), h.anchor_h[a]), (float)p.neth);
+			}
+			bx = (float)(((double)bx - (double)deltaw / 2. / p.netw) / (double)ratiow);
+			by = (float)(((double)by - (double)deltah / 2. / p.neth) / (double)ratioh);
+			bw = __fmul_rn(bw, __fdiv_rn(1.0f, ratiow));
+			bh = __fmul_rn(bh, __fdiv_rn(1.0f, ratioh));
+			if (!p.relative)
+			{
+				bx = __fmul_rn(bx, (float)p.img_w); bw = __fmul_rn(bw, (float)p.img_w);
+				by = __fmul_rn(by, (float)p.img_h); bh = __fmul_rn(bh, (float)p.img_h);
+			}
+			if (lane == 0)
+			{
+				const size_t d = (size_t)b * p.max_dets + slot;
+				*reinterpret_cast<float4 *>(p.boxes + d * 4) = make_float4(bx, by, bw, bh);
+				p.objectness[d] = obj;
+			}
+		}
+		cluster.sync();                                          // the lists are complete; every CTA has read the old count
+		if (rank == 0 && threadIdx.x == 0) { p.count[b] = found; }
 	}
-	if (threadIdx.x == 0) { p.row_count[b] = base; }
+	const int n = min(found, p.max_dets);
+
+	if (p.nms)
+	{
+		const int warp_max = min(DET_WARP_MAX, p.max_dets);
+		float4 * s_boxes = reinterpret_cast<float4 *>(det_smem + (((size_t)p.lists * p.max_dets * DET_LIST_BYTES + 15) & ~(size_t)15));
+		for (int k0 = 0; k0 < p.classes; k0 += DET_CLUSTER * p.lists)
+		{
+			// warps 0 .. lists-1 of every CTA: one class each
+			const int k = k0 + warp * DET_CLUSTER + rank;
+			float * s_score = reinterpret_cast<float *>(det_smem + (size_t)warp * p.max_dets * DET_LIST_BYTES);
+			uint16_t * s_idx = reinterpret_cast<uint16_t *>(s_score + p.max_dets);
+			uint16_t * s_order = s_idx + p.max_dets;
+			int m = 0;
+			if (warp < p.lists && k < p.classes)
+			{
+				for (int d0 = 0; d0 < n; d0 += 4 * 32)
+				{
+					float s[4];
+					#pragma unroll
+					for (int j = 0; j < 4; ++j)
+					{
+						const int d = d0 + j * 32 + lane;
+						s[j] = (d < n) ? __ldcg(probs + (size_t)d * p.classes + k) : 0.0f;
+					}
+					#pragma unroll
+					for (int j = 0; j < 4; ++j)
+					{
+						const unsigned mask = __ballot_sync(0xffffffffu, s[j] > 0.0f);
+						if (s[j] > 0.0f)
+						{
+							const int at = m + __popc(mask & ((1u << lane) - 1u));
+							s_score[at] = s[j];
+							s_idx[at] = (uint16_t)(d0 + j * 32 + lane);
+						}
+						m += __popc(mask);
+					}
+				}
+				__syncwarp();
+				if (m > 1 && m <= DET_WARP_MAX) { suppress_warp(p, m, s_score, s_idx, s_order, s_boxes + warp * warp_max, boxes, probs, k); }
+			}
+			if (lane == 0) { s_m[warp] = m; }
+			__syncthreads();
+			for (int w = 0; w < p.lists; ++w)                    // crowded classes: the whole CTA, one after the other
+			{
+				const int mw = s_m[w];
+				if (mw <= DET_WARP_MAX) { continue; }
+				float * score = reinterpret_cast<float *>(det_smem + (size_t)w * p.max_dets * DET_LIST_BYTES);
+				uint16_t * idx = reinterpret_cast<uint16_t *>(score + p.max_dets);
+				suppress_cta(p, mw, score, idx, idx + p.max_dets, boxes, probs, k0 + w * DET_CLUSTER + rank);
+			}
+			__syncthreads();
+		}
+		cluster.sync();
+	}
+
+	if (p.rows != nullptr)
+	{
+		// rows per detection, then the prefix sums every CTA needs for its own detections
+		int * s_rows = reinterpret_cast<int *>(det_smem);        // rows of detection d: kept by the CTA whose warp counts it
+		int * s_start = s_rows + p.max_dets;
+		for (int d = all_warp; d < n; d += DET_ALL_WARPS)
+		{
+			int c = 0;
+			for (int k = lane; k < p.classes; k += 32) { c += (__ldcg(probs + (size_t)d * p.classes + k) > 0.0f) ? 1 : 0; }
+			c = __reduce_add_sync(0xffffffffu, c);
+			if (lane == 0) { s_rows[d] = c; }
+		}
+		cluster.sync();
+		int base = 0;
+		for (int d0 = 0; d0 < n; d0 += DET_THREADS)
+		{
+			const int d = d0 + threadIdx.x;
+			int c = 0;
+			if (d < n) { c = cluster.map_shared_rank(s_rows, (d % DET_ALL_WARPS) / DET_WARPS)[d]; }
+			int incl = c;
+			#pragma unroll
+			for (int o = 1; o < 32; o <<= 1)
+			{
+				const int u = __shfl_up_sync(0xffffffffu, incl, o);
+				if (lane >= o) { incl += u; }
+			}
+			if (lane == 31) { s_cnt[warp] = incl; }
+			__syncthreads();
+			int before = 0, all = 0;
+			#pragma unroll
+			for (int w = 0; w < DET_WARPS; ++w)
+			{
+				if (w < warp) { before += s_cnt[w]; }
+				all += s_cnt[w];
+			}
+			if (d < n) { s_start[d] = base + before + incl - c; }
+			base += all;
+			__syncthreads();
+		}
+		for (int d = all_warp; d < n; d += DET_ALL_WARPS)
+		{
+			int slot = s_start[d];
+			const size_t dd = (size_t)b * p.max_dets + d;
+			const float4 box = __ldcg(boxes + d);
+			const float obj = __ldcg(p.objectness + dd);
+			for (int k0 = 0; k0 < p.classes; k0 += 32)
+			{
+				const int k = k0 + lane;
+				const float s = (k < p.classes) ? __ldcg(probs + (size_t)d * p.classes + k) : 0.0f;
+				const unsigned mask = __ballot_sync(0xffffffffu, s > 0.0f);
+				const int at = slot + __popc(mask & ((1u << lane) - 1u));
+				if (s > 0.0f && at < p.max_rows)
+				{
+					float * r = p.rows + ((size_t)b * p.max_rows + at) * 7;
+					r[0] = box.x; r[1] = box.y; r[2] = box.z; r[3] = box.w; r[4] = obj; r[5] = (float)k; r[6] = s;
+				}
+				slot += __popc(mask);
+			}
+		}
+		if (rank == 0 && threadIdx.x == 0) { p.row_count[b] = base; }
+		cluster.sync();                                          // nobody's counts may go while another CTA still reads them
+	}
 }
 
 static int check_dets(const xnor_b200_detections * d, int batch)
@@ -280,6 +462,56 @@ static int check_dets(const xnor_b200_detections * d, int batch)
 	if (d->max_dets > XNOR_B200_MAX_DETECTIONS) { return XNOR_B200_ERR_TOO_LARGE; }
 	if ((((uintptr_t)d->boxes) & 15u) != 0) { return XNOR_B200_ERR_ALIGNMENT; }
 	return XNOR_B200_OK;
+}
+
+static int add_head(const xnor_b200_yolo_head & head, int classes, DetectParams & p)
+{
+	if (head.output == nullptr) { return XNOR_B200_ERR_NULL; }
+	if (head.w <= 0 || head.h <= 0 || head.n <= 0 || head.n > DET_MAX_ANCHORS || head.classes != classes) { return XNOR_B200_ERR_INVALID; }
+	if ((long long)head.w * head.h * head.n >= (1 << 28)) { return XNOR_B200_ERR_TOO_LARGE; }
+	YoloHeadParams & h = p.heads[p.n_heads++];
+	h.head = head.output;
+	h.lw = head.w; h.lh = head.h; h.n = head.n; h.new_coords = head.new_coords;
+	for (int a = 0; a < DET_MAX_ANCHORS; ++a)
+	{
+		h.anchor_w[a] = (a < head.n) ? head.anchors[2 * a] : 0.0f;
+		h.anchor_h[a] = (a < head.n) ? head.anchors[2 * a + 1] : 0.0f;
+	}
+	return XNOR_B200_OK;
+}
+
+static int set_decode(DetectParams & p, int netw, int neth, int img_w, int img_h, float thresh, int relative, int letter, int append)
+{
+	if (netw <= 0 || neth <= 0 || img_w <= 0 || img_h <= 0) { return XNOR_B200_ERR_INVALID; }
+	p.netw = netw; p.neth = neth; p.img_w = img_w; p.img_h = img_h;
+	p.thresh = thresh; p.relative = relative; p.letter = letter; p.append = append;
+	return XNOR_B200_OK;
+}
+
+static int set_rows(DetectParams & p, float * rows, int max_rows, int * row_count)
+{
+	if (rows == nullptr || row_count == nullptr) { return XNOR_B200_ERR_NULL; }
+	if (max_rows <= 0) { return XNOR_B200_ERR_INVALID; }
+	p.rows = rows; p.row_count = row_count; p.max_rows = max_rows;
+	return XNOR_B200_OK;
+}
+
+static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int batch, void * stream)
+{
+	if (batch > 65535) { return XNOR_B200_ERR_TOO_LARGE; }
+	p.boxes = d->boxes; p.objectness = d->objectness; p.probs = d->probs; p.count = d->count;
+	p.max_dets = d->max_dets; p.classes = d->classes;
+	// shared memory: the hit list, then the candidate lists (as many as the classes of a CTA and the budget ask for), then two
+	// ints per detection
+	const int want = min(DET_WARPS, (p.classes + DET_CLUSTER - 1) / DET_CLUSTER);
+	const int list_bytes = p.max_dets * DET_LIST_BYTES;
+	const int box_bytes = min(DET_WARP_MAX, p.max_dets) * (int)sizeof(float4);
+	p.lists = max(1, min(want, DET_SMEM_BUDGET / (list_bytes + box_bytes)));
+	const size_t smem = p.nms ? round_up((size_t)p.lists * list_bytes, 16) + (size_t)p.lists * box_bytes : (size_t)list_bytes;
+	const int rc = ensure_dynamic_smem((const void *)detect_kernel, smem);
+	if (rc != XNOR_B200_OK) { return rc; }
+	detect_kernel<<<dim3(DET_CLUSTER, (unsigned)batch, 1), DET_THREADS, smem, (cudaStream_t)stream>>>(p);
+	return check_launch();
 }
 
 }  // namespace xnor
@@ -292,49 +524,64 @@ extern "C" int xnor_b200_yolo_detections(const xnor_b200_yolo_head * head, int b
 	if (head == nullptr || head->output == nullptr) { return XNOR_B200_ERR_NULL; }
 	int rc = check_dets(dets, batch);
 	if (rc != XNOR_B200_OK) { return rc; }
-	if (head->w <= 0 || head->h <= 0 || head->n <= 0 || head->n > DET_MAX_ANCHORS || head->classes != dets->classes) { return XNOR_B200_ERR_INVALID; }
-	if (netw <= 0 || neth <= 0 || img_w <= 0 || img_h <= 0) { return XNOR_B200_ERR_INVALID; }
-	if ((long long)head->w * head->h * head->n > 0x7fffffffLL) { return XNOR_B200_ERR_TOO_LARGE; }
-	YoloParams p;
-	p.head = head->output;
-	p.batch = batch; p.lw = head->w; p.lh = head->h; p.n = head->n; p.classes = head->classes;
-	for (int a = 0; a < DET_MAX_ANCHORS; ++a)
-	{
-		p.anchor_w[a] = (a < head->n) ? head->anchors[2 * a] : 0.0f;
-		p.anchor_h[a] = (a < head->n) ? head->anchors[2 * a + 1] : 0.0f;
-	}
-	p.netw = netw; p.neth = neth; p.img_w = img_w; p.img_h = img_h;
-	p.thresh = thresh; p.relative = relative; p.letter = letter; p.new_coords = head->new_coords; p.append = append;
-	p.boxes = dets->boxes; p.objectness = dets->objectness; p.probs = dets->probs; p.count = dets->count; p.max_dets = dets->max_dets;
-	yolo_detections_kernel<<<batch, DET_THREADS, 0, (cudaStream_t)stream>>>(p);
-	return check_launch();
+	DetectParams p = {};
+	rc = add_head(*head, dets->classes, p);
+	if (rc != XNOR_B200_OK) { return rc; }
+	rc = set_decode(p, netw, neth, img_w, img_h, thresh, relative, letter, append);
+	return (rc != XNOR_B200_OK) ? rc : launch_detect(p, dets, batch, stream);
 }
 
 extern "C" int xnor_b200_nms_sort(const xnor_b200_detections * dets, int batch, float nms_thresh, void * stream)
 {
-	int rc = check_dets(dets, batch);
+	const int rc = check_dets(dets, batch);
 	if (rc != XNOR_B200_OK) { return rc; }
-	if (batch > 65535) { return XNOR_B200_ERR_TOO_LARGE; }
-	NmsParams p;
-	p.boxes = dets->boxes; p.probs = dets->probs; p.count = dets->count;
-	p.max_dets = dets->max_dets; p.classes = dets->classes; p.thresh = nms_thresh;
-	const size_t smem = (size_t)dets->max_dets * 4 * sizeof(int);
-	rc = ensure_dynamic_smem((const void *)nms_sort_kernel, smem);
-	if (rc != XNOR_B200_OK) { return rc; }
-	nms_sort_kernel<<<dim3((unsigned)dets->classes, (unsigned)batch, 1), DET_THREADS, smem, (cudaStream_t)stream>>>(p);
-	return check_launch();
+	DetectParams p = {};
+	p.nms = 1;
+	p.nms_thresh = nms_thresh;
+	return launch_detect(p, dets, batch, stream);
 }
 
 extern "C" int xnor_b200_detection_rows(const xnor_b200_detections * dets, int batch, float * rows, int max_rows, int * row_count, void * stream)
 {
 	int rc = check_dets(dets, batch);
 	if (rc != XNOR_B200_OK) { return rc; }
-	if (rows == nullptr || row_count == nullptr) { return XNOR_B200_ERR_NULL; }
-	if (max_rows <= 0) { return XNOR_B200_ERR_INVALID; }
-	RowsParams p;
-	p.boxes = dets->boxes; p.objectness = dets->objectness; p.probs = dets->probs; p.count = dets->count;
-	p.max_dets = dets->max_dets; p.classes = dets->classes;
-	p.rows = rows; p.row_count = row_count; p.max_rows = max_rows;
-	detection_rows_kernel<<<batch, DET_THREADS, 0, (cudaStream_t)stream>>>(p);
-	return check_launch();
+	DetectParams p = {};
+	rc = set_rows(p, rows, max_rows, row_count);
+	return (rc != XNOR_B200_OK) ? rc : launch_detect(p, dets, batch, stream);
+}
+
+extern "C" int xnor_b200_detect(const xnor_b200_yolo_head * heads, int n_heads, int batch, int netw, int neth, int img_w, int img_h,
+		float thresh, int relative, int letter, float nms_thresh, const xnor_b200_detections * dets,
+		float * rows, int max_rows, int * row_count, void * stream)
+{
+	if (heads == nullptr) { return XNOR_B200_ERR_NULL; }
+	int rc = check_dets(dets, batch);
+	if (rc != XNOR_B200_OK) { return rc; }
+	if (n_heads <= 0) { return XNOR_B200_ERR_INVALID; }
+	if (n_heads > DET_MAX_HEADS) { return XNOR_B200_ERR_TOO_LARGE; }
+	DetectParams p = {};
+	for (int i = 0; i < n_heads; ++i)
+	{
+		rc = add_head(heads[i], dets->classes, p);
+		if (rc != XNOR_B200_OK) { return rc; }
+	}
+	rc = set_decode(p, netw, neth, img_w, img_h, thresh, relative, letter, 0);
+	if (rc != XNOR_B200_OK) { return rc; }
+	rc = set_rows(p, rows, max_rows, row_count);
+	if (rc != XNOR_B200_OK) { return rc; }
+	p.nms = (nms_thresh > 0.0f) ? 1 : 0;
+	p.nms_thresh = nms_thresh;
+	return launch_detect(p, dets, batch, stream);
+}
+
+extern "C" int xnor_b200_rows_to_host(const float * rows, int max_rows, const int * row_count, int batch, int take, float * host_rows,
+		int * host_count, void * stream)
+{
+	if (rows == nullptr || row_count == nullptr || host_rows == nullptr || host_count == nullptr) { return XNOR_B200_ERR_NULL; }
+	if (batch <= 0 || take <= 0 || take > max_rows) { return XNOR_B200_ERR_INVALID; }
+	cudaError_t e = cudaMemcpyAsync(host_count, row_count, (size_t)batch * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+	if (e != cudaSuccess) { return cuda_fail(e); }
+	const size_t row = 7 * sizeof(float);
+	e = cudaMemcpy2DAsync(host_rows, take * row, rows, max_rows * row, take * row, (size_t)batch, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+	return (e == cudaSuccess) ? XNOR_B200_OK : cuda_fail(e);
 }

@@ -894,11 +894,23 @@ class DetectionBuffers:
         self.row_count = torch.zeros(batch, dtype=torch.int32, device=device)
         self.desc = capi.Detections(self.boxes.data_ptr(), self.objectness.data_ptr(), self.probs.data_ptr(), self.count.data_ptr(),
                                     max_dets, classes)
+        # where rows_host receives the counts and the first rows: page-locked, so that both copies are queued and waited for once
+        self.take = min(max_rows, 512)
+        pin = self.rows.is_cuda
+        self.host_count = torch.empty(batch, dtype=torch.int32, pin_memory=pin)
+        self.host_rows = torch.empty(batch, self.take, 7, dtype=torch.float32, pin_memory=pin)
 
     def rows_host(self) -> List[np.ndarray]:
-        """Per image the rows {x, y, w, h, objectness, class, probability} (one device-to-host copy of the counts, one of the rows)."""
-        counts = self.row_count.cpu().numpy()
-        rows = self.rows.cpu().numpy()
+        """Per image the rows {x, y, w, h, objectness, class, probability}.  The counts and each image's first `take` rows come over
+        together (most frames have fewer: the whole list would be eight times the bytes); only a longer list costs a second copy."""
+        stream = torch.cuda.current_stream(self.rows.device)
+        capi.check(capi.lib().xnor_b200_rows_to_host(self.rows.data_ptr(), self.max_rows, self.row_count.data_ptr(), self.batch, self.take,
+                                                    self.host_rows.data_ptr(), self.host_count.data_ptr(), stream.cuda_stream),
+                   "xnor_b200_rows_to_host")
+        stream.synchronize()
+        counts, rows = self.host_count.numpy(), self.host_rows.numpy()
+        if int(counts.max()) > self.take:
+            rows = self.rows.cpu().numpy()
         return [rows[b, :min(int(counts[b]), self.max_rows)].copy() for b in range(self.batch)]
 
 
@@ -915,6 +927,12 @@ def yolo_head_desc(l: Layer, output: torch.Tensor) -> capi.YoloHead:
     return hd
 
 
+def _checked_head(h: torch.Tensor) -> torch.Tensor:
+    if not (h.is_cuda and h.is_contiguous() and h.dtype == torch.float32):
+        raise ValueError("head outputs must be contiguous fp32 device tensors")
+    return h
+
+
 def get_network_boxes(net: Network, heads: List[torch.Tensor], img_w: int, img_h: int, thresh: float, dets: DetectionBuffers,
                       relative: int = 1, letter: int = 0) -> DetectionBuffers:
     """get_network_boxes (src-lib/darknet_network.cpp:1250) on the device: every [yolo] head of the network, in layer order, appended
@@ -925,9 +943,7 @@ def get_network_boxes(net: Network, heads: List[torch.Tensor], img_w: int, img_h
         raise ValueError("one activated output per [yolo] layer is needed")
     stream = torch.cuda.current_stream().cuda_stream
     for k, (l, h) in enumerate(zip(yolo_layers, heads)):
-        if not (h.is_cuda and h.is_contiguous() and h.dtype == torch.float32):
-            raise ValueError("head outputs must be contiguous fp32 device tensors")
-        hd = yolo_head_desc(l, h)
+        hd = yolo_head_desc(l, _checked_head(h))
         capi.check(capi.lib().xnor_b200_yolo_detections(C.byref(hd), net.batch, net.w, net.h, img_w, img_h, thresh, relative, letter,
                                                        1 if k else 0, C.byref(dets.desc), stream), "xnor_b200_yolo_detections")
     return dets
@@ -947,6 +963,20 @@ def detection_rows(dets: DetectionBuffers) -> None:
                                                   dets.row_count.data_ptr(), torch.cuda.current_stream().cuda_stream), "xnor_b200_detection_rows")
 
 
+def detect(net: Network, heads: List[torch.Tensor], img_w: int, img_h: int, thresh: float, nms_thresh: float, dets: DetectionBuffers,
+           relative: int = 1, letter: int = 0) -> DetectionBuffers:
+    """get_network_boxes, do_nms_sort (nms_thresh > 0) and detection_rows in one launch."""
+    import ctypes as C
+    yolo_layers = [l for l in net.layers if l.type == "yolo"]
+    if len(yolo_layers) != len(heads) or not yolo_layers:
+        raise ValueError("one activated output per [yolo] layer is needed")
+    descs = (capi.YoloHead * len(heads))(*[yolo_head_desc(l, _checked_head(h)) for l, h in zip(yolo_layers, heads)])
+    capi.check(capi.lib().xnor_b200_detect(descs, len(heads), net.batch, net.w, net.h, img_w, img_h, thresh, relative, letter, nms_thresh,
+                                          C.byref(dets.desc), dets.rows.data_ptr(), dets.max_rows, dets.row_count.data_ptr(),
+                                          torch.cuda.current_stream().cuda_stream), "xnor_b200_detect")
+    return dets
+
+
 def network_detections(net: Network, x: torch.Tensor, thresh: float = 0.25, nms_thresh: float = 0.45,
                        dets: Optional[DetectionBuffers] = None, img_w: Optional[int] = None, img_h: Optional[int] = None) -> DetectionBuffers:
     """Forward + decode + suppress + compact, all on the device: what a caller of Darknet's predict API does with
@@ -955,11 +985,7 @@ def network_detections(net: Network, x: torch.Tensor, thresh: float = 0.25, nms_
     if dets is None:
         classes = int(next(l for l in net.layers if l.type == "yolo").opts.get("classes", 20))
         dets = DetectionBuffers(net.batch, classes, device=x.device)
-    get_network_boxes(net, heads, img_w or net.w, img_h or net.h, thresh, dets)
-    if nms_thresh > 0:
-        do_nms_sort(dets, nms_thresh)
-    detection_rows(dets)
-    return dets
+    return detect(net, heads, img_w or net.w, img_h or net.h, thresh, nms_thresh, dets)
 
 
 def load_network_custom(cfg: str, weights: str, batch: int = 1, device: str = "cuda:0", sign_chains: bool = True,

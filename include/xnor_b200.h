@@ -392,6 +392,16 @@ XNOR_B200_API int xnor_b200_nms_sort(const xnor_b200_detections * dets, int batc
 XNOR_B200_API int xnor_b200_detection_rows(const xnor_b200_detections * dets, int batch, float * rows, int max_rows, int * row_count,
 		void * stream);
 
+/* The three calls above in one launch: decode every head in order (at most 4, append = 0), suppress (nms_thresh > 0), compact. */
+XNOR_B200_API int xnor_b200_detect(const xnor_b200_yolo_head * heads, int n_heads, int batch, int netw, int neth, int img_w, int img_h,
+		float thresh, int relative, int letter, float nms_thresh, const xnor_b200_detections * dets,
+		float * rows, int max_rows, int * row_count, void * stream);
+
+/* Queues the copies of row_count [batch] and of each image's first `take` rows to host memory (page-locked for the copies to be
+ * asynchronous): host_count [batch], host_rows [batch][take][7]. */
+XNOR_B200_API int xnor_b200_rows_to_host(const float * rows, int max_rows, const int * row_count, int batch, int take, float * host_rows,
+		int * host_count, void * stream);
+
 /* Bytes of the library-resident scratch array behind xnor_b200_conv_forward_static. */
 #define XNOR_B200_STATIC_SCRATCH_BYTES (8u << 20)
 

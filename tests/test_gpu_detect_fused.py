@@ -1,0 +1,71 @@
+"""xnor_b200_detect (decode, suppress and compact in one launch) against a plain CPU restatement, at list lengths around the
+kernel's own limits: none, one scan step, a class crowded past what one warp ranks, more detections than slots."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from darknet_b200 import cfgs, network  # noqa: E402
+
+
+def iou(a, b):
+    f = np.float32
+
+    def overlap(x1, w1, x2, w2):
+        return f(min(f(x1 + f(w1 / f(2))), f(x2 + f(w2 / f(2)))) - max(f(x1 - f(w1 / f(2))), f(x2 - f(w2 / f(2)))))
+    w, h = overlap(a[0], a[2], b[0], b[2]), overlap(a[1], a[3], b[1], b[3])
+    if w <= 0 or h <= 0:
+        return f(0)
+    inter = f(w * h)
+    return f(inter / f(f(f(a[2] * a[3]) + f(b[2] * b[3])) - inter))
+
+
+def expected_rows(boxes, obj, probs, thresh):
+    probs = probs.copy()
+    for k in range(probs.shape[1]):
+        order = [d for d in np.argsort(-probs[:, k], kind="stable") if probs[d, k] > 0]
+        for r, i in enumerate(order):
+            if probs[i, k] == 0:
+                continue
+            for j in order[r + 1:]:
+                if probs[j, k] > 0 and iou(boxes[i], boxes[j]) > thresh:
+                    probs[j, k] = 0
+    return np.array([[*boxes[d], obj[d], k, probs[d, k]] for d in range(len(obj)) for k in range(probs.shape[1]) if probs[d, k] > 0],
+                    np.float32).reshape(-1, 7), probs
+
+
+@pytest.mark.parametrize("share,size,max_dets,favourite", [(0.0, 32, 64, 0), (0.1, 96, 700, 5), (0.02, 64, 256, 0), (0.2, 96, 700, 0), (0.6, 96, 2048, 3), (0.9, 96, 128, 1),
+                                                           (1.0, 128, 4096, 2)])
+def test_detect_equals_the_restatement(tmp_path, share, size, max_dets, favourite):
+    cfg = tmp_path / "net.cfg"
+    cfg.write_text(cfgs.yolov3_tiny_xnor_cfg(size, size))
+    batch = 2
+    net = network.parse_network_cfg(str(cfg), batch, "cuda:0")
+    g = torch.Generator().manual_seed(int(share * 100) + size)
+    heads = []
+    for l in (l for l in net.layers if l.type == "yolo"):
+        h = torch.rand(batch, 3, 85, l.h * l.w, generator=g) * 0.3
+        h[:, :, 2:4] -= 0.15
+        h[:, :, 4] = torch.where(torch.rand(batch, 3, l.h * l.w, generator=g) < share, 0.9 + 0.1 * h[:, :, 4], 0.1 * h[:, :, 4])
+        h[:, :, 5:] = torch.where(torch.rand(batch, 3, 80, l.h * l.w, generator=g) < 0.02, h[:, :, 5:] + 0.6, h[:, :, 5:])
+        if favourite:
+            h[:, :, 5 + favourite] += 0.65                          # one class that nearly every detection belongs to
+        heads.append(h.reshape(batch, 255, l.h, l.w).cuda().contiguous())
+    apart = network.DetectionBuffers(batch, 80, max_dets=max_dets, max_rows=20000)
+    network.get_network_boxes(net, heads, size, size, 0.5, apart)
+    torch.cuda.synchronize()
+    count = apart.count.cpu().numpy()
+    boxes, obj, probs = (t.cpu().numpy() for t in (apart.boxes, apart.objectness, apart.probs))
+    fused = network.DetectionBuffers(batch, 80, max_dets=max_dets, max_rows=20000)
+    network.detect(net, heads, size, size, 0.5, 0.45, fused)
+    network.do_nms_sort(apart, 0.45)
+    network.detection_rows(apart)
+    got, same = fused.rows_host(), apart.rows_host()
+    assert np.array_equal(fused.count.cpu().numpy(), count)
+    for b in range(batch):
+        n = min(int(count[b]), max_dets)
+        assert int(count[b]) == sum(int((h.view(batch, 3, 85, -1)[b, :, 4] > 0.5).sum()) for h in heads)
+        want, kept = expected_rows(boxes[b, :n], obj[b, :n], probs[b, :n], np.float32(0.45))
+        assert np.array_equal(got[b], want) and np.array_equal(same[b], want)
+        assert np.array_equal(fused.probs[b, :n].cpu().numpy(), kept)
