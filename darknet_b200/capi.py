@@ -27,6 +27,7 @@ EXPORTS = (
     "xnor_b200_pack_input_pooled", "xnor_b200_conv_forward_pooled", "xnor_b200_float_conv_small", "xnor_b200_float_conv3_io", "xnor_b200_float_conv_map_weights_bytes",
     "xnor_b200_float_conv_map_prepare", "xnor_b200_float_conv_map", "xnor_b200_float_conv_map_yolo", "xnor_b200_float_conv_1x1_tc", "xnor_b200_yolo_activate", "xnor_b200_region_activate", "xnor_b200_conv_forward_io", "xnor_b200_conv_takes_masks", "xnor_b200_tap_major_weights",
     "xnor_b200_yolo_detections", "xnor_b200_nms_sort", "xnor_b200_detection_rows", "xnor_b200_detect", "xnor_b200_rows_to_host",
+    "xnor_b200_avgpool", "xnor_b200_softmax", "xnor_b200_run_ops", "xnor_b200_float_conv3_words", "xnor_b200_float_conv_tc", "xnor_b200_conv_words", "xnor_b200_conv_words_weights", "xnor_b200_conv_words_weights_bytes", "xnor_b200_sign_words", "xnor_b200_grid_block_words", "xnor_b200_grid_front",
     "xnor_b200_measure_popc_peak", "xnor_b200_measure_bmma_peak", "xnor_b200_measure_umma_i8_peak", "xnor_b200_measure_umma_mxf4_peak",
 )
 
@@ -54,6 +55,28 @@ class ConvIO(C.Structure):
                 ("input_packed", C.c_int), ("window_major", C.c_int), ("sinks", C.POINTER(SignSink)), ("n_sinks", C.c_int),
                 ("input_masks", C.c_void_p), ("tap_major_weights", C.c_int), ("shortcut_signs", C.c_void_p),
                 ("shortcut_sink", C.POINTER(SignSink))]
+
+
+class WordsSource(C.Structure):
+    """struct xnor_b200_words_source"""
+    _fields_ = [("words", C.c_void_p)] + [(n, C.c_int) for n in ("blocks", "h", "w", "pool_stride", "pool_pad", "upsample", "pitch")]
+
+
+class WordsIO(C.Structure):
+    """struct xnor_b200_words_io"""
+    _fields_ = [("sources", WordsSource * 2), ("n_sources", C.c_int), ("output", C.c_void_p), ("output_signs", C.c_void_p),
+                ("shortcut_in", C.c_void_p), ("shortcut_out", C.c_void_p), ("shortcut_signs", C.c_void_p), ("pitch", C.c_int)]
+
+
+(OP_CONV3, OP_SIGN_WORDS, OP_CONV_WORDS, OP_FLOAT_MAP, OP_FLOAT_TC, OP_YOLO, OP_REGION, OP_AVGPOOL, OP_SOFTMAX, OP_FORK,
+ OP_BACK) = range(1, 12)
+OP_INPUT, OP_HEAD = 1, 2
+
+
+class Op(C.Structure):
+    """struct xnor_b200_op"""
+    _fields_ = [("kind", C.c_int), ("arg", C.c_int), ("pitch", C.c_int), ("desc", ConvDesc), ("io", WordsIO), ("input", C.c_void_p),
+                ("output", C.c_void_p), ("weights", C.c_void_p), ("mean_arr", C.c_void_p), ("biases", C.c_void_p)]
 
 
 ROUTE_AUTO, ROUTE_INTEGER, ROUTE_TENSOR, ROUTE_TILED = 0, 1, 2, 3
@@ -129,6 +152,11 @@ def lib() -> C.CDLL:
     L.xnor_b200_conv_forward_pooled.argtypes = [dp, pp, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]
     L.xnor_b200_float_conv_small.argtypes = [dp, vp, vp, vp, vp, vp]
     L.xnor_b200_float_conv3_io.argtypes = [dp, ci, vp, vp, vp, vp, vp, vp, vp]
+    L.xnor_b200_avgpool.argtypes = [vp, vp, ci, ci, vp]
+    L.xnor_b200_softmax.argtypes = [vp, vp, ci, ci, vp]
+    L.xnor_b200_run_ops.argtypes = [C.POINTER(Op), ci, vp, C.POINTER(vp), ci, vp, vp, vp, vp]
+    L.xnor_b200_float_conv_tc.argtypes = [dp, vp, vp, vp, vp, ci, vp]
+    L.xnor_b200_float_conv3_words.argtypes = [dp, ci, vp, vp, vp, vp, ci, vp]
     L.xnor_b200_conv_takes_masks.argtypes = [dp]
     L.xnor_b200_tap_major_weights.argtypes = [dp, vp, vp, vp]
     L.xnor_b200_float_conv_map_weights_bytes.argtypes = [dp]
@@ -143,6 +171,14 @@ def lib() -> C.CDLL:
     L.xnor_b200_yolo_detections.argtypes = [C.POINTER(YoloHead), ci, ci, ci, ci, ci, C.c_float, ci, ci, ci, C.POINTER(Detections), vp]
     L.xnor_b200_nms_sort.argtypes = [C.POINTER(Detections), ci, C.c_float, vp]
     L.xnor_b200_detection_rows.argtypes = [C.POINTER(Detections), ci, vp, ci, vp, vp]
+    L.xnor_b200_conv_words_weights_bytes.restype = sz
+    L.xnor_b200_conv_words_weights_bytes.argtypes = [dp]
+    L.xnor_b200_conv_words_weights.argtypes = [dp, vp, vp, vp]
+    L.xnor_b200_conv_words.argtypes = [dp, C.POINTER(WordsIO), vp, vp, vp, vp]
+    L.xnor_b200_sign_words.argtypes = [vp, ci, ci, ci, ci, ci, vp, vp]
+    L.xnor_b200_grid_block_words.restype = sz
+    L.xnor_b200_grid_block_words.argtypes = [ci, ci, ci]
+    L.xnor_b200_grid_front.argtypes = [ci]
     L.xnor_b200_detect.argtypes = [C.POINTER(YoloHead), ci, ci, ci, ci, ci, ci, C.c_float, ci, ci, C.c_float, C.POINTER(Detections), vp, ci, vp, vp]
     L.xnor_b200_rows_to_host.argtypes = [vp, ci, vp, ci, ci, vp, vp, vp]
     L.xnor_b200_conv_forward_static.argtypes = [dp, vp, vp, vp, vp, vp, vp, vp, vp]
@@ -160,8 +196,14 @@ def check(code: int, where: str) -> None:
         raise XnorError(code, where)
 
 
+# True while set_tuning pins kernels of the packed-operand route: the callers that would otherwise take the sign-word route ask
+packed_route_pinned = False
+
+
 def set_tuning(**fields) -> None:
     """xnor_b200_set_tuning: pins kernel choices process-wide (tests and benchmarks); no arguments = library defaults."""
+    global packed_route_pinned
+    packed_route_pinned = any(fields.get(k) for k in ("gemm_route", "tc_kernel", "pack_ctas_per_sm", "pack_two_pass"))
     if not fields:
         check(lib().xnor_b200_set_tuning(None), "xnor_b200_set_tuning")
         return

@@ -7,7 +7,7 @@
 // its output (16 planes of the full-resolution image), not by arithmetic, so one pass that reads the image once
 // and writes every output plane once, coalesced, is the whole optimisation; a GEMM formulation would only add an
 // im2col buffer.  Accumulation order is (channel, ky, kx) with fused multiply-adds, bias added last.
-#include "xnor_common.cuh"
+#include "grid_words.cuh"
 
 namespace xnor
 {
@@ -103,19 +103,31 @@ float_conv_small_kernel(const FloatConvParams p)
 	}
 }
 
-// ---- 3 input channels, 3x3, stride 1, pad 1: a thread computes a 2x2 block of outputs for 8 filters ----------
-// The first layer of every xnor network.  One thread loads the 4x4x3 input patch of its block once (48 values in
-// registers) and reads each weight once per block as part of a 16-byte vector, so the kernel runs at FMA speed
-// instead of one shared-memory load per multiply.  Three ways to finish, chosen by the caller:
+// ---- 3 input channels, 3x3, stride 1, pad 1: a thread computes a 4x4 block of outputs, four filters at a time --------------
+// The first layer of every xnor network.  Bound by the FMA pipe (27 multiply-adds a value) as long as nothing else is: a CTA
+// stages its 32x32 tile with its border in shared memory once; a thread keeps four filters' accumulators for its 16 pixels, so
+// that a 16-byte read of weights feeds 64 multiply-adds.  (A 16-byte shared-memory read delivers 512 bytes to a warp and holds the
+// SM's one port for four cycles even when every lane reads the same address.  Packed multiply-adds, fma.rn.f32x2, run at the
+// same rate -- 61 TFLOP/s measured against 62 -- and need every second pair of columns copied together: 1350 us.)
+// 16 filters at 416x416, 256 images, pooled signs: 1489 us with 2x2 pixels and the patch from global memory, 1070 us now; the
+// multiply-adds alone take 620 us at the measured rate.
+//
+// Every map of a multiple of 32 rows and columns is covered without idle threads.  Ways to finish, chosen by the caller:
 //   * fp32 output at full resolution (bias, leaky/linear);
 //   * the [maxpool] size 2 / stride 2 that follows the layer applied in registers, fp32 output at half resolution
 //     (leaky is monotonic, so max(act(v)) == act(max(v)) value for value);
-//   * only the SIGN of that pooled output, as x-packed bit planes uint32 [image][filter][H/2][ceil(W/2/32)] -- what
-//     a following xnor layer needs and nothing more (max > 0 exactly when one of the four values is > 0).
+//   * only the SIGN of either, which is what a following xnor layer needs (max > 0 exactly when one of the four values is > 0):
+//     as grid words (one 32-channel word per pixel on the padded grid of grid_words.cuh), as channel masks per pixel, or -- pooled
+//     only -- as x-packed bit planes uint32 [image][filter][H/2][ceil(W/2/32)].
 // Each output value is formed exactly as in float_conv_small_kernel: fmaf over (channel, ky, kx) from zero, then
-// + bias, so the three variants and that kernel agree bit for bit.
-constexpr int FB_THREADS = 256;          // 8 warps: warp w = block row w of the tile, lane = block column
-constexpr int FB_FILTERS = 8;            // filters per thread (blockIdx.y picks the group)
+// + bias, so all variants and that kernel agree bit for bit.
+constexpr int FB_THREADS = 64;           // 2 warps; a warp covers 32 columns x 16 rows of the tile, a lane 4 x 4
+constexpr int FB_TILE = 32;
+constexpr int FB_PITCH = FB_TILE + 4;    // columns -1 .. 32 and two more, so that rows stay 16-byte aligned
+constexpr int FB_ROWS = FB_TILE + 2;
+constexpr int FB_FILTERS = 4;            // filters at a time
+constexpr int FB_MAX_FILTERS = 32;       // most filters per CTA: one sign word
+constexpr int FB_SMALL_TILES = 4;        // tiles per SM up to which a CTA takes 8 filters only
 
 struct FloatBlockParams
 {
@@ -124,172 +136,217 @@ struct FloatBlockParams
 	const float * biases;    // [n] or nullptr
 	float * out;             // fp32 output (full or pooled) or nullptr
 	uint32_t * planes;       // pooled sign planes or nullptr
-	uint8_t * masks;         // pooled sign masks [image][H/2][W/2][ceil(N/8)] (bit f%8 of byte f/8) or nullptr
+	uint8_t * masks;         // sign masks [image][pixels][ceil(N/8)] (bit f%8 of byte f/8) or nullptr
+	uint32_t * words;        // sign words on the grid, or nullptr
+	int block_words, front, pitch;
 	int H, W, N;
-	int BH, BW;              // 2x2 blocks per column / row: ceil(H/2), ceil(W/2)
-	int xtiles;              // ceil(BW / 32)
-	int pooled;              // 1: one value per block
+	int OH, OW;              // output map (half the input's when pooled)
+	int plane_words;         // ceil(OW / 32)
+	int xtiles;
+	int fpc;                 // filters per CTA: a multiple of 8, at most FB_MAX_FILTERS (blockIdx.y picks them)
+	int pooled;
 	int leaky;
 };
 
-__global__ void __launch_bounds__(FB_THREADS)
-float_conv3_block_kernel(const FloatBlockParams p)
+__global__ void __launch_bounds__(FB_THREADS, 8)
+float_conv3_block_kernel(const __grid_constant__ FloatBlockParams p)
 {
-	__shared__ __align__(16) float s_w[27 * FB_FILTERS];      // [tap][filter of this group]
-	__shared__ float s_b[FB_FILTERS];
-	const int f0 = blockIdx.y * FB_FILTERS;
-	for (int i = threadIdx.x; i < 27 * FB_FILTERS; i += FB_THREADS)
+	__shared__ __align__(16) float s_in[3][FB_ROWS][FB_PITCH];
+	__shared__ __align__(16) float s_w[27 * FB_MAX_FILTERS];       // [group of 4 filters][tap][filter]
+	__shared__ float s_b[FB_MAX_FILTERS];
+	const int tid = threadIdx.x;
+	const int lane = tid & 31, warp = tid >> 5;
+	const int f0 = blockIdx.y * p.fpc;
+	const int nf = min(p.fpc, p.N - f0);
+	const int groups = (nf + FB_FILTERS - 1) / FB_FILTERS;
+	for (int i = tid; i < groups * 27 * FB_FILTERS; i += FB_THREADS)
 	{
-		const int k = i / FB_FILTERS;
-		const int f = f0 + (i - k * FB_FILTERS);
-		s_w[i] = (f < p.N) ? p.weights[(size_t)f * 27 + k] : 0.0f;
+		const int g = i / (27 * FB_FILTERS);
+		const int k = (i - g * 27 * FB_FILTERS) / FB_FILTERS;
+		const int f = g * FB_FILTERS + i % FB_FILTERS;
+		s_w[i] = (f < nf) ? __ldg(p.weights + (size_t)(f0 + f) * 27 + k) : 0.0f;
 	}
-	if (threadIdx.x < FB_FILTERS)
+	for (int f = tid; f < groups * FB_FILTERS; f += FB_THREADS) { s_b[f] = (p.biases != nullptr && f < nf) ? __ldg(p.biases + f0 + f) : 0.0f; }
+	const int ty = blockIdx.x / p.xtiles;
+	const int tx = blockIdx.x - ty * p.xtiles;
+	const int y0 = ty * FB_TILE, x0 = tx * FB_TILE;
+	const float * img = p.in + (size_t)blockIdx.z * 3 * p.H * p.W;
+	// The tile with its border.  Rows: a warp takes every second one, 17 loads in flight; the columns left and right of the tile are
+	// dealt over all threads behind them.  Tiles inside the image need no checks.
 	{
-		const int f = f0 + threadIdx.x;
-		s_b[threadIdx.x] = (p.biases != nullptr && f < p.N) ? p.biases[f] : 0.0f;
+		constexpr int ROUNDS = FB_ROWS / 2;
+		const bool inside = (y0 > 0 && x0 > 0 && y0 + FB_TILE < p.H && x0 + FB_TILE < p.W);
+		const float * at = img + (ptrdiff_t)(y0 - 1 + warp) * p.W + x0 + lane;
+		const size_t step = 2 * (size_t)p.W;
+		const bool in_x = (x0 + lane < p.W);
+		#pragma unroll 1
+		for (int c = 0; c < 3; ++c, at += (size_t)p.H * p.W)
+		{
+			float v[ROUNDS];
+			const float * row = at;
+			#pragma unroll
+			for (int r = 0; r < ROUNDS; ++r, row += step)
+			{
+				const int iy = y0 - 1 + r * 2 + warp;
+				v[r] = (inside || (iy >= 0 && iy < p.H && in_x)) ? __ldg(row) : 0.0f;
+			}
+			float * dst = &s_in[c][warp][lane + 1];
+			#pragma unroll
+			for (int r = 0; r < ROUNDS; ++r) { dst[r * 2 * FB_PITCH] = v[r]; }
+		}
+		for (int i = tid; i < 3 * FB_ROWS * 2; i += FB_THREADS)
+		{
+			const int right = i & 1, row = i >> 1;
+			const int c = row / FB_ROWS, r = row - c * FB_ROWS;
+			const int iy = y0 - 1 + r, ix = right ? x0 + FB_TILE : x0 - 1;
+			s_in[c][r][right ? FB_TILE + 1 : 0] = (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) ? __ldg(img + ((size_t)c * p.H + iy) * p.W + ix) : 0.0f;
+		}
 	}
 	__syncthreads();
 
-	const int lane = threadIdx.x & 31;
-	const int warp = threadIdx.x >> 5;
-	const int xt = blockIdx.x % p.xtiles;
-	const int yt = blockIdx.x / p.xtiles;
-	const int bx = xt * 32 + lane;
-	const int by = yt * 8 + warp;
-	const bool live = (bx < p.BW && by < p.BH);
-	const float * img = p.in + (size_t)blockIdx.z * 3 * p.H * p.W;
-
-	// the 4x4 patch of each channel: rows 2by-1 .. 2by+2, columns 2bx-1 .. 2bx+2
-	float v[3][4][4];
+	const int bx = (lane & 7) * 4;                               // first column and row of this thread's block inside the tile
+	const int by = warp * 16 + (lane >> 3) * 4;
+	const int gx = x0 + bx, gy = y0 + by;
+	const bool live = (gx < p.W && gy < p.H);
+	uint32_t bits[16];                                           // sign bits of the filters so far, newest lowest, per pixel (pooled: the first four)
 	#pragma unroll
-	for (int c = 0; c < 3; ++c)
+	for (int i = 0; i < 16; ++i) { bits[i] = 0; }
+	#pragma unroll 1
+	for (int g = 0; g < groups; ++g)
 	{
+		float acc[FB_FILTERS][4][4];                             // [filter][row][column]
 		#pragma unroll
-		for (int r = 0; r < 4; ++r)
+		for (int f = 0; f < FB_FILTERS; ++f)
 		{
-			const int iy = 2 * by - 1 + r;
 			#pragma unroll
-			for (int q = 0; q < 4; ++q)
-			{
-				const int ix = 2 * bx - 1 + q;
-				const bool ok = live && iy >= 0 && iy < p.H && ix >= 0 && ix < p.W;
-				v[c][r][q] = ok ? __ldg(img + ((size_t)c * p.H + iy) * p.W + ix) : 0.0f;
-			}
+			for (int i = 0; i < 16; ++i) { acc[f][i / 4][i % 4] = 0.0f; }
 		}
-	}
-	float acc[FB_FILTERS][4];              // [filter][2*dy + dx]
-	#pragma unroll
-	for (int f = 0; f < FB_FILTERS; ++f)
-	{
+		const float4 * wg = reinterpret_cast<const float4 *>(s_w + g * 27 * FB_FILTERS);
 		#pragma unroll
-		for (int o = 0; o < 4; ++o) { acc[f][o] = 0.0f; }
-	}
-	#pragma unroll
-	for (int c = 0; c < 3; ++c)
-	{
-		#pragma unroll
-		for (int ky = 0; ky < 3; ++ky)
+		for (int c = 0; c < 3; ++c)
 		{
+			float v[6][6];
 			#pragma unroll
-			for (int kx = 0; kx < 3; ++kx)
+			for (int r = 0; r < 6; ++r)
 			{
-				const int k = (c * 3 + ky) * 3 + kx;
-				const float4 wa = *reinterpret_cast<const float4 *>(s_w + k * FB_FILTERS);
-				const float4 wb = *reinterpret_cast<const float4 *>(s_w + k * FB_FILTERS + 4);
-				const float w[FB_FILTERS] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+				const float4 a = *reinterpret_cast<const float4 *>(&s_in[c][by + r][bx]);
+				const float2 b = *reinterpret_cast<const float2 *>(&s_in[c][by + r][bx + 4]);
+				v[r][0] = a.x; v[r][1] = a.y; v[r][2] = a.z; v[r][3] = a.w; v[r][4] = b.x; v[r][5] = b.y;
+			}
+			#pragma unroll
+			for (int k = 0; k < 9; ++k)
+			{
+				const int ky = k / 3, kx = k % 3;
+				const float4 w4 = wg[c * 9 + k];
+				const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 				#pragma unroll
 				for (int f = 0; f < FB_FILTERS; ++f)
 				{
-					acc[f][0] = fmaf(v[c][ky][kx], w[f], acc[f][0]);
-					acc[f][1] = fmaf(v[c][ky][kx + 1], w[f], acc[f][1]);
-					acc[f][2] = fmaf(v[c][ky + 1][kx], w[f], acc[f][2]);
-					acc[f][3] = fmaf(v[c][ky + 1][kx + 1], w[f], acc[f][3]);
+					#pragma unroll
+					for (int i = 0; i < 16; ++i) { acc[f][i / 4][i % 4] = fmaf(v[ky + i / 4][kx + i % 4], w[f], acc[f][i / 4][i % 4]); }
 				}
 			}
 		}
-	}
-
-	const bool col1 = (2 * bx + 1 < p.W);
-	const bool row1 = (2 * by + 1 < p.H);
-	if (p.masks != nullptr && !p.pooled)
-	{
-		// sign of this thread's 8 filters at each of its four pixels, one byte of each pixel's channel mask; with 32
-		// filters the four bytes of a pixel are the channel-packed sign word an xnor layer over 32 channels reads
-		uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
 		#pragma unroll
 		for (int f = 0; f < FB_FILTERS; ++f)
 		{
-			const uint32_t on = (f0 + f < p.N) ? 1u : 0u;
-			m0 |= (on & (acc[f][0] + s_b[f] > 0.0f ? 1u : 0u)) << f;
-			m1 |= (on & (acc[f][1] + s_b[f] > 0.0f ? 1u : 0u)) << f;
-			m2 |= (on & (acc[f][2] + s_b[f] > 0.0f ? 1u : 0u)) << f;
-			m3 |= (on & (acc[f][3] + s_b[f] > 0.0f ? 1u : 0u)) << f;
-		}
-		if (live)
-		{
-			uint8_t * dst = p.masks + (((size_t)blockIdx.z * p.H + 2 * by) * p.W + 2 * bx) * gridDim.y + blockIdx.y;
-			dst[0] = (uint8_t)m0;
-			if (col1) { dst[gridDim.y] = (uint8_t)m1; }
-			if (row1)
+			const int fl = g * FB_FILTERS + f;
+			const float b = s_b[fl];
+			if (p.pooled)
 			{
-				dst[(size_t)p.W * gridDim.y] = (uint8_t)m2;
-				if (col1) { dst[(size_t)(p.W + 1) * gridDim.y] = (uint8_t)m3; }
+				// adding the bias keeps the order of values, so the largest sum is the largest value plus the bias
+				float top[4];
+				#pragma unroll
+				for (int i = 0; i < 4; ++i)
+				{
+					const int y = (i >> 1) * 2, x = (i & 1) * 2;
+					top[i] = fmaxf(fmaxf(acc[f][y][x], acc[f][y][x + 1]), fmaxf(acc[f][y + 1][x], acc[f][y + 1][x + 1]));
+				}
+				if (p.out == nullptr && p.planes == nullptr)
+				{
+					// value > 0 is the sign bit of -bias - top, whatever the signs of zeros
+					#pragma unroll
+					for (int i = 0; i < 4; ++i) { bits[i] = __funnelshift_l(__float_as_uint(__fsub_rn(-b, top[i])), bits[i], 1); }
+					continue;
+				}
+				#pragma unroll
+				for (int y = 0; y < 2; ++y)
+				{
+					const int oy = (gy >> 1) + y;
+					float m[2] = {top[2 * y] + b, top[2 * y + 1] + b};
+					if (p.out != nullptr)
+					{
+						if (!live || oy >= p.OH || fl >= nf) { continue; }
+						float * dst = p.out + (((size_t)blockIdx.z * p.N + f0 + fl) * p.OH + oy) * p.OW + (gx >> 1);
+						#pragma unroll
+						for (int i = 0; i < 2; ++i)
+						{
+							if (p.leaky) { m[i] = (m[i] > 0.0f) ? m[i] : m[i] * 0.1f; }
+							if ((gx >> 1) + i < p.OW) { dst[i] = m[i]; }
+						}
+					}
+					else
+					{
+						// two bits of the lane's 16-column half word, gathered over the eight lanes of its rows
+						uint32_t half = (m[0] > 0.0f ? 1u : 0u) | ((m[1] > 0.0f && (gx >> 1) + 1 < p.OW) ? 2u : 0u);
+						half = live ? half << (2 * (lane & 7)) : 0u;
+						half |= __shfl_xor_sync(0xffffffffu, half, 1);
+						half |= __shfl_xor_sync(0xffffffffu, half, 2);
+						half |= __shfl_xor_sync(0xffffffffu, half, 4);
+						if ((lane & 7) == 0 && oy < p.OH && fl < nf)
+						{
+							uint16_t * row = reinterpret_cast<uint16_t *>(p.planes + (((size_t)blockIdx.z * p.N + f0 + fl) * p.OH + oy) * p.plane_words);
+							row[tx] = (uint16_t)half;
+							if (tx == p.xtiles - 1 && tx % 2 == 0) { row[tx + 1] = 0; }
+						}
+					}
+				}
+				continue;
 			}
+			if (p.out != nullptr)
+			{
+				if (!live || fl >= nf) { continue; }
+				float r[4][4];
+				#pragma unroll
+				for (int i = 0; i < 16; ++i) { r[i / 4][i % 4] = acc[f][i / 4][i % 4] + b; }
+				float * dst = p.out + (((size_t)blockIdx.z * p.N + f0 + fl) * p.H + gy) * p.W + gx;
+				#pragma unroll
+				for (int y = 0; y < 4; ++y)
+				{
+					#pragma unroll
+					for (int x = 0; x < 4; ++x) { if (p.leaky) { r[y][x] = (r[y][x] > 0.0f) ? r[y][x] : r[y][x] * 0.1f; } }
+					if (gy + y >= p.H) { break; }
+					if (p.W % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0)
+					{
+						*reinterpret_cast<float4 *>(dst + (size_t)y * p.W) = make_float4(r[y][0], r[y][1], r[y][2], r[y][3]);
+						continue;
+					}
+					#pragma unroll
+					for (int x = 0; x < 4; ++x) { if (gx + x < p.W) { dst[(size_t)y * p.W + x] = r[y][x]; } }
+				}
+				continue;
+			}
+			#pragma unroll
+			for (int i = 0; i < 16; ++i) { bits[i] = __funnelshift_l(__float_as_uint(__fsub_rn(-b, acc[f][i / 4][i % 4])), bits[i], 1); }
 		}
-		return;
 	}
-	if (p.masks != nullptr)
-	{
-		// pooled sign of this thread's 8 filters as one byte of the pixel's channel mask
-		uint32_t m = 0;
-		#pragma unroll
-		for (int f = 0; f < FB_FILTERS; ++f)
-		{
-			const float r0 = acc[f][0] + s_b[f], r1 = acc[f][1] + s_b[f], r2 = acc[f][2] + s_b[f], r3 = acc[f][3] + s_b[f];
-			m |= ((f0 + f < p.N) && (r0 > 0.0f || r1 > 0.0f || r2 > 0.0f || r3 > 0.0f) ? 1u : 0u) << f;
-		}
-		if (live) { p.masks[(((size_t)blockIdx.z * p.BH + by) * p.BW + bx) * gridDim.y + blockIdx.y] = (uint8_t)m; }
-		return;
-	}
+	if (p.out != nullptr || p.planes != nullptr || !live) { return; }
+	// this CTA's bytes of every pixel's mask or word; filters that do not exist have weights 0 and bias 0: not > 0
+	const int bytes = (p.words != nullptr) ? 4 : (p.N + 7) / 8;
 	#pragma unroll
-	for (int f = 0; f < FB_FILTERS; ++f)
+	for (int i = 0; i < 16; ++i)
 	{
-		const float r0 = acc[f][0] + s_b[f], r1 = acc[f][1] + s_b[f], r2 = acc[f][2] + s_b[f], r3 = acc[f][3] + s_b[f];
-		if (p.planes != nullptr)
-		{
-			// pooled sign: the block lies inside the image whenever it is live (H and W are even in this mode)
-			const uint32_t word = __ballot_sync(0xffffffffu, live && (r0 > 0.0f || r1 > 0.0f || r2 > 0.0f || r3 > 0.0f));
-			if (lane == 0 && by < p.BH && f0 + f < p.N)
-			{
-				p.planes[(((size_t)blockIdx.z * p.N + f0 + f) * p.BH + by) * p.xtiles + xt] = word;
-			}
-			continue;
-		}
-		if (!live || f0 + f >= p.N) { continue; }
-		if (p.pooled)
-		{
-			float m = fmaxf(fmaxf(r0, r1), fmaxf(r2, r3));
-			if (p.leaky) { m = (m > 0.0f) ? m : m * 0.1f; }
-			p.out[(((size_t)blockIdx.z * p.N + f0 + f) * p.BH + by) * p.BW + bx] = m;
-		}
-		else
-		{
-			float a0 = r0, a1 = r1, a2 = r2, a3 = r3;
-			if (p.leaky)
-			{
-				a0 = (a0 > 0.0f) ? a0 : a0 * 0.1f; a1 = (a1 > 0.0f) ? a1 : a1 * 0.1f;
-				a2 = (a2 > 0.0f) ? a2 : a2 * 0.1f; a3 = (a3 > 0.0f) ? a3 : a3 * 0.1f;
-			}
-			float * dst = p.out + (((size_t)blockIdx.z * p.N + f0 + f) * p.H + 2 * by) * p.W + 2 * bx;
-			dst[0] = a0;
-			if (col1) { dst[1] = a1; }
-			if (row1)
-			{
-				dst[p.W] = a2;
-				if (col1) { dst[p.W + 1] = a3; }
-			}
-		}
+		if (p.pooled && i >= 4) { break; }
+		const int oy = p.pooled ? (gy >> 1) + (i >> 1) : gy + (i >> 2);
+		const int ox = p.pooled ? (gx >> 1) + (i & 1) : gx + (i & 3);
+		if (oy >= p.OH || ox >= p.OW) { continue; }
+		const uint32_t word = __brev(bits[i]) >> (32 - groups * FB_FILTERS);         // filter f at bit f
+		uint8_t * dst = (p.words != nullptr)
+				? reinterpret_cast<uint8_t *>(p.words + (size_t)(f0 >> 5) * p.block_words + p.front + ((size_t)blockIdx.z * (p.OH + 1) + oy) * p.pitch + ox) + ((f0 & 31) >> 3)
+				: p.masks + (((size_t)blockIdx.z * p.OH + oy) * p.OW + ox) * bytes + (f0 >> 3);
+		// a CTA that has all of a word's filters writes the whole word
+		if (p.words != nullptr && (p.fpc == FB_MAX_FILTERS || p.fpc >= p.N)) { *reinterpret_cast<uint32_t *>(dst) = word; }
+		else { for (int q = 0; q * 8 < nf; ++q) { dst[q] = (uint8_t)(word >> (8 * q)); } }
 	}
 }
 
@@ -330,27 +387,56 @@ extern "C" int xnor_b200_float_conv_small(const xnor_b200_conv_desc * desc, cons
 	return check_launch();
 }
 
-extern "C" int xnor_b200_float_conv3_io(const xnor_b200_conv_desc * desc, int pool, const float * input, const float * weights,
-		const float * biases, float * output, uint32_t * output_sign_planes, uint8_t * output_sign_masks, void * stream)
+static int launch_conv3(const xnor_b200_conv_desc * desc, int pool, const float * input, const float * weights, const float * biases,
+		FloatBlockParams & p, void * stream)
 {
 	if (desc == nullptr || input == nullptr || weights == nullptr) { return XNOR_B200_ERR_NULL; }
-	if ((output != nullptr) + (output_sign_planes != nullptr) + (output_sign_masks != nullptr) != 1) { return XNOR_B200_ERR_NULL; }
+	if ((p.out != nullptr) + (p.planes != nullptr) + (p.masks != nullptr) + (p.words != nullptr) != 1) { return XNOR_B200_ERR_NULL; }
 	int rc = validate_desc(desc);
 	if (rc != XNOR_B200_OK) { return rc; }
 	if (desc->c != 3 || desc->size != 3 || desc->stride != 1 || desc->pad != 1) { return XNOR_B200_ERR_INVALID; }
 	if (pool != 0 && pool != 2) { return XNOR_B200_ERR_INVALID; }
 	if (pool == 2 && (desc->h % 2 != 0 || desc->w % 2 != 0)) { return XNOR_B200_ERR_INVALID; }
-	if (output_sign_planes != nullptr && pool != 2) { return XNOR_B200_ERR_INVALID; }
-	FloatBlockParams p;
-	p.in = input; p.weights = weights; p.biases = biases; p.out = output; p.planes = output_sign_planes; p.masks = output_sign_masks;
+	if (p.planes != nullptr && pool != 2) { return XNOR_B200_ERR_INVALID; }
+	p.in = input; p.weights = weights; p.biases = biases;
 	p.H = desc->h; p.W = desc->w; p.N = desc->n;
-	p.BH = (desc->h + 1) / 2; p.BW = (desc->w + 1) / 2;
-	p.xtiles = (p.BW + 31) / 32;
 	p.pooled = (pool == 2) ? 1 : 0;
+	p.OH = p.pooled ? desc->h / 2 : desc->h;
+	p.OW = p.pooled ? desc->w / 2 : desc->w;
+	p.plane_words = (p.OW + 31) / 32;
+	p.xtiles = (desc->w + FB_TILE - 1) / FB_TILE;
 	p.leaky = (desc->activation == XNOR_B200_LEAKY) ? 1 : 0;
-	const long long tiles = (long long)p.xtiles * ((p.BH + 7) / 8);
-	const int groups = (desc->n + FB_FILTERS - 1) / FB_FILTERS;
+	if (p.words != nullptr)
+	{
+		if (p.pitch == 0) { p.pitch = p.OW + 1; }
+		if (p.pitch <= p.OW) { return XNOR_B200_ERR_INVALID; }
+		if (xnor_b200_grid_block_words(desc->batch, p.OH, p.pitch) == 0) { return XNOR_B200_ERR_TOO_LARGE; }
+		p.front = grid_front(p.pitch);
+		p.block_words = grid_block_words(desc->batch, p.OH, p.pitch);
+	}
+	const long long tiles = (long long)p.xtiles * ((desc->h + FB_TILE - 1) / FB_TILE);
+	// All of a pixel's filters in one CTA read the tile once and write whole words; with few tiles, eight filters each, so that
+	// the GPU fills (one image of 416x416, 16 filters: 169 tiles).
+	p.fpc = (tiles * desc->batch <= (long long)FB_SMALL_TILES * sm_count()) ? 8 : FB_MAX_FILTERS;
+	const int groups = (desc->n + p.fpc - 1) / p.fpc;
 	if (tiles > 0x7fffffffLL || groups > 65535 || desc->batch > 65535) { return XNOR_B200_ERR_TOO_LARGE; }
 	float_conv3_block_kernel<<<dim3((unsigned)tiles, (unsigned)groups, (unsigned)desc->batch), FB_THREADS, 0, (cudaStream_t)stream>>>(p);
 	return check_launch();
+}
+
+extern "C" int xnor_b200_float_conv3_io(const xnor_b200_conv_desc * desc, int pool, const float * input, const float * weights,
+		const float * biases, float * output, uint32_t * output_sign_planes, uint8_t * output_sign_masks, void * stream)
+{
+	FloatBlockParams p = {};
+	p.out = output; p.planes = output_sign_planes; p.masks = output_sign_masks;
+	return launch_conv3(desc, pool, input, weights, biases, p, stream);
+}
+
+extern "C" int xnor_b200_float_conv3_words(const xnor_b200_conv_desc * desc, int pool, const float * input, const float * weights,
+		const float * biases, uint32_t * words, int pitch, void * stream)
+{
+	FloatBlockParams p = {};
+	p.words = words;
+	p.pitch = pitch;
+	return launch_conv3(desc, pool, input, weights, biases, p, stream);
 }

@@ -1,5 +1,7 @@
-// Float 1x1 / stride-1 convolutions at batch (the heads behind the xnor path: yolo and region heads, 255..1024 filters
-// over 256..1024 channels and tens of thousands of pixels) on the tcgen05 tensor cores, at fp32 accuracy.
+// Float 1x1 and 3x3 stride-1 convolutions at batch (the layers behind the xnor path: yolo and region heads, 255..1024 filters
+// over 256..1024 channels and tens of thousands of pixels, and the 3x3 layer in front of a head) on the tcgen05 tensor cores, at
+// fp32 accuracy.  A 3x3 layer is the same GEMM with K = (tap, channel): a K block of 32 channels lies in one tap, so its pixel
+// rows are the 1x1 layer's, shifted, with zeros where the tap leaves the map.
 //
 // Replaces, for those layers, the float branch of forward_convolutional_layer_gpu (src-lib/convolutional_kernels.cu:373-434:
 // a cuBLAS/cuDNN GEMM per image) + add_bias_gpu + activate_array_ongpu.  out[b][f][p] = bias[f] + sum_c w[f][c] * x[b][c][p].
@@ -15,7 +17,9 @@
 // src-lib/convolutional_layer.cpp:350).
 //
 // Same skeleton as xnor_gemm_tc.cu: one CTA = 128 pixels (TMEM lanes; the batch is folded into the pixel index) x 128
-// filters (TMEM columns), warp 0 allocates tensor memory and one lane issues, 16 producer warps -- two threads per operand
+// filters (TMEM columns), warp 0 allocates tensor memory and issues (the warp stays converged and one elected lane issues: a
+// divergent lane takes longer to bring an instruction's operands to the uniform registers than the tensor core to execute it),
+// 16 producer warps -- two threads per operand
 // row, 16 channels of every K block each (pixel row: one coalesced load per channel across the warp; filter row: 64
 // contiguous bytes) -- split their values and write hi and lo straight into K-major SWIZZLE_128B tiles (32 tf32 = one 128-byte row); 12
 // tcgen05.mma.kind::tf32 (M=128, N=128, K=8) per K block of 32 channels; the same warps then add the bias, apply leaky and
@@ -40,12 +44,15 @@ constexpr int FT_THREADS = 32 + 32 * FT_PRODUCER_WARPS;
 struct FtParams
 {
 	const float * x;      // [batch][C][HW]
-	const float * w;      // [N][C]
+	const float * w;      // [N][taps][C]
 	const float * bias;   // [N] or nullptr
 	float * out;          // [batch][N][HW]
 	int C, HW, N;
 	int total;            // batch * HW
-	int kblocks;          // ceil(C / 32)
+	int H, W, taps;       // taps 1 or 9
+	int cblocks;          // ceil(C / 32): K blocks per tap
+	int kblocks;          // taps * cblocks
+	int yolo_entries;     // > 0: the [yolo] layer's activation step is applied to the result (xnor_b200_yolo_activate)
 	int leaky;
 	int tiles_f;
 	int w_vec;            // 1: weight rows may be read with 16-byte loads
@@ -88,7 +95,7 @@ float_conv_tc_kernel(const FtParams p)
 	volatile int * s_failed = &s_failed_storage;
 
 	const int tid = threadIdx.x;
-	const int warp = tid >> 5;
+	const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 	const int lane = tid & 31;
 	const uint32_t ring = (smem_u32(ft_smem_raw) + 1023u) & ~1023u;
 	const int tile_p = blockIdx.x / p.tiles_f;
@@ -115,19 +122,19 @@ float_conv_tc_kernel(const FtParams p)
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-	const uint32_t tmem_base = tmem_base_slot;
+	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
 
 	if (warp == 0)
 	{
-		if (lane == 0)
 		{
+			const bool leader = elect_one();
 			// instruction descriptor: D = f32, A = B = tf32, both K-major, N = 128, M = 128
 			const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(FT_NF >> 3) << 17) | ((uint32_t)(TC_PIX >> 4) << 24);
 			bool ok = true;
 			for (int kb = 0; kb < p.kblocks && ok; ++kb)
 			{
 				const int s = kb % FT_STAGES;
-				ok = mbar_wait(&bar_full[s], (uint32_t)((kb / FT_STAGES) & 1), s_failed, p.spin_limit);
+				ok = __all_sync(0xffffffffu, mbar_wait(&bar_full[s], (uint32_t)((kb / FT_STAGES) & 1), s_failed, p.spin_limit));
 				if (!ok) { break; }
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 				const uint32_t a_hi = ring + (uint32_t)s * FT_STAGE_BYTES;
@@ -143,17 +150,17 @@ float_conv_tc_kernel(const FtParams p)
 						const uint64_t adesc = make_smem_desc((term == 0 ? a_lo : a_hi) + k * 32);
 						const uint64_t bdesc = make_smem_desc((term == 1 ? b_lo : b_hi) + k * 32);
 						const uint32_t accumulate = (kb >= FT_ACCS || k > 0 || term > 0) ? 1u : 0u;
-						asm volatile(
+						if (leader) asm volatile(
 							"{\n\t.reg .pred p;\n\t"
 							"setp.ne.b32 p, %4, 0;\n\t"
 							"tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
 							:: "r"(tmem_base + (uint32_t)((kb % FT_ACCS) * FT_NF)), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 					}
 				}
-				asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+				if (leader) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
 						:: "r"(smem_u32(&bar_empty[s])) : "memory");
 			}
-			if (ok)
+			if (ok && leader)
 			{
 				asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
 						:: "r"(smem_u32(&bar_done)) : "memory");
@@ -176,18 +183,30 @@ float_conv_tc_kernel(const FtParams p)
 		const int img = (is_pix && row_ok) ? g / p.HW : 0;
 		const int pix = (is_pix && row_ok) ? g - img * p.HW : 0;
 		// element c of the row is base[c * stride]
-		const float * base = is_pix ? p.x + (size_t)img * p.C * p.HW + pix : p.w + (size_t)(row_ok ? f : 0) * p.C;
+		const float * base = is_pix ? p.x + (size_t)img * p.C * p.HW + pix : p.w + (size_t)(row_ok ? f : 0) * p.C * p.taps;
 		const size_t stride = is_pix ? (size_t)p.HW : 1;
+		const int py = pix / p.W, px = pix - py * p.W;
 		float nxt[FT_CH];
-		auto fetch = [&](int kb)
+		int tap = 0, cb = 0;                                      // of the K block that is fetched next
+		auto fetch = [&]()
 		{
-			const int c0 = kb * 32 + part * FT_CH;
-			if (!is_pix && p.w_vec && row_ok && c0 + FT_CH <= p.C)
+			const int c0 = cb * 32 + part * FT_CH;
+			const float * at = base;
+			bool ok = row_ok;
+			if (p.taps == 9 && is_pix)
+			{
+				const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+				ok = ok && py + dy >= 0 && py + dy < p.H && px + dx >= 0 && px + dx < p.W;
+				at += dy * p.W + dx;
+			}
+			if (!is_pix) { at += (size_t)tap * p.C; }
+			if (++cb == p.cblocks) { cb = 0; ++tap; }
+			if (!is_pix && p.w_vec && ok && c0 + FT_CH <= p.C)
 			{
 				#pragma unroll
 				for (int q = 0; q < FT_CH / 4; ++q)
 				{
-					const float4 t = __ldg(reinterpret_cast<const float4 *>(base + c0) + q);
+					const float4 t = __ldg(reinterpret_cast<const float4 *>(at + c0) + q);
 					nxt[4 * q] = t.x; nxt[4 * q + 1] = t.y; nxt[4 * q + 2] = t.z; nxt[4 * q + 3] = t.w;
 				}
 				return;
@@ -195,10 +214,10 @@ float_conv_tc_kernel(const FtParams p)
 			#pragma unroll
 			for (int k = 0; k < FT_CH; ++k)
 			{
-				nxt[k] = (row_ok && c0 + k < p.C) ? __ldg(base + (size_t)(c0 + k) * stride) : 0.0f;
+				nxt[k] = (ok && c0 + k < p.C) ? __ldg(at + (size_t)(c0 + k) * stride) : 0.0f;
 			}
 		};
-		fetch(0);
+		fetch();
 		bool ok = true;
 		for (int kb = 0; kb < p.kblocks; ++kb)
 		{
@@ -206,7 +225,7 @@ float_conv_tc_kernel(const FtParams p)
 			float cur[FT_CH];
 			#pragma unroll
 			for (int k = 0; k < FT_CH; ++k) { cur[k] = nxt[k]; }
-			if (kb + 1 < p.kblocks) { fetch(kb + 1); }
+			if (kb + 1 < p.kblocks) { fetch(); }
 			if (kb >= FT_STAGES)
 			{
 				ok = mbar_wait(&bar_empty[s], (uint32_t)((kb / FT_STAGES - 1) & 1), s_failed, p.spin_limit);
@@ -262,6 +281,12 @@ float_conv_tc_kernel(const FtParams p)
 				{
 					float v = __fadd_rn(acc[j], s_bias[fl]);
 					v = fmaxf(v, __fmul_rn(v, slope));
+					if (p.yolo_entries > 0)
+					{
+						// logistic on every entry of an anchor but its width and height (head_activate.cu)
+						const int e = (f0 + fl) % p.yolo_entries;
+						if (e != 2 && e != 3) { v = 1.0f / (1.0f + expf(-v)); }
+					}
 					out_pix[(size_t)fl * p.HW] = v;
 				}
 			}
@@ -284,20 +309,25 @@ float_conv_tc_kernel(const FtParams p)
 
 using namespace xnor;
 
-extern "C" int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
-		const float * biases, float * output, void * stream)
+extern "C" int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
+		const float * biases, float * output, int yolo_entries, void * stream)
 {
 	if (desc == nullptr || input == nullptr || weights == nullptr || output == nullptr) { return XNOR_B200_ERR_NULL; }
 	int rc = validate_desc(desc);
 	if (rc != XNOR_B200_OK) { return rc; }
-	if (desc->size != 1 || desc->stride != 1 || desc->pad != 0) { return XNOR_B200_ERR_INVALID; }
+	const bool one = (desc->size == 1 && desc->pad == 0), three = (desc->size == 3 && desc->pad == 1 && desc->c % 32 == 0);
+	if (desc->stride != 1 || !(one || three)) { return XNOR_B200_ERR_INVALID; }
+	if (yolo_entries < 0 || (yolo_entries > 0 && (yolo_entries < 5 || desc->n % yolo_entries != 0))) { return XNOR_B200_ERR_INVALID; }
 	const long long total = (long long)desc->batch * desc->h * desc->w;
 	if (total > 0x7fffffffLL - TC_PIX) { return XNOR_B200_ERR_TOO_LARGE; }
 	FtParams p;
 	p.x = input; p.w = weights; p.bias = biases; p.out = output;
-	p.C = desc->c; p.HW = desc->h * desc->w; p.N = desc->n;
+	p.C = desc->c; p.H = desc->h; p.W = desc->w; p.HW = desc->h * desc->w; p.N = desc->n;
 	p.total = (int)total;
-	p.kblocks = (desc->c + 31) / 32;
+	p.taps = desc->size * desc->size;
+	p.cblocks = (desc->c + 31) / 32;
+	p.kblocks = p.taps * p.cblocks;
+	p.yolo_entries = yolo_entries;
 	p.leaky = (desc->activation == XNOR_B200_LEAKY) ? 1 : 0;
 	p.tiles_f = (desc->n + FT_NF - 1) / FT_NF;
 	p.w_vec = (desc->c % 4 == 0 && (((uintptr_t)weights) & 15u) == 0) ? 1 : 0;
@@ -312,4 +342,11 @@ extern "C" int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, con
 	if (rc != XNOR_B200_OK) { return rc; }
 	float_conv_tc_kernel<<<(unsigned)grid, FT_THREADS, FT_SMEM_BYTES, (cudaStream_t)stream>>>(p);
 	return check_launch();
+}
+
+extern "C" int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
+		const float * biases, float * output, void * stream)
+{
+	if (desc != nullptr && desc->size != 1) { return XNOR_B200_ERR_INVALID; }
+	return xnor_b200_float_conv_tc(desc, input, weights, biases, output, 0, stream);
 }

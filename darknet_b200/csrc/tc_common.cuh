@@ -85,6 +85,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t * bar, uint32_t parity, volat
 	return false;
 }
 
+// Wait that does not look at the CTA's failure flag (used while draining on the way out).
+__device__ __forceinline__ bool mbar_wait_plain(uint64_t * bar, uint32_t parity, uint32_t limit)
+{
+	const uint32_t addr = smem_u32(bar);
+	for (uint32_t spin = 0; spin < limit; ++spin)
+	{
+		uint32_t done;
+		asm volatile(
+			"{\n\t.reg .pred p;\n\t"
+			"mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+			"selp.u32 %0, 1, 0, p;\n\t}"
+			: "=r"(done) : "r"(addr), "r"(parity) : "memory");
+		if (done) { return true; }
+	}
+	return false;
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t * bar, uint32_t bytes)
+{
+	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+	uint32_t e;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+	return e != 0;
+}
+
 // 16 bits -> 16 bytes, each 0x00 (bit clear) or 0xFF (bit set), with one byte-permute per 4 bytes: PRMT picks
 // every output byte from an 8-byte pool by a 4-bit selector taken from the packed word itself.  The pool
 // alternates 0x00, 0xFF, so only the selector's lowest bit matters, and since 0x00 / 0xFF are their own sign

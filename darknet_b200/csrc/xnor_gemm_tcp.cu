@@ -56,28 +56,6 @@ constexpr int TP_SMEM_BYTES = TP_STAGES * TP_STAGE_BYTES + TP_RAW_STAGES * TP_RA
 constexpr int TP_TMEM_COLS = 512;
 constexpr int TP_SF_COL = 2 * TP_NF;          // scale factors of the pixel operand (4 columns used); the filter operand's at + 8
 
-// Wait that does not look at the CTA's failure flag (used while draining on the way out).
-__device__ __forceinline__ bool mbar_wait_plain(uint64_t * bar, uint32_t parity, uint32_t limit)
-{
-	const uint32_t addr = smem_u32(bar);
-	for (uint32_t spin = 0; spin < limit; ++spin)
-	{
-		uint32_t done;
-		asm volatile(
-			"{\n\t.reg .pred p;\n\t"
-			"mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-			"selp.u32 %0, 1, 0, p;\n\t}"
-			: "=r"(done) : "r"(addr), "r"(parity) : "memory");
-		if (done) { return true; }
-	}
-	return false;
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t * bar, uint32_t bytes)
-{
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
 // One 2-D box of a row-major byte matrix -> shared memory; x = byte offset inside the rows (a multiple of 16), y = first row.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap * map, int x, int y, uint64_t * bar)
 {

@@ -231,3 +231,59 @@ def tap_major_weights(l: ConvolutionalLayer) -> None:
 
 def conv_takes_masks(l: ConvolutionalLayer) -> bool:
     return bool(capi.lib().xnor_b200_conv_takes_masks(C.byref(l.desc)))
+
+
+def conv_words_weights_bytes(l: ConvolutionalLayer) -> int:
+    """Size of the filters' copy that xnor_b200_conv_words reads; 0 for a shape it does not take."""
+    return capi.lib().xnor_b200_conv_words_weights_bytes(C.byref(l.desc))
+
+
+def conv_words_weights(l: ConvolutionalLayer) -> Optional[torch.Tensor]:
+    """The layer's filters in the order of xnor_b200_conv_words, made from align_bit_weights_gpu; None for a shape it does not take."""
+    nbytes = conv_words_weights_bytes(l)
+    if nbytes == 0:
+        return None
+    out = torch.empty(nbytes // 4, dtype=torch.int32, device=l.device)
+    capi.check(capi.lib().xnor_b200_conv_words_weights(C.byref(l.desc), l.align_bit_weights_gpu.data_ptr(), out.data_ptr(), _stream()),
+               "xnor_b200_conv_words_weights")
+    return out
+
+
+class GridWords:
+    """A sign tensor on the position grid (include/xnor_b200.h): int32 [ceil(c/32)][block words], zero-filled."""
+
+    def __init__(self, batch: int, c: int, h: int, w: int, pitch: int = 0, device="cuda:0") -> None:
+        self.batch, self.c, self.h, self.w, self.pitch = batch, c, h, w, pitch or w + 1
+        self.blocks = (c + 31) // 32
+        self.words = torch.zeros(self.blocks, capi.lib().xnor_b200_grid_block_words(batch, h, self.pitch), dtype=torch.int32, device=device)
+
+    def source(self, pool_stride: int = 0, pool_pad: int = 0, upsample: int = 0) -> capi.WordsSource:
+        """This tensor as an input of conv_words, with what lies between it and the layer."""
+        return capi.WordsSource(self.words.data_ptr(), self.blocks, self.h, self.w, pool_stride, pool_pad, upsample, self.pitch)
+
+
+def sign_words(x: torch.Tensor, pitch: int = 0) -> GridWords:
+    """The signs of an fp32 tensor [batch][c][h][w]."""
+    b, c, h, w = x.shape
+    out = GridWords(b, c, h, w, pitch, x.device)
+    capi.check(capi.lib().xnor_b200_sign_words(x.data_ptr(), b, c, h, w, out.pitch, out.words.data_ptr(), _stream()), "xnor_b200_sign_words")
+    return out
+
+
+def conv_words(l: ConvolutionalLayer, weights: torch.Tensor, sources, output=None, signs: Optional[GridWords] = None, shortcut_in=None,
+               shortcut_out=None, pitch: int = 0) -> None:
+    """xnor_b200_conv_words: the layer from its inputs' sign words in one launch.  signs receives the signs of what is written
+    last: the output, or with a shortcut the sum."""
+    io = capi.WordsIO()
+    for i, s in enumerate(sources):
+        io.sources[i] = s
+    io.n_sources = len(sources)
+    io.output = _ptr(output)
+    io.shortcut_in, io.shortcut_out = _ptr(shortcut_in), _ptr(shortcut_out)
+    if signs is not None and shortcut_out is not None:
+        io.shortcut_signs = signs.words.data_ptr()
+    elif signs is not None:
+        io.output_signs = signs.words.data_ptr()
+    io.pitch = signs.pitch if signs is not None else pitch
+    capi.check(capi.lib().xnor_b200_conv_words(C.byref(l.desc), C.byref(io), weights.data_ptr(), l.mean_arr_gpu.data_ptr(),
+                                              l.biases_gpu.data_ptr(), _stream()), "xnor_b200_conv_words")

@@ -30,6 +30,7 @@ import torch.nn.functional as F
 
 from . import capi
 from . import layer as L
+from . import network_plan
 
 
 # ---- cfg -----------------------------------------------------------------------------------------
@@ -86,6 +87,7 @@ class Layer:
     pool_desc: Optional[capi.PoolDesc] = None
     # xnor conv whose only reader is another xnor conv (directly or through a maxpool): hands over sign bits
     weights_blocked_gpu: Optional[torch.Tensor] = None     # float conv on a small map: weights re-blocked at load time
+    weights_tap_major_gpu: Optional[torch.Tensor] = None   # float conv that runs as a GEMM on the tensor cores: weights [n][taps][c]
     branch_start: bool = False       # first / last layer of a head branch that runs on the side stream
     branch_end: bool = False
     yolo_entries: int = 0            # float conv in front of a [yolo] layer: the head's logistic step runs in the conv epilogue
@@ -136,6 +138,7 @@ class Network:
     packed_from_cache: int = 0             # xnor layers whose packed weights came from the cache file beside the .weights file
     sink_max_batch: int = 1 << 30          # batch up to which direct sign sinks are linked (measured: a gain at every batch for yolov3-tiny, within 2% either way for the other two networks at batch 32-256)
     sink_links: int = 0
+    plan: Optional[object] = None          # network_plan.Plan: the forward as one native call
 
 
 def parse_network_cfg(path: str, batch: int = 1, device: str = "cuda:0") -> Network:
@@ -404,6 +407,8 @@ def calculate_binary_weights(net: Network, packed: Optional[Dict[int, dict]] = N
     if net.fuse_first_conv:
         link_first_conv(net)
     fold_maxpools(net)
+    if net.sign_chains and net.fuse_first_conv:
+        net.plan = network_plan.build(net)
     torch.cuda.synchronize(dev)
 
 
@@ -676,16 +681,21 @@ def _map_conv_desc(net: Network, l: Layer) -> capi.ConvDesc:
 
 def prepare_float_map_convs(net: Network) -> None:
     """Re-blocks the weights of the float convolutions that the small-map kernel takes (many channels, stride 1,
-    3x3/pad 1 or 1x1, few output pixels in the whole batch).  Runs after fuse_conv_batchnorm."""
+    3x3/pad 1 or 1x1, few output pixels in the whole batch), and lays out those of the others for the tensor-core GEMM.
+    Runs after fuse_conv_batchnorm."""
     import ctypes as C
     for l in net.layers:
         if l.type != "convolutional" or l.xnor or l.activation not in ("leaky", "linear"):
             continue
-        if l.c * l.size * l.size <= 128 or net.batch * l.out_h * l.out_w > net.float_map_max_pixels:
+        if l.c * l.size * l.size <= 128:
             continue
         desc = _map_conv_desc(net, l)
         nbytes = capi.lib().xnor_b200_float_conv_map_weights_bytes(C.byref(desc))
-        if nbytes == 0:
+        if nbytes == 0 or net.batch * l.out_h * l.out_w > net.float_map_max_pixels:
+            # many pixels: one GEMM over the whole batch on the tensor cores, K = (tap, channel)
+            if l.stride == 1 and ((l.size == 1 and l.pad == 0) or (l.size == 3 and l.pad == 1 and l.c % 32 == 0)):
+                w = l.weights_gpu
+                l.weights_tap_major_gpu = w if l.size == 1 else w.reshape(l.n, l.c, 9).permute(0, 2, 1).contiguous()
             continue
         nxt = net.layers[l.index + 1] if l.index + 1 < len(net.layers) else None
         if (nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
@@ -697,13 +707,31 @@ def prepare_float_map_convs(net: Network) -> None:
                                                               torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_map_prepare")
 
 
-def _float_conv_1x1_tc(l: Layer, x: torch.Tensor) -> torch.Tensor:
-    """1x1 / stride-1 float convolution + bias + leaky/linear through xnor_b200_float_conv_1x1_tc."""
+def _float_conv_tc(l: Layer, x: torch.Tensor) -> torch.Tensor:
+    """1x1 or 3x3 stride-1 float convolution + bias + leaky/linear through xnor_b200_float_conv_tc."""
     import ctypes as C
-    desc = capi.ConvDesc(x.shape[0], l.c, l.h, l.w, l.n, 1, 1, 0, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
+    desc = capi.ConvDesc(x.shape[0], l.c, l.h, l.w, l.n, l.size, 1, l.pad, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
     out = torch.empty(x.shape[0], l.n, l.out_h, l.out_w, dtype=torch.float32, device=x.device)
-    capi.check(capi.lib().xnor_b200_float_conv_1x1_tc(C.byref(desc), x.data_ptr(), l.weights_gpu.data_ptr(), l.biases_gpu.data_ptr(),
-                                                     out.data_ptr(), torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_1x1_tc")
+    capi.check(capi.lib().xnor_b200_float_conv_tc(C.byref(desc), x.data_ptr(), l.weights_tap_major_gpu.data_ptr(), l.biases_gpu.data_ptr(),
+                                                 out.data_ptr(), 0, torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_tc")
+    return out
+
+
+def _avgpool(x: torch.Tensor) -> torch.Tensor:
+    b, c, h, w = x.shape
+    if not (x.is_cuda and x.is_contiguous()):
+        return x.mean((2, 3), keepdim=True)
+    out = torch.empty(b, c, 1, 1, dtype=torch.float32, device=x.device)
+    capi.check(capi.lib().xnor_b200_avgpool(x.data_ptr(), out.data_ptr(), b * c, h * w, torch.cuda.current_stream().cuda_stream), "xnor_b200_avgpool")
+    return out
+
+
+def _softmax(x: torch.Tensor) -> torch.Tensor:
+    if not (x.is_cuda and x.is_contiguous()):
+        return torch.softmax(x.reshape(x.shape[0], -1), 1).reshape(x.shape)
+    out = torch.empty_like(x)
+    capi.check(capi.lib().xnor_b200_softmax(x.data_ptr(), out.data_ptr(), x.shape[0], x[0].numel(), torch.cuda.current_stream().cuda_stream),
+               "xnor_b200_softmax")
     return out
 
 
@@ -773,7 +801,11 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
     """The layer loop of forward_network_gpu (src-lib/network_kernels.cu:30-65).  Returns the outputs of the
     network's head layers (yolo / region / softmax).  heads_host: pinned host tensors, one per head; each head is
     copied there as soon as it exists, on the stream that made it (Darknet's yolo layer pulls its output to the host
-    in every forward, src-lib/yolo_layer.cpp:1439-1489), so the copy of an early head overlaps the rest of the network."""
+    in every forward, src-lib/yolo_layer.cpp:1439-1489), so the copy of an early head overlaps the rest of the network.
+    A network that was lowered to native operations (network_plan) runs as one call; the loop below runs the others, and every
+    network while xnor_b200_set_tuning pins kernels of the packed-operand route."""
+    if net.plan is not None and net.plan.takes(x):
+        return net.plan.run(x, heads_host)
     heads: List[torch.Tensor] = []
     cur = x
     side_ctx = None
@@ -823,10 +855,10 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
                 # a head whose yolo activation runs in this kernel can be written straight into the caller's pinned host tensor
                 direct = heads_host is not None and l.yolo_entries > 0 and net.heads_direct_to_host
                 cur = _float_conv_map(net, l, cur.contiguous(), heads_host[len(heads)] if direct else None)
-            elif l.size == 1 and l.stride == 1 and l.pad == 0 and l.activation in ("leaky", "linear"):
-                # a 1x1 convolution over many pixels: one GEMM over the whole batch on the tensor cores (three tf32 products
-                # per operand pair), bias and activation in its epilogue
-                cur = _float_conv_1x1_tc(l, cur.contiguous())
+            elif l.weights_tap_major_gpu is not None:
+                # many pixels: one GEMM over the whole batch on the tensor cores (three tf32 products per operand pair), bias and
+                # activation in its epilogue
+                cur = _float_conv_tc(l, cur.contiguous())
             elif l.size == 1 and l.stride == 1 and l.pad == 0:
                 # other activations: a plain matrix product per image (cuBLAS sgemm, fp32)
                 b = cur.shape[0]
@@ -851,9 +883,9 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
         elif l.type == "upsample":
             cur = F.interpolate(cur, scale_factor=l.stride, mode="nearest")
         elif l.type == "avgpool":
-            cur = cur.mean((2, 3), keepdim=True)
+            cur = _avgpool(cur)
         elif l.type == "softmax":
-            cur = torch.softmax(cur.reshape(cur.shape[0], -1), 1).reshape(cur.shape)
+            cur = _softmax(cur)
             heads.append(cur)
             if heads_host is not None:
                 heads_host[len(heads) - 1].copy_(cur, non_blocking=True)
@@ -1026,6 +1058,8 @@ def load_network_custom(cfg: str, weights: str, batch: int = 1, device: str = "c
 
 def own_launches_per_forward(net: Network) -> int:
     """Kernels of libxnor_b200.so that one forward launches, after every fusion that load_network_custom set up."""
+    if net.plan is not None:
+        return sum(1 for op in net.plan.ops if op.kind not in (capi.OP_FORK, capi.OP_BACK))
     n = 0
     for l in net.layers:
         if l.type == "convolutional":
@@ -1036,9 +1070,9 @@ def own_launches_per_forward(net: Network) -> int:
                 n += 1 if (l.packed_input or from_planes) else 2
             elif (l.c == 3 and l.size == 3 and l.stride == 1 and l.pad == 1) or l.c * l.size * l.size <= 128 or l.weights_blocked_gpu is not None:
                 n += 1
-            elif l.size == 1 and l.stride == 1 and l.pad == 0 and l.activation in ("leaky", "linear"):
-                n += 1                                    # tensor-core 1x1 float convolution
-        elif (l.type == "yolo" and not l.yolo_done) or l.type == "region":
+            elif l.weights_tap_major_gpu is not None:
+                n += 1                                    # tensor-core float convolution
+        elif (l.type == "yolo" and not l.yolo_done) or l.type in ("region", "avgpool", "softmax"):
             n += 1
     return n
 

@@ -1,0 +1,290 @@
+"""A loaded network lowered to one array of native operations (xnor_b200_run_ops).
+
+Between xnor convolutions only signs travel: every tensor that an xnor convolution reads is kept as grid words (one 32-channel
+sign word per pixel), written by the layer that makes it and read through whatever [maxpool], [upsample] or [route] lies in
+between (xnor_b200_conv_words).  fp32 tensors exist where a float layer or a fused [shortcut] reads them.
+
+    plan = build(net)                 # once, at the end of calculate_binary_weights; None: a layer that has no native operation
+    heads = plan.run(x, heads_host)   # forward_network_gpu
+"""
+from __future__ import annotations
+
+import ctypes as C
+from typing import Dict, List, Optional, Tuple
+
+import torch
+
+from . import capi
+from . import layer as L
+
+
+class Unsupported(Exception):
+    """The network keeps to the layer-by-layer forward."""
+
+
+class Plan:
+    def __init__(self, net) -> None:
+        self.net = net
+        self.shape = (net.batch, net.c, net.h, net.w)
+        self.ops: List[capi.Op] = []
+        self.keep: List = []                       # tensors the operations point at
+        self.head_layers: List = []
+        self.head_direct: List[bool] = []          # a head whose last operation may store into page-locked host memory
+        self.signs: Dict[int, L.GridWords] = {}    # layer index -> its (or for a blank [shortcut] the sum's) signs
+        self.floats: Dict[int, torch.Tensor] = {}  # layer index -> fp32 tensor of a float layer
+        self.events: List[torch.cuda.Event] = []
+
+    def finish(self) -> None:
+        self.array = (capi.Op * len(self.ops))(*self.ops)
+        self.n_ops = len(self.ops)
+        self.heads_type = C.c_void_p * max(1, len(self.head_layers))
+        self.head_shapes = [(self.net.batch, l.out_c, l.out_h, l.out_w) for l in self.head_layers]
+        self.side = self.fork = self.join = None
+        if any(op.kind == capi.OP_FORK for op in self.ops):
+            if self.net.side_stream is None:
+                self.net.side_stream = torch.cuda.Stream(self.net.device)
+            self.events = [torch.cuda.Event(), torch.cuda.Event()]
+            for e in self.events:
+                e.record(self.net.side_stream)     # a torch event exists from its first record on
+            self.side = self.net.side_stream.cuda_stream
+            self.fork, self.join = (e.cuda_event for e in self.events)
+
+    def takes(self, x: torch.Tensor) -> bool:
+        return (x.is_cuda and x.dtype == torch.float32 and x.shape == self.shape and x.is_contiguous() and not capi.packed_route_pinned)
+
+    def run(self, x: torch.Tensor, heads_host: Optional[List[torch.Tensor]]) -> List[torch.Tensor]:
+        direct = heads_host is not None and self.net.heads_direct_to_host
+        heads = [heads_host[i] if direct and self.head_direct[i] else torch.empty(s, dtype=torch.float32, device=x.device)
+                 for i, s in enumerate(self.head_shapes)]
+        pointers = self.heads_type(*[h.data_ptr() for h in heads])
+        capi.check(capi.lib().xnor_b200_run_ops(self.array, self.n_ops, x.data_ptr(), pointers, len(heads),
+                                               torch._C._cuda_getCurrentRawStream(x.device.index), self.side, self.fork, self.join),
+                   "xnor_b200_run_ops")
+        for l, h in zip(self.head_layers, heads):
+            l.output_gpu = h
+        if heads_host is not None:
+            for h, host in zip(heads, heads_host):
+                if h is not host:
+                    host.copy_(h, non_blocking=True)
+        return heads
+
+
+# One input of an xnor convolution: (layer whose signs are read, pool stride, pool padding, upsample)
+Source = Tuple[int, int, int, int]
+
+
+def _sources(net, k: int, pool: Tuple[int, int] = (0, 0), up: int = 0) -> List[Source]:
+    """What the sign words of layer k's output are made of, walked backwards."""
+    l = net.layers[k]
+    if l.type == "convolutional" or (l.type == "shortcut" and l.blank):
+        if l.out_c % 32 != 0 and not (l.type == "convolutional" and not l.xnor):
+            raise Unsupported("filters that fill no whole sign words")
+        return [(k, pool[0], pool[1], up)]
+    if l.type == "maxpool" and pool == (0, 0) and up == 0 and l.size == 2 and l.stride in (1, 2) and l.pad in (0, 1) and k > 0:
+        return _sources(net, k - 1, (l.stride, l.pad), 0)
+    if l.type == "upsample" and pool == (0, 0) and up == 0 and l.stride == 2 and k > 0:
+        return _sources(net, k - 1, (0, 0), 2)
+    if l.type == "route":
+        return [s for i in l.input_layers for s in _sources(net, i, pool, up)]
+    raise Unsupported(f"[{l.type}] in front of an xnor layer")
+
+
+def _float_layer(net, k: int) -> int:
+    """The layer whose fp32 tensor is layer k's output (a [route] of one layer hands it on)."""
+    l = net.layers[k]
+    if l.type == "route" and len(l.input_layers) == 1:
+        return _float_layer(net, l.input_layers[0])
+    if l.type in ("convolutional", "avgpool") or (l.type == "shortcut" and l.blank):
+        return k
+    raise Unsupported(f"[{l.type}] in front of a float layer")
+
+
+def _first_conv(l) -> bool:
+    return (not l.xnor and l.index == 0 and l.c == 3 and l.size == 3 and l.stride == 1 and l.pad == 1 and l.n <= 32
+            and l.activation in ("leaky", "linear"))
+
+
+def build(net) -> Optional[Plan]:
+    try:
+        return _build(net)
+    except Unsupported:
+        return None
+
+
+def _build(net) -> Plan:
+    layers = net.layers
+    plan = Plan(net)
+    # ---- who reads what: signs per layer, fp32 per layer --------------------------------------------------------------
+    sources: Dict[int, List[Source]] = {}
+    float_in: Dict[int, int] = {}
+    pooled_first = False                           # the [maxpool] behind the first convolution is applied by its kernel
+    for k, l in enumerate(layers):
+        if l.type == "convolutional" and l.xnor:
+            if l.xnor_layer is None or L.conv_words_weights_bytes(l.xnor_layer) == 0 or k == 0:
+                raise Unsupported("xnor layer of another shape")
+            sources[k] = _sources(net, k - 1)
+            if len(sources[k]) > 2 or (len(sources[k]) == 2 and any(layers[s[0]].out_c % 32 != 0 for s in sources[k])):
+                raise Unsupported("more than two sources")
+            if l.stride == 2 and any(s[1] or s[3] for s in sources[k]):
+                raise Unsupported("a pool in front of a stride-2 layer")
+        elif l.type == "convolutional" and not _first_conv(l):
+            float_in[k] = _float_layer(net, k - 1)
+        elif l.type in ("avgpool", "yolo", "region", "softmax"):
+            float_in[k] = _float_layer(net, k - 1)
+        elif l.type == "shortcut":
+            if not l.blank:
+                raise Unsupported("[shortcut] that is not fused")
+            float_in[k] = _float_layer(net, l.input_layers[0])
+    sign_read = {s[0] for ss in sources.values() for s in ss}
+    fp32_read = set(float_in.values())
+    readers: Dict[int, List[int]] = {}
+    for k, l in enumerate(layers):
+        for i in (l.input_layers if l.type == "route" else [k - 1] + (l.input_layers if l.type == "shortcut" else [])):
+            readers.setdefault(i, []).append(k)
+    first = layers[0]
+    if not _first_conv(first) or 0 in fp32_read:
+        raise Unsupported("a first convolution of another shape")
+    firsts = [s for ss in sources.values() for s in ss if s[0] == 0]
+    pools = {s[1:3] for s in firsts}
+    if pools == {(2, 1)} and readers[0] == [1] and first.out_h % 2 == 0 and first.out_w % 2 == 0 and all(s[3] == 0 for s in firsts):
+        pooled_first = True
+    # ---- grids: rows of a multiple of 8 pixels keep whole memory sectors where a layer of that map writes fp32 -----------
+    wide = {(l.out_h, l.out_w) for k, l in enumerate(layers) if k in fp32_read and k in _xnor_outputs(net) and l.out_w % 8 == 0}
+
+    def pitch(h: int, w: int) -> int:
+        return w + 8 if (h, w) in wide else w + 1
+
+    def grid(k: int) -> L.GridWords:
+        if k not in plan.signs:
+            l = layers[k]
+            h, w = (l.out_h // 2, l.out_w // 2) if k == 0 and pooled_first else (l.out_h, l.out_w)
+            plan.signs[k] = L.GridWords(net.batch, l.out_c, h, w, pitch(h, w), net.device)
+        return plan.signs[k]
+
+    # ---- operations in layer order ---------------------------------------------------------------------------------------
+    for k, l in enumerate(layers):
+        if l.branch_start:
+            plan.ops.append(capi.Op(kind=capi.OP_FORK))
+        if l.type == "convolutional" and l.xnor:
+            _xnor_conv(plan, k, sources[k], grid, sign_read, fp32_read)
+        elif l.type == "convolutional" and _first_conv(l):
+            g = grid(k)
+            plan.ops.append(capi.Op(kind=capi.OP_CONV3, arg=2 if pooled_first else 0, pitch=g.pitch, desc=_desc(net, l), input=capi.OP_INPUT,
+                                    output=g.words.data_ptr(), weights=l.weights_gpu.data_ptr(), biases=l.biases_gpu.data_ptr()))
+        elif l.type == "convolutional":
+            _float_conv(plan, k, float_in[k], fp32_read)
+        elif l.type == "avgpool":
+            src = layers[float_in[k]]
+            plan.floats[k] = torch.empty(net.batch, l.out_c, 1, 1, device=net.device)
+            plan.ops.append(capi.Op(kind=capi.OP_AVGPOOL, desc=capi.ConvDesc(net.batch, src.out_c, src.out_h, src.out_w),
+                                    input=_tensor(plan, float_in[k]).data_ptr(), output=plan.floats[k].data_ptr()))
+        elif l.type in ("yolo", "region", "softmax"):
+            _head(plan, k, float_in[k])
+        if l.branch_end:
+            plan.ops.append(capi.Op(kind=capi.OP_BACK))
+    if not plan.head_layers:
+        raise Unsupported("no head")
+    for k, l in enumerate(layers):
+        l.output_gpu = plan.floats.get(k, l.output_gpu)
+    plan.finish()
+    return plan
+
+
+def _xnor_outputs(net) -> set:
+    return {k for k, l in enumerate(net.layers) if (l.type == "convolutional" and l.xnor) or (l.type == "shortcut" and l.blank)}
+
+
+def _desc(net, l) -> capi.ConvDesc:
+    return capi.ConvDesc(net.batch, l.c, l.h, l.w, l.n, l.size, l.stride, l.pad, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
+
+
+def _tensor(plan: Plan, k: int) -> torch.Tensor:
+    """The fp32 tensor of layer k."""
+    l = plan.net.layers[k]
+    if k in plan.floats:
+        return plan.floats[k]
+    if l.type == "shortcut":
+        return l.output_gpu
+    return l.xnor_layer.output_gpu
+
+
+def _xnor_conv(plan: Plan, k: int, sources: List[Source], grid, sign_read: set, fp32_read: set) -> None:
+    layers = plan.net.layers
+    l = layers[k]
+    xl = l.xnor_layer
+    weights = L.conv_words_weights(xl)
+    plan.keep.append(weights)
+    io = capi.WordsIO()
+    io.n_sources = len(sources)
+    for i, (s, pool_stride, pool_pad, up) in enumerate(sources):
+        g = grid(s)
+        if s == 0 and g.h != layers[0].out_h:
+            pool_stride = pool_pad = 0                             # pooled by the first convolution's kernel
+        io.sources[i] = g.source(pool_stride, pool_pad, up)
+    fused = k + 1 < len(layers) and layers[k + 1].blank
+    if k in fp32_read:
+        io.output = xl.output_gpu.data_ptr()
+    out = k
+    if fused:
+        out = k + 1
+        if k in sign_read:
+            raise Unsupported("signs of a layer and of its fused shortcut")
+        io.shortcut_in = _tensor(plan, _float_layer(plan.net, layers[out].input_layers[0])).data_ptr()
+        if out in fp32_read:
+            io.shortcut_out = layers[out].output_gpu.data_ptr()
+        if out in sign_read:
+            io.shortcut_signs = grid(out).words.data_ptr()
+    elif k in sign_read:
+        io.output_signs = grid(k).words.data_ptr()
+    g = plan.signs.get(out)
+    io.pitch = g.pitch if g is not None else 0
+    plan.ops.append(capi.Op(kind=capi.OP_CONV_WORDS, desc=xl.desc, io=io, weights=weights.data_ptr(), mean_arr=xl.mean_arr_gpu.data_ptr(),
+                            biases=xl.biases_gpu.data_ptr()))
+
+
+def _float_conv(plan: Plan, k: int, src: int, fp32_read: set) -> None:
+    """A float convolution behind the path; in front of a [yolo] layer with that layer's activation, into the head."""
+    net, l = plan.net, plan.net.layers[k]
+    nxt = net.layers[k + 1] if k + 1 < len(net.layers) else None
+    op = capi.Op(desc=_desc(net, l), input=_tensor(plan, src).data_ptr(), biases=l.biases_gpu.data_ptr())
+    head = nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
+    entries = 5 + int(nxt.opts.get("classes", 20)) if head else 0
+    head = head and l.n % entries == 0
+    if l.weights_blocked_gpu is not None:
+        op.kind, op.weights = capi.OP_FLOAT_MAP, l.weights_blocked_gpu.data_ptr()
+        if not l.yolo_entries:
+            head = False
+    elif l.weights_tap_major_gpu is not None:
+        op.kind, op.weights = capi.OP_FLOAT_TC, l.weights_tap_major_gpu.data_ptr()
+    else:
+        raise Unsupported("a float convolution of another shape")
+    if head:
+        op.arg = entries
+        op.output = capi.OP_HEAD + len(plan.head_layers)           # the [yolo] layer behind it adds itself
+    else:
+        plan.floats[k] = torch.empty(net.batch, l.n, l.out_h, l.out_w, device=net.device)
+        op.output = plan.floats[k].data_ptr()
+    plan.ops.append(op)
+
+
+def _head(plan: Plan, k: int, src: int) -> None:
+    net, l = plan.net, plan.net.layers[k]
+    slot = capi.OP_HEAD + len(plan.head_layers)
+    conv = plan.ops[-1]
+    plan.head_layers.append(l)
+    if l.type == "yolo" and conv.output == slot:
+        plan.head_direct.append(conv.kind == capi.OP_FLOAT_MAP)
+        return
+    plan.head_direct.append(False)
+    op = capi.Op(desc=capi.ConvDesc(net.batch, l.c, l.h, l.w), input=_tensor(plan, src).data_ptr(), output=slot)
+    if l.type == "softmax":
+        op.kind = capi.OP_SOFTMAX
+    elif l.type == "yolo" and float(l.opts.get("scale_x_y", 1)) == 1.0:
+        op.kind, op.arg = capi.OP_YOLO, int(l.opts.get("classes", 20))
+        op.desc.n = len(l.opts["mask"].split(","))
+    elif l.type == "region" and int(l.opts.get("coords", 4)) >= 2:
+        op.kind, op.arg, op.pitch = capi.OP_REGION, int(l.opts.get("classes", 20)), int(l.opts.get("coords", 4))
+        op.desc.n, op.desc.activation = int(l.opts.get("num", 1)), int(l.opts.get("softmax", 0))
+    else:
+        raise Unsupported("a head of another kind")
+    plan.ops.append(op)

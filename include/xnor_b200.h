@@ -285,6 +285,60 @@ XNOR_B200_API int xnor_b200_conv_forward_io(const xnor_b200_conv_desc * desc, co
 		const uint8_t * align_bit_weights, const float * mean_arr, const float * biases,
 		void * scratch, size_t scratch_bytes, void * stream);
 
+/* ---- the same layer from sign words, without a packed operand ------------------------------------------------------
+ * For layers of size 3 / pad 1 or size 1 / pad 0, stride 1 or 2: one launch reads the previous layers' sign words where they
+ * lie, through whatever stands in between, and writes sign words, fp32 or the fused shortcut sum.  Results are those of
+ * xnor_b200_conv_forward bit for bit.
+ *
+ * Grid words: the signs of a tensor [batch][c][h][w] as uint32 [ceil(c/32)][xnor_b200_grid_block_words(batch, h, pitch)], bit
+ * ch % 32 of a word = value > 0, the pixel (image, y, x) at word xnor_b200_grid_front(pitch) + (image * (h + 1) + y) * pitch + x of
+ * each block; every other word is 0.  pitch > w is the buffer's own; w + 1 is the shortest.  Zero-fill a buffer once (or let
+ * xnor_b200_sign_words write it whole); 16-byte aligned. */
+XNOR_B200_API size_t xnor_b200_grid_block_words(int batch, int h, int pitch);
+XNOR_B200_API int xnor_b200_grid_front(int pitch);
+
+/* One run of the input's channels: `blocks` blocks of 32 in grid words of the map h x w.  In between: a [maxpool] size 2
+ * (pool_stride 1 or 2, pool_pad = its padding, 0 or 1; pool_stride 0 = none) or an [upsample] stride 2 (upsample = 2), either in
+ * front of a stride-1 layer only.  pitch: of the buffer, 0 = w + 1. */
+typedef struct xnor_b200_words_source
+{
+	const uint32_t * words;
+	int blocks, h, w;
+	int pool_stride, pool_pad;
+	int upsample;
+	int pitch;
+} xnor_b200_words_source;
+
+/* sources: one, or two for a [route] concatenation (c % 32 == 0 then).  Outputs: `output` and / or output_signs (n % 32 == 0);
+ * or shortcut_out = shortcut_in + output and / or its sign words in shortcut_signs, with the layer's own `output` if wanted.
+ * fp32 tensors [batch][n][out_h * out_w], sign words on the output's grid (only the pixels are written).
+ * pitch: of the output's grid, 0 = out_w + 1.  The kernel walks that grid; a source of the same map and pitch is read fastest, and
+ * where fp32 tensors of rows of a multiple of 8 pixels are written, a multiple of 8 keeps them on whole memory sectors. */
+typedef struct xnor_b200_words_io
+{
+	xnor_b200_words_source sources[2];
+	int n_sources;
+	float * output;
+	uint32_t * output_signs;
+	const float * shortcut_in;
+	float * shortcut_out;
+	uint32_t * shortcut_signs;
+	int pitch;
+} xnor_b200_words_io;
+
+/* The filters in the order this kernel reads them, made once at load time from xnor_b200_binary_align_weights(invert = 0):
+ * bytes of the copy (0: a shape it does not take), and the copy itself. */
+XNOR_B200_API size_t xnor_b200_conv_words_weights_bytes(const xnor_b200_conv_desc * desc);
+XNOR_B200_API int xnor_b200_conv_words_weights(const xnor_b200_conv_desc * desc, const uint8_t * align_bit_weights, uint32_t * conv_weights,
+		void * stream);
+
+/* repack_input + float_to_bit of every image (src-lib/gemm.cpp:2202-2220, :1510), any channel count: fp32 [batch][c][h][w] -> grid
+ * words, padding included. */
+XNOR_B200_API int xnor_b200_sign_words(const float * input, int batch, int c, int h, int w, int pitch, uint32_t * words, void * stream);
+
+XNOR_B200_API int xnor_b200_conv_words(const xnor_b200_conv_desc * desc, const xnor_b200_words_io * io, const uint32_t * conv_weights,
+		const float * mean_arr, const float * biases, void * stream);
+
 /* The float convolution in front of the path (3 input channels -> 16/32 filters in the xnor networks): the float
  * branch of forward_convolutional_layer_gpu (src-lib/convolutional_kernels.cu:373-434, cuDNN or im2col + sgemm) +
  * add_bias_gpu + leaky activate_array_ongpu (src-lib/activation_kernels.cu:34) as one direct-convolution kernel
@@ -310,6 +364,11 @@ XNOR_B200_API int xnor_b200_float_conv_small(const xnor_b200_conv_desc * desc, c
 XNOR_B200_API int xnor_b200_float_conv3_io(const xnor_b200_conv_desc * desc, int pool, const float * input, const float * weights,
 		const float * biases, float * output, uint32_t * output_sign_planes, uint8_t * output_sign_masks, void * stream);
 
+/* The signs of the same layer (with pool = 2 of its pooled output) as grid words of that map (see xnor_b200_conv_words; pitch 0 =
+ * width + 1), the words source of the xnor layer behind it.  The buffer has been zero-filled once; only the pixels are written. */
+XNOR_B200_API int xnor_b200_float_conv3_words(const xnor_b200_conv_desc * desc, int pool, const float * input, const float * weights,
+		const float * biases, uint32_t * words, int pitch, void * stream);
+
 /* The float convolutions behind the path (many channels on a small map: the 3x3 256->512 layer on 13x13 and the
  * 1x1 layers in front of the yolo heads): the same float branch of forward_convolutional_layer_gpu
  * (src-lib/convolutional_kernels.cu:373-434) + add_bias_gpu + activate_array_ongpu, for stride 1 and either
@@ -330,6 +389,10 @@ XNOR_B200_API int xnor_b200_float_conv_map(const xnor_b200_conv_desc * desc, con
  * convolution to fp32 rounding (a few 1e-7 relative), not with cuBLAS bit for bit. */
 XNOR_B200_API int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
 		const float * biases, float * output, void * stream);
+/* The same kernel for 1x1 / pad 0 and 3x3 / pad 1 (c % 32 == 0) stride-1 layers, weights [n][size * size][c] (Darknet's [n][c][taps]
+ * with taps and channels exchanged; the same thing for 1x1); yolo_entries as below. */
+XNOR_B200_API int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
+		const float * biases, float * output, int yolo_entries, void * stream);
 /* Same, for the convolution right in front of a [yolo] layer: yolo_entries = 4 + 1 + classes (n must be a multiple of
  * it) also applies that layer's activation step (xnor_b200_yolo_activate below) to the result; 0 = plain call. */
 XNOR_B200_API int xnor_b200_float_conv_map_yolo(const xnor_b200_conv_desc * desc, const float * input, const float * blocked_weights,
@@ -401,6 +464,48 @@ XNOR_B200_API int xnor_b200_detect(const xnor_b200_yolo_head * heads, int n_head
  * asynchronous): host_count [batch], host_rows [batch][take][7]. */
 XNOR_B200_API int xnor_b200_rows_to_host(const float * rows, int max_rows, const int * row_count, int batch, int take, float * host_rows,
 		int * host_count, void * stream);
+
+/* avgpool_layer (src-lib/avgpool_layer.cpp:42-60): the mean of every plane.  input [planes][hw], output [planes]. */
+XNOR_B200_API int xnor_b200_avgpool(const float * input, float * output, int planes, int hw, void * stream);
+/* softmax over the n values of every image (src-lib/blas.cpp softmax_cpu, temperature 1, one group). */
+XNOR_B200_API int xnor_b200_softmax(const float * input, float * output, int batch, int n, void * stream);
+
+/* ---- a network's forward in one call -------------------------------------------------------------------------------
+ * The launches of the layer loop (forward_network_gpu, src-lib/network_kernels.cu:30-65) as an array that the caller fills once
+ * per network; xnor_b200_run_ops issues them in order. */
+#define XNOR_B200_OP_CONV3       1   /* xnor_b200_float_conv3_words(desc, arg = pool, input, weights, biases, output, pitch)          */
+#define XNOR_B200_OP_SIGN_WORDS  2   /* xnor_b200_sign_words(input, desc.batch, desc.c, desc.h, desc.w, pitch, output)                */
+#define XNOR_B200_OP_CONV_WORDS  3   /* xnor_b200_conv_words(desc, io, weights, mean_arr, biases)                                     */
+#define XNOR_B200_OP_FLOAT_MAP   4   /* xnor_b200_float_conv_map_yolo(desc, input, weights, biases, output, arg = yolo_entries)       */
+#define XNOR_B200_OP_FLOAT_TC    5   /* xnor_b200_float_conv_tc(desc, input, weights, biases, output, arg = yolo_entries)             */
+#define XNOR_B200_OP_YOLO        6   /* xnor_b200_yolo_activate(input, output, desc.batch, desc.n = anchors, arg = classes, desc.h*w) */
+#define XNOR_B200_OP_REGION      7   /* xnor_b200_region_activate(..., desc.n = anchors, pitch = coords, arg = classes, desc.activation = softmax) */
+#define XNOR_B200_OP_AVGPOOL     8   /* xnor_b200_avgpool(input, output, desc.batch * desc.c, desc.h * desc.w)                        */
+#define XNOR_B200_OP_SOFTMAX     9   /* xnor_b200_softmax(input, output, desc.batch, desc.c * desc.h * desc.w)                        */
+#define XNOR_B200_OP_FORK       10   /* the operations up to OP_BACK run on the side stream, beside those behind OP_BACK              */
+#define XNOR_B200_OP_BACK       11
+
+/* Values of input / output that stand for the run's own tensors. */
+#define XNOR_B200_OP_INPUT       1   /* the network's input                 */
+#define XNOR_B200_OP_HEAD        2   /* + i: head i                         */
+
+typedef struct xnor_b200_op
+{
+	int kind, arg, pitch;
+	xnor_b200_conv_desc desc;
+	xnor_b200_words_io io;
+	const void * input;
+	void * output;
+	const void * weights;
+	const float * mean_arr;
+	const float * biases;
+} xnor_b200_op;
+
+/* heads: n_heads tensors the operations write (device memory, or page-locked host memory for the head convolutions).  side_stream
+ * and the two events (cudaEvent_t) are needed when the operations fork, at most once; the caller's stream has joined the side
+ * stream when the call returns. */
+XNOR_B200_API int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const float * input, void * const * heads, int n_heads, void * stream,
+		void * side_stream, void * fork_event, void * join_event);
 
 /* Bytes of the library-resident scratch array behind xnor_b200_conv_forward_static. */
 #define XNOR_B200_STATIC_SCRATCH_BYTES (8u << 20)
