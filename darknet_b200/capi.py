@@ -69,14 +69,15 @@ class WordsIO(C.Structure):
 
 
 (OP_CONV3, OP_SIGN_WORDS, OP_CONV_WORDS, OP_FLOAT_MAP, OP_FLOAT_TC, OP_YOLO, OP_REGION, OP_AVGPOOL, OP_SOFTMAX, OP_FORK,
- OP_BACK) = range(1, 12)
+ OP_BACK, OP_CONV) = range(1, 13)
 OP_INPUT, OP_HEAD = 1, 2
 
 
 class Op(C.Structure):
     """struct xnor_b200_op"""
     _fields_ = [("kind", C.c_int), ("arg", C.c_int), ("pitch", C.c_int), ("desc", ConvDesc), ("io", WordsIO), ("input", C.c_void_p),
-                ("output", C.c_void_p), ("weights", C.c_void_p), ("mean_arr", C.c_void_p), ("biases", C.c_void_p)]
+                ("output", C.c_void_p), ("weights", C.c_void_p), ("mean_arr", C.c_void_p), ("biases", C.c_void_p),
+                ("scratch", C.c_void_p), ("scratch_bytes", C.c_size_t)]
 
 
 ROUTE_AUTO, ROUTE_INTEGER, ROUTE_TENSOR, ROUTE_TILED = 0, 1, 2, 3

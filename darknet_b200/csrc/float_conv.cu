@@ -252,6 +252,7 @@ float_conv3_block_kernel(const __grid_constant__ FloatBlockParams p)
 		{
 			const int fl = g * FB_FILTERS + f;
 			const float b = s_b[fl];
+			const float minus_b = __fsub_rn(0.0f, b);            // +0 for a bias of zero: below, +0 - +0 must not come out as -0
 			if (p.pooled)
 			{
 				// adding the bias keeps the order of values, so the largest sum is the largest value plus the bias
@@ -264,9 +265,9 @@ float_conv3_block_kernel(const __grid_constant__ FloatBlockParams p)
 				}
 				if (p.out == nullptr && p.planes == nullptr)
 				{
-					// value > 0 is the sign bit of -bias - top, whatever the signs of zeros
+					// value > 0 is the sign bit of (0 - bias) - top, whatever the signs of zeros
 					#pragma unroll
-					for (int i = 0; i < 4; ++i) { bits[i] = __funnelshift_l(__float_as_uint(__fsub_rn(-b, top[i])), bits[i], 1); }
+					for (int i = 0; i < 4; ++i) { bits[i] = __funnelshift_l(__float_as_uint(__fsub_rn(minus_b, top[i])), bits[i], 1); }
 					continue;
 				}
 				#pragma unroll
@@ -327,7 +328,7 @@ float_conv3_block_kernel(const __grid_constant__ FloatBlockParams p)
 				continue;
 			}
 			#pragma unroll
-			for (int i = 0; i < 16; ++i) { bits[i] = __funnelshift_l(__float_as_uint(__fsub_rn(-b, acc[f][i / 4][i % 4])), bits[i], 1); }
+			for (int i = 0; i < 16; ++i) { bits[i] = __funnelshift_l(__float_as_uint(__fsub_rn(minus_b, acc[f][i / 4][i % 4])), bits[i], 1); }
 		}
 	}
 	if (p.out != nullptr || p.planes != nullptr || !live) { return; }

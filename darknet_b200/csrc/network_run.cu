@@ -102,6 +102,10 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 			case XNOR_B200_OP_REGION: rc = xnor_b200_region_activate(in, out, d.batch, d.n, op.pitch, op.arg, d.activation, d.h * d.w, at); break;
 			case XNOR_B200_OP_AVGPOOL: rc = xnor_b200_avgpool(in, out, d.batch * d.c, d.h * d.w, at); break;
 			case XNOR_B200_OP_SOFTMAX: rc = xnor_b200_softmax(in, out, d.batch, d.c * d.h * d.w, at); break;
+			case XNOR_B200_OP_CONV:
+				rc = xnor_b200_conv_forward(&d, in, (const uint8_t *)op.weights, op.mean_arr, op.biases, out, op.io.shortcut_in, op.io.shortcut_out,
+						op.scratch, op.scratch_bytes, at);
+				break;
 			case XNOR_B200_OP_FORK:
 			{
 				// what follows runs on the side stream, behind everything issued so far

@@ -484,6 +484,7 @@ XNOR_B200_API int xnor_b200_softmax(const float * input, float * output, int bat
 #define XNOR_B200_OP_SOFTMAX     9   /* xnor_b200_softmax(input, output, desc.batch, desc.c * desc.h * desc.w)                        */
 #define XNOR_B200_OP_FORK       10   /* the operations up to OP_BACK run on the side stream, beside those behind OP_BACK              */
 #define XNOR_B200_OP_BACK       11
+#define XNOR_B200_OP_CONV       12   /* xnor_b200_conv_forward(desc, input, weights, mean_arr, biases, output, io.shortcut_in, io.shortcut_out, scratch) */
 
 /* Values of input / output that stand for the run's own tensors. */
 #define XNOR_B200_OP_INPUT       1   /* the network's input                 */
@@ -499,6 +500,8 @@ typedef struct xnor_b200_op
 	const void * weights;
 	const float * mean_arr;
 	const float * biases;
+	void * scratch;
+	size_t scratch_bytes;
 } xnor_b200_op;
 
 /* heads: n_heads tensors the operations write (device memory, or page-locked host memory for the head convolutions).  side_stream

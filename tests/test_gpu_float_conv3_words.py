@@ -1,0 +1,44 @@
+"""xnor_b200_float_conv3_words (signs of the first convolution on the position grid) and the sign masks against the fp32 output,
+with sums and biases that are exactly zero: zero is not positive, whatever its sign."""
+import ctypes as C
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import torch.nn.functional as F  # noqa: E402
+
+from darknet_b200 import capi, layer as L  # noqa: E402
+
+
+@pytest.mark.parametrize("pool", [0, 2])
+@pytest.mark.parametrize("batch,h,w,n,pitch", [(1, 32, 32, 32, 0), (2, 34, 30, 16, 0), (1, 2, 2, 8, 0), (3, 64, 96, 20, 56), (40, 96, 98, 32, 104)])
+def test_signs_of_zero_sums_and_zero_biases(batch, h, w, n, pitch, pool):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + h)
+    x = torch.randint(0, 3, (batch, 3, h, w), generator=g, device="cuda").float() / 4
+    wt = torch.randint(-1, 2, (n, 27), generator=g, device="cuda").float() / 4
+    b = torch.randint(-1, 2, (n,), generator=g, device="cuda").float() / 8
+    b[::3] = -0.0
+    desc = capi.ConvDesc(batch, 3, h, w, n, 3, 1, 1, capi.LEAKY)
+    oh, ow = (h // 2, w // 2) if pool else (h, w)
+    if not pool and pitch:
+        pitch = ow + 8
+    grid = L.GridWords(batch, n, oh, ow, pitch)
+    capi.check(capi.lib().xnor_b200_float_conv3_words(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), grid.words.data_ptr(),
+                                                     grid.pitch, None), "conv3_words")
+    masks = torch.zeros(batch, oh, ow, (n + 7) // 8, dtype=torch.uint8, device="cuda")
+    capi.check(capi.lib().xnor_b200_float_conv3_io(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), None, None,
+                                                  masks.data_ptr(), None), "conv3_io")
+    y = F.conv2d(x.double(), wt.double().view(n, 3, 3, 3), b.double(), 1, 1)
+    y = F.max_pool2d(y, 2, 2) if pool else y
+    assert int((y == 0).sum()) > 0 or y.numel() < 64
+    bits = F.pad(y > 0, (0, 0, 0, 0, 0, 32 - n)).to(torch.int64)
+    want = (bits << torch.arange(32, device="cuda").view(1, 32, 1, 1)).sum(1)
+    front = capi.lib().xnor_b200_grid_front(grid.pitch)
+    body = grid.words[0, front:front + batch * (oh + 1) * grid.pitch].view(batch, oh + 1, grid.pitch).to(torch.int64) & 0xFFFFFFFF
+    assert torch.equal(body[:, :oh, :ow], want)
+    assert int(body[:, oh].sum()) == 0 and int(body[:, :, ow:].sum()) == 0
+    got = sum(masks[..., i].to(torch.int64) << (8 * i) for i in range(masks.shape[-1]))
+    assert torch.equal(got, want)
