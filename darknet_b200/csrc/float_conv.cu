@@ -154,6 +154,7 @@ float_conv3_block_kernel(const __grid_constant__ FloatBlockParams p)
 	__shared__ __align__(16) float s_in[3][FB_ROWS][FB_PITCH];
 	__shared__ __align__(16) float s_w[27 * FB_MAX_FILTERS];       // [group of 4 filters][tap][filter]
 	__shared__ float s_b[FB_MAX_FILTERS];
+	pdl_trigger();
 	const int tid = threadIdx.x;
 	const int lane = tid & 31, warp = tid >> 5;
 	const int f0 = blockIdx.y * p.fpc;

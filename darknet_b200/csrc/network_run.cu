@@ -6,6 +6,8 @@
 namespace xnor
 {
 
+thread_local bool g_behind_kernel = false;
+
 // A pointer of an operation: an address, or (small values) the network's input or one of its heads.
 static const void * resolve(const void * at, const void * input, void * const * heads, int n_heads)
 {
@@ -84,6 +86,7 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 	if (ops == nullptr || input == nullptr || (n_heads > 0 && heads == nullptr)) { return XNOR_B200_ERR_NULL; }
 	void * at = stream;
 	bool forked = false;
+	struct Reset { ~Reset() { g_behind_kernel = false; } } reset;
 	for (int i = 0; i < n_ops; ++i)
 	{
 		const xnor_b200_op & op = ops[i];
@@ -91,6 +94,8 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 		float * out = (float *)resolve(op.output, input, heads, n_heads);
 		const xnor_b200_conv_desc & d = op.desc;
 		int rc = XNOR_B200_OK;
+		// behind a fork or a return the stream's last entry is no kernel of this call
+		g_behind_kernel = (i > 0 && ops[i - 1].kind != XNOR_B200_OP_FORK && ops[i - 1].kind != XNOR_B200_OP_BACK);
 		switch (op.kind)
 		{
 			case XNOR_B200_OP_CONV3: rc = xnor_b200_float_conv3_words(&d, op.arg, in, (const float *)op.weights, op.biases, (uint32_t *)out, op.pitch, at); break;

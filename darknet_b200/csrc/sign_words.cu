@@ -34,6 +34,7 @@ template <int VEC>
 __global__ void __launch_bounds__(SW_THREADS)
 sign_words_grid_kernel(const __grid_constant__ SignWordsParams p)
 {
+	pdl_trigger();
 	const int idx = blockIdx.x * SW_THREADS + threadIdx.x;
 	if (idx < p.items)
 	{

@@ -88,7 +88,34 @@ struct GemmExtra
 // True when launch_xnor_gemm would run such a layer on the short-K kernel, i.e. when `planes` may be used.
 bool gemm_takes_planes(int M, int n_total, int c, int size, int stride, int pad);
 
+// Set by xnor_b200_run_ops for an operation whose predecessor on the stream is another kernel of the same forward: the kernels that
+// know how (launch_behind) then start while that one finishes.
+extern thread_local bool g_behind_kernel;
+
 #ifdef __CUDACC__
+// The kernel's prologue may run before the previous kernel on the stream has finished; everything from here on runs behind it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel on the stream may be launched once every CTA of this one has come here.  Only behind pdl_wait (or in a kernel
+// that is never launched through launch_behind), so that what a prologue reads is finished: it lies two kernels back.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class Kernel, class Params>
+int launch_behind(Kernel kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Params & params)
+{
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(grid, 1, 1);
+	cfg.blockDim = dim3(threads, 1, 1);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = stream;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = g_behind_kernel ? 1 : 0;
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, params);
+	return (e == cudaSuccess) ? check_launch() : cuda_fail(e);
+}
+
 // Pixel (row-major index inside the image) of column `pixcol` of an image.
 __device__ __forceinline__ int col_to_pixel(const GemmExtra & x, int pixcol)
 {

@@ -92,6 +92,7 @@ struct XcParams
 	int kwords;              // nb * taps
 	uint32_t last_mask;      // channels that exist in the last block
 	FastDiv d_img, d_pitch;  // positions per image, positions per row
+	FastDiv d_kw;            // K words of a full stage (kw_full)
 	int pitch, rows;         // of the position grid
 	int total_pos, halo;     // positions of the batch; positions in front of a tile that its window needs
 	int planes, slots_plane; // parity planes, window positions of one
@@ -296,25 +297,30 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	// this filter group's words: [K word][128]
 	const uint32_t * my_filters = p.weights + (size_t)(f0 >> 7) * p.kwords * 128 + (f0 & 127);
 
-	if (tid == 0)
+	// What this prologue reads (filters, means, biases) was written long before the previous kernel; behind a kernel of the same
+	// forward it runs while that one finishes (griddepcontrol.wait below).
+	if (warp == XC_COPY_WARP)
 	{
-		for (int s = 0; s < XC_RAW_STAGES; ++s)
+		if (lane < XC_RAW_STAGES)
 		{
-			mbar_init(&raw_full[s], 2);                           // the copies (with their bytes), and the window table
-			mbar_init(&raw_empty[s], XC_EXP_WARPS);
+			mbar_init(&raw_full[lane], 2);                        // the copies (with their bytes), and the window table
+			mbar_init(&raw_empty[lane], XC_EXP_WARPS);
 		}
-		for (int s = 0; s < XC_MAX_STAGES; ++s)
+		if (lane < XC_MAX_STAGES)
 		{
-			mbar_init(&op_full[s], XC_EXP_WARPS);
-			mbar_init(&op_empty[s], 1);
+			mbar_init(&op_full[lane], XC_EXP_WARPS);
+			mbar_init(&op_empty[lane], 1);
 		}
-		for (int a = 0; a < ACC; ++a)
+		if (lane < ACC)
 		{
-			mbar_init(&acc_full[a], 1);
-			mbar_init(&acc_empty[a], 4 * CHUNKS);
+			mbar_init(&acc_full[lane], 1);
+			mbar_init(&acc_empty[lane], 4 * CHUNKS);
 		}
-		mbar_init(&drain_bar, 1);
-		s_failed_storage = 0;
+		if (lane == 31)
+		{
+			mbar_init(&drain_bar, 1);
+			s_failed_storage = 0;
+		}
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	if (warp == XC_MMA_WARP)
@@ -332,11 +338,43 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			s_koff[i] = (uint32_t)o0 | ((uint32_t)(o1 - o0) << 16);
 		}
 	}
+	float mean = 0.0f, bias = -0.0f;                               // v + -0.0 is v
+	if (tid < NF && f0 + tid < p.M)
+	{
+		mean = __ldg(p.mean_arr + f0 + tid);
+		if (p.bias != nullptr) { bias = __ldg(p.bias + f0 + tid); }
+	}
+	if (!STREAM)
+	{
+		// a warp takes 32 filters of every STEP-th K word, eight loads in flight per thread
+		constexpr int STEP = XC_THREADS / NF;
+		const int f = tid % NF;
+		const int total = p.stages_k * p.kw_full;
+		const int g_words = p.G * p.taps;
+		for (int k0 = tid / NF; k0 < total; k0 += 8 * STEP)
+		{
+			uint32_t bits[8];
+			int at[8];                                            // stage and word of the stage
+			#pragma unroll
+			for (int q = 0; q < 8; ++q)
+			{
+				bits[q] = 0;
+				const int kk = k0 + q * STEP;
+				const int st = fdiv(kk, p.d_kw);
+				at[q] = kk - st * p.kw_full | (st << 8);
+				const int k = st * g_words + (at[q] & 255);
+				if (kk < total && (at[q] & 255) < g_words && k < p.kwords) { bits[q] = __ldg(my_filters + (size_t)k * 128 + f); }
+			}
+			#pragma unroll
+			for (int q = 0; q < 8; ++q)
+			{
+				if (k0 + q * STEP < total) { put_filter<NF>(p, b_base + (uint32_t)((at[q] >> 8) * p.b_stage_bytes), at[q] >> 8, at[q] & 255, f, bits[q]); }
+			}
+		}
+		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+	}
 	if (tid < NF)
 	{
-		const int f = f0 + tid;
-		const float mean = (f < p.M) ? __ldg(p.mean_arr + f) : 0.0f;
-		const float bias = (f < p.M && p.bias != nullptr) ? __ldg(p.bias + f) : -0.0f;      // v + -0.0 is v
 		s_mean[tid] = mean;
 		s_bias[tid] = bias;
 		if (MODE == 0)
@@ -349,39 +387,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				const int mid = lo + ((hi - lo) >> 1);
 				if (positive(mid)) { hi = mid; } else { lo = mid; }
 			}
-			s_thr[tid] = (f < p.M) ? (float)hi : 3.0e38f;
+			s_thr[tid] = (f0 + tid < p.M) ? (float)hi : 3.0e38f;
 		}
-	}
-	if (!STREAM)
-	{
-		// eight loads in flight per thread; (stage, word of the stage) advance without divisions
-		constexpr int STEP = XC_THREADS / NF;
-		const int f = tid % NF;
-		const int total = p.stages_k * p.kw_full;
-		const int g_words = p.G * p.taps;
-		int st = 0, j = tid / NF;
-		while (j >= p.kw_full) { j -= p.kw_full; ++st; }
-		for (int k0 = tid / NF; k0 < total; k0 += 8 * STEP)
-		{
-			uint32_t bits[8];
-			int st2 = st, j2 = j;
-			#pragma unroll
-			for (int q = 0; q < 8; ++q)
-			{
-				const int k = st2 * g_words + j2;
-				bits[q] = (k0 + q * STEP < total && j2 < g_words && k < p.kwords) ? __ldg(my_filters + (size_t)k * 128 + f) : 0u;
-				j2 += STEP;
-				while (j2 >= p.kw_full) { j2 -= p.kw_full; ++st2; }
-			}
-			#pragma unroll
-			for (int q = 0; q < 8; ++q)
-			{
-				if (k0 + q * STEP < total) { put_filter<NF>(p, b_base + (uint32_t)(st * p.b_stage_bytes), st, j, f, bits[q]); }
-				j += STEP;
-				while (j >= p.kw_full) { j -= p.kw_full; ++st; }
-			}
-		}
-		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
@@ -395,9 +402,16 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			:: "r"(taddr), "r"(0x7F7F7F7Fu) : "memory");
 		asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 	}
-	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-	__syncthreads();
-	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+	if (warp < 4 || warp == XC_MMA_WARP)
+	{
+		// the scale factors are in place: only the issuer has to know
+		asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+		asm volatile("bar.sync 1, 160;" ::: "memory");
+		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+	}
+	// Everything the previous kernel wrote, and everything it read and this one overwrites, from here on.
+	pdl_wait();
+	if (tid == 0) { pdl_trigger(); }
 
 	if (warp < XC_EPI_WARPS)
 	{
@@ -737,6 +751,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	{
 		// ---- bulk copies ------------------------------------------------------------------------------------------------------
 		const bool leader = elect_one();
+		asm volatile("fence.proxy.async.global;" ::: "memory");            // the previous kernel's stores -> this one's bulk copies
 		int rs = 0;
 		uint32_t rs_phase = 1, k = 0;
 		bool ok = true;
@@ -1019,8 +1034,7 @@ static int launch_conv(XcParams & p, const XcPlan & q, cudaStream_t stream)
 {
 	int rc = ensure_dynamic_smem((const void *)xnor_conv_kernel<NF, MODE, STREAM>, q.smem);
 	if (rc != XNOR_B200_OK) { return rc; }
-	xnor_conv_kernel<NF, MODE, STREAM><<<q.grid, XC_THREADS, q.smem, stream>>>(p);
-	return check_launch();
+	return launch_behind(xnor_conv_kernel<NF, MODE, STREAM>, (unsigned)q.grid, XC_THREADS, q.smem, stream, p);
 }
 
 static XcPlan best_plan(const XcParams & p, int mode)
@@ -1052,6 +1066,7 @@ static int launch_mode(XcParams & p, cudaStream_t stream)
 	if (best.cost >= 1e30) { return XNOR_B200_ERR_TOO_LARGE; }
 	p.pt = best.pt;
 	p.G = best.g; p.stages_k = best.stages_k; p.ring = best.ring; p.kw_full = best.kw_full;
+	p.d_kw = make_div((uint32_t)best.kw_full);
 	p.a_stage_bytes = best.a_stage; p.b_stage_bytes = best.b_stage;
 	p.raw_words = best.raw_words; p.raw_stage_bytes = best.raw_stage;
 	p.slots_plane = best.slots_plane;

@@ -49,13 +49,39 @@ class ConvolutionalLayer:
         self.mean_arr_gpu = torch.zeros(n, dtype=torch.float32, device=self.device)
         self.align_bit_weights_gpu: Optional[torch.Tensor] = None
         self.tap_major_weights_gpu: Optional[torch.Tensor] = None    # xnor_b200_tap_major_weights copy, for channel-mask input
-        self.output_gpu = torch.empty(batch, n, g.out_h, g.out_w, dtype=torch.float32, device=self.device)
-        # zero-filled: when producers write this operand through sinks, padding taps and row tails are never written
-        self.scratch = torch.zeros(capi.lib().xnor_b200_scratch_bytes(C.byref(self.desc)), dtype=torch.uint8, device=self.device)
+        self._output: Optional[torch.Tensor] = None
+        self._scratch: Optional[torch.Tensor] = None
         self.window_major = False      # operand rows in 2x2-window-major pixel order (set when a sink of this layer pools)
         self.bin_conv_shortcut_in_gpu: Optional[torch.Tensor] = None
         self.bin_conv_shortcut_out_gpu: Optional[torch.Tensor] = None
         self.shortcut_signs_gpu: Optional[torch.Tensor] = None       # sign words of the fused shortcut sum, when a layer reads them
+        self.conv_words_gpu: Optional[torch.Tensor] = None           # the filters as xnor_b200_conv_words reads them, where that route is taken
+        self.input_words: Optional[GridWords] = None                 # ... and the input's sign words
+        self._ops = self._ops_of = None                              # forward_convolutional_layer_gpu: its launches, and the tensors they name
+        self._input_floats = batch * c * h * w
+
+    # The two large buffers are made when something first asks for them: a layer inside a network that hands signs on needs neither
+    # (at batch 256 the packed operands of tiny-yolo are 1.5 GB, their allocation and zero fill most of the load time).
+    @property
+    def output_gpu(self) -> torch.Tensor:
+        if self._output is None:
+            self._output = torch.empty(self.batch, self.n, self.out_h, self.out_w, dtype=torch.float32, device=self.device)
+        return self._output
+
+    @output_gpu.setter
+    def output_gpu(self, t: torch.Tensor) -> None:
+        self._output = t
+
+    @property
+    def scratch(self) -> torch.Tensor:
+        if self._scratch is None:
+            # zero-filled: when producers write this operand through sinks, padding taps and row tails are never written
+            self._scratch = torch.zeros(capi.lib().xnor_b200_scratch_bytes(C.byref(self.desc)), dtype=torch.uint8, device=self.device)
+        return self._scratch
+
+    @scratch.setter
+    def scratch(self, t: torch.Tensor) -> None:
+        self._scratch = t
 
     def load_weights(self, weights: torch.Tensor, biases: torch.Tensor) -> None:
         self.weights_gpu.copy_(weights.reshape(self.n, -1))
@@ -78,12 +104,31 @@ def binarize_weights(weights: torch.Tensor, n: int, size: int):
     return binary, mean
 
 
-def binary_align_weights(l: ConvolutionalLayer, invert: bool = False) -> None:
-    """binary_align_weights (src-lib/convolutional_layer.cpp:1339): fills align_bit_weights_gpu and mean_arr_gpu."""
+def binary_align_weights(l: ConvolutionalLayer, invert: bool = False, single_calls: bool = True) -> None:
+    """binary_align_weights (src-lib/convolutional_layer.cpp:1339): fills align_bit_weights_gpu and mean_arr_gpu.
+    single_calls: also what forward_convolutional_layer_gpu needs (a network that runs the layer its own way does without)."""
     l.align_bit_weights_gpu = torch.empty(l.geom.weights_bytes, dtype=torch.uint8, device=l.device)
     capi.check(capi.lib().xnor_b200_binary_align_weights(C.byref(l.desc), l.weights_gpu.data_ptr(),
                                                         l.align_bit_weights_gpu.data_ptr(), l.mean_arr_gpu.data_ptr(),
                                                         int(invert), _stream()), "xnor_b200_binary_align_weights")
+    l._ops = l._ops_of = None
+    if single_calls and not invert and takes_words(l):
+        l.conv_words_gpu = conv_words_weights(l)
+        if l.input_words is None and l.conv_words_gpu is not None:
+            l.input_words = GridWords(l.batch, l.c, l.h, l.w, device=l.device)
+    else:
+        l.conv_words_gpu = None
+
+
+def takes_words(l: ConvolutionalLayer) -> bool:
+    """Whether a single layer call runs as sign words + xnor_b200_conv_words or as packed operand + GEMM.  Measured on B200 over 44
+    shapes (7..208 pixels a side, 8..1024 channels and filters, batch 1..64): 3x3 layers 0.07 to 1.05 of the packed route's time,
+    1x1 layers whose channels fill no whole words 0.07 to 1.08.  1x1 layers over whole words gain from a few million fp32 values
+    or some hundred million binary operations on (0.6 to 1.06) and lose below (1.0 to 1.4: two kernels of 3 us each do all of it)."""
+    if l.size == 1 and l.c % 32 == 0:
+        floats = l.batch * (l.c * l.h * l.w // (l.stride * l.stride) + l.outputs)
+        return floats > 4_000_000 or 2 * l.batch * l.outputs * l.c > 250_000_000
+    return True
 
 
 def pack_input(l: ConvolutionalLayer, x: torch.Tensor) -> torch.Tensor:
@@ -128,6 +173,18 @@ def pack_input_pooled(l: ConvolutionalLayer, pool: capi.PoolDesc, x: torch.Tenso
 def forward_convolutional_layer_gpu(l: ConvolutionalLayer, x: torch.Tensor, pool: Optional[capi.PoolDesc] = None) -> torch.Tensor:
     """The xnor branch of forward_convolutional_layer_gpu (src-lib/convolutional_kernels.cu:204-262), whole batch.
     With `pool`, x is the input of a [maxpool] layer that sits directly in front of this convolution."""
+    if pool is None and x.is_cuda and not capi.packed_route_pinned:
+        named = l._ops_of
+        if (named is None or named[0] is not l.output_gpu or named[1] is not l.bin_conv_shortcut_in_gpu
+                or named[2] is not l.bin_conv_shortcut_out_gpu or named[3] is not l.align_bit_weights_gpu or named[4] is not l.biases_gpu):
+            _layer_ops(l)
+        if x.dtype != torch.float32 or x.numel() != l._input_floats or not x.is_contiguous():
+            raise ValueError("input must be a contiguous fp32 tensor of batch*c*h*w elements")
+        rc = capi.lib().xnor_b200_run_ops(l._ops, len(l._ops), x.data_ptr(), None, 0, torch._C._cuda_getCurrentRawStream(x.device.index),
+                                          None, None, None)
+        if rc:
+            capi.check(rc, "xnor_b200_run_ops")
+        return l.output_gpu
     if l.align_bit_weights_gpu is None:
         raise RuntimeError("binary_align_weights() has not been called for this layer")
     expect = l.batch * l.c * (l.h * l.w if pool is None else pool.in_h * pool.in_w)
@@ -144,6 +201,30 @@ def forward_convolutional_layer_gpu(l: ConvolutionalLayer, x: torch.Tensor, pool
                                                 _ptr(l.bin_conv_shortcut_in_gpu), _ptr(l.bin_conv_shortcut_out_gpu),
                                                 l.scratch.data_ptr(), l.scratch.numel(), _stream()), "xnor_b200_conv_forward")
     return l.output_gpu
+
+
+def _layer_ops(l: ConvolutionalLayer) -> None:
+    """The launches of forward_convolutional_layer_gpu, kept until the weights or a tensor they name are replaced."""
+    if l.align_bit_weights_gpu is None:
+        raise RuntimeError("binary_align_weights() has not been called for this layer")
+    shortcut_in, shortcut_out = l.bin_conv_shortcut_in_gpu, l.bin_conv_shortcut_out_gpu
+    op = capi.Op(desc=l.desc, mean_arr=l.mean_arr_gpu.data_ptr(), biases=l.biases_gpu.data_ptr())
+    op.io.shortcut_in, op.io.shortcut_out = _ptr(shortcut_in) if shortcut_out is not None else None, _ptr(shortcut_out)
+    if l.conv_words_gpu is not None and l._ops_of is not None and l._ops_of[3] is not l.align_bit_weights_gpu:
+        l.conv_words_gpu = None                                     # other packed weights than the ones it was made from
+    if l.conv_words_gpu is not None:
+        signs = capi.Op(kind=capi.OP_SIGN_WORDS, desc=l.desc, input=capi.OP_INPUT, output=l.input_words.words.data_ptr(), pitch=l.input_words.pitch)
+        op.kind, op.weights = capi.OP_CONV_WORDS, l.conv_words_gpu.data_ptr()
+        op.io.n_sources = 1
+        op.io.sources[0] = l.input_words.source()
+        op.io.output = l.output_gpu.data_ptr()
+        l._ops = (capi.Op * 2)(signs, op)
+    else:
+        op.kind, op.weights = capi.OP_CONV, l.align_bit_weights_gpu.data_ptr()
+        op.input, op.output = capi.OP_INPUT, l.output_gpu.data_ptr()
+        op.scratch, op.scratch_bytes = l.scratch.data_ptr(), l.scratch.numel()
+        l._ops = (capi.Op * 1)(op)
+    l._ops_of = (l.output_gpu, shortcut_in, shortcut_out, l.align_bit_weights_gpu, l.biases_gpu)
 
 
 class Sink:

@@ -377,9 +377,8 @@ def calculate_binary_weights(net: Network, packed: Optional[Dict[int, dict]] = N
             xl.mean_arr_gpu.copy_(torch.from_numpy(cached["mean"]))
             net.packed_from_cache += 1
         else:
-            L.binary_align_weights(xl)
+            L.binary_align_weights(xl, single_calls=False)
         l.xnor_layer = xl
-        l.output_gpu = xl.output_gpu
         net.xnor_launches_per_forward += 2
         if j + 1 < len(net.layers):
             sc = net.layers[j + 1]
