@@ -416,6 +416,12 @@ static int launch_conv3(const xnor_b200_conv_desc * desc, int pool, const float 
 		p.front = grid_front(p.pitch);
 		p.block_words = grid_block_words(desc->batch, p.OH, p.pitch);
 	}
+	if (p.words != nullptr)
+	{
+		// signs only: on the tensor cores, where the shape allows
+		rc = launch_float_conv3_signs(*desc, pool, input, weights, biases, p.words, p.pitch, (cudaStream_t)stream);
+		if (rc != XNOR_B200_ERR_TOO_LARGE) { return rc; }
+	}
 	const long long tiles = (long long)p.xtiles * ((desc->h + FB_TILE - 1) / FB_TILE);
 	// All of a pixel's filters in one CTA read the tile once and write whole words; with few tiles, eight filters each, so that
 	// the GPU fills (one image of 416x416, 16 filters: 169 tiles).

@@ -1,0 +1,557 @@
+// Signs of the first convolution (3 channels, 3x3, stride 1, pad 1, up to 32 filters) on the tcgen05 tensor cores, exactly.
+//
+// What the layer behind it wants is one bit per value: fl(sum) + bias > 0, the sum formed by fmaf over (channel, ky, kx) from zero.
+// 27 multiply-adds a value on the FMA pipe are 620 us for 16 filters at 416x416 and 256 images (1070 us with everything around
+// them).  Here the values are first formed approximately, as fp16 products with fp32 accumulation, together with a bound on how far
+// off they can be; wherever the value is farther from zero than that, the sign is known, and the rest -- about half a percent --
+// are formed again in fp32, in the order above.  Every bit is therefore the exact one.
+//
+//   |approximate - exact| <= (xmax + 1e-4) * (1.02e-3 * sum|w| + 1e-6)
+//
+// with the filter scaled by a power of two to max|w| in [0.5, 1) and xmax the largest input of the unit: 2^-10 for the two fp16
+// roundings of a product, 2^-25 each for subnormal operands, the rest for the accumulation here and there.  Inputs or filters that
+// fp16 cannot hold make the bound infinite, and every value is formed again.
+//
+// One MMA row is a 2x2 block of pixels, its columns the block's four values of every filter, K the 4x4 patch: with N = 4 * filters
+// and 8 (pair of pixels x 4) halves of 16 bytes that is 4 instructions per 512 pixels.  The operand is never gathered: an input
+// pixel pair (2q - 1, 2q) is 16 bytes [c0 c1 c2 0 | c0 c1 c2 0] in a plane [block row][pair], one plane for even and one for odd
+// pixel rows, and a patch row is another start address (as in xnor_conv.cu; position = (image * (BH + 1) + by) * (BW + 1) + bx).
+//
+// Roles (one CTA per SM): warps 0..15 epilogue, 16..22 converters (global fp32 -> planes), 23 issuer.
+// Bound by HBM (12 bytes a pixel) and by the converters' and the epilogue's issue slots.
+#include "grid_words.cuh"
+#include "tc_common.cuh"
+
+namespace xnor
+{
+
+constexpr int F3_EPI_WARPS = 16;
+constexpr int F3_CONV_WARPS = 7;
+constexpr int F3_MMA_WARP = F3_EPI_WARPS + F3_CONV_WARPS;
+constexpr int F3_THREADS = (F3_MMA_WARP + 1) * 32;
+constexpr int F3_BATCH = 2;                    // window slots a converter thread has in flight
+constexpr int F3_STAGES = 3;
+constexpr int F3_MAX_PT = 8;                  // tiles of 128 blocks per unit
+constexpr int F3_MAX_UNITS_AHEAD = 16;        // entries of the ring of unit maxima: stages + accumulators + 1 are under way
+constexpr int F3_QUEUE = 64;                  // values of a warp that wait to be formed exactly
+constexpr int F3_SMEM_MAX = 200 * 1024;
+
+struct F3Params
+{
+	const float * in;        // [batch][3][H][W]
+	const float * weights;   // [n][27]
+	const float * biases;    // [n] or nullptr
+	uint32_t * words;        // position 0 of the output grid
+	int H, W, N;
+	int BH, BW, pitch;       // 2x2 blocks; pitch = BW + 1
+	int OH, OW, out_pitch;
+	FastDiv d_img, d_pitch;  // positions per image, per row
+	int total_pos, pt, units;
+	int plane_slots;         // window positions of a unit: pt * 128 + pitch + 2
+	int stage_bytes;
+	int vec;                 // 1: rows of whole, aligned pairs
+	int * status;
+	uint32_t spin_limit;
+};
+
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi)
+{
+	uint32_t r;
+	asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+	return r;
+}
+
+// The larger value, NaN if either is
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+	float r;
+	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+
+__device__ __forceinline__ uint64_t f3_desc(uint32_t start, uint32_t lbo)
+{
+	return (uint64_t)(start | (lbo << 16)) | ((uint64_t)(8u | (1u << 14)) << 32);
+}
+
+// The exact value, formed as float_conv_small_kernel does.
+__device__ __forceinline__ float exact_value(const F3Params & p, int img, int oy, int ox, const float * w, float bias)
+{
+	const float * base = p.in + (size_t)img * 3 * p.H * p.W;
+	float acc = 0.0f;
+	#pragma unroll 1
+	for (int c = 0; c < 3; ++c)
+	{
+		float v[9];
+		#pragma unroll
+		for (int k = 0; k < 9; ++k)
+		{
+			const int iy = oy - 1 + k / 3, ix = ox - 1 + k % 3;
+			v[k] = (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) ? __ldg(base + ((size_t)c * p.H + iy) * p.W + ix) : 0.0f;
+		}
+		#pragma unroll
+		for (int k = 0; k < 9; ++k) { acc = fmaf(v[k], w[c * 9 + k], acc); }
+	}
+	return acc + bias;
+}
+
+// NF filters (16 or 32), POOL: the 2x2 max-pool behind the layer is applied.
+template <int NF, bool POOL>
+__global__ void __launch_bounds__(F3_THREADS, 1)
+float_conv3_signs_kernel(const __grid_constant__ F3Params p)
+{
+	constexpr int NN = 4 * NF;                                  // MMA columns: POOL: filter * 4 + pixel of the block, else pixel * NF + filter
+	constexpr int ACC = 512 / NN;
+	extern __shared__ __align__(128) uint8_t f3_smem[];         // [stage][odd rows | even rows][slot] of 16 bytes
+	__shared__ __align__(128) uint4 s_b[8 * NN];                // filter operand [16-byte half of K][column]
+	__shared__ float s_w[NF * 27];
+	__shared__ float s_bias[NF];                                // as given
+	__shared__ __align__(16) float s_sb[NF];                    // scaled like the filter
+	__shared__ __align__(16) float s_tol[NF];                   // bound = (xmax + 1e-4) * tol
+	__shared__ float s_xmax[F3_MAX_UNITS_AHEAD][F3_CONV_WARPS];
+	__shared__ uint2 s_queue[F3_EPI_WARPS][F3_QUEUE];
+	__shared__ uint64_t st_full[F3_STAGES], st_empty[F3_STAGES], acc_full[ACC], acc_empty[ACC], drain_bar;
+	__shared__ uint32_t tmem_base_slot;
+	__shared__ int s_failed_storage;
+	volatile int * s_failed = &s_failed_storage;
+
+	const int tid = threadIdx.x;
+	const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+	const int lane = tid & 31;
+	const uint32_t limit = p.spin_limit;
+	const uint32_t a_base = smem_u32(f3_smem);
+	const int my_units = (p.units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+	pdl_trigger();
+
+	if (tid == 0)
+	{
+		for (int s = 0; s < F3_STAGES; ++s)
+		{
+			mbar_init(&st_full[s], F3_CONV_WARPS);
+			mbar_init(&st_empty[s], 1);
+		}
+		for (int a = 0; a < ACC; ++a)
+		{
+			mbar_init(&acc_full[a], 1);
+			mbar_init(&acc_empty[a], 4);
+		}
+		mbar_init(&drain_bar, 1);
+		s_failed_storage = 0;
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == F3_MMA_WARP)
+	{
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+	}
+	for (int i = tid; i < NF * 27; i += F3_THREADS) { s_w[i] = (i < p.N * 27) ? __ldg(p.weights + i) : 0.0f; }
+	__syncthreads();
+	if (tid < NF)
+	{
+		float big = 0.0f, sum = 0.0f;
+		bool fits = true;
+		for (int k = 0; k < 27; ++k)
+		{
+			const float w = fabsf(s_w[tid * 27 + k]);
+			fits = fits && (w < 1e30f);
+			big = fmaxf(big, w);
+		}
+		int e = 0;
+		if (big > 0.0f) { frexpf(big, &e); }
+		fits = fits && e > -100;
+		const float scale = fits ? ldexpf(1.0f, -e) : 0.0f;
+		for (int k = 0; k < 27; ++k) { sum += fabsf(s_w[tid * 27 + k] * scale); }
+		const float bias = (p.biases != nullptr && tid < p.N) ? __ldg(p.biases + tid) : 0.0f;
+		s_bias[tid] = bias;
+		s_sb[tid] = bias * scale;
+		s_tol[tid] = fits ? 1.02e-3f * sum + 1e-6f : INFINITY;
+		for (int h = 0; h < 8; ++h)
+		{
+			// half h: patch row h / 2 counted odd, even, odd, even; pair h % 2
+			const int row = h >> 1;
+			for (int s = 0; s < 4; ++s)
+			{
+				float v[8];
+				for (int q = 0; q < 8; ++q)
+				{
+					const int ky = row - (s >> 1), kx = (h & 1) * 2 + (q >> 2) - (s & 1), c = q & 3;
+					v[q] = (c < 3 && ky >= 0 && ky < 3 && kx >= 0 && kx < 3) ? s_w[tid * 27 + (c * 3 + ky) * 3 + kx] * scale : 0.0f;
+				}
+				s_b[h * NN + (POOL ? tid * 4 + s : s * NF + tid)] = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
+			}
+		}
+	}
+	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+	__syncthreads();
+	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
+
+	if (warp < F3_EPI_WARPS)
+	{
+		// ---- epilogue: warp w takes the tiles w / 4, w / 4 + 4, ... of this CTA, lane quarter w % 4 -----------------------------
+		const int quarter = warp & 3;
+		const int my_tiles = my_units * p.pt;
+		int tile = warp >> 2;
+		int nu = 0, t = tile;                                    // unit of this CTA, tile of the unit
+		while (t >= p.pt) { t -= p.pt; ++nu; }
+		int a = tile % ACC;
+		uint32_t phase = (uint32_t)((tile / ACC) & 1);
+		int have_unit = -1;
+		float xmax = 0.0f;
+		int q_head = 0, q_count = 0;                             // this warp's ring of values to be formed exactly
+		// output word of a position and pixel of its block
+		auto word_at = [&](int img, int y, int x) { return p.words + ((size_t)img * (p.OH + 1) + y) * p.out_pitch + x; };
+		auto resolve = [&](int n)
+		{
+			// the n oldest values; POOL: four lanes form one, a pixel of the block each
+			constexpr int LANES = POOL ? 4 : 1;
+			__syncwarp();
+			if (lane < n * LANES)
+			{
+				const uint2 item = s_queue[warp][(q_head + lane / LANES) % F3_QUEUE];
+				const int f = (int)(item.y & 255u), s = POOL ? (lane & 3) : (int)(item.y >> 8);
+				const int pos = (int)item.x;
+				const int img = fdiv(pos, p.d_img);
+				const int r = pos - img * (int)p.d_img.d;
+				const int by = fdiv(r, p.d_pitch), bx = r - by * p.pitch;
+				const int oy = 2 * by + (s >> 1), ox = 2 * bx + (s & 1);
+				if (exact_value(p, img, oy, ox, s_w + f * 27, s_bias[f]) > 0.0f)
+				{
+					atomicOr(POOL ? word_at(img, by, bx) : word_at(img, oy, ox), 1u << f);
+				}
+			}
+			q_head = (q_head + n) % F3_QUEUE;
+			q_count -= n;
+		};
+		auto enqueue = [&](uint32_t unsure, int pos, int s)
+		{
+			// one value per lane and round; the words they belong to have been stored
+			constexpr int BATCH = POOL ? 8 : 32;
+			__syncwarp();
+			while (true)
+			{
+				const unsigned who = __ballot_sync(0xffffffffu, unsure != 0);
+				if (who == 0) { break; }
+				if (unsure != 0)
+				{
+					const int f = __ffs(unsure) - 1;
+					unsure &= unsure - 1;
+					s_queue[warp][(q_head + q_count + __popc(who & ((1u << lane) - 1u))) % F3_QUEUE] = make_uint2((uint32_t)pos, (uint32_t)(f | (s << 8)));
+				}
+				q_count += __popc(who);
+				while (q_count >= BATCH) { resolve(BATCH); }
+			}
+		};
+		while (tile < my_tiles)
+		{
+			if (!__all_sync(0xffffffffu, mbar_wait<32>(&acc_full[a], phase, s_failed, limit))) { break; }
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			if (nu != have_unit)
+			{
+				have_unit = nu;
+				xmax = (lane < F3_CONV_WARPS) ? s_xmax[nu % F3_MAX_UNITS_AHEAD][lane] : 0.0f;
+				#pragma unroll
+				for (int o = 4; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
+				xmax = __shfl_sync(0xffffffffu, xmax, 0) + 1e-4f;
+			}
+			const int pos = (((int)blockIdx.x + nu * (int)gridDim.x) * p.pt + t) * TC_PIX + quarter * 32 + lane;
+			const int img = fdiv(pos, p.d_img);
+			const int r = pos - img * (int)p.d_img.d;
+			const int by = fdiv(r, p.d_pitch), bx = r - by * p.pitch;
+			const bool ok = (pos < p.total_pos && by < p.BH && bx < p.BW);
+			const uint32_t tacc = tmem_base + (uint32_t)(a * NN) + ((uint32_t)(quarter * 32) << 16);
+			if (POOL)
+			{
+				uint32_t word = 0, unsure = 0;
+				#pragma unroll
+				for (int h = 0; h < NN / 32; ++h)
+				{
+					uint32_t d[32];
+					tmem_load<32>(tacc + (uint32_t)(h * 32), d);
+					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					if (h == NN / 32 - 1)
+					{
+						asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+						__syncwarp();
+						if (lane == 0) { mbar_arrive(&acc_empty[a]); }
+					}
+					const float4 b0 = *reinterpret_cast<const float4 *>(s_sb + h * 8), b1 = *reinterpret_cast<const float4 *>(s_sb + h * 8 + 4);
+					const float4 t0 = *reinterpret_cast<const float4 *>(s_tol + h * 8), t1 = *reinterpret_cast<const float4 *>(s_tol + h * 8 + 4);
+					const float sb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+					const float tol[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+					#pragma unroll
+					for (int i = 0; i < 8; ++i)
+					{
+						const int f = h * 8 + i;
+						const float top = fmaxf(fmaxf(__uint_as_float(d[4 * i]), __uint_as_float(d[4 * i + 1])), fmaxf(__uint_as_float(d[4 * i + 2]), __uint_as_float(d[4 * i + 3])));
+						const float v = top + sb[i];
+						const float bound = xmax * tol[i];
+						word |= (v > bound) ? (1u << f) : 0u;
+						unsure |= !(fabsf(v) > bound) ? (1u << f) : 0u;
+					}
+				}
+				// filters past the last have weights and bias zero: exact value 0, no sign
+				if (ok) { *word_at(img, by, bx) = word; }
+				if (!ok) { unsure = 0; }
+				if (p.N < 32) { unsure &= (1u << p.N) - 1u; }
+				if (__any_sync(0xffffffffu, unsure != 0)) { enqueue(unsure, pos, 0); }
+			}
+			else
+			{
+				#pragma unroll 1
+				for (int s = 0; s < 4; ++s)
+				{
+					uint32_t d[NF];
+					tmem_load<NF>(tacc + (uint32_t)(s * NF), d);
+					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					if (s == 3)
+					{
+						asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+						__syncwarp();
+						if (lane == 0) { mbar_arrive(&acc_empty[a]); }
+					}
+					uint32_t word = 0, unsure = 0;
+					#pragma unroll
+					for (int f0 = 0; f0 < NF; f0 += 4)
+					{
+						const float4 b4 = *reinterpret_cast<const float4 *>(s_sb + f0), t4 = *reinterpret_cast<const float4 *>(s_tol + f0);
+						const float sb[4] = {b4.x, b4.y, b4.z, b4.w}, tol[4] = {t4.x, t4.y, t4.z, t4.w};
+						#pragma unroll
+						for (int i = 0; i < 4; ++i)
+						{
+							const float v = __uint_as_float(d[f0 + i]) + sb[i];
+							const float bound = xmax * tol[i];
+							word |= (v > bound) ? (1u << (f0 + i)) : 0u;
+							unsure |= !(fabsf(v) > bound) ? (1u << (f0 + i)) : 0u;
+						}
+					}
+					const int oy = 2 * by + (s >> 1), ox = 2 * bx + (s & 1);
+					const bool in = ok && oy < p.OH && ox < p.OW;
+					if (in) { *word_at(img, oy, ox) = word; }
+					if (!in) { unsure = 0; }
+					if (p.N < 32) { unsure &= (1u << p.N) - 1u; }
+					if (__any_sync(0xffffffffu, unsure != 0)) { enqueue(unsure, pos, s); }
+				}
+			}
+			tile += F3_EPI_WARPS / 4;
+			a += F3_EPI_WARPS / 4;
+			while (a >= ACC) { a -= ACC; phase ^= 1u; }
+			t += F3_EPI_WARPS / 4;
+			while (t >= p.pt) { t -= p.pt; ++nu; }
+		}
+		while (q_count > 0) { resolve(min(q_count, POOL ? 8 : 32)); }
+	}
+	else if (warp < F3_MMA_WARP)
+	{
+		// ---- converters: a slot is the pair of pixels (2q - 1, 2q) of an odd and of an even row -----------------------------
+		const int cw = warp - F3_EPI_WARPS;
+		const size_t plane = (size_t)p.H * p.W;
+		const int groups = (p.plane_slots + 31) >> 5;
+		int es = 0;
+		uint32_t es_phase = 1;
+		bool ok = true;
+		for (int nu = 0; nu < my_units && ok; ++nu)
+		{
+			const int pos0 = ((int)blockIdx.x + nu * (int)gridDim.x) * p.pt * TC_PIX;
+			const uint32_t odd = a_base + (uint32_t)(es * p.stage_bytes);
+			const uint32_t even = odd + (uint32_t)(p.plane_slots * 16);
+			float xmax = 0.0f;
+			if (nu >= F3_STAGES)
+			{
+				ok = __all_sync(0xffffffffu, mbar_wait<32>(&st_empty[es], es_phase, s_failed, limit));
+				if (!ok) { break; }
+			}
+			// F3_BATCH slots at a time: all of their loads first, for the kernel lives on bytes in flight (a load followed by the
+			// shuffle that uses it, slot by slot, took 350 us where this takes ~F3_NOW~: 64 images of 416x416)
+			for (int g0 = cw; g0 < groups; g0 += F3_CONV_WARPS * F3_BATCH)
+			{
+				float2 v[F3_BATCH][6];                            // [slot][odd, even row x channel]: pixels 2q and 2q + 1
+				float e[F3_BATCH][6];                             // pixel 2q - 1 where no neighbouring lane has it
+				bool mid[F3_BATCH];
+				#pragma unroll
+				for (int i = 0; i < F3_BATCH; ++i)
+				{
+					const int s = (g0 + i * F3_CONV_WARPS) * 32 + lane;
+					const int pos = pos0 + s;
+					const int img = fdiv(pos, p.d_img);
+					const int r = pos - img * (int)p.d_img.d;
+					const int by = fdiv(r, p.d_pitch), q = r - by * p.pitch;
+					const bool in = (s < p.plane_slots && pos < p.total_pos);
+					const int ye = 2 * by, x = 2 * q;
+					const float * at = p.in + (size_t)img * 3 * plane + (ptrdiff_t)(ye - 1) * p.W + x;
+					mid[i] = (q > 0);
+					#pragma unroll
+					for (int k = 0; k < 2; ++k)
+					{
+						const int y = ye - 1 + k;
+						const bool row_ok = in && y >= 0 && y < p.H;
+						const bool own = row_ok && x < p.W, edge = row_ok && q > 0 && x - 1 < p.W && (lane == 0 || !p.vec);
+						#pragma unroll
+						for (int c = 0; c < 3; ++c)
+						{
+							const float * src = at + (ptrdiff_t)k * p.W + (size_t)c * plane;
+							v[i][k * 3 + c] = make_float2(0.0f, 0.0f);
+							e[i][k * 3 + c] = 0.0f;
+							if (p.vec) { if (own) { v[i][k * 3 + c] = __ldg(reinterpret_cast<const float2 *>(src)); } }
+							else if (own) { v[i][k * 3 + c].x = __ldg(src); }
+							if (edge) { e[i][k * 3 + c] = __ldg(src - 1); }
+						}
+					}
+				}
+				#pragma unroll
+				for (int i = 0; i < F3_BATCH; ++i)
+				{
+					const int s = (g0 + i * F3_CONV_WARPS) * 32 + lane;
+					#pragma unroll
+					for (int k = 0; k < 2; ++k)
+					{
+						float l[3], h[3];
+						#pragma unroll
+						for (int c = 0; c < 3; ++c)
+						{
+							// rows outside the image and slots behind the end were left at zero, in the neighbour as here
+							const float left = __shfl_up_sync(0xffffffffu, v[i][k * 3 + c].y, 1);
+							l[c] = (lane == 0 || !p.vec) ? e[i][k * 3 + c] : (mid[i] ? left : 0.0f);
+							h[c] = v[i][k * 3 + c].x;
+							xmax = max_nan(xmax, max_nan(fabsf(h[c]), fabsf(l[c])));
+						}
+						if (s < p.plane_slots)
+						{
+							asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"((k == 0 ? odd : even) + (uint32_t)s * 16u),
+									"r"(pack_half2(l[0], l[1])), "r"(pack_half2(l[2], 0.0f)), "r"(pack_half2(h[0], h[1])), "r"(pack_half2(h[2], 0.0f)));
+						}
+					}
+				}
+			}
+			if (!(xmax < 60000.0f)) { xmax = INFINITY; }                    // beyond fp16, or not a number
+			#pragma unroll
+			for (int o = 16; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
+			if (lane == 0) { s_xmax[nu % F3_MAX_UNITS_AHEAD][cw] = xmax; }
+			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+			__syncwarp();
+			if (lane == 0) { mbar_arrive(&st_full[es]); }
+			if (++es == F3_STAGES) { es = 0; es_phase ^= 1u; }
+		}
+	}
+	else
+	{
+		// ---- issuer -----------------------------------------------------------------------------------------------------
+		const bool leader = elect_one();
+		// D = f32, A = B = f16, both K-major
+		const uint32_t idesc = (1u << 4) | ((uint32_t)(NN >> 3) << 17) | ((uint32_t)(TC_PIX >> 4) << 24);
+		const uint32_t b16 = smem_u32(s_b) >> 4;
+		int es = 0, a = 0, used = 0;
+		uint32_t es_phase = 0, a_phase = 1;
+		bool ok = true;
+		for (int nu = 0; nu < my_units && ok; ++nu)
+		{
+			ok = __all_sync(0xffffffffu, mbar_wait<0>(&st_full[es], es_phase, s_failed, limit));
+			if (!ok) { break; }
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			uint32_t odd = (a_base + (uint32_t)(es * p.stage_bytes)) >> 4;
+			for (int t = 0; t < p.pt; ++t, odd += TC_PIX)
+			{
+				if (used >= ACC)
+				{
+					ok = __all_sync(0xffffffffu, mbar_wait<32>(&acc_empty[a], a_phase, s_failed, limit));
+					if (!ok) { break; }
+					asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+				}
+				else { ++used; }
+				const uint32_t even = odd + (uint32_t)p.plane_slots;
+				#pragma unroll
+				for (int k = 0; k < 4; ++k)                       // patch rows 2by - 1, 2by, 2by + 1, 2by + 2
+				{
+					const uint32_t start = ((k & 1) ? even : odd) + ((k >> 1) ? (uint32_t)p.pitch : 0u);
+					if (leader)
+					{
+						asm volatile(
+							"{\n\t.reg .pred p;\n\t"
+							"setp.ne.b32 p, %4, 0;\n\t"
+							"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+							:: "r"(tmem_base + (uint32_t)(a * NN)), "l"(f3_desc(start, 1u)), "l"(f3_desc(b16 + (uint32_t)(2 * k * NN), (uint32_t)NN)), "r"(idesc),
+							   "r"(k != 0 ? 1u : 0u), "r"(0u) : "memory");
+					}
+				}
+				if (leader)
+				{
+					asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&acc_full[a])) : "memory");
+				}
+				if (++a == ACC) { a = 0; a_phase ^= 1u; }
+			}
+			if (!ok) { break; }
+			if (leader)
+			{
+				asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&st_empty[es])) : "memory");
+			}
+			if (++es == F3_STAGES) { es = 0; es_phase ^= 1u; }
+		}
+		if (!ok)
+		{
+			if (leader)
+			{
+				asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&drain_bar)) : "memory");
+			}
+			mbar_wait_plain(&drain_bar, 0, limit);
+		}
+		__syncwarp();
+	}
+
+	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+	__syncthreads();
+	if (*s_failed != 0 && tid == 0) { atomicExch(p.status, 1); }
+	if (warp == F3_MMA_WARP)
+	{
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512u) : "memory");
+	}
+}
+
+template <int NF, bool POOL>
+static int launch_f3(const F3Params & p, size_t smem, cudaStream_t stream)
+{
+	const int rc = ensure_dynamic_smem((const void *)float_conv3_signs_kernel<NF, POOL>, smem);
+	if (rc != XNOR_B200_OK) { return rc; }
+	const int grid = (p.units < sm_count()) ? p.units : sm_count();
+	float_conv3_signs_kernel<NF, POOL><<<grid, F3_THREADS, smem, stream>>>(p);
+	return check_launch();
+}
+
+// Up to 32 filters and maps whose rows fit the stages; returns ERR_TOO_LARGE for what has to go to the kernel of float_conv.cu.
+int launch_float_conv3_signs(const xnor_b200_conv_desc & d, int pool, const float * input, const float * weights, const float * biases,
+		uint32_t * words, int pitch, cudaStream_t stream)
+{
+	F3Params p = {};
+	p.in = input; p.weights = weights; p.biases = biases;
+	p.H = d.h; p.W = d.w; p.N = d.n;
+	p.BH = (d.h + 1) / 2; p.BW = (d.w + 1) / 2; p.pitch = p.BW + 1;
+	p.OH = pool ? d.h / 2 : d.h; p.OW = pool ? d.w / 2 : d.w; p.out_pitch = pitch;
+	p.words = words + grid_front(pitch);
+	const long long total = (long long)d.batch * (p.BH + 1) * p.pitch;
+	if (d.n > 32 || total > 0x7fff0000LL) { return XNOR_B200_ERR_TOO_LARGE; }
+	p.total_pos = (int)total;
+	p.d_img = make_div((uint32_t)((p.BH + 1) * p.pitch));
+	p.d_pitch = make_div((uint32_t)p.pitch);
+	p.vec = (d.w % 2 == 0 && ((uintptr_t)input & 7u) == 0) ? 1 : 0;
+	// Tiles per unit: a unit costs its blocks and the row below them, and the busiest SM has ceil(units / SMs) of them.
+	double best = 1e30;
+	for (int pt = 1; pt <= F3_MAX_PT; ++pt)
+	{
+		const int slots = pt * TC_PIX + p.pitch + 2;
+		if ((size_t)F3_STAGES * round_up((size_t)slots * 32, 128) > F3_SMEM_MAX) { break; }
+		const int units = (int)((total + pt * TC_PIX - 1) / (pt * TC_PIX));
+		const double cost = (double)((units + sm_count() - 1) / sm_count()) * (slots + 60.0);
+		if (cost < best) { best = cost; p.pt = pt; p.units = units; p.plane_slots = slots; }
+	}
+	if (p.pt == 0) { return XNOR_B200_ERR_TOO_LARGE; }
+	p.stage_bytes = (int)round_up((size_t)p.plane_slots * 32, 128);
+	TcParams common = {};
+	const int rc = tc_fill_launch_fields(common);
+	if (rc != XNOR_B200_OK) { return rc; }
+	p.status = common.status; p.spin_limit = common.spin_limit;
+	const size_t smem = (size_t)F3_STAGES * p.stage_bytes;
+	if (d.n <= 16) { return pool ? launch_f3<16, true>(p, smem, stream) : launch_f3<16, false>(p, smem, stream); }
+	return pool ? launch_f3<32, true>(p, smem, stream) : launch_f3<32, false>(p, smem, stream);
+}
+
+}  // namespace xnor

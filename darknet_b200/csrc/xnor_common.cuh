@@ -163,6 +163,10 @@ int launch_xnor_gemm_tc(int M, int n_total, int n_per_image, int K,
 // Sticky device-side status (bounded wait expired in the tensor-core kernel); synchronous copy from the device.
 int read_tc_error(int * out, bool clear);
 
+// Signs of the first float convolution on the tensor cores (float_conv3_tc.cu); ERR_TOO_LARGE: a shape it does not take.
+int launch_float_conv3_signs(const xnor_b200_conv_desc & d, int pool, const float * input, const float * weights, const float * biases,
+		uint32_t * words, int pitch, cudaStream_t stream);
+
 // pool == nullptr: the tensor in memory is the convolution input; otherwise it is max-pooled on the fly.
 // from_signs != 0: `input` is not fp32 but the sign words [image][c/32][in_h*in_w] left by a sign-only GEMM epilogue.
 int launch_pack_input(const xnor_b200_conv_desc & d, const xnor_b200_pool_desc * pool, const float * input,
