@@ -6,34 +6,38 @@
 // off they can be; wherever the value is farther from zero than that, the sign is known, and the rest -- about half a percent --
 // are formed again in fp32, in the order above.  Every bit is therefore the exact one.
 //
-//   |approximate - exact| <= (xmax + 1e-4) * (1.02e-3 * sum|w| + 1e-6)
+//   |approximate - exact| <= (xmax + 1e-4) * 1.03e-3
 //
-// with the filter scaled by a power of two to max|w| in [0.5, 1) and xmax the largest input of the unit: 2^-10 for the two fp16
-// roundings of a product, 2^-25 each for subnormal operands, the rest for the accumulation here and there.  Inputs or filters that
-// fp16 cannot hold make the bound infinite, and every value is formed again.
+// (compared in fp16, hence 1.032e-3 + 1.2e-7) for a filter scaled to sum|w| = 1 and xmax the largest input of the unit: 2^-10 for the
+// two fp16 roundings of a product, 2^-25 each for subnormal operands, the rest for the scaling and the accumulation here and there.
+// Inputs or filters that fp16 cannot hold make the bound infinite or the value NaN, and every value is formed again.
 //
-// One MMA row is a 2x2 block of pixels, its columns the block's four values of every filter, K the 4x4 patch: with N = 4 * filters
-// and 8 (pair of pixels x 4) halves of 16 bytes that is 4 instructions per 512 pixels.  The operand is never gathered: an input
-// pixel pair (2q - 1, 2q) is 16 bytes [c0 c1 c2 0 | c0 c1 c2 0] in a plane [block row][pair], one plane for even and one for odd
-// pixel rows, and a patch row is another start address (as in xnor_conv.cu; position = (image * (BH + 1) + by) * (BW + 1) + bx).
+// One MMA row is a 2x2 block of pixels, its columns the block's four values of every filter, K the patch of pixels around it: with
+// N = 4 * filters and 12 halves of 16 bytes that is 6 instructions per 512 pixels.  The operand is never gathered: an input pixel
+// pair (2q, 2q + 1) is 16 bytes [c0 c1 c2 1 | c0 c1 c2 1] in a plane [block row][pair], one plane for even and one for odd pixel
+// rows, and a row or a neighbouring pair is another start address (as in xnor_conv.cu; position = (image * (BH + 1) + by) * (BW + 1) +
+// bx, the pair behind a row is zero).  The ones carry the bias, as three fp16 parts in the filter operand.
 //
-// Roles (one CTA per SM): warps 0..15 epilogue, 16..22 converters (global fp32 -> planes), 23 issuer.
-// Bound by HBM (12 bytes a pixel) and by the converters' and the epilogue's issue slots.
+// Roles (one CTA per SM): warps 0..11 (unpooled 0..15) epilogue, then converters (global fp32 -> planes), 23 issuer.
+// Measured at 416x416, 16 filters, pooled, 64 images: 90 us; 350 with every load followed by its use, 104 with unaligned pairs
+// (2q - 1, 2q), a shuffle for each, and bias and bound per filter in the epilogue.  Clock traces: converters and epilogue, bound by
+// issue slots and by the latency of the doubtful values, take turns as the bound; HBM would be 22 us.
 #include "grid_words.cuh"
 #include "tc_common.cuh"
+
+#include <cuda_fp16.h>
 
 namespace xnor
 {
 
-constexpr int F3_EPI_WARPS = 16;
-constexpr int F3_CONV_WARPS = 7;
-constexpr int F3_MMA_WARP = F3_EPI_WARPS + F3_CONV_WARPS;
+constexpr int F3_MMA_WARP = 23;
 constexpr int F3_THREADS = (F3_MMA_WARP + 1) * 32;
 constexpr int F3_BATCH = 2;                    // window slots a converter thread has in flight
 constexpr int F3_STAGES = 3;
 constexpr int F3_MAX_PT = 8;                  // tiles of 128 blocks per unit
 constexpr int F3_MAX_UNITS_AHEAD = 16;        // entries of the ring of unit maxima: stages + accumulators + 1 are under way
 constexpr int F3_QUEUE = 64;                  // values of a warp that wait to be formed exactly
+constexpr int F3_HALVES = 12;                 // 16-byte pieces of K: four patch rows x three pairs
 constexpr int F3_SMEM_MAX = 200 * 1024;
 
 struct F3Params
@@ -47,7 +51,7 @@ struct F3Params
 	int OH, OW, out_pitch;
 	FastDiv d_img, d_pitch;  // positions per image, per row
 	int total_pos, pt, units;
-	int plane_slots;         // window positions of a unit: pt * 128 + pitch + 2
+	int plane_slots;         // window positions of a unit, from one in front of it on: pt * 128 + pitch + 2
 	int stage_bytes;
 	int vec;                 // 1: rows of whole, aligned pairs
 	int * status;
@@ -61,11 +65,37 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi)
 	return r;
 }
 
-// The larger value, NaN if either is
-__device__ __forceinline__ float max_nan(float a, float b)
+// Largest magnitude so far of the two halves each, NaN if one is
+__device__ __forceinline__ uint32_t max_half2(uint32_t a, uint32_t b)
+{
+	uint32_t r;
+	asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b & 0x7fff7fffu));
+	return r;
+}
+
+__device__ __forceinline__ uint32_t larger_half2(uint32_t a, uint32_t b)
+{
+	uint32_t r;
+	asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+	return r;
+}
+
+// 0xffff in each half where a > b (not where either is NaN)
+__device__ __forceinline__ uint32_t above_half2(uint32_t a, uint32_t b)
+{
+	return __hgt2_mask(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+}
+
+// Bits 0..3, 8..11 and 16..19, 24..27 -> 0..15
+__device__ __forceinline__ uint32_t spread(uint32_t v)
+{
+	return (v & 0x0f0fu) | ((v >> 12) & 0xf0f0u);
+}
+
+__device__ __forceinline__ float half_of(float v)
 {
 	float r;
-	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	asm("{\n\t.reg .b16 h;\n\tcvt.rn.f16.f32 h, %1;\n\tcvt.f32.f16 %0, h;\n\t}" : "=f"(r) : "f"(v));
 	return r;
 }
 
@@ -78,20 +108,16 @@ __device__ __forceinline__ uint64_t f3_desc(uint32_t start, uint32_t lbo)
 __device__ __forceinline__ float exact_value(const F3Params & p, int img, int oy, int ox, const float * w, float bias)
 {
 	const float * base = p.in + (size_t)img * 3 * p.H * p.W;
-	float acc = 0.0f;
-	#pragma unroll 1
-	for (int c = 0; c < 3; ++c)
+	float v[27];                                                  // all loads at once: one memory latency
+	#pragma unroll
+	for (int k = 0; k < 27; ++k)
 	{
-		float v[9];
-		#pragma unroll
-		for (int k = 0; k < 9; ++k)
-		{
-			const int iy = oy - 1 + k / 3, ix = ox - 1 + k % 3;
-			v[k] = (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) ? __ldg(base + ((size_t)c * p.H + iy) * p.W + ix) : 0.0f;
-		}
-		#pragma unroll
-		for (int k = 0; k < 9; ++k) { acc = fmaf(v[k], w[c * 9 + k], acc); }
+		const int iy = oy - 1 + (k % 9) / 3, ix = ox - 1 + k % 3;
+		v[k] = (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) ? __ldg(base + ((size_t)(k / 9) * p.H + iy) * p.W + ix) : 0.0f;
 	}
+	float acc = 0.0f;
+	#pragma unroll
+	for (int k = 0; k < 27; ++k) { acc = fmaf(v[k], w[k], acc); }
 	return acc + bias;
 }
 
@@ -100,16 +126,17 @@ template <int NF, bool POOL>
 __global__ void __launch_bounds__(F3_THREADS, 1)
 float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 {
+	// the 23 warps beside the issuer: a pooled block leaves one word of 16 bits, an unpooled one four words, for the same input
+	constexpr int EPI_WARPS = POOL ? 12 : 16;
+	constexpr int CONV_WARPS = F3_MMA_WARP - EPI_WARPS;
 	constexpr int NN = 4 * NF;                                  // MMA columns: POOL: filter * 4 + pixel of the block, else pixel * NF + filter
 	constexpr int ACC = 512 / NN;
 	extern __shared__ __align__(128) uint8_t f3_smem[];         // [stage][odd rows | even rows][slot] of 16 bytes
-	__shared__ __align__(128) uint4 s_b[8 * NN];                // filter operand [16-byte half of K][column]
+	__shared__ __align__(128) uint4 s_b[F3_HALVES * NN];                // filter operand [16-byte half of K][column]
 	__shared__ float s_w[NF * 27];
 	__shared__ float s_bias[NF];                                // as given
-	__shared__ __align__(16) float s_sb[NF];                    // scaled like the filter
-	__shared__ __align__(16) float s_tol[NF];                   // bound = (xmax + 1e-4) * tol
-	__shared__ float s_xmax[F3_MAX_UNITS_AHEAD][F3_CONV_WARPS];
-	__shared__ uint2 s_queue[F3_EPI_WARPS][F3_QUEUE];
+	__shared__ float s_xmax[F3_MAX_UNITS_AHEAD][CONV_WARPS];
+	__shared__ uint2 s_queue[EPI_WARPS][F3_QUEUE];
 	__shared__ uint64_t st_full[F3_STAGES], st_empty[F3_STAGES], acc_full[ACC], acc_empty[ACC], drain_bar;
 	__shared__ uint32_t tmem_base_slot;
 	__shared__ int s_failed_storage;
@@ -127,7 +154,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	{
 		for (int s = 0; s < F3_STAGES; ++s)
 		{
-			mbar_init(&st_full[s], F3_CONV_WARPS);
+			mbar_init(&st_full[s], CONV_WARPS);
 			mbar_init(&st_empty[s], 1);
 		}
 		for (int a = 0; a < ACC; ++a)
@@ -148,35 +175,30 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	__syncthreads();
 	if (tid < NF)
 	{
-		float big = 0.0f, sum = 0.0f;
-		bool fits = true;
-		for (int k = 0; k < 27; ++k)
-		{
-			const float w = fabsf(s_w[tid * 27 + k]);
-			fits = fits && (w < 1e30f);
-			big = fmaxf(big, w);
-		}
-		int e = 0;
-		if (big > 0.0f) { frexpf(big, &e); }
-		fits = fits && e > -100;
-		const float scale = fits ? ldexpf(1.0f, -e) : 0.0f;
-		for (int k = 0; k < 27; ++k) { sum += fabsf(s_w[tid * 27 + k] * scale); }
+		float sum = 0.0f;
+		for (int k = 0; k < 27; ++k) { sum += fabsf(s_w[tid * 27 + k]); }
 		const float bias = (p.biases != nullptr && tid < p.N) ? __ldg(p.biases + tid) : 0.0f;
 		s_bias[tid] = bias;
-		s_sb[tid] = bias * scale;
-		s_tol[tid] = fits ? 1.02e-3f * sum + 1e-6f : INFINITY;
-		for (int h = 0; h < 8; ++h)
+		// a filter of zeros stays as it is; one whose scale fp32 cannot hold, or whose bias fp16 cannot, gets a bias of NaN
+		const float scale = (sum > 0.0f) ? 1.0f / sum : 1.0f;
+		const bool fits = (sum < 1e30f) && (scale < 1e30f) && (fabsf(bias * scale) < 60000.0f);
+		float part[3];
+		part[0] = fits ? bias * scale : NAN;
+		part[1] = part[0] - half_of(part[0]);
+		part[2] = part[1] - half_of(part[1]);
+		for (int h = 0; h < F3_HALVES; ++h)
 		{
-			// half h: patch row h / 2 counted odd, even, odd, even; pair h % 2
-			const int row = h >> 1;
+			// half h: patch rows 0, 2 (odd pixel rows), 1, 3 (even ones), three pairs each
+			const int row = (h / 6) + 2 * ((h / 3) & 1), pair = h % 3;
 			for (int s = 0; s < 4; ++s)
 			{
 				float v[8];
 				for (int q = 0; q < 8; ++q)
 				{
-					const int ky = row - (s >> 1), kx = (h & 1) * 2 + (q >> 2) - (s & 1), c = q & 3;
-					v[q] = (c < 3 && ky >= 0 && ky < 3 && kx >= 0 && kx < 3) ? s_w[tid * 27 + (c * 3 + ky) * 3 + kx] * scale : 0.0f;
+					const int ky = row - (s >> 1), kx = 2 * (pair - 1) + (q >> 2) - (s & 1) + 1, c = q & 3;
+					v[q] = (fits && c < 3 && ky >= 0 && ky < 3 && kx >= 0 && kx < 3) ? s_w[tid * 27 + (c * 3 + ky) * 3 + kx] * scale : 0.0f;
 				}
+				if (h < 3) { v[3] = part[h]; }
 				s_b[h * NN + (POOL ? tid * 4 + s : s * NF + tid)] = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
 			}
 		}
@@ -187,7 +209,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
 
-	if (warp < F3_EPI_WARPS)
+	if (warp < EPI_WARPS)
 	{
 		// ---- epilogue: warp w takes the tiles w / 4, w / 4 + 4, ... of this CTA, lane quarter w % 4 -----------------------------
 		const int quarter = warp & 3;
@@ -198,7 +220,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 		int a = tile % ACC;
 		uint32_t phase = (uint32_t)((tile / ACC) & 1);
 		int have_unit = -1;
-		float xmax = 0.0f;
+		uint32_t limit2 = 0;                                     // the bound of the unit, in both halves
 		int q_head = 0, q_count = 0;                             // this warp's ring of values to be formed exactly
 		// output word of a position and pixel of its block
 		auto word_at = [&](int img, int y, int x) { return p.words + ((size_t)img * (p.OH + 1) + y) * p.out_pitch + x; };
@@ -250,10 +272,12 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 			if (nu != have_unit)
 			{
 				have_unit = nu;
-				xmax = (lane < F3_CONV_WARPS) ? s_xmax[nu % F3_MAX_UNITS_AHEAD][lane] : 0.0f;
+				float xmax = (lane < CONV_WARPS) ? s_xmax[nu % F3_MAX_UNITS_AHEAD][lane] : 0.0f;
 				#pragma unroll
-				for (int o = 4; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
-				xmax = __shfl_sync(0xffffffffu, xmax, 0) + 1e-4f;
+				for (int o = 8; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
+				// values are compared as fp16, so a little more for their rounding; infinity stays infinity
+				const float bound = (__shfl_sync(0xffffffffu, xmax, 0) + 1e-4f) * 1.032e-3f + 1.2e-7f;
+				limit2 = pack_half2(bound, bound);
 			}
 			const int pos = (((int)blockIdx.x + nu * (int)gridDim.x) * p.pt + t) * TC_PIX + quarter * 32 + lane;
 			const int img = fdiv(pos, p.d_img);
@@ -263,7 +287,9 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 			const uint32_t tacc = tmem_base + (uint32_t)(a * NN) + ((uint32_t)(quarter * 32) << 16);
 			if (POOL)
 			{
-				uint32_t word = 0, unsure = 0;
+				uint32_t pos_bits[NN / 64], sure_bits[NN / 64];        // of 16 filters: the low half 0..3 | 8..11, the high half 4..7 | 12..15
+				#pragma unroll
+				for (int g = 0; g < NN / 64; ++g) { pos_bits[g] = 0; sure_bits[g] = 0; }
 				#pragma unroll
 				for (int h = 0; h < NN / 32; ++h)
 				{
@@ -276,21 +302,26 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 						__syncwarp();
 						if (lane == 0) { mbar_arrive(&acc_empty[a]); }
 					}
-					const float4 b0 = *reinterpret_cast<const float4 *>(s_sb + h * 8), b1 = *reinterpret_cast<const float4 *>(s_sb + h * 8 + 4);
-					const float4 t0 = *reinterpret_cast<const float4 *>(s_tol + h * 8), t1 = *reinterpret_cast<const float4 *>(s_tol + h * 8 + 4);
-					const float sb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-					const float tol[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+					// filters i and i + 4 of these eight side by side
 					#pragma unroll
-					for (int i = 0; i < 8; ++i)
+					for (int i = 0; i < 4; ++i)
 					{
-						const int f = h * 8 + i;
-						const float top = fmaxf(fmaxf(__uint_as_float(d[4 * i]), __uint_as_float(d[4 * i + 1])), fmaxf(__uint_as_float(d[4 * i + 2]), __uint_as_float(d[4 * i + 3])));
-						const float v = top + sb[i];
-						const float bound = xmax * tol[i];
-						word |= (v > bound) ? (1u << f) : 0u;
-						unsure |= !(fabsf(v) > bound) ? (1u << f) : 0u;
+						uint32_t v = pack_half2(__uint_as_float(d[4 * i]), __uint_as_float(d[4 * i + 16]));
+						#pragma unroll
+						for (int s = 1; s < 4; ++s) { v = larger_half2(v, pack_half2(__uint_as_float(d[4 * i + s]), __uint_as_float(d[4 * i + 16 + s]))); }
+						const uint32_t bit = (1u << i) | (1u << (i + 16));
+						pos_bits[h / 2] |= (above_half2(v, limit2) & bit) << (8 * (h & 1));
+						sure_bits[h / 2] |= (above_half2(v & 0x7fff7fffu, limit2) & bit) << (8 * (h & 1));
 					}
 				}
+				uint32_t word = 0, unsure = 0;
+				#pragma unroll
+				for (int g = 0; g < NN / 64; ++g)
+				{
+					word |= spread(pos_bits[g]) << (16 * g);
+					unsure |= spread(sure_bits[g]) << (16 * g);
+				}
+				unsure = ~unsure & ((NF == 32) ? 0xffffffffu : 0xffffu);
 				// filters past the last have weights and bias zero: exact value 0, no sign
 				if (ok) { *word_at(img, by, bx) = word; }
 				if (!ok) { unsure = 0; }
@@ -311,21 +342,22 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 						__syncwarp();
 						if (lane == 0) { mbar_arrive(&acc_empty[a]); }
 					}
+					// filters f and f + NF / 2 side by side
 					uint32_t word = 0, unsure = 0;
 					#pragma unroll
-					for (int f0 = 0; f0 < NF; f0 += 4)
+					for (int f = 0; f < NF / 2; ++f)
 					{
-						const float4 b4 = *reinterpret_cast<const float4 *>(s_sb + f0), t4 = *reinterpret_cast<const float4 *>(s_tol + f0);
-						const float sb[4] = {b4.x, b4.y, b4.z, b4.w}, tol[4] = {t4.x, t4.y, t4.z, t4.w};
-						#pragma unroll
-						for (int i = 0; i < 4; ++i)
-						{
-							const float v = __uint_as_float(d[f0 + i]) + sb[i];
-							const float bound = xmax * tol[i];
-							word |= (v > bound) ? (1u << (f0 + i)) : 0u;
-							unsure |= !(fabsf(v) > bound) ? (1u << (f0 + i)) : 0u;
-						}
+						const uint32_t v = pack_half2(__uint_as_float(d[f]), __uint_as_float(d[f + NF / 2]));
+						const uint32_t bit = (1u << f) | (1u << (f + 16));
+						word |= above_half2(v, limit2) & bit;
+						unsure |= above_half2(v & 0x7fff7fffu, limit2) & bit;
 					}
+					if (NF == 16)
+					{
+						word = (word & 0xffu) | ((word >> 8) & 0xff00u);
+						unsure = (unsure & 0xffu) | ((unsure >> 8) & 0xff00u);
+					}
+					unsure = ~unsure & ((NF == 32) ? 0xffffffffu : 0xffffu);
 					const int oy = 2 * by + (s >> 1), ox = 2 * bx + (s & 1);
 					const bool in = ok && oy < p.OH && ox < p.OW;
 					if (in) { *word_at(img, oy, ox) = word; }
@@ -334,97 +366,100 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 					if (__any_sync(0xffffffffu, unsure != 0)) { enqueue(unsure, pos, s); }
 				}
 			}
-			tile += F3_EPI_WARPS / 4;
-			a += F3_EPI_WARPS / 4;
+			tile += EPI_WARPS / 4;
+			a += EPI_WARPS / 4;
 			while (a >= ACC) { a -= ACC; phase ^= 1u; }
-			t += F3_EPI_WARPS / 4;
+			t += EPI_WARPS / 4;
 			while (t >= p.pt) { t -= p.pt; ++nu; }
 		}
 		while (q_count > 0) { resolve(min(q_count, POOL ? 8 : 32)); }
 	}
 	else if (warp < F3_MMA_WARP)
 	{
-		// ---- converters: a slot is the pair of pixels (2q - 1, 2q) of an odd and of an even row -----------------------------
-		const int cw = warp - F3_EPI_WARPS;
+		// ---- converters: a slot is the pair of pixels (2q, 2q + 1) of an odd and of an even row ------------------------------
+		const int cw = warp - EPI_WARPS;
 		const size_t plane = (size_t)p.H * p.W;
 		const int groups = (p.plane_slots + 31) >> 5;
+		const int H = p.H, W = p.W, plane_slots = p.plane_slots, total_pos = p.total_pos, pitch = p.pitch;
+		const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
+		const bool vec = (p.vec != 0);
 		int es = 0;
 		uint32_t es_phase = 1;
 		bool ok = true;
 		for (int nu = 0; nu < my_units && ok; ++nu)
 		{
-			const int pos0 = ((int)blockIdx.x + nu * (int)gridDim.x) * p.pt * TC_PIX;
+			const int pos0 = ((int)blockIdx.x + nu * (int)gridDim.x) * p.pt * TC_PIX - 1;
 			const uint32_t odd = a_base + (uint32_t)(es * p.stage_bytes);
-			const uint32_t even = odd + (uint32_t)(p.plane_slots * 16);
-			float xmax = 0.0f;
+			const uint32_t even = odd + (uint32_t)(plane_slots * 16);
+			uint32_t top = 0;                                     // largest magnitudes, two halves
 			if (nu >= F3_STAGES)
 			{
 				ok = __all_sync(0xffffffffu, mbar_wait<32>(&st_empty[es], es_phase, s_failed, limit));
 				if (!ok) { break; }
 			}
-			// F3_BATCH slots at a time: all of their loads first, for the kernel lives on bytes in flight (a load followed by the
-			// shuffle that uses it, slot by slot, took 350 us where this takes ~F3_NOW~: 64 images of 416x416)
-			for (int g0 = cw; g0 < groups; g0 += F3_CONV_WARPS * F3_BATCH)
+			// F3_BATCH slots at a time, all of their loads first: the kernel lives on bytes in flight
+			for (int g0 = cw; g0 < groups; g0 += CONV_WARPS * F3_BATCH)
 			{
-				float2 v[F3_BATCH][6];                            // [slot][odd, even row x channel]: pixels 2q and 2q + 1
-				float e[F3_BATCH][6];                             // pixel 2q - 1 where no neighbouring lane has it
-				bool mid[F3_BATCH];
+				float2 v[F3_BATCH][6];                            // [slot][odd, even row x channel]
 				#pragma unroll
 				for (int i = 0; i < F3_BATCH; ++i)
 				{
-					const int s = (g0 + i * F3_CONV_WARPS) * 32 + lane;
+					const int s = (g0 + i * CONV_WARPS) * 32 + lane;
 					const int pos = pos0 + s;
-					const int img = fdiv(pos, p.d_img);
-					const int r = pos - img * (int)p.d_img.d;
-					const int by = fdiv(r, p.d_pitch), q = r - by * p.pitch;
-					const bool in = (s < p.plane_slots && pos < p.total_pos);
+					const int img = fdiv(max(pos, 0), d_img);
+					const int r = pos - img * (int)d_img.d;
+					const int by = fdiv(max(r, 0), d_pitch), q = r - by * pitch;
 					const int ye = 2 * by, x = 2 * q;
-					const float * at = p.in + (size_t)img * 3 * plane + (ptrdiff_t)(ye - 1) * p.W + x;
-					mid[i] = (q > 0);
+					const bool in = (s < plane_slots && pos >= 0 && pos < total_pos && x < W);
+					const bool odd_ok = in && ye > 0 && ye - 1 < H, even_ok = in && ye < H;
+					const float * at = p.in + (size_t)img * 3 * plane + (ptrdiff_t)ye * W + x;
 					#pragma unroll
-					for (int k = 0; k < 2; ++k)
+					for (int c = 0; c < 3; ++c, at += plane)
 					{
-						const int y = ye - 1 + k;
-						const bool row_ok = in && y >= 0 && y < p.H;
-						const bool own = row_ok && x < p.W, edge = row_ok && q > 0 && x - 1 < p.W && (lane == 0 || !p.vec);
-						#pragma unroll
-						for (int c = 0; c < 3; ++c)
+						v[i][c] = make_float2(0.0f, 0.0f);
+						v[i][3 + c] = make_float2(0.0f, 0.0f);
+						if (vec)
 						{
-							const float * src = at + (ptrdiff_t)k * p.W + (size_t)c * plane;
-							v[i][k * 3 + c] = make_float2(0.0f, 0.0f);
-							e[i][k * 3 + c] = 0.0f;
-							if (p.vec) { if (own) { v[i][k * 3 + c] = __ldg(reinterpret_cast<const float2 *>(src)); } }
-							else if (own) { v[i][k * 3 + c].x = __ldg(src); }
-							if (edge) { e[i][k * 3 + c] = __ldg(src - 1); }
+							if (odd_ok) { v[i][c] = __ldg(reinterpret_cast<const float2 *>(at - W)); }
+							if (even_ok) { v[i][3 + c] = __ldg(reinterpret_cast<const float2 *>(at)); }
+						}
+						else
+						{
+							if (odd_ok) { v[i][c].x = __ldg(at - W); }
+							if (odd_ok && x + 1 < W) { v[i][c].y = __ldg(at - W + 1); }
+							if (even_ok) { v[i][3 + c].x = __ldg(at); }
+							if (even_ok && x + 1 < W) { v[i][3 + c].y = __ldg(at + 1); }
 						}
 					}
 				}
 				#pragma unroll
 				for (int i = 0; i < F3_BATCH; ++i)
 				{
-					const int s = (g0 + i * F3_CONV_WARPS) * 32 + lane;
+					const int s = (g0 + i * CONV_WARPS) * 32 + lane;
 					#pragma unroll
 					for (int k = 0; k < 2; ++k)
 					{
-						float l[3], h[3];
-						#pragma unroll
-						for (int c = 0; c < 3; ++c)
+						const float2 c0 = v[i][3 * k], c1 = v[i][3 * k + 1], c2 = v[i][3 * k + 2];
+						const uint32_t left = pack_half2(c0.x, c1.x), right = pack_half2(c0.y, c1.y), third = pack_half2(c2.x, c2.y);
+						top = max_half2(top, left);
+						top = max_half2(top, right);
+						top = max_half2(top, third);
+						if (s < plane_slots)
 						{
-							// rows outside the image and slots behind the end were left at zero, in the neighbour as here
-							const float left = __shfl_up_sync(0xffffffffu, v[i][k * 3 + c].y, 1);
-							l[c] = (lane == 0 || !p.vec) ? e[i][k * 3 + c] : (mid[i] ? left : 0.0f);
-							h[c] = v[i][k * 3 + c].x;
-							xmax = max_nan(xmax, max_nan(fabsf(h[c]), fabsf(l[c])));
-						}
-						if (s < p.plane_slots)
-						{
+							constexpr uint32_t ONE = 0x3c00u;
 							asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"((k == 0 ? odd : even) + (uint32_t)s * 16u),
-									"r"(pack_half2(l[0], l[1])), "r"(pack_half2(l[2], 0.0f)), "r"(pack_half2(h[0], h[1])), "r"(pack_half2(h[2], 0.0f)));
+									"r"(left), "r"(__byte_perm(third, ONE, 0x5410)), "r"(right), "r"(__byte_perm(third, ONE, 0x5432)));
 						}
 					}
 				}
 			}
-			if (!(xmax < 60000.0f)) { xmax = INFINITY; }                    // beyond fp16, or not a number
+			float xmax;
+			{
+				// (a little more than the fp16 maximum for what its rounding may have taken; NaN counts as infinity)
+				float lo, hi;
+				asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, h;\n\t}" : "=f"(lo), "=f"(hi) : "r"(top));
+				xmax = (lo <= 65504.0f && hi <= 65504.0f) ? fmaxf(lo, hi) * 1.001f : INFINITY;
+			}
 			#pragma unroll
 			for (int o = 16; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
 			if (lane == 0) { s_xmax[nu % F3_MAX_UNITS_AHEAD][cw] = xmax; }
@@ -461,16 +496,19 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 				else { ++used; }
 				const uint32_t even = odd + (uint32_t)p.plane_slots;
 				#pragma unroll
-				for (int k = 0; k < 4; ++k)                       // patch rows 2by - 1, 2by, 2by + 1, 2by + 2
+				for (int k = 0; k < F3_HALVES / 2; ++k)
 				{
-					const uint32_t start = ((k & 1) ? even : odd) + ((k >> 1) ? (uint32_t)p.pitch : 0u);
+					// per plane: (row 0, pairs 0 and 1), (row 0, pair 2 and row 1, pair 0), (row 1, pairs 1 and 2)
+					const uint32_t from = (k < 3) ? odd : even;
+					const uint32_t start = from + ((k % 3 == 0) ? 0u : (k % 3 == 1) ? 2u : (uint32_t)p.pitch + 1u);
+					const uint32_t lbo = (k % 3 == 1) ? (uint32_t)p.pitch - 2u : 1u;
 					if (leader)
 					{
 						asm volatile(
 							"{\n\t.reg .pred p;\n\t"
 							"setp.ne.b32 p, %4, 0;\n\t"
 							"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-							:: "r"(tmem_base + (uint32_t)(a * NN)), "l"(f3_desc(start, 1u)), "l"(f3_desc(b16 + (uint32_t)(2 * k * NN), (uint32_t)NN)), "r"(idesc),
+							:: "r"(tmem_base + (uint32_t)(a * NN)), "l"(f3_desc(start, lbo)), "l"(f3_desc(b16 + (uint32_t)(2 * k * NN), (uint32_t)NN)), "r"(idesc),
 							   "r"(k != 0 ? 1u : 0u), "r"(0u) : "memory");
 					}
 				}
@@ -510,7 +548,8 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 template <int NF, bool POOL>
 static int launch_f3(const F3Params & p, size_t smem, cudaStream_t stream)
 {
-	const int rc = ensure_dynamic_smem((const void *)float_conv3_signs_kernel<NF, POOL>, smem);
+	// (at least 64 KB: with the static part a smaller request would pass the 48 KB that need no asking)
+	const int rc = ensure_dynamic_smem((const void *)float_conv3_signs_kernel<NF, POOL>, smem < 65536 ? 65536 : smem);
 	if (rc != XNOR_B200_OK) { return rc; }
 	const int grid = (p.units < sm_count()) ? p.units : sm_count();
 	float_conv3_signs_kernel<NF, POOL><<<grid, F3_THREADS, smem, stream>>>(p);
@@ -528,7 +567,7 @@ int launch_float_conv3_signs(const xnor_b200_conv_desc & d, int pool, const floa
 	p.OH = pool ? d.h / 2 : d.h; p.OW = pool ? d.w / 2 : d.w; p.out_pitch = pitch;
 	p.words = words + grid_front(pitch);
 	const long long total = (long long)d.batch * (p.BH + 1) * p.pitch;
-	if (d.n > 32 || total > 0x7fff0000LL) { return XNOR_B200_ERR_TOO_LARGE; }
+	if (d.n > 32 || p.pitch < 3 || total > 0x7fff0000LL) { return XNOR_B200_ERR_TOO_LARGE; }
 	p.total_pos = (int)total;
 	p.d_img = make_div((uint32_t)((p.BH + 1) * p.pitch));
 	p.d_pitch = make_div((uint32_t)p.pitch);

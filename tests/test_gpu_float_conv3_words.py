@@ -42,3 +42,25 @@ def test_signs_of_zero_sums_and_zero_biases(batch, h, w, n, pitch, pool):
     assert int(body[:, oh].sum()) == 0 and int(body[:, :, ow:].sum()) == 0
     got = sum(masks[..., i].to(torch.int64) << (8 * i) for i in range(masks.shape[-1]))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("pool,n", [(2, 16), (0, 32)])
+@pytest.mark.parametrize("x_scale,w_scale", [(1.0, 1.0), (1e6, 1.0), (1e-7, 1.0), (1.0, 1e-9), (255.0, 1e5), (1.0, 1e33)])
+def test_signs_at_every_scale(x_scale, w_scale, pool, n):
+    """Values that fp16 cannot hold, or holds with few bits, still get the sign of the fp32 sum (the masks, formed in fp32)."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    x = torch.randn(2, 3, 70, 90, generator=g, device="cuda") * x_scale
+    wt = torch.randn(n, 27, generator=g, device="cuda") * w_scale
+    wt[1] = 0.0
+    b = torch.randn(n, generator=g, device="cuda") * (0.3 * x_scale * w_scale)
+    b[2] = 1e30
+    desc = capi.ConvDesc(2, 3, 70, 90, n, 3, 1, 1, capi.LINEAR)
+    oh, ow = (35, 45) if pool else (70, 90)
+    grid = L.GridWords(2, n, oh, ow)
+    masks = torch.zeros(2, oh, ow, n // 8, dtype=torch.uint8, device="cuda")
+    capi.check(capi.lib().xnor_b200_float_conv3_words(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), grid.words.data_ptr(), 0, None), "words")
+    capi.check(capi.lib().xnor_b200_float_conv3_io(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), None, None, masks.data_ptr(), None), "io")
+    front = capi.lib().xnor_b200_grid_front(ow + 1)
+    body = grid.words[0, front:front + 2 * (oh + 1) * (ow + 1)].view(2, oh + 1, ow + 1)[:, :oh, :ow].to(torch.int64) & 0xFFFFFFFF
+    assert torch.equal(body, sum(masks[..., i].to(torch.int64) << (8 * i) for i in range(n // 8)))
