@@ -16,19 +16,26 @@
 // reference's own GPU path does (it asks cuDNN for tensor-op math, i.e. single tf32 products, on every convolution:
 // src-lib/convolutional_layer.cpp:350).
 //
-// Same skeleton as xnor_gemm_tc.cu: one CTA = 128 pixels (TMEM lanes; the batch is folded into the pixel index) x 128
-// filters (TMEM columns), warp 0 allocates tensor memory and issues (the warp stays converged and one elected lane issues: a
-// divergent lane takes longer to bring an instruction's operands to the uniform registers than the tensor core to execute it),
-// 16 producer warps -- two threads per operand
-// row, 16 channels of every K block each (pixel row: one coalesced load per channel across the warp; filter row: 64
-// contiguous bytes) -- split their values and write hi and lo straight into K-major SWIZZLE_128B tiles (32 tf32 = one 128-byte row); 12
-// tcgen05.mma.kind::tf32 (M=128, N=128, K=8) per K block of 32 channels; the same warps then add the bias, apply leaky and
-// store 32 consecutive pixels of one filter per warp-store.  Every barrier wait is bounded (status word shared with the
-// xnor tensor-core kernels).
+// One tile of 128 pixels (TMEM lanes; the batch is folded into the pixel index) x 128 filters (TMEM columns) per CTA.  Warp 0 issues
+// (converged, one elected lane: a divergent lane takes longer to bring an instruction's operands to the uniform registers than the
+// tensor core to execute it): 12 tcgen05.mma.kind::tf32 (M=128, N=128, K=8, 73 cycles each) per K block of 32 channels.  Warps 1..16
+// produce the pixel operand -- four threads per row, 8 channels of every K block each, two blocks in flight -- and split it into the
+// hi and lo K-major SWIZZLE_128B tiles.  Warp 17 brings the filter operand, which load time has split and laid out in the same form,
+// with one 32 KB bulk copy per block.  With few tiles the K blocks are dealt to a cluster of up to four CTAs per tile; the partial
+// sums meet in the first one's shared memory and are added in order.  The epilogue adds the bias, applies leaky or the [yolo]
+// layer's logistic and stores 32 consecutive pixels of one filter per warp-store.  Every barrier wait is bounded (status word
+// shared with the xnor tensor-core kernels).
+// Measured: 3x3 256 -> 512 on 13x13 at batch 64 162 us (one block in flight and the filters split on the way: 300), at batch 8 30 us
+// (101 without the cluster); 1x1 1024 -> 425 on 13x13 at batch 256 269 us (475).  Bound by the tensor pipe (880 cycles per K block) and
+// by shared-memory bandwidth (64 KB written and 96 KB read per K block: 1280 cycles).
 #include "tc_common.cuh"
+
+#include <cooperative_groups.h>
 
 namespace xnor
 {
+
+namespace cg = cooperative_groups;
 
 constexpr int FT_NF = 128;                                 // filters per tile
 constexpr int FT_ACCS = 4;                                 // accumulators that take the K blocks in turn
@@ -36,15 +43,17 @@ constexpr int FT_STAGES = 3;
 constexpr int FT_TILE_BYTES = 128 * 128;                   // 128 rows x 32 tf32
 constexpr int FT_STAGE_BYTES = 4 * FT_TILE_BYTES;          // pixel hi, pixel lo, filter hi, filter lo
 constexpr int FT_SMEM_BYTES = FT_STAGES * FT_STAGE_BYTES + 1024;
-constexpr int FT_TPR = 2;                                  // producer threads per operand row: each takes 32 / FT_TPR channels of a K block
-constexpr int FT_CH = 32 / FT_TPR;
-constexpr int FT_PRODUCER_WARPS = 8 * FT_TPR;
-constexpr int FT_THREADS = 32 + 32 * FT_PRODUCER_WARPS;
+constexpr int FT_PARTS = 4;                                // producer threads per pixel row: each takes 8 channels of a K block
+constexpr int FT_CH = 32 / FT_PARTS;
+constexpr int FT_PRODUCER_WARPS = 4 * FT_PARTS;
+constexpr int FT_COPY_WARP = FT_PRODUCER_WARPS + 1;
+constexpr int FT_THREADS = 32 * (FT_COPY_WARP + 1);
+constexpr int FT_MAX_SPLIT = 4;                            // CTAs that share a tile's K blocks: their sums fill the first one's stages
 
 struct FtParams
 {
 	const float * x;      // [batch][C][HW]
-	const float * w;      // [N][taps][C]
+	const float * w;      // RAW: [N][C] (1x1); else [filter tile][K block][hi, lo][128 rows x 32 channels, swizzled]
 	const float * bias;   // [N] or nullptr
 	float * out;          // [batch][N][HW]
 	int C, HW, N;
@@ -55,7 +64,7 @@ struct FtParams
 	int yolo_entries;     // > 0: the [yolo] layer's activation step is applied to the result (xnor_b200_yolo_activate)
 	int leaky;
 	int tiles_f;
-	int w_vec;            // 1: weight rows may be read with 16-byte loads
+	int split;            // CTAs per tile
 	int * status;
 	uint32_t spin_limit;
 };
@@ -82,6 +91,24 @@ __device__ __forceinline__ void split_row(uint32_t row_swz_hi, uint32_t lo_offse
 	}
 }
 
+// The partial sums of the accumulators that were used, added in fp32: 32 columns of this warp's lanes
+__device__ __forceinline__ void tile_sums(uint32_t tmem, int used, float (&acc)[32])
+{
+	#pragma unroll
+	for (int j = 0; j < 32; ++j) { acc[j] = 0.0f; }
+	#pragma unroll 1
+	for (int a = 0; a < used; ++a)
+	{
+		uint32_t d[32];
+		tmem_load<32>(tmem + (uint32_t)(a * FT_NF), d);
+		asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+		#pragma unroll
+		for (int j = 0; j < 32; ++j) { acc[j] = (a == 0) ? __uint_as_float(d[j]) : __fadd_rn(acc[j], __uint_as_float(d[j])); }
+	}
+}
+
+// RAW: the filters come as Darknet keeps them and are split by the producers as well (callers without a prepared copy, 1x1 only).
+template <bool RAW>
 __global__ void __launch_bounds__(FT_THREADS, 1)
 float_conv_tc_kernel(const FtParams p)
 {
@@ -98,15 +125,22 @@ float_conv_tc_kernel(const FtParams p)
 	const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 	const int lane = tid & 31;
 	const uint32_t ring = (smem_u32(ft_smem_raw) + 1023u) & ~1023u;
-	const int tile_p = blockIdx.x / p.tiles_f;
-	const int f0 = (blockIdx.x - tile_p * p.tiles_f) * FT_NF;
+	const int tile = blockIdx.x / p.split;
+	const int rank = blockIdx.x - tile * p.split;
+	const int tile_p = tile / p.tiles_f;
+	const int tile_f = tile - tile_p * p.tiles_f;
+	const int f0 = tile_f * FT_NF;
+	// this CTA's K blocks
+	const int per = (p.kblocks + p.split - 1) / p.split;
+	const int kb0 = rank * per;
+	const int kbn = max(0, min(p.kblocks - kb0, per));
 	const int g0 = tile_p * TC_PIX;                          // first pixel of the tile, batch folded in
 
 	if (tid == 0)
 	{
 		for (int s = 0; s < FT_STAGES; ++s)
 		{
-			mbar_init(&bar_full[s], FT_PRODUCER_WARPS);
+			mbar_init(&bar_full[s], FT_PRODUCER_WARPS + (RAW ? 0 : 1));
 			mbar_init(&bar_empty[s], 1);
 		}
 		mbar_init(&bar_done, 1);
@@ -131,7 +165,7 @@ float_conv_tc_kernel(const FtParams p)
 			// instruction descriptor: D = f32, A = B = tf32, both K-major, N = 128, M = 128
 			const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(FT_NF >> 3) << 17) | ((uint32_t)(TC_PIX >> 4) << 24);
 			bool ok = true;
-			for (int kb = 0; kb < p.kblocks && ok; ++kb)
+			for (int kb = 0; kb < kbn && ok; ++kb)
 			{
 				const int s = kb % FT_STAGES;
 				ok = __all_sync(0xffffffffu, mbar_wait(&bar_full[s], (uint32_t)((kb / FT_STAGES) & 1), s_failed, p.spin_limit));
@@ -168,75 +202,98 @@ float_conv_tc_kernel(const FtParams p)
 		}
 		__syncwarp();
 	}
-	else
+	else if (warp <= FT_PRODUCER_WARPS)
 	{
-		// ---- producers: per part (FT_CH channels of every K block) four warps of pixel rows and four of filter rows -------
-		const int part = (warp - 1) >> 3;
-		const int r = (tid - 32) - part * 256;
-		const bool is_pix = r < TC_PIX;
-		const int row = is_pix ? r : r - TC_PIX;
-		const uint32_t row_swz0 = (ring + (is_pix ? 0u : 2u * FT_TILE_BYTES) + (uint32_t)row * 128u)
-				^ ((uint32_t)((row & 7) ^ (part * (FT_CH / 4))) << 4);
-		const int g = g0 + row;
-		const int f = f0 + row;
-		const bool row_ok = is_pix ? (g < p.total) : (f < p.N);
-		const int img = (is_pix && row_ok) ? g / p.HW : 0;
-		const int pix = (is_pix && row_ok) ? g - img * p.HW : 0;
-		// element c of the row is base[c * stride]
-		const float * base = is_pix ? p.x + (size_t)img * p.C * p.HW + pix : p.w + (size_t)(row_ok ? f : 0) * p.C * p.taps;
-		const size_t stride = is_pix ? (size_t)p.HW : 1;
+		// ---- producers ------------------------------------------------------------------------------------------------
+		const int part = (warp - 1) >> 2;
+		const int row = ((warp - 1) & 3) * 32 + lane;
+		const uint32_t row_swz0 = (ring + (uint32_t)row * 128u) ^ ((uint32_t)((row & 7) ^ (part * (FT_CH / 4))) << 4);
+		const int g = g0 + row, f = f0 + row;
+		const bool row_ok = g < p.total;
+		const int img = row_ok ? g / p.HW : 0;
+		const int pix = row_ok ? g - img * p.HW : 0;
+		const float * base = p.x + (size_t)img * p.C * p.HW + pix;
 		const int py = pix / p.W, px = pix - py * p.W;
-		float nxt[FT_CH];
-		int tap = 0, cb = 0;                                      // of the K block that is fetched next
-		auto fetch = [&]()
+		int tap = kb0 / p.cblocks, cb = kb0 - tap * p.cblocks;    // of the K block that is fetched next
+		float buf[2][FT_CH], fil[2][RAW ? FT_CH : 1];
+		auto fetch = [&](float (&v)[FT_CH], float (&w)[RAW ? FT_CH : 1])
 		{
 			const int c0 = cb * 32 + part * FT_CH;
-			const float * at = base;
+			const float * at = base + (size_t)c0 * p.HW;
 			bool ok = row_ok;
-			if (p.taps == 9 && is_pix)
+			if (p.taps == 9)
 			{
-				const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+				const int dy = tap / 3 - 1, dx = tap - (tap / 3) * 3 - 1;
 				ok = ok && py + dy >= 0 && py + dy < p.H && px + dx >= 0 && px + dx < p.W;
 				at += dy * p.W + dx;
 			}
-			if (!is_pix) { at += (size_t)tap * p.C; }
 			if (++cb == p.cblocks) { cb = 0; ++tap; }
-			if (!is_pix && p.w_vec && ok && c0 + FT_CH <= p.C)
+			#pragma unroll
+			for (int k = 0; k < FT_CH; ++k, at += p.HW)
+			{
+				v[k] = 0.0f;
+				if (ok && c0 + k < p.C) { v[k] = __ldg(at); }
+			}
+			if constexpr (RAW)
 			{
 				#pragma unroll
-				for (int q = 0; q < FT_CH / 4; ++q)
-				{
-					const float4 t = __ldg(reinterpret_cast<const float4 *>(at + c0) + q);
-					nxt[4 * q] = t.x; nxt[4 * q + 1] = t.y; nxt[4 * q + 2] = t.z; nxt[4 * q + 3] = t.w;
-				}
-				return;
-			}
-			#pragma unroll
-			for (int k = 0; k < FT_CH; ++k)
-			{
-				nxt[k] = (ok && c0 + k < p.C) ? __ldg(at + (size_t)(c0 + k) * stride) : 0.0f;
+				for (int k = 0; k < FT_CH; ++k) { w[k] = (f < p.N && c0 + k < p.C) ? __ldg(p.w + (size_t)f * p.C + c0 + k) : 0.0f; }
 			}
 		};
-		fetch();
+		if (kbn > 0) { fetch(buf[0], fil[0]); }
+		if (kbn > 1) { fetch(buf[1], fil[1]); }
 		bool ok = true;
-		for (int kb = 0; kb < p.kblocks; ++kb)
+		for (int kb = 0; kb < kbn && ok; kb += 2)
+		{
+			#pragma unroll
+			for (int u = 0; u < 2; ++u)
+			{
+				if (kb + u >= kbn) { break; }
+				const int s = (kb + u) % FT_STAGES;
+				if (kb + u >= FT_STAGES)
+				{
+					ok = mbar_wait(&bar_empty[s], (uint32_t)(((kb + u) / FT_STAGES - 1) & 1), s_failed, p.spin_limit);
+					if (!ok) { break; }
+				}
+				split_row(row_swz0 + (uint32_t)s * FT_STAGE_BYTES, (uint32_t)FT_TILE_BYTES, buf[u]);
+				if constexpr (RAW) { split_row(row_swz0 + (uint32_t)s * FT_STAGE_BYTES + 2u * FT_TILE_BYTES, (uint32_t)FT_TILE_BYTES, fil[u]); }
+				if (kb + u + 2 < kbn) { fetch(buf[u], fil[u]); }
+				asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+				__syncwarp();
+				if (lane == 0) { mbar_arrive(&bar_full[s]); }
+			}
+		}
+		if (part == 0) { s_bias[row] = (f < p.N && p.bias != nullptr) ? __ldg(p.bias + f) : 0.0f; }
+	}
+	else if (!RAW)
+	{
+		// ---- filter operand: one bulk copy per K block ------------------------------------------------------------------------
+		const bool leader = elect_one();
+		const float * src = p.w + ((size_t)tile_f * p.kblocks + kb0) * (2 * FT_TILE_BYTES / 4);
+		bool ok = true;
+		int issued = 0;
+		for (int kb = 0; kb < kbn; ++kb, src += 2 * FT_TILE_BYTES / 4)
 		{
 			const int s = kb % FT_STAGES;
-			float cur[FT_CH];
-			#pragma unroll
-			for (int k = 0; k < FT_CH; ++k) { cur[k] = nxt[k]; }
-			if (kb + 1 < p.kblocks) { fetch(); }
 			if (kb >= FT_STAGES)
 			{
-				ok = mbar_wait(&bar_empty[s], (uint32_t)((kb / FT_STAGES - 1) & 1), s_failed, p.spin_limit);
+				ok = __all_sync(0xffffffffu, mbar_wait<32>(&bar_empty[s], (uint32_t)((kb / FT_STAGES - 1) & 1), s_failed, p.spin_limit));
 				if (!ok) { break; }
 			}
-			split_row(row_swz0 + (uint32_t)s * FT_STAGE_BYTES, (uint32_t)FT_TILE_BYTES, cur);
-			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+			if (leader)
+			{
+				mbar_expect_tx(&bar_full[s], 2u * FT_TILE_BYTES);
+				asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+						:: "r"(ring + (uint32_t)s * FT_STAGE_BYTES + 2u * FT_TILE_BYTES), "l"(src), "r"(2u * FT_TILE_BYTES), "r"(smem_u32(&bar_full[s])) : "memory");
+			}
+			++issued;
 			__syncwarp();
-			if (lane == 0) { mbar_arrive(&bar_full[s]); }
 		}
-		if (!is_pix && part == 0) { s_bias[row] = (row_ok && p.bias != nullptr) ? __ldg(p.bias + f) : 0.0f; }
+		// no copy may be in flight when the CTA leaves: bar_done covers it unless something failed
+		if (!ok)
+		{
+			for (int s = 0; s < FT_STAGES && s < issued; ++s) { mbar_wait_plain(&bar_full[s], (uint32_t)(((issued - 1 - s) / FT_STAGES) & 1), p.spin_limit); }
+		}
 	}
 
 	if (tid == 0) { mbar_wait<64>(&bar_done, 0, s_failed, p.spin_limit); }
@@ -244,52 +301,57 @@ float_conv_tc_kernel(const FtParams p)
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const bool failed = (*s_failed != 0);
-
-	if (!failed && warp != 0)
+	const int used = min(FT_ACCS, kbn);
+	cg::cluster_group cluster = cg::this_cluster();
+	if (p.split > 1)
 	{
-		// warp w reads the TMEM lanes of quarter w % 4; the warps of a quarter share the four 32-filter chunks
+		// every CTA of the tile is through with its stages; the sums of ranks 1.. go to rank 0's
+		cluster.sync();
+		if (rank > 0 && warp >= 1 && warp <= FT_PRODUCER_WARPS)
+		{
+			float * theirs = cluster.map_shared_rank(reinterpret_cast<float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))), 0) + (size_t)(rank - 1) * FT_NF * TC_PIX;
+			const int quarter = warp & 3;
+			const int chunk = (warp - 1) >> 2;
+			float acc[32];
+			tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, acc);
+			#pragma unroll
+			for (int j = 0; j < 32; ++j) { theirs[(chunk * 32 + j) * TC_PIX + quarter * 32 + lane] = acc[j]; }
+		}
+		cluster.sync();
+	}
+
+	if (!failed && rank == 0 && warp >= 1 && warp <= FT_PRODUCER_WARPS)
+	{
+		// warp w reads the TMEM lanes of quarter w % 4 and one of the four 32-filter chunks
 		const int quarter = warp & 3;
-		const int share = (warp - 1) >> 2;
-		constexpr int SHARES = FT_PRODUCER_WARPS / 4;
+		const int chunk = (warp - 1) >> 2;
 		const int g = g0 + quarter * 32 + lane;
 		const bool col_ok = g < p.total;
 		const int img = col_ok ? g / p.HW : 0;
 		const int pix = col_ok ? g - img * p.HW : 0;
-		float * out_pix = p.out + ((size_t)img * p.N + f0) * p.HW + pix;
+		float * out_pix = p.out + ((size_t)img * p.N + f0 + chunk * 32) * p.HW + pix;
 		const float slope = p.leaky ? 0.1f : 1.0f;
-		#pragma unroll 1
-		for (int chunk = share; chunk < FT_NF / 32; chunk += SHARES)
+		float acc[32];
+		tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, acc);
+		const float * sums = reinterpret_cast<const float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))) + (size_t)chunk * 32 * TC_PIX + quarter * 32 + lane;
+		for (int r = 1; r < p.split; ++r, sums += FT_NF * TC_PIX)
 		{
-			// the partial sums of the accumulators that were used, added in fp32
-			float acc[32];
-			const int used = min(FT_ACCS, p.kblocks);
-			#pragma unroll 1
-			for (int a = 0; a < used; ++a)
-			{
-				uint32_t d[32];
-				tmem_load<32>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * FT_NF + chunk * 32), d);
-				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-				#pragma unroll
-				for (int j = 0; j < 32; ++j) { acc[j] = (a == 0) ? __uint_as_float(d[j]) : __fadd_rn(acc[j], __uint_as_float(d[j])); }
-			}
-			if (!col_ok) { continue; }
 			#pragma unroll
-			for (int j = 0; j < 32; ++j)
+			for (int j = 0; j < 32; ++j) { acc[j] = __fadd_rn(acc[j], sums[j * TC_PIX]); }
+		}
+		int e = (p.yolo_entries > 0) ? (f0 + chunk * 32) % p.yolo_entries : 0;
+		#pragma unroll
+		for (int j = 0; j < 32; ++j)
+		{
+			float v = __fadd_rn(acc[j], s_bias[chunk * 32 + j]);
+			v = fmaxf(v, __fmul_rn(v, slope));
+			if (p.yolo_entries > 0)
 			{
-				const int fl = chunk * 32 + j;
-				if (f0 + fl < p.N)
-				{
-					float v = __fadd_rn(acc[j], s_bias[fl]);
-					v = fmaxf(v, __fmul_rn(v, slope));
-					if (p.yolo_entries > 0)
-					{
-						// logistic on every entry of an anchor but its width and height (head_activate.cu)
-						const int e = (f0 + fl) % p.yolo_entries;
-						if (e != 2 && e != 3) { v = 1.0f / (1.0f + expf(-v)); }
-					}
-					out_pix[(size_t)fl * p.HW] = v;
-				}
+				// logistic on every entry of an anchor but its width and height (head_activate.cu)
+				if (e != 2 && e != 3) { v = 1.0f / (1.0f + expf(-v)); }
+				if (++e == p.yolo_entries) { e = 0; }
 			}
+			if (col_ok && f0 + chunk * 32 + j < p.N) { out_pix[(size_t)j * p.HW] = v; }
 		}
 	}
 	else if (failed && tid == 0)
@@ -305,19 +367,40 @@ float_conv_tc_kernel(const FtParams p)
 	}
 }
 
-}  // namespace xnor
+// Darknet's [n][c][taps] -> the swizzled hi and lo tiles of every K block (tap, 32 channels)
+__global__ void float_conv_tc_weights_kernel(const float * __restrict__ w, float * __restrict__ out, int n, int C, int taps, int cblocks)
+{
+	const int kb = blockIdx.x, tile_f = blockIdx.y;
+	const int tap = kb / cblocks, c0 = (kb - tap * cblocks) * 32;
+	float * dst = out + ((size_t)tile_f * gridDim.x + kb) * (2 * FT_TILE_BYTES / 4);
+	for (int i = threadIdx.x; i < 128 * 32; i += blockDim.x)
+	{
+		const int row = i >> 5, k = i & 31;
+		const int f = tile_f * FT_NF + row, c = c0 + k;
+		const float v = (f < n && c < C) ? w[((size_t)f * C + c) * taps + tap] : 0.0f;
+		const float hi = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
+		const int at = row * 32 + (((k >> 2) ^ (row & 7)) << 2) + (k & 3);
+		dst[at] = hi;
+		dst[FT_TILE_BYTES / 4 + at] = __fsub_rn(v, hi);
+	}
+}
 
-using namespace xnor;
+// 1x1 / pad 0, or 3x3 / pad 1 over whole K blocks; stride 1
+static bool ft_shape_ok(const xnor_b200_conv_desc * d)
+{
+	return d->stride == 1 && ((d->size == 1 && d->pad == 0) || (d->size == 3 && d->pad == 1 && d->c % 32 == 0));
+}
 
-extern "C" int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
-		const float * biases, float * output, int yolo_entries, void * stream)
+template <bool RAW>
+static int launch_float_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights, const float * biases, float * output,
+		int yolo_entries, cudaStream_t stream)
 {
 	if (desc == nullptr || input == nullptr || weights == nullptr || output == nullptr) { return XNOR_B200_ERR_NULL; }
 	int rc = validate_desc(desc);
 	if (rc != XNOR_B200_OK) { return rc; }
-	const bool one = (desc->size == 1 && desc->pad == 0), three = (desc->size == 3 && desc->pad == 1 && desc->c % 32 == 0);
-	if (desc->stride != 1 || !(one || three)) { return XNOR_B200_ERR_INVALID; }
+	if (!ft_shape_ok(desc)) { return XNOR_B200_ERR_INVALID; }
 	if (yolo_entries < 0 || (yolo_entries > 0 && (yolo_entries < 5 || desc->n % yolo_entries != 0))) { return XNOR_B200_ERR_INVALID; }
+	if (!RAW && ((uintptr_t)weights & 15u) != 0) { return XNOR_B200_ERR_ALIGNMENT; }
 	const long long total = (long long)desc->batch * desc->h * desc->w;
 	if (total > 0x7fffffffLL - TC_PIX) { return XNOR_B200_ERR_TOO_LARGE; }
 	FtParams p;
@@ -330,23 +413,68 @@ extern "C" int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const f
 	p.yolo_entries = yolo_entries;
 	p.leaky = (desc->activation == XNOR_B200_LEAKY) ? 1 : 0;
 	p.tiles_f = (desc->n + FT_NF - 1) / FT_NF;
-	p.w_vec = (desc->c % 4 == 0 && (((uintptr_t)weights) & 15u) == 0) ? 1 : 0;
 	TcParams tp = TcParams();
 	rc = tc_fill_launch_fields(tp);
 	if (rc != XNOR_B200_OK) { return rc; }
 	p.status = tp.status;
 	p.spin_limit = tp.spin_limit;
-	const long long grid = (long long)p.tiles_f * ((total + TC_PIX - 1) / TC_PIX);
-	if (grid > 0x7fffffffLL) { return XNOR_B200_ERR_TOO_LARGE; }
-	rc = ensure_dynamic_smem((const void *)float_conv_tc_kernel, FT_SMEM_BYTES);
+	const long long tiles = (long long)p.tiles_f * ((total + TC_PIX - 1) / TC_PIX);
+	if (tiles * FT_MAX_SPLIT > 0x7fffffffLL) { return XNOR_B200_ERR_TOO_LARGE; }
+	// as many CTAs per tile as leave the grid one wave and each of them a few K blocks (about 3 us go into joining the sums)
+	p.split = 1;
+	for (int s = 2; s <= FT_MAX_SPLIT; ++s) { if (tiles * s <= sm_count() && p.kblocks >= 4 * s) { p.split = s; } }
+	rc = ensure_dynamic_smem((const void *)float_conv_tc_kernel<RAW>, FT_SMEM_BYTES);
 	if (rc != XNOR_B200_OK) { return rc; }
-	float_conv_tc_kernel<<<(unsigned)grid, FT_THREADS, FT_SMEM_BYTES, (cudaStream_t)stream>>>(p);
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3((unsigned)(tiles * p.split), 1, 1);
+	cfg.blockDim = dim3(FT_THREADS, 1, 1);
+	cfg.dynamicSmemBytes = FT_SMEM_BYTES;
+	cfg.stream = stream;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeClusterDimension;
+	attr[0].val.clusterDim.x = (unsigned)p.split;
+	attr[0].val.clusterDim.y = 1;
+	attr[0].val.clusterDim.z = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, float_conv_tc_kernel<RAW>, p);
+	return (e == cudaSuccess) ? check_launch() : cuda_fail(e);
+}
+
+}  // namespace xnor
+
+using namespace xnor;
+
+extern "C" size_t xnor_b200_float_conv_tc_weights_bytes(const xnor_b200_conv_desc * desc)
+{
+	if (desc == nullptr || validate_desc(desc) != XNOR_B200_OK || !ft_shape_ok(desc)) { return 0; }
+	const size_t tiles_f = (size_t)(desc->n + FT_NF - 1) / FT_NF;
+	return tiles_f * (size_t)((desc->c + 31) / 32 * desc->size * desc->size) * 2 * FT_TILE_BYTES;
+}
+
+extern "C" int xnor_b200_float_conv_tc_prepare(const xnor_b200_conv_desc * desc, const float * weights, float * tc_weights, void * stream)
+{
+	if (desc == nullptr || weights == nullptr || tc_weights == nullptr) { return XNOR_B200_ERR_NULL; }
+	const int rc = validate_desc(desc);
+	if (rc != XNOR_B200_OK) { return rc; }
+	if (!ft_shape_ok(desc)) { return XNOR_B200_ERR_INVALID; }
+	if (((uintptr_t)tc_weights & 15u) != 0) { return XNOR_B200_ERR_ALIGNMENT; }
+	const int taps = desc->size * desc->size, cblocks = (desc->c + 31) / 32, tiles_f = (desc->n + FT_NF - 1) / FT_NF;
+	if (tiles_f > 65535) { return XNOR_B200_ERR_TOO_LARGE; }
+	float_conv_tc_weights_kernel<<<dim3((unsigned)(taps * cblocks), (unsigned)tiles_f, 1), 256, 0, (cudaStream_t)stream>>>(
+			weights, tc_weights, desc->n, desc->c, taps, cblocks);
 	return check_launch();
+}
+
+extern "C" int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * tc_weights,
+		const float * biases, float * output, int yolo_entries, void * stream)
+{
+	return launch_float_tc<false>(desc, input, tc_weights, biases, output, yolo_entries, (cudaStream_t)stream);
 }
 
 extern "C" int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
 		const float * biases, float * output, void * stream)
 {
 	if (desc != nullptr && desc->size != 1) { return XNOR_B200_ERR_INVALID; }
-	return xnor_b200_float_conv_tc(desc, input, weights, biases, output, 0, stream);
+	return launch_float_tc<true>(desc, input, weights, biases, output, 0, (cudaStream_t)stream);
 }

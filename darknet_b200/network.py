@@ -87,7 +87,7 @@ class Layer:
     pool_desc: Optional[capi.PoolDesc] = None
     # xnor conv whose only reader is another xnor conv (directly or through a maxpool): hands over sign bits
     weights_blocked_gpu: Optional[torch.Tensor] = None     # float conv on a small map: weights re-blocked at load time
-    weights_tap_major_gpu: Optional[torch.Tensor] = None   # float conv that runs as a GEMM on the tensor cores: weights [n][taps][c]
+    weights_tc_gpu: Optional[torch.Tensor] = None          # float conv that runs as a GEMM on the tensor cores: its filters, laid out for it
     branch_start: bool = False       # first / last layer of a head branch that runs on the side stream
     branch_end: bool = False
     yolo_entries: int = 0            # float conv in front of a [yolo] layer: the head's logistic step runs in the conv epilogue
@@ -130,7 +130,7 @@ class Network:
     sum_signs_min_batch: int = 4           # from this batch on the sign of a fused shortcut sum is handed to the next xnor layer (the call runs on the tensor-core kernel; measured on darknet53: +5 % at batch 4, -7 % at batch 2, -26 % at batch 1)
     sum_sign_links: int = 0
     fuse_first_conv: bool = True
-    float_map_max_pixels: int = 1024       # batch*out_h*out_w up to which float convs use the cluster split-K kernel (measured: it wins at 676 pixels, loses to cuDNN/cuBLAS at 1352)
+    float_map_max_pixels: int = 1024       # batch*out_h*out_w beyond which no float convolution takes the small-map kernels (tuning runs; see _map_conv_wins)
     sign_links: int = 0
     heads_direct_to_host: bool = True      # with heads_host: a fused head convolution stores into the pinned host tensor itself
     side_branches: bool = True             # a head branch that nothing later reads runs on a second stream
@@ -243,10 +243,10 @@ def load_weights(net: Network, path: str) -> None:
         fh.read(8 if major * 10 + minor >= 2 else 4)
 
         def take(count: int) -> np.ndarray:
-            buf = fh.read(4 * count)
-            if len(buf) != 4 * count:
+            values = np.fromfile(fh, "<f4", count)
+            if values.size != count:
                 raise ValueError("weights file ended early")
-            return np.frombuffer(buf, "<f4").astype(np.float32)
+            return values.astype(np.float32, copy=False)
 
         for l in net.layers:
             if l.type != "convolutional":
@@ -348,7 +348,8 @@ def fuse_conv_batchnorm(net: Network) -> None:
             std = np.sqrt(l.rolling_variance.astype(np.float64) + 0.00001)
             l.biases = (l.biases.astype(np.float64) - l.scales.astype(np.float64) * l.rolling_mean.astype(np.float64) / std).astype(np.float32)
             pre = l.scales.astype(np.float64) / std
-            l.weights = (l.weights.astype(np.float64) * pre[:, None, None, None]).astype(np.float32)
+            # double products rounded once, in one pass (numpy converts blockwise; whole double copies cost three)
+            l.weights = np.multiply(l.weights, pre[:, None, None, None], out=np.empty_like(l.weights), dtype=np.float64, casting="same_kind")
             l.batch_normalize = 0
 
 
@@ -678,6 +679,17 @@ def _map_conv_desc(net: Network, l: Layer) -> capi.ConvDesc:
     return capi.ConvDesc(net.batch, l.c, l.h, l.w, l.n, l.size, l.stride, l.pad, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
 
 
+def _map_conv_wins(net: Network, l: Layer) -> bool:
+    """Whether a float convolution runs on the small-map kernel rather than as a tensor-core GEMM.  Measured on B200 (us, map / GEMM):
+    3x3 256 -> 512: 21 / 25 at 169 pixels, 31 / 25 at 338, 101 / 30 at 1352; 1x1 512 -> 255: 7 / 15 at 169, 16 / 15 at 627;
+    1x1 256 -> 255: 9 / 13 at 676, 22 / 13 at 2508; 1x1 1024 -> 512: 27 / 18 at 196.  The map kernels work in runs of 32 pixels of
+    one image (1x1 512 -> 1000 on 64 maps of one pixel: 116 / 21)."""
+    pixels = net.batch * (-(-l.out_h * l.out_w // 32) * 32)
+    if net.batch * l.out_h * l.out_w > net.float_map_max_pixels:
+        return False
+    return pixels <= 256 if l.size == 3 else (l.c <= 512 and pixels <= 704)
+
+
 def prepare_float_map_convs(net: Network) -> None:
     """Re-blocks the weights of the float convolutions that the small-map kernel takes (many channels, stride 1,
     3x3/pad 1 or 1x1, few output pixels in the whole batch), and lays out those of the others for the tensor-core GEMM.
@@ -690,11 +702,13 @@ def prepare_float_map_convs(net: Network) -> None:
             continue
         desc = _map_conv_desc(net, l)
         nbytes = capi.lib().xnor_b200_float_conv_map_weights_bytes(C.byref(desc))
-        if nbytes == 0 or net.batch * l.out_h * l.out_w > net.float_map_max_pixels:
+        if nbytes == 0 or not _map_conv_wins(net, l):
             # many pixels: one GEMM over the whole batch on the tensor cores, K = (tap, channel)
-            if l.stride == 1 and ((l.size == 1 and l.pad == 0) or (l.size == 3 and l.pad == 1 and l.c % 32 == 0)):
-                w = l.weights_gpu
-                l.weights_tap_major_gpu = w if l.size == 1 else w.reshape(l.n, l.c, 9).permute(0, 2, 1).contiguous()
+            nbytes = capi.lib().xnor_b200_float_conv_tc_weights_bytes(C.byref(desc))
+            if nbytes:
+                l.weights_tc_gpu = torch.empty(nbytes // 4, dtype=torch.float32, device=l.weights_gpu.device)
+                capi.check(capi.lib().xnor_b200_float_conv_tc_prepare(C.byref(desc), l.weights_gpu.data_ptr(), l.weights_tc_gpu.data_ptr(),
+                                                                     torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_tc_prepare")
             continue
         nxt = net.layers[l.index + 1] if l.index + 1 < len(net.layers) else None
         if (nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
@@ -711,7 +725,7 @@ def _float_conv_tc(l: Layer, x: torch.Tensor) -> torch.Tensor:
     import ctypes as C
     desc = capi.ConvDesc(x.shape[0], l.c, l.h, l.w, l.n, l.size, 1, l.pad, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
     out = torch.empty(x.shape[0], l.n, l.out_h, l.out_w, dtype=torch.float32, device=x.device)
-    capi.check(capi.lib().xnor_b200_float_conv_tc(C.byref(desc), x.data_ptr(), l.weights_tap_major_gpu.data_ptr(), l.biases_gpu.data_ptr(),
+    capi.check(capi.lib().xnor_b200_float_conv_tc(C.byref(desc), x.data_ptr(), l.weights_tc_gpu.data_ptr(), l.biases_gpu.data_ptr(),
                                                  out.data_ptr(), 0, torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_tc")
     return out
 
@@ -804,7 +818,7 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
     A network that was lowered to native operations (network_plan) runs as one call; the loop below runs the others, and every
     network while xnor_b200_set_tuning pins kernels of the packed-operand route."""
     if net.plan is not None and net.plan.takes(x):
-        return net.plan.run(x, heads_host)
+        return net.plan.run(net, x, heads_host)
     heads: List[torch.Tensor] = []
     cur = x
     side_ctx = None
@@ -854,7 +868,7 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
                 # a head whose yolo activation runs in this kernel can be written straight into the caller's pinned host tensor
                 direct = heads_host is not None and l.yolo_entries > 0 and net.heads_direct_to_host
                 cur = _float_conv_map(net, l, cur.contiguous(), heads_host[len(heads)] if direct else None)
-            elif l.weights_tap_major_gpu is not None:
+            elif l.weights_tc_gpu is not None:
                 # many pixels: one GEMM over the whole batch on the tensor cores (three tf32 products per operand pair), bias and
                 # activation in its epilogue
                 cur = _float_conv_tc(l, cur.contiguous())
@@ -1069,7 +1083,7 @@ def own_launches_per_forward(net: Network) -> int:
                 n += 1 if (l.packed_input or from_planes) else 2
             elif (l.c == 3 and l.size == 3 and l.stride == 1 and l.pad == 1) or l.c * l.size * l.size <= 128 or l.weights_blocked_gpu is not None:
                 n += 1
-            elif l.weights_tap_major_gpu is not None:
+            elif l.weights_tc_gpu is not None:
                 n += 1                                    # tensor-core float convolution
         elif (l.type == "yolo" and not l.yolo_done) or l.type in ("region", "avgpool", "softmax"):
             n += 1

@@ -5,7 +5,7 @@ sign word per pixel), written by the layer that makes it and read through whatev
 between (xnor_b200_conv_words).  fp32 tensors exist where a float layer or a fused [shortcut] reads them.
 
     plan = build(net)                 # once, at the end of calculate_binary_weights; None: a layer that has no native operation
-    heads = plan.run(x, heads_host)   # forward_network_gpu
+    heads = plan.run(net, x, heads_host)   # forward_network_gpu
 """
 from __future__ import annotations
 
@@ -24,7 +24,7 @@ class Unsupported(Exception):
 
 class Plan:
     def __init__(self, net) -> None:
-        self.net = net
+        self.net = net                             # while it is built: a plan that kept it would be a cycle, and its memory wait for the collector
         self.shape = (net.batch, net.c, net.h, net.w)
         self.ops: List[capi.Op] = []
         self.keep: List = []                       # tensors the operations point at
@@ -48,12 +48,13 @@ class Plan:
                 e.record(self.net.side_stream)     # a torch event exists from its first record on
             self.side = self.net.side_stream.cuda_stream
             self.fork, self.join = (e.cuda_event for e in self.events)
+        self.net = None
 
     def takes(self, x: torch.Tensor) -> bool:
         return (x.is_cuda and x.dtype == torch.float32 and x.shape == self.shape and x.is_contiguous() and not capi.packed_route_pinned)
 
-    def run(self, x: torch.Tensor, heads_host: Optional[List[torch.Tensor]]) -> List[torch.Tensor]:
-        direct = heads_host is not None and self.net.heads_direct_to_host
+    def run(self, net, x: torch.Tensor, heads_host: Optional[List[torch.Tensor]]) -> List[torch.Tensor]:
+        direct = heads_host is not None and net.heads_direct_to_host
         heads = [heads_host[i] if direct and self.head_direct[i] else torch.empty(s, dtype=torch.float32, device=x.device)
                  for i, s in enumerate(self.head_shapes)]
         pointers = self.heads_type(*[h.data_ptr() for h in heads])
@@ -254,8 +255,8 @@ def _float_conv(plan: Plan, k: int, src: int, fp32_read: set) -> None:
         op.kind, op.weights = capi.OP_FLOAT_MAP, l.weights_blocked_gpu.data_ptr()
         if not l.yolo_entries:
             head = False
-    elif l.weights_tap_major_gpu is not None:
-        op.kind, op.weights = capi.OP_FLOAT_TC, l.weights_tap_major_gpu.data_ptr()
+    elif l.weights_tc_gpu is not None:
+        op.kind, op.weights = capi.OP_FLOAT_TC, l.weights_tc_gpu.data_ptr()
     else:
         raise Unsupported("a float convolution of another shape")
     if head:

@@ -389,9 +389,12 @@ XNOR_B200_API int xnor_b200_float_conv_map(const xnor_b200_conv_desc * desc, con
  * convolution to fp32 rounding (a few 1e-7 relative), not with cuBLAS bit for bit. */
 XNOR_B200_API int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
 		const float * biases, float * output, void * stream);
-/* The same kernel for 1x1 / pad 0 and 3x3 / pad 1 (c % 32 == 0) stride-1 layers, weights [n][size * size][c] (Darknet's [n][c][taps]
- * with taps and channels exchanged; the same thing for 1x1); yolo_entries as below. */
-XNOR_B200_API int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,
+/* The same kernel for 1x1 / pad 0 and 3x3 / pad 1 (c % 32 == 0) stride-1 layers over filters that were split and laid out once at load
+ * time: _weights_bytes of that copy (0: a shape it does not take), _prepare fills it (16-byte aligned) from Darknet's [n][c*size*size]
+ * weights, batch-norm folded.  yolo_entries as below. */
+XNOR_B200_API size_t xnor_b200_float_conv_tc_weights_bytes(const xnor_b200_conv_desc * desc);
+XNOR_B200_API int xnor_b200_float_conv_tc_prepare(const xnor_b200_conv_desc * desc, const float * weights, float * tc_weights, void * stream);
+XNOR_B200_API int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * tc_weights,
 		const float * biases, float * output, int yolo_entries, void * stream);
 /* Same, for the convolution right in front of a [yolo] layer: yolo_entries = 4 + 1 + classes (n must be a multiple of
  * it) also applies that layer's activation step (xnor_b200_yolo_activate below) to the result; 0 = plain call. */
