@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 import torch.nn.functional as F  # noqa: E402
 
-from darknet_b200 import capi, synth  # noqa: E402
+import synth  # noqa: E402
+from darknet_b200 import capi  # noqa: E402
 
 
 @pytest.mark.parametrize("batch,c,h,w,n,size,leaky,entries", [
