@@ -47,7 +47,6 @@ constexpr int XC_EXP_THREADS = XC_EXP_WARPS * 32;
 constexpr int XC_ITEMS = 8;                   // words of a stage per expander thread
 constexpr int XC_MAX_STAGES = 4;
 constexpr int XC_RAW_STAGES = 3;              // stages whose bits are on their way
-constexpr int XC_TABLES = XC_RAW_STAGES + 1;  // window tables: one per unit that can be under way
 constexpr int XC_MAX_ACC = 14;
 constexpr long long XC_STREAM_BYTES = 32 << 20;   // fp32 tensors above this size do not expect their reader to find them in the L2
 constexpr int XC_TMEM_COLS = 512;
@@ -84,8 +83,9 @@ struct XcParams
 	uint32_t * sc_signs;
 	int M, K;                // filters; channels * taps: the largest magnitude an accumulator can have
 	int leaky;
+	float minus_zero;        // -0.0f
 	int stream_values;       // the fp32 tensors are too large to be found in the L2 again
-	int OH, OW, n_pix;       // output map
+	int batch, OH, OW, n_pix;   // images, output map
 	int out_front, out_block_words;   // of sign words on the output's grid
 	int stride, taps;
 	int nb, G, stages_k;     // channel blocks, blocks per stage, stages per unit
@@ -219,6 +219,30 @@ __device__ __forceinline__ void st_policy(float * at, float v, uint64_t policy)
 	asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" :: "l"(at), "f"(v), "l"(policy));
 }
 
+// Two fp32 operations in one instruction, each rounded as the plain one is.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+	uint64_t v;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+	return v;
+}
+
+__device__ __forceinline__ void unpack2(uint64_t v, float & lo, float & hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+	uint64_t v;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+	return v;
+}
+
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+	uint64_t v;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+	return v;
+}
+
 // The run of a source's words (from its block start, 16-byte aligned) that holds the window of unit u, and where in it the
 // window's first position lies (linear sources).
 struct XcRun
@@ -285,10 +309,9 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	const int lane = tid & 31;
 	const uint32_t limit = p.spin_limit;
 	const uint32_t a_base = smem_u32(xc_smem);
-	// ring of pixel stages, then the filters (all of them, or a ring beside the pixel stages), the raw ring, the window tables
+	// ring of pixel stages, then the filters (all of them, or a ring beside the pixel stages), the raw ring
 	const uint32_t b_base = a_base + (uint32_t)(p.ring * p.a_stage_bytes);
 	const uint32_t raw_base = b_base + (uint32_t)((STREAM ? p.ring : p.stages_k) * p.b_stage_bytes);
-	int * s_table = reinterpret_cast<int *>(xc_smem + (raw_base - a_base) + (size_t)XC_RAW_STAGES * p.raw_stage_bytes);
 	const int fg = blockIdx.x % p.fgroups;
 	const int f0 = fg * NF;
 	const int unit0 = blockIdx.x / p.fgroups;
@@ -303,7 +326,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	{
 		if (lane < XC_RAW_STAGES)
 		{
-			mbar_init(&raw_full[lane], 2);                        // the copies (with their bytes), and the window table
+			mbar_init(&raw_full[lane], 1);                        // the copies (with their bytes)
 			mbar_init(&raw_empty[lane], XC_EXP_WARPS);
 		}
 		if (lane < XC_MAX_STAGES)
@@ -424,7 +447,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const int fb = chunk * 32;
 		constexpr int TILE_STEP = 4 / CHUNKS;
 		const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
-		const int pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos, pt = p.pt;
+		const int pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos, pt = p.pt, batch = p.batch;
 		const size_t n_pix = (size_t)p.n_pix;
 		const int left = p.M - f0 - fb;                          // filters of this chunk that exist
 		const size_t img_elems = (size_t)p.M * n_pix;
@@ -438,10 +461,15 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			const int x = r - y * pitch;
 			it.ok = (pos < total_pos && y < OH && x < OW && left > 0);
 			it.pos = pos;
-			it.elem = (MODE == 0) ? 0 : (size_t)img * img_elems + (size_t)(f0 + fb) * n_pix + (size_t)(y * OW + x);
+			// off the map: the address of a pixel beside it, so that loads need no condition
+			it.elem = (MODE == 0) ? 0 : (size_t)min(img, batch - 1) * img_elems + (size_t)(f0 + fb) * n_pix + (size_t)(min(y, OH - 1) * OW + min(x, OW - 1));
 			return it;
 		};
 		const float slope = p.leaky ? 0.1f : 1.0f;               // leaky(v) = max(v, 0.1 v), linear(v) = max(v, v)
+		const uint64_t slope2 = pack2(slope, slope);
+		// a * b is a * b + -0 with a zero that the compiler does not know: it joins a packed product and the sum behind it into one rounding
+		const uint64_t minus_zero2 = pack2(p.minus_zero, p.minus_zero);
+		const uint32_t step = (uint32_t)p.n_pix * 4u;            // bytes from one filter's plane to the next
 		uint32_t * words = (MODE == 2) ? p.sc_signs : p.signs;
 		if (words != nullptr) { words += (size_t)((f0 + fb) >> 5) * p.out_block_words + p.out_front; }
 		float * const out = p.out;
@@ -462,13 +490,19 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		{
 			if constexpr (MODE == 2)
 			{
-				const float * at = sc_in + it.elem + (size_t)h * n_pix;
-				#pragma unroll
-				for (int i = 0; i < 8; ++i)
+				// No condition per value: a load behind one was waited for on the spot, four times the latency per 32 values.  Filters
+				// that do not exist read the last one that does.
+				const char * at = reinterpret_cast<const char *>(sc_in + it.elem);
+				if (left >= 32)
 				{
-					sc[h + i] = 0.0f;
-					if (it.ok && h + i < left) { sc[h + i] = ld_policy(at, policy); }
-					at += n_pix;
+					at += (size_t)step * (uint32_t)h;
+					#pragma unroll
+					for (int i = 0; i < 8; ++i) { sc[h + i] = ld_policy(reinterpret_cast<const float *>(at + (size_t)step * (uint32_t)i), policy); }
+				}
+				else
+				{
+					#pragma unroll
+					for (int i = 0; i < 8; ++i) { sc[h + i] = ld_policy(reinterpret_cast<const float *>(at + (size_t)step * (uint32_t)min(h + i, left - 1)), policy); }
 				}
 			}
 		};
@@ -476,8 +510,11 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		if (tile < my_tiles)
 		{
 			it = locate(pos_of());
-			#pragma unroll
-			for (int h = 0; h < 32; h += 8) { load8(it, h); }
+			if (left > 0)
+			{
+				#pragma unroll
+				for (int h = 0; h < 32; h += 8) { load8(it, h); }
+			}
 		}
 		while (tile < my_tiles)
 		{
@@ -515,9 +552,11 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			}
 			else
 			{
-				if (tile < my_tiles) { next = locate(pos_of()); }
-				float * dst = ((MODE == 2) ? sc_out : out) + it.elem;
-				float * own = (MODE == 2 && out != nullptr) ? out + it.elem : nullptr;
+				const bool more = (tile < my_tiles && left > 0);
+				if (more) { next = locate(pos_of()); }
+				char * const dst = reinterpret_cast<char *>(((MODE == 2) ? sc_out : out) + it.elem);
+				char * const own = reinterpret_cast<char *>((MODE == 2 && out != nullptr) ? out + it.elem : nullptr);
+				const bool store = it.ok && (MODE == 1 || sc_out != nullptr);       // else only the sum's signs are wanted
 				#pragma unroll
 				for (int h = 0; h < 32; h += 16)
 				{
@@ -533,46 +572,57 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					#pragma unroll
 					for (int u0 = 0; u0 < 16; u0 += 8)
 					{
+						const int j0 = h + u0;
+						uint64_t w[4];                           // eight values, in pairs
+						#pragma unroll
+						for (int i = 0; i < 4; i += 2)
+						{
+							const ulonglong2 m = *reinterpret_cast<const ulonglong2 *>(s_mean + fb + j0 + 2 * i);
+							const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(s_bias + fb + j0 + 2 * i);
+							const int at = u0 + 2 * i;
+							w[i] = add2(fma2(pack2(__uint_as_float(d[at]), __uint_as_float(d[at + 1])), m.x, minus_zero2), b.x);
+							w[i + 1] = add2(fma2(pack2(__uint_as_float(d[at + 2]), __uint_as_float(d[at + 3])), m.y, minus_zero2), b.y);
+						}
 						float v[8];
 						#pragma unroll
-						for (int i = 0; i < 8; i += 4)
+						for (int i = 0; i < 4; ++i)
 						{
-							const float4 m4 = *reinterpret_cast<const float4 *>(s_mean + fb + h + u0 + i);
-							const float4 b4 = *reinterpret_cast<const float4 *>(s_bias + fb + h + u0 + i);
-							v[i + 0] = __fadd_rn(__fmul_rn(__uint_as_float(d[u0 + i + 0]), m4.x), b4.x);
-							v[i + 1] = __fadd_rn(__fmul_rn(__uint_as_float(d[u0 + i + 1]), m4.y), b4.y);
-							v[i + 2] = __fadd_rn(__fmul_rn(__uint_as_float(d[u0 + i + 2]), m4.z), b4.z);
-							v[i + 3] = __fadd_rn(__fmul_rn(__uint_as_float(d[u0 + i + 3]), m4.w), b4.w);
+							float lo, hi;
+							unpack2(fma2(w[i], slope2, minus_zero2), lo, hi);
+							unpack2(w[i], v[2 * i], v[2 * i + 1]);
+							v[2 * i] = fmaxf(v[2 * i], lo);
+							v[2 * i + 1] = fmaxf(v[2 * i + 1], hi);
 						}
-						#pragma unroll
-						for (int i = 0; i < 8; ++i) { v[i] = fmaxf(v[i], __fmul_rn(v[i], slope)); }
 						if (MODE == 2)
 						{
 							if (own != nullptr && it.ok)
 							{
 								#pragma unroll
-								for (int i = 0; i < 8; ++i) { if (h + u0 + i < left) { st_policy(own + (size_t)(h + u0 + i) * n_pix, v[i], policy); } }
+								for (int i = 0; i < 8; ++i) { if (j0 + i < left) { st_policy(reinterpret_cast<float *>(own + (size_t)step * (uint32_t)(j0 + i)), v[i], policy); } }
 							}
 							#pragma unroll
-							for (int i = 0; i < 8; ++i) { v[i] = __fadd_rn(sc[MODE == 2 ? h + u0 + i : 0], v[i]); }
-							load8(next, h + u0);
+							for (int i = 0; i < 8; ++i) { v[i] = __fadd_rn(sc[MODE == 2 ? j0 + i : 0], v[i]); }
+							if (more) { load8(next, j0); }
 						}
-						if (MODE == 2 && sc_out == nullptr) {}                       // only the sum's signs are wanted
-						else if (it.ok && left >= 32)
+						if (store && left >= 32)
 						{
 							#pragma unroll
-							for (int i = 0; i < 8; ++i) { st_policy(dst, v[i], policy); dst += n_pix; }
+							for (int i = 0; i < 8; ++i) { st_policy(reinterpret_cast<float *>(dst + (size_t)step * (uint32_t)(j0 + i)), v[i], policy); }
 						}
-						else if (it.ok)
+						else if (store)
 						{
 							#pragma unroll
-							for (int i = 0; i < 8; ++i) { if (h + u0 + i < left) { st_policy(dst + (size_t)(h + u0 + i) * n_pix, v[i], policy); } }
+							for (int i = 0; i < 8; ++i) { if (j0 + i < left) { st_policy(reinterpret_cast<float *>(dst + (size_t)step * (uint32_t)(j0 + i)), v[i], policy); } }
 						}
-						// v > 0 is the sign bit of 0 - v (zeros of either sign give +0), shifted in from above
-						#pragma unroll
-						for (int i = 0; i < 8; ++i) { word = __funnelshift_r(word, __float_as_uint(__fsub_rn(0.0f, v[i])) >> 31, 1); }
+						if (words != nullptr)
+						{
+							// v > 0 is the sign bit of 0 - v (zeros of either sign give +0), shifted in from below and turned round at the end
+							#pragma unroll
+							for (int i = 0; i < 8; ++i) { word = __funnelshift_l(__float_as_uint(__fsub_rn(0.0f, v[i])), word, 1); }
+						}
 					}
 				}
+				word = __brev(word);
 			}
 			if (words != nullptr && it.ok) { words[it.pos] = word; }
 			it = next;
@@ -586,7 +636,6 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const int ew = warp - XC_EPI_WARPS;
 		const int et = ew * 32 + lane;
 		const int slots_plane = p.slots_plane, G = p.G, nb = p.nb, stages_k = p.stages_k, ring = p.ring, units = p.units;
-		const int table_len = p.n_src * slots_plane;
 		const int blocks0 = p.src[0].blocks;
 		const int mode = p.src[0].mode;                          // OR4 and SINGLE may meet in one layer (a route); both work as OR4
 		const bool tabled = (mode != XC_LINEAR);
@@ -621,12 +670,33 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		int es = 0, rs = 0;
 		uint32_t es_phase = 1, rs_phase = 0;                     // es_phase: parity of the wait for an emptied stage
 		bool ok = true;
-		int n_unit = 0;
-		for (int u = unit0; u < units && ok; u += unit_step, ++n_unit)
+		for (int u = unit0; u < units && ok; u += unit_step)
 		{
-			const uint32_t table_addr = smem_u32(s_table + (n_unit % XC_TABLES) * table_len);
-			const uint32_t shift0 = tabled ? 0u : (uint32_t)run_of(p, p.src[0], u).shift * 4u;
-			const uint32_t shift1 = (tabled || p.n_src == 1) ? 0u : (uint32_t)run_of(p, p.src[1], u).shift * 4u;
+			const XcRun run0 = run_of(p, p.src[0], u);
+			const XcRun run1 = (p.n_src == 1) ? run0 : run_of(p, p.src[1], u);
+			const uint32_t shift0 = (uint32_t)run0.shift * 4u, shift1 = (uint32_t)run1.shift * 4u;
+			// tabled: where in a raw stage this thread's words of the unit lie (-1: padding)
+			int e[XC_ITEMS];
+			auto find = [&](const XcSource & src, int run_start)
+			{
+				const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
+				const int pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos;
+				const int scale = src.scale, src_pitch = src.pitch, src_rows = src.h + 1, base = src.front - run_start;
+				const int pos0 = u * p.pt * TC_PIX - p.halo;
+				#pragma unroll
+				for (int j = 0; j < XC_ITEMS; ++j)
+				{
+					if (j >= n_items) { break; }
+					const int pos = pos0 + (int)(from[j] & 0xffffu);
+					const int img = fdiv(pos, d_img);
+					const int r = pos - img * (int)d_img.d;
+					const int y = fdiv(r, d_pitch);
+					const int x = r - y * pitch;
+					const int sy = (scale == 2) ? 2 * y : (scale == 1) ? y : y >> 1;
+					const int sx = (scale == 2) ? 2 * x : (scale == 1) ? x : x >> 1;
+					e[j] = (pos >= 0 && pos < total_pos && y < OH && x < OW) ? (base + (img * src_rows + sy) * src_pitch + sx + (int)(from[j] >> 16)) * 4 : -1;
+				}
+			};
 			for (int st = 0; st < stages_k; ++st, ++k)
 			{
 				const int cb0 = st * G;
@@ -659,7 +729,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				}
 				else
 				{
-					const uint32_t tab = table_addr + (second ? (uint32_t)slots_plane * 4u : 0u);
+					if (st == 0 || cb0 == blocks0) { if (second) { find(p.src[1], run1.start); } else { find(p.src[0], run0.start); } }
 					const uint32_t down = second ? down1 : down0;
 					const uint32_t right = (down != 0u) ? 4u : 0u;
 					#pragma unroll
@@ -667,16 +737,13 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					{
 						if (j0 >= n_items) { break; }
 						uint32_t w0[2], w1[2], w2[2], w3[2], keep[2];
-						int e[2];
-						#pragma unroll
-						for (int q = 0; q < 2; ++q) { if (has(j0 + q)) { e[q] = (int)ld_shared_u32(tab + (from[j0 + q] & 0xffffu) * 4u); } }
 						#pragma unroll
 						for (int q = 0; q < 2; ++q)
 						{
 							if (!has(j0 + q)) { continue; }
 							// padding (-1) reads the run's first words and drops them
-							const uint32_t at = raw + ((uint32_t)max(e[q], 0) + (from[j0 + q] >> 16)) * 4u;
-							keep[q] = ~(uint32_t)(e[q] >> 31);
+							const uint32_t at = raw + (uint32_t)max(e[j0 + q], 0);
+							keep[q] = ~(uint32_t)(e[j0 + q] >> 31);
 							w0[q] = ld_shared_u32(at);
 							w1[q] = ld_shared_u32(at + right);
 							w2[q] = ld_shared_u32(at + down);
@@ -755,8 +822,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		int rs = 0;
 		uint32_t rs_phase = 1, k = 0;
 		bool ok = true;
-		int n_unit = 0;
-		for (int u = unit0; u < p.units && ok; u += unit_step, ++n_unit)
+		for (int u = unit0; u < p.units && ok; u += unit_step)
 		{
 			const XcRun run0 = run_of(p, p.src[0], u);
 			const XcRun run1 = (p.n_src > 1) ? run_of(p, p.src[1], u) : run0;
@@ -787,33 +853,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 						bulk_load(dst + (uint32_t)(p.G * p.raw_words * 4), my_filters + (size_t)cb0 * p.taps * 128, (uint32_t)fil_words * 4u, &raw_full[rs]);
 					}
 				}
-				if (st == 0 && p.tabled)
-				{
-					// which word of the run each position of the window is (-1: padding); the copies are on their way meanwhile
-					int * tab = s_table + (n_unit % XC_TABLES) * (p.n_src * p.slots_plane);
-					const int slots_plane = p.slots_plane, pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos;
-					const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
-					const int pos0 = u * p.pt * TC_PIX - p.halo;
-					for (int si = 0; si < p.n_src; ++si, tab += slots_plane)
-					{
-						const int scale = p.src[si].scale, src_pitch = p.src[si].pitch, src_rows = p.src[si].h + 1;
-						const int base = p.src[si].front - (si ? run1.start : run0.start);
-						#pragma unroll 4
-						for (int s = lane; s < slots_plane; s += 32)
-						{
-							const int pos = pos0 + s;
-							const int img = fdiv(pos, d_img);
-							const int r = pos - img * (int)d_img.d;
-							const int y = fdiv(r, d_pitch);
-							const int x = r - y * pitch;
-							const int sy = (scale == 2) ? 2 * y : (scale == 1) ? y : y >> 1;
-							const int sx = (scale == 2) ? 2 * x : (scale == 1) ? x : x >> 1;
-							tab[s] = (pos >= 0 && pos < total_pos && y < OH && x < OW) ? base + (img * src_rows + sy) * src_pitch + sx : -1;
-						}
-					}
-				}
 				__syncwarp();
-				if (lane == 0) { mbar_arrive(&raw_full[rs]); }
 				if (++rs == XC_RAW_STAGES) { rs = 0; rs_phase ^= 1u; }
 			}
 		}
@@ -974,8 +1014,7 @@ static bool plan_sizes(const XcParams & p, int nf, int pt, int stream, XcPlan * 
 	}
 	if (p.tabled && (long long)q.g * q.raw_words > 0xffff) { return false; }
 	q.raw_stage = (q.g * q.raw_words + (stream ? q.kw_full * nf : 0)) * 4;
-	const size_t table = p.tabled ? XC_TABLES * (size_t)p.n_src * q.slots_plane * sizeof(int) : 0;
-	const size_t fixed = (size_t)XC_RAW_STAGES * q.raw_stage + table;
+	const size_t fixed = (size_t)XC_RAW_STAGES * q.raw_stage;
 	for (q.ring = XC_MAX_STAGES; q.ring >= 2; --q.ring)
 	{
 		q.smem = (size_t)q.ring * q.a_stage + (size_t)(stream ? q.ring : q.stages_k) * q.b_stage + fixed;
@@ -1012,6 +1051,8 @@ static void fill_params(const xnor_b200_conv_desc & d, XcParams & p, int pitch)
 {
 	p.OH = conv_out_dim(d.h, d.size, d.stride, d.pad);
 	p.OW = conv_out_dim(d.w, d.size, d.stride, d.pad);
+	p.minus_zero = -0.0f;
+	p.batch = d.batch;
 	p.n_pix = p.OH * p.OW;
 	p.M = d.n; p.K = d.c * d.size * d.size;
 	p.stride = d.stride; p.taps = d.size * d.size;
