@@ -47,6 +47,7 @@ constexpr int XC_EXP_THREADS = XC_EXP_WARPS * 32;
 constexpr int XC_ITEMS = 8;                   // words of a stage per expander thread
 constexpr int XC_MAX_STAGES = 4;
 constexpr int XC_RAW_STAGES = 3;              // stages whose bits are on their way
+constexpr int XC_TABLES = XC_RAW_STAGES + 1;  // window tables: one per unit that can be under way
 constexpr int XC_MAX_ACC = 14;
 constexpr long long XC_STREAM_BYTES = 32 << 20;   // fp32 tensors above this size do not expect their reader to find them in the L2
 constexpr int XC_TMEM_COLS = 512;
@@ -309,9 +310,10 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	const int lane = tid & 31;
 	const uint32_t limit = p.spin_limit;
 	const uint32_t a_base = smem_u32(xc_smem);
-	// ring of pixel stages, then the filters (all of them, or a ring beside the pixel stages), the raw ring
+	// ring of pixel stages, then the filters (all of them, or a ring beside the pixel stages), the raw ring, the window tables
 	const uint32_t b_base = a_base + (uint32_t)(p.ring * p.a_stage_bytes);
 	const uint32_t raw_base = b_base + (uint32_t)((STREAM ? p.ring : p.stages_k) * p.b_stage_bytes);
+	int * s_table = reinterpret_cast<int *>(xc_smem + (raw_base - a_base) + (size_t)XC_RAW_STAGES * p.raw_stage_bytes);
 	const int fg = blockIdx.x % p.fgroups;
 	const int f0 = fg * NF;
 	const int unit0 = blockIdx.x / p.fgroups;
@@ -326,7 +328,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	{
 		if (lane < XC_RAW_STAGES)
 		{
-			mbar_init(&raw_full[lane], 1);                        // the copies (with their bytes)
+			mbar_init(&raw_full[lane], 2);                        // the copies (with their bytes), and the window table
 			mbar_init(&raw_empty[lane], XC_EXP_WARPS);
 		}
 		if (lane < XC_MAX_STAGES)
@@ -636,6 +638,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const int ew = warp - XC_EPI_WARPS;
 		const int et = ew * 32 + lane;
 		const int slots_plane = p.slots_plane, G = p.G, nb = p.nb, stages_k = p.stages_k, ring = p.ring, units = p.units;
+		const int table_len = p.n_src * slots_plane;
 		const int blocks0 = p.src[0].blocks;
 		const int mode = p.src[0].mode;                          // OR4 and SINGLE may meet in one layer (a route); both work as OR4
 		const bool tabled = (mode != XC_LINEAR);
@@ -670,33 +673,12 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		int es = 0, rs = 0;
 		uint32_t es_phase = 1, rs_phase = 0;                     // es_phase: parity of the wait for an emptied stage
 		bool ok = true;
-		for (int u = unit0; u < units && ok; u += unit_step)
+		int n_unit = 0;
+		for (int u = unit0; u < units && ok; u += unit_step, ++n_unit)
 		{
-			const XcRun run0 = run_of(p, p.src[0], u);
-			const XcRun run1 = (p.n_src == 1) ? run0 : run_of(p, p.src[1], u);
-			const uint32_t shift0 = (uint32_t)run0.shift * 4u, shift1 = (uint32_t)run1.shift * 4u;
-			// tabled: where in a raw stage this thread's words of the unit lie (-1: padding)
-			int e[XC_ITEMS];
-			auto find = [&](const XcSource & src, int run_start)
-			{
-				const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
-				const int pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos;
-				const int scale = src.scale, src_pitch = src.pitch, src_rows = src.h + 1, base = src.front - run_start;
-				const int pos0 = u * p.pt * TC_PIX - p.halo;
-				#pragma unroll
-				for (int j = 0; j < XC_ITEMS; ++j)
-				{
-					if (j >= n_items) { break; }
-					const int pos = pos0 + (int)(from[j] & 0xffffu);
-					const int img = fdiv(pos, d_img);
-					const int r = pos - img * (int)d_img.d;
-					const int y = fdiv(r, d_pitch);
-					const int x = r - y * pitch;
-					const int sy = (scale == 2) ? 2 * y : (scale == 1) ? y : y >> 1;
-					const int sx = (scale == 2) ? 2 * x : (scale == 1) ? x : x >> 1;
-					e[j] = (pos >= 0 && pos < total_pos && y < OH && x < OW) ? (base + (img * src_rows + sy) * src_pitch + sx + (int)(from[j] >> 16)) * 4 : -1;
-				}
-			};
+			const uint32_t table_addr = smem_u32(s_table + (n_unit % XC_TABLES) * table_len);
+			const uint32_t shift0 = tabled ? 0u : (uint32_t)run_of(p, p.src[0], u).shift * 4u;
+			const uint32_t shift1 = (tabled || p.n_src == 1) ? 0u : (uint32_t)run_of(p, p.src[1], u).shift * 4u;
 			for (int st = 0; st < stages_k; ++st, ++k)
 			{
 				const int cb0 = st * G;
@@ -729,7 +711,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				}
 				else
 				{
-					if (st == 0 || cb0 == blocks0) { if (second) { find(p.src[1], run1.start); } else { find(p.src[0], run0.start); } }
+					const uint32_t tab = table_addr + (second ? (uint32_t)slots_plane * 4u : 0u);
 					const uint32_t down = second ? down1 : down0;
 					const uint32_t right = (down != 0u) ? 4u : 0u;
 					#pragma unroll
@@ -737,13 +719,16 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					{
 						if (j0 >= n_items) { break; }
 						uint32_t w0[2], w1[2], w2[2], w3[2], keep[2];
+						int e[2];
+						#pragma unroll
+						for (int q = 0; q < 2; ++q) { if (has(j0 + q)) { e[q] = (int)ld_shared_u32(tab + (from[j0 + q] & 0xffffu) * 4u); } }
 						#pragma unroll
 						for (int q = 0; q < 2; ++q)
 						{
 							if (!has(j0 + q)) { continue; }
 							// padding (-1) reads the run's first words and drops them
-							const uint32_t at = raw + (uint32_t)max(e[j0 + q], 0);
-							keep[q] = ~(uint32_t)(e[j0 + q] >> 31);
+							const uint32_t at = raw + ((uint32_t)max(e[q], 0) + (from[j0 + q] >> 16)) * 4u;
+							keep[q] = ~(uint32_t)(e[q] >> 31);
 							w0[q] = ld_shared_u32(at);
 							w1[q] = ld_shared_u32(at + right);
 							w2[q] = ld_shared_u32(at + down);
@@ -822,7 +807,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		int rs = 0;
 		uint32_t rs_phase = 1, k = 0;
 		bool ok = true;
-		for (int u = unit0; u < p.units && ok; u += unit_step)
+		int n_unit = 0;
+		for (int u = unit0; u < p.units && ok; u += unit_step, ++n_unit)
 		{
 			const XcRun run0 = run_of(p, p.src[0], u);
 			const XcRun run1 = (p.n_src > 1) ? run_of(p, p.src[1], u) : run0;
@@ -853,7 +839,37 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 						bulk_load(dst + (uint32_t)(p.G * p.raw_words * 4), my_filters + (size_t)cb0 * p.taps * 128, (uint32_t)fil_words * 4u, &raw_full[rs]);
 					}
 				}
+				if (st == 0 && p.tabled)
+				{
+					// which word of the run each position of the window is (-1: padding); the copies are on their way meanwhile
+					int * tab = s_table + (n_unit % XC_TABLES) * (p.n_src * p.slots_plane);
+					const int slots_plane = p.slots_plane, pitch = p.pitch, rows = p.rows, OH = p.OH, OW = p.OW, batch = p.batch;
+					const int y_step = fdiv(32, p.d_pitch), x_step = 32 - y_step * pitch;
+					const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
+					const int pos0 = u * p.pt * TC_PIX - p.halo;
+					for (int si = 0; si < p.n_src; ++si, tab += slots_plane)
+					{
+						const int down = 2 - p.src[si].scale, src_pitch = p.src[si].pitch, src_rows = p.src[si].h + 1;
+						const int base = p.src[si].front - (si ? run1.start : run0.start);
+						// walked in steps of 32 positions: a division per entry made this warp the bound of pooled layers
+						const int q = pos0 + lane + (int)d_img.d;            // the window starts at most one row and a pixel before the batch
+						int img = fdiv(q, d_img) - 1;
+						const int r = q - (img + 1) * (int)d_img.d;
+						int y = fdiv(r, d_pitch);
+						int x = r - y * pitch;
+						for (int s = lane; s < slots_plane; s += 32)
+						{
+							const int sy = (2 * y) >> down, sx = (2 * x) >> down;
+							tab[s] = ((unsigned)img < (unsigned)batch && y < OH && x < OW) ? base + (img * src_rows + sy) * src_pitch + sx : -1;
+							x += x_step;
+							y += y_step;
+							if (x >= pitch) { x -= pitch; ++y; }
+							while (y >= rows) { y -= rows; ++img; }
+						}
+					}
+				}
 				__syncwarp();
+				if (lane == 0) { mbar_arrive(&raw_full[rs]); }
 				if (++rs == XC_RAW_STAGES) { rs = 0; rs_phase ^= 1u; }
 			}
 		}
@@ -1014,7 +1030,8 @@ static bool plan_sizes(const XcParams & p, int nf, int pt, int stream, XcPlan * 
 	}
 	if (p.tabled && (long long)q.g * q.raw_words > 0xffff) { return false; }
 	q.raw_stage = (q.g * q.raw_words + (stream ? q.kw_full * nf : 0)) * 4;
-	const size_t fixed = (size_t)XC_RAW_STAGES * q.raw_stage;
+	const size_t table = p.tabled ? XC_TABLES * (size_t)p.n_src * q.slots_plane * sizeof(int) : 0;
+	const size_t fixed = (size_t)XC_RAW_STAGES * q.raw_stage + table;
 	for (q.ring = XC_MAX_STAGES; q.ring >= 2; --q.ring)
 	{
 		q.smem = (size_t)q.ring * q.a_stage + (size_t)(stream ? q.ring : q.stages_k) * q.b_stage + fixed;
