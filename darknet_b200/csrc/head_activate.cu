@@ -23,9 +23,52 @@ yolo_activate_kernel(const float * __restrict__ in, float * __restrict__ out, si
 
 // [region] head (src-lib/region_layer.cpp:494-537): per image, anchor and cell the logistic function on x, y and the
 // objectness entry, w and h raw, and -- with softmax=1 -- a softmax over the class entries (max subtracted, temperature
-// 1: softmax_cpu in src-lib/blas.cpp).  The tensor is [batch][anchors][coords + 1 + classes][h*w]; a thread owns one
-// (image, anchor, cell), so every access of a warp is 32 consecutive cells of one entry plane.  The class scores
-// are read twice (running maximum and sum in one pass, normalised values in the second, from L1/L2).
+// 1: softmax_cpu in src-lib/blas.cpp).  The tensor is [batch][anchors][coords + 1 + classes][h*w].
+//
+// region_group_kernel: one anchor of one image per block, its entries side by side in shared memory.  Bound by memory: planes of
+// 13x13 cells start on no boundary, so reading them plane by plane takes a third more sectors and leaves partly written ones; the
+// whole group is one run that is read and written once, in order.
+constexpr int RG_THREADS = 256;
+constexpr size_t RG_MAX_BYTES = 100 * 1024;              // two blocks on an SM
+
+__global__ void __launch_bounds__(RG_THREADS)
+region_group_kernel(const float * __restrict__ in, float * __restrict__ out, int coords, int classes, int hw)
+{
+	extern __shared__ float s_group[];
+	const int total = (coords + 1 + classes) * hw;
+	const size_t base = (size_t)blockIdx.x * total;
+	#pragma unroll 8
+	for (int i = threadIdx.x; i < total; i += RG_THREADS) { s_group[i] = in[base + i]; }
+	__syncthreads();
+	for (int i = threadIdx.x; i < 3 * hw; i += RG_THREADS)
+	{
+		const int e = i / hw;
+		float * at = s_group + (e == 2 ? coords : e) * hw + (i - e * hw);
+		*at = 1.0f / (1.0f + expf(-*at));
+	}
+	float * cls = s_group + (coords + 1) * hw;
+	for (int cell = threadIdx.x; cell < hw; cell += RG_THREADS)
+	{
+		float top = -INFINITY, sum = 0.0f;
+		#pragma unroll 8
+		for (int c = 0; c < classes; ++c) { top = fmaxf(top, cls[c * hw + cell]); }
+		#pragma unroll 4
+		for (int c = 0; c < classes; ++c)
+		{
+			const float v = expf(cls[c * hw + cell] - top);
+			cls[c * hw + cell] = v;
+			sum += v;
+		}
+		#pragma unroll 4
+		for (int c = 0; c < classes; ++c) { cls[c * hw + cell] = cls[c * hw + cell] / sum; }
+	}
+	__syncthreads();
+	#pragma unroll 8
+	for (int i = threadIdx.x; i < total; i += RG_THREADS) { out[base + i] = s_group[i]; }
+}
+
+// Without a softmax, and groups that do not fit: a thread owns one (image, anchor, cell), so every access of a warp is 32
+// consecutive cells of one entry plane; the class scores are read three times, from the L1 / L2.
 __global__ void __launch_bounds__(256)
 region_activate_kernel(const float * __restrict__ in, float * __restrict__ out, size_t cells, int coords, int classes, int softmax, int hw)
 {
@@ -65,6 +108,14 @@ extern "C" int xnor_b200_region_activate(const float * input, float * output, in
 	if (input == nullptr || output == nullptr) { return XNOR_B200_ERR_NULL; }
 	if (batch <= 0 || anchors <= 0 || coords < 2 || classes < 0 || hw <= 0 || input == output) { return XNOR_B200_ERR_INVALID; }
 	const size_t cells = (size_t)batch * anchors * hw;
+	const size_t group_bytes = (size_t)(coords + 1 + classes) * hw * sizeof(float);
+	if (softmax && group_bytes <= RG_MAX_BYTES && (long long)batch * anchors <= 0x7fffffffLL)
+	{
+		const int rc = ensure_dynamic_smem((const void *)region_group_kernel, group_bytes);
+		if (rc != XNOR_B200_OK) { return rc; }
+		region_group_kernel<<<(unsigned)(batch * anchors), RG_THREADS, group_bytes, (cudaStream_t)stream>>>(input, output, coords, classes, hw);
+		return check_launch();
+	}
 	const int grid = (int)min((cells + 255) / 256, (size_t)sm_count() * 8);
 	region_activate_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(input, output, cells, coords, classes, softmax, hw);
 	return check_launch();

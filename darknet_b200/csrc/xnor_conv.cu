@@ -843,28 +843,24 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				{
 					// which word of the run each position of the window is (-1: padding); the copies are on their way meanwhile
 					int * tab = s_table + (n_unit % XC_TABLES) * (p.n_src * p.slots_plane);
-					const int slots_plane = p.slots_plane, pitch = p.pitch, rows = p.rows, OH = p.OH, OW = p.OW, batch = p.batch;
-					const int y_step = fdiv(32, p.d_pitch), x_step = 32 - y_step * pitch;
+					const int slots_plane = p.slots_plane, pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos;
 					const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
 					const int pos0 = u * p.pt * TC_PIX - p.halo;
 					for (int si = 0; si < p.n_src; ++si, tab += slots_plane)
 					{
 						const int down = 2 - p.src[si].scale, src_pitch = p.src[si].pitch, src_rows = p.src[si].h + 1;
 						const int base = p.src[si].front - (si ? run1.start : run0.start);
-						// walked in steps of 32 positions: a division per entry made this warp the bound of pooled layers
-						const int q = pos0 + lane + (int)d_img.d;            // the window starts at most one row and a pixel before the batch
-						int img = fdiv(q, d_img) - 1;
-						const int r = q - (img + 1) * (int)d_img.d;
-						int y = fdiv(r, d_pitch);
-						int x = r - y * pitch;
+						// a division per entry: four independent ones at a time beat one chain of steps of 32 positions (104x104 83 / 115 us)
+						#pragma unroll 2
 						for (int s = lane; s < slots_plane; s += 32)
 						{
+							const int pos = pos0 + s;
+							const int img = fdiv(pos, d_img);
+							const int r = pos - img * (int)d_img.d;
+							const int y = fdiv(r, d_pitch);
+							const int x = r - y * pitch;
 							const int sy = (2 * y) >> down, sx = (2 * x) >> down;
-							tab[s] = ((unsigned)img < (unsigned)batch && y < OH && x < OW) ? base + (img * src_rows + sy) * src_pitch + sx : -1;
-							x += x_step;
-							y += y_step;
-							if (x >= pitch) { x -= pitch; ++y; }
-							while (y >= rows) { y -= rows; ++img; }
+							tab[s] = (pos >= 0 && pos < total_pos && y < OH && x < OW) ? base + (img * src_rows + sy) * src_pitch + sx : -1;
 						}
 					}
 				}
