@@ -940,22 +940,28 @@ class DetectionBuffers:
         self.desc = capi.Detections(self.boxes.data_ptr(), self.objectness.data_ptr(), self.probs.data_ptr(), self.count.data_ptr(),
                                     max_dets, classes)
         # where rows_host receives the counts and the first rows: page-locked, so that both copies are queued and waited for once
-        self.take = min(max_rows, 512)
-        pin = self.rows.is_cuda
-        self.host_count = torch.empty(batch, dtype=torch.int32, pin_memory=pin)
-        self.host_rows = torch.empty(batch, self.take, 7, dtype=torch.float32, pin_memory=pin)
+        self.host_count = torch.empty(batch, dtype=torch.int32, pin_memory=self.rows.is_cuda)
+        self._take_rows(512)
+
+    def _take_rows(self, rows: int) -> None:
+        """Makes room for the first `rows` rows of every image on the host."""
+        self.take = min(self.max_rows, rows)
+        self.host_rows = torch.empty(self.batch, self.take, 7, dtype=torch.float32, pin_memory=self.rows.is_cuda)
 
     def rows_host(self) -> List[np.ndarray]:
         """Per image the rows {x, y, w, h, objectness, class, probability}.  The counts and each image's first `take` rows come over
-        together (most frames have fewer: the whole list would be eight times the bytes); only a longer list costs a second copy."""
+        together (most frames have fewer: the whole list would be eight times the bytes); a longer list costs a second copy, 40 us with
+        its wait, and widens the first one for the frames to come, which show much the same scene."""
         stream = torch.cuda.current_stream(self.rows.device)
         capi.check(capi.lib().xnor_b200_rows_to_host(self.rows.data_ptr(), self.max_rows, self.row_count.data_ptr(), self.batch, self.take,
                                                     self.host_rows.data_ptr(), self.host_count.data_ptr(), stream.cuda_stream),
                    "xnor_b200_rows_to_host")
         stream.synchronize()
         counts, rows = self.host_count.numpy(), self.host_rows.numpy()
-        if int(counts.max()) > self.take:
+        longest = min(int(counts.max()), self.max_rows)
+        if longest > self.take:
             rows = self.rows.cpu().numpy()
+            self._take_rows(1 << (longest - 1).bit_length())
         return [rows[b, :min(int(counts[b]), self.max_rows)].copy() for b in range(self.batch)]
 
 

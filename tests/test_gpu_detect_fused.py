@@ -69,3 +69,16 @@ def test_detect_equals_the_restatement(tmp_path, share, size, max_dets, favourit
         want, kept = expected_rows(boxes[b, :n], obj[b, :n], probs[b, :n], np.float32(0.45))
         assert np.array_equal(got[b], want) and np.array_equal(same[b], want)
         assert np.array_equal(fused.probs[b, :n].cpu().numpy(), kept)
+
+
+@pytest.mark.parametrize("counts,max_rows", [([0, 512], 4096), ([513, 3], 4096), ([2049, 700], 4096), ([900, 901], 900)])
+def test_rows_host_of_long_lists(counts, max_rows):
+    """Lists longer than the first copy: whole the first time, and from then on in one copy."""
+    dets = network.DetectionBuffers(2, 4, max_rows=max_rows)
+    for _ in range(2):
+        dets.rows.normal_()
+        dets.row_count.copy_(torch.tensor(counts, dtype=torch.int32))
+        got = dets.rows_host()
+        for b, n in enumerate(counts):
+            assert got[b].shape == (min(n, max_rows), 7) and (got[b] == dets.rows[b, :min(n, max_rows)].cpu().numpy()).all()
+        assert min(max(counts), max_rows) <= dets.take <= max_rows
