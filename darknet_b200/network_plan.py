@@ -173,7 +173,12 @@ def _build(net) -> Plan:
             plan.ops.append(capi.Op(kind=capi.OP_CONV3, arg=2 if pooled_first else 0, pitch=g.pitch, desc=_desc(net, l), input=capi.OP_INPUT,
                                     output=g.words.data_ptr(), weights=l.weights_gpu.data_ptr(), biases=l.biases_gpu.data_ptr()))
         elif l.type == "convolutional":
-            _float_conv(plan, k, float_in[k], fp32_read)
+            _float_conv(plan, k, float_in[k], k in sign_read)
+            if k in sign_read:
+                # an xnor layer reads it: the kernel leaves fp32, its signs are taken in a pass of their own
+                g = grid(k)
+                plan.ops.append(capi.Op(kind=capi.OP_SIGN_WORDS, desc=capi.ConvDesc(net.batch, l.n, l.out_h, l.out_w), pitch=g.pitch,
+                                        input=plan.floats[k].data_ptr(), output=g.words.data_ptr()))
         elif l.type == "avgpool":
             src = layers[float_in[k]]
             plan.floats[k] = torch.empty(net.batch, l.out_c, 1, 1, device=net.device)
@@ -185,10 +190,23 @@ def _build(net) -> Plan:
             plan.ops.append(capi.Op(kind=capi.OP_BACK))
     if not plan.head_layers:
         raise Unsupported("no head")
+    _check_signs_are_written(plan)
     for k, l in enumerate(layers):
         l.output_gpu = plan.floats.get(k, l.output_gpu)
     plan.finish()
     return plan
+
+
+def _check_signs_are_written(plan: Plan) -> None:
+    """Grid words start as zeros: an operation in front of the one that writes them would quietly read "nothing is > 0"."""
+    written = set()
+    for op in plan.ops:
+        if op.kind == capi.OP_CONV_WORDS:
+            if any(s.words not in written for s in op.io.sources[:op.io.n_sources]):
+                raise Unsupported("a sign tensor that no operation writes")
+            written |= {op.io.output_signs, op.io.shortcut_signs}
+        elif op.kind in (capi.OP_CONV3, capi.OP_SIGN_WORDS):
+            written.add(op.output)
 
 
 def _xnor_outputs(net) -> set:
@@ -243,12 +261,12 @@ def _xnor_conv(plan: Plan, k: int, sources: List[Source], grid, sign_read: set, 
                             biases=xl.biases_gpu.data_ptr()))
 
 
-def _float_conv(plan: Plan, k: int, src: int, fp32_read: set) -> None:
+def _float_conv(plan: Plan, k: int, src: int, signs_wanted: bool) -> None:
     """A float convolution behind the path; in front of a [yolo] layer with that layer's activation, into the head."""
     net, l = plan.net, plan.net.layers[k]
     nxt = net.layers[k + 1] if k + 1 < len(net.layers) else None
     op = capi.Op(desc=_desc(net, l), input=_tensor(plan, src).data_ptr(), biases=l.biases_gpu.data_ptr())
-    head = nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
+    head = not signs_wanted and nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
     entries = 5 + int(nxt.opts.get("classes", 20)) if head else 0
     head = head and l.n % entries == 0
     if l.weights_blocked_gpu is not None:
