@@ -695,6 +695,7 @@ def prepare_float_map_convs(net: Network) -> None:
     3x3/pad 1 or 1x1, few output pixels in the whole batch), and lays out those of the others for the tensor-core GEMM.
     Runs after fuse_conv_batchnorm."""
     import ctypes as C
+    readers = _readers(net)
     for l in net.layers:
         if l.type != "convolutional" or l.xnor or l.activation not in ("leaky", "linear"):
             continue
@@ -711,7 +712,7 @@ def prepare_float_map_convs(net: Network) -> None:
                                                                      torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_tc_prepare")
             continue
         nxt = net.layers[l.index + 1] if l.index + 1 < len(net.layers) else None
-        if (nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
+        if (nxt is not None and nxt.type == "yolo" and readers[l.index] == [l.index + 1] and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
                 and l.n % (5 + int(nxt.opts.get("classes", 20))) == 0):
             l.yolo_entries = 5 + int(nxt.opts.get("classes", 20))
             nxt.yolo_done = True

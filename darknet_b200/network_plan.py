@@ -173,7 +173,7 @@ def _build(net) -> Plan:
             plan.ops.append(capi.Op(kind=capi.OP_CONV3, arg=2 if pooled_first else 0, pitch=g.pitch, desc=_desc(net, l), input=capi.OP_INPUT,
                                     output=g.words.data_ptr(), weights=l.weights_gpu.data_ptr(), biases=l.biases_gpu.data_ptr()))
         elif l.type == "convolutional":
-            _float_conv(plan, k, float_in[k], k in sign_read)
+            _float_conv(plan, k, float_in[k], readers.get(k) == [k + 1])
             if k in sign_read:
                 # an xnor layer reads it: the kernel leaves fp32, its signs are taken in a pass of their own
                 g = grid(k)
@@ -261,12 +261,12 @@ def _xnor_conv(plan: Plan, k: int, sources: List[Source], grid, sign_read: set, 
                             biases=xl.biases_gpu.data_ptr()))
 
 
-def _float_conv(plan: Plan, k: int, src: int, signs_wanted: bool) -> None:
-    """A float convolution behind the path; in front of a [yolo] layer with that layer's activation, into the head."""
+def _float_conv(plan: Plan, k: int, src: int, one_reader: bool) -> None:
+    """A float convolution behind the path; in front of a [yolo] layer that alone reads it with that layer's activation, into the head."""
     net, l = plan.net, plan.net.layers[k]
     nxt = net.layers[k + 1] if k + 1 < len(net.layers) else None
     op = capi.Op(desc=_desc(net, l), input=_tensor(plan, src).data_ptr(), biases=l.biases_gpu.data_ptr())
-    head = not signs_wanted and nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
+    head = one_reader and nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
     entries = 5 + int(nxt.opts.get("classes", 20)) if head else 0
     head = head and l.n % entries == 0
     if l.weights_blocked_gpu is not None:

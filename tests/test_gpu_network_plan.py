@@ -63,3 +63,10 @@ def test_a_float_convolution_between_xnor_layers(between, tmp_path):
     close = float((values.abs() <= 2e-6 * values.abs().max()).float().mean())
     differ = float(((got[0] - want[0]).abs() > 1e-4).float().mean())
     assert differ <= 1e-3 + 576 * close < 0.1 and float(want[0].std()) > 0
+
+
+@pytest.mark.parametrize("batch,width,height", [(2, 64, 48), (1, 16, 16)], ids=["gemm", "small map"])
+def test_a_route_may_read_the_convolution_in_front_of_a_yolo_layer(batch, width, height, tmp_path):
+    net, got, want = both(tmp_path, [cfgs._conv(32, 3), cfgs._conv(160, 3, xnor=1), HEAD, YOLO, "[route]\nlayers=-2\n", YOLO], batch, width, height)
+    assert net.plan is not None and torch.equal(got[0], got[1])
+    assert_heads_close(got, want)

@@ -68,3 +68,11 @@ def test_a_float_convolution_read_by_an_xnor_layer_gets_its_signs_made(between, 
     assert signs.input == float_conv.output and (signs.desc.c, signs.desc.h, signs.desc.w) == (64, 64, 64)
     read, written = sign_buffers(net.plan)
     assert read == written
+
+
+def test_a_route_may_read_the_convolution_in_front_of_a_yolo_layer(tmp_path, monkeypatch):
+    """Its raw values are kept for the [route]; the [yolo] layer's activation is then a pass of its own."""
+    net = lowered([conv(32, 3), conv(160, 3, xnor=1), head_conv(), YOLO, "[route]\nlayers=-2\n", YOLO], tmp_path, monkeypatch)
+    convs, heads = [[op for op in net.plan.ops if op.kind == k] for k in (capi.OP_FLOAT_TC, capi.OP_YOLO)]
+    assert len(convs) == 1 and convs[0].arg == 0 and convs[0].output not in (capi.OP_HEAD, capi.OP_HEAD + 1)
+    assert [op.output for op in heads] == [capi.OP_HEAD, capi.OP_HEAD + 1] and all(op.input == convs[0].output for op in heads)
