@@ -69,7 +69,7 @@ class WordsIO(C.Structure):
 
 
 (OP_CONV3, OP_SIGN_WORDS, OP_CONV_WORDS, OP_FLOAT_MAP, OP_FLOAT_TC, OP_YOLO, OP_REGION, OP_AVGPOOL, OP_SOFTMAX, OP_FORK,
- OP_BACK, OP_CONV) = range(1, 13)
+ OP_BACK, OP_CONV, OP_FILTERS) = range(1, 14)
 OP_INPUT, OP_HEAD = 1, 2
 
 

@@ -94,8 +94,8 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 		float * out = (float *)resolve(op.output, input, heads, n_heads);
 		const xnor_b200_conv_desc & d = op.desc;
 		int rc = XNOR_B200_OK;
-		// behind a fork or a return the stream's last entry is no kernel of this call
-		g_behind_kernel = (i > 0 && ops[i - 1].kind != XNOR_B200_OP_FORK && ops[i - 1].kind != XNOR_B200_OP_BACK);
+		// behind a fork, a return or filters (seldom made again) the stream's last entry may be no kernel of this call
+		g_behind_kernel = (i > 0 && ops[i - 1].kind != XNOR_B200_OP_FORK && ops[i - 1].kind != XNOR_B200_OP_BACK && ops[i - 1].kind != XNOR_B200_OP_FILTERS);
 		switch (op.kind)
 		{
 			case XNOR_B200_OP_CONV3: rc = xnor_b200_float_conv3_words(&d, op.arg, in, (const float *)op.weights, op.biases, (uint32_t *)out, op.pitch, at); break;
@@ -111,6 +111,17 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 				rc = xnor_b200_conv_forward(&d, in, (const uint8_t *)op.weights, op.mean_arr, op.biases, out, op.io.shortcut_in, op.io.shortcut_out,
 						op.scratch, op.scratch_bytes, at);
 				break;
+			case XNOR_B200_OP_FILTERS:
+			{
+				cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+				if (op.arg == 0)
+				{
+					const cudaError_t e = cudaStreamIsCapturing((cudaStream_t)at, &capture);
+					if (e != cudaSuccess) { return cuda_fail(e); }
+				}
+				if (op.arg != 0 || capture != cudaStreamCaptureStatusNone) { rc = xnor_b200_conv_words_weights(&d, (const uint8_t *)op.weights, (uint32_t *)out, at); }
+				break;
+			}
 			case XNOR_B200_OP_FORK:
 			{
 				// what follows runs on the side stream, behind everything issued so far

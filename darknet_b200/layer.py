@@ -55,8 +55,11 @@ class ConvolutionalLayer:
         self.bin_conv_shortcut_in_gpu: Optional[torch.Tensor] = None
         self.bin_conv_shortcut_out_gpu: Optional[torch.Tensor] = None
         self.shortcut_signs_gpu: Optional[torch.Tensor] = None       # sign words of the fused shortcut sum, when a layer reads them
-        self.conv_words_gpu: Optional[torch.Tensor] = None           # the filters as xnor_b200_conv_words reads them, where that route is taken
-        self.input_words: Optional[GridWords] = None                 # ... and the input's sign words
+        # align_bit_weights_gpu as xnor_b200_conv_words reads it, where that route is taken; made again before a call when it was
+        # replaced or written to through torch since
+        self.conv_words_gpu: Optional[torch.Tensor] = None
+        self._words_of = (None, None)                                # the tensor it was made from and that tensor's version (None: keeps none)
+        self.input_words: Optional[GridWords] = None                 # the input's sign words
         self._ops = self._ops_of = None                              # forward_convolutional_layer_gpu: its launches, and the tensors they name
         self._input_floats = batch * c * h * w
 
@@ -114,10 +117,16 @@ def binary_align_weights(l: ConvolutionalLayer, invert: bool = False, single_cal
     l._ops = l._ops_of = None
     if single_calls and not invert and takes_words(l):
         l.conv_words_gpu = conv_words_weights(l)
+        l._words_of = (l.align_bit_weights_gpu, _version(l.align_bit_weights_gpu))
         if l.input_words is None and l.conv_words_gpu is not None:
             l.input_words = GridWords(l.batch, l.c, l.h, l.w, device=l.device)
     else:
         l.conv_words_gpu = None
+
+
+def _version(t: torch.Tensor) -> Optional[int]:
+    """Counts the writes to a tensor through torch; None for one made under inference_mode, which does not count them."""
+    return None if t.is_inference() else t._version
 
 
 def takes_words(l: ConvolutionalLayer) -> bool:
@@ -180,10 +189,18 @@ def forward_convolutional_layer_gpu(l: ConvolutionalLayer, x: torch.Tensor, pool
             _layer_ops(l)
         if x.dtype != torch.float32 or x.numel() != l._input_floats or not x.is_contiguous():
             raise ValueError("input must be a contiguous fp32 tensor of batch*c*h*w elements")
+        of, version = l._words_of
+        changed = l.conv_words_gpu is not None and (of is not l.align_bit_weights_gpu or version is None or of._version != version)
+        if changed:
+            l._ops[0].arg = 1                                       # makes the filters again
         rc = capi.lib().xnor_b200_run_ops(l._ops, len(l._ops), x.data_ptr(), None, 0, torch._C._cuda_getCurrentRawStream(x.device.index),
                                           None, None, None)
         if rc:
             capi.check(rc, "xnor_b200_run_ops")
+        if changed:
+            l._ops[0].arg = 0
+            if not torch.cuda.is_current_stream_capturing():        # captured work has not run
+                l._words_of = (l.align_bit_weights_gpu, _version(l.align_bit_weights_gpu))
         return l.output_gpu
     if l.align_bit_weights_gpu is None:
         raise RuntimeError("binary_align_weights() has not been called for this layer")
@@ -210,15 +227,14 @@ def _layer_ops(l: ConvolutionalLayer) -> None:
     shortcut_in, shortcut_out = l.bin_conv_shortcut_in_gpu, l.bin_conv_shortcut_out_gpu
     op = capi.Op(desc=l.desc, mean_arr=l.mean_arr_gpu.data_ptr(), biases=l.biases_gpu.data_ptr())
     op.io.shortcut_in, op.io.shortcut_out = _ptr(shortcut_in) if shortcut_out is not None else None, _ptr(shortcut_out)
-    if l.conv_words_gpu is not None and l._ops_of is not None and l._ops_of[3] is not l.align_bit_weights_gpu:
-        l.conv_words_gpu = None                                     # other packed weights than the ones it was made from
     if l.conv_words_gpu is not None:
+        filters = capi.Op(kind=capi.OP_FILTERS, desc=l.desc, weights=l.align_bit_weights_gpu.data_ptr(), output=l.conv_words_gpu.data_ptr())
         signs = capi.Op(kind=capi.OP_SIGN_WORDS, desc=l.desc, input=capi.OP_INPUT, output=l.input_words.words.data_ptr(), pitch=l.input_words.pitch)
         op.kind, op.weights = capi.OP_CONV_WORDS, l.conv_words_gpu.data_ptr()
         op.io.n_sources = 1
         op.io.sources[0] = l.input_words.source()
         op.io.output = l.output_gpu.data_ptr()
-        l._ops = (capi.Op * 2)(signs, op)
+        l._ops = (capi.Op * 3)(filters, signs, op)
     else:
         op.kind, op.weights = capi.OP_CONV, l.align_bit_weights_gpu.data_ptr()
         op.input, op.output = capi.OP_INPUT, l.output_gpu.data_ptr()

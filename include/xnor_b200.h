@@ -488,6 +488,8 @@ XNOR_B200_API int xnor_b200_softmax(const float * input, float * output, int bat
 #define XNOR_B200_OP_FORK       10   /* the operations up to OP_BACK run on the side stream, beside those behind OP_BACK              */
 #define XNOR_B200_OP_BACK       11
 #define XNOR_B200_OP_CONV       12   /* xnor_b200_conv_forward(desc, input, weights, mean_arr, biases, output, io.shortcut_in, io.shortcut_out, scratch) */
+#define XNOR_B200_OP_FILTERS    13   /* xnor_b200_conv_words_weights(desc, weights, output), where arg != 0 or the stream is being captured
+                                      * (a captured forward then follows later changes of the packed weights)                         */
 
 /* Values of input / output that stand for the run's own tensors. */
 #define XNOR_B200_OP_INPUT       1   /* the network's input                 */
