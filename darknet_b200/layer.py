@@ -60,7 +60,7 @@ class ConvolutionalLayer:
         self.conv_words_gpu: Optional[torch.Tensor] = None
         self._words_of = (None, None)                                # the tensor it was made from and that tensor's version (None: keeps none)
         self.input_words: Optional[GridWords] = None                 # the input's sign words
-        self._ops = self._ops_of = None                              # forward_convolutional_layer_gpu: its launches, and the tensors they name
+        self._ops = self._conv_op = self._ops_of = None              # forward_convolutional_layer_gpu: its launches, the last of them, what they name
         self._input_floats = batch * c * h * w
 
     # The two large buffers are made when something first asks for them: a layer inside a network that hands signs on needs neither
@@ -114,7 +114,6 @@ def binary_align_weights(l: ConvolutionalLayer, invert: bool = False, single_cal
     capi.check(capi.lib().xnor_b200_binary_align_weights(C.byref(l.desc), l.weights_gpu.data_ptr(),
                                                         l.align_bit_weights_gpu.data_ptr(), l.mean_arr_gpu.data_ptr(),
                                                         int(invert), _stream()), "xnor_b200_binary_align_weights")
-    l._ops = l._ops_of = None
     if single_calls and not invert and takes_words(l):
         l.conv_words_gpu = conv_words_weights(l)
         l._words_of = (l.align_bit_weights_gpu, _version(l.align_bit_weights_gpu))
@@ -183,10 +182,12 @@ def forward_convolutional_layer_gpu(l: ConvolutionalLayer, x: torch.Tensor, pool
     """The xnor branch of forward_convolutional_layer_gpu (src-lib/convolutional_kernels.cu:204-262), whole batch.
     With `pool`, x is the input of a [maxpool] layer that sits directly in front of this convolution."""
     if pool is None and x.is_cuda and not capi.packed_route_pinned:
-        named = l._ops_of
-        if (named is None or named[0] is not l.output_gpu or named[1] is not l.bin_conv_shortcut_in_gpu
-                or named[2] is not l.bin_conv_shortcut_out_gpu or named[3] is not l.align_bit_weights_gpu or named[4] is not l.biases_gpu):
+        if l._ops_of != _named(l):
             _layer_ops(l)
+        if l.bin_conv_shortcut_out_gpu is not None or l._conv_op.io.shortcut_out:
+            # a caller may name other tensors on every call
+            l._conv_op.io.shortcut_in = _ptr(l.bin_conv_shortcut_in_gpu) if l.bin_conv_shortcut_out_gpu is not None else None
+            l._conv_op.io.shortcut_out = _ptr(l.bin_conv_shortcut_out_gpu)
         if x.dtype != torch.float32 or x.numel() != l._input_floats or not x.is_contiguous():
             raise ValueError("input must be a contiguous fp32 tensor of batch*c*h*w elements")
         of, version = l._words_of
@@ -220,13 +221,18 @@ def forward_convolutional_layer_gpu(l: ConvolutionalLayer, x: torch.Tensor, pool
     return l.output_gpu
 
 
-def _layer_ops(l: ConvolutionalLayer) -> None:
-    """The launches of forward_convolutional_layer_gpu, kept until the weights or a tensor they name are replaced."""
+def _named(l: ConvolutionalLayer) -> tuple:
+    """What the launches of forward_convolutional_layer_gpu name: the sizes, and where the layer's tensors lie.  Looked up on every call,
+    so that they never name memory of a tensor that was replaced."""
     if l.align_bit_weights_gpu is None:
         raise RuntimeError("binary_align_weights() has not been called for this layer")
-    shortcut_in, shortcut_out = l.bin_conv_shortcut_in_gpu, l.bin_conv_shortcut_out_gpu
+    return (bytes(l.desc), l.align_bit_weights_gpu.data_ptr(), l.mean_arr_gpu.data_ptr(), l.biases_gpu.data_ptr(), l.output_gpu.data_ptr(),
+            (l.scratch if l.conv_words_gpu is None else l.conv_words_gpu).data_ptr(), l.input_words)
+
+
+def _layer_ops(l: ConvolutionalLayer) -> None:
+    """The launches of forward_convolutional_layer_gpu."""
     op = capi.Op(desc=l.desc, mean_arr=l.mean_arr_gpu.data_ptr(), biases=l.biases_gpu.data_ptr())
-    op.io.shortcut_in, op.io.shortcut_out = _ptr(shortcut_in) if shortcut_out is not None else None, _ptr(shortcut_out)
     if l.conv_words_gpu is not None:
         filters = capi.Op(kind=capi.OP_FILTERS, desc=l.desc, weights=l.align_bit_weights_gpu.data_ptr(), output=l.conv_words_gpu.data_ptr())
         signs = capi.Op(kind=capi.OP_SIGN_WORDS, desc=l.desc, input=capi.OP_INPUT, output=l.input_words.words.data_ptr(), pitch=l.input_words.pitch)
@@ -234,13 +240,13 @@ def _layer_ops(l: ConvolutionalLayer) -> None:
         op.io.n_sources = 1
         op.io.sources[0] = l.input_words.source()
         op.io.output = l.output_gpu.data_ptr()
-        l._ops = (capi.Op * 3)(filters, signs, op)
+        ops = (capi.Op * 3)(filters, signs, op)
     else:
         op.kind, op.weights = capi.OP_CONV, l.align_bit_weights_gpu.data_ptr()
         op.input, op.output = capi.OP_INPUT, l.output_gpu.data_ptr()
         op.scratch, op.scratch_bytes = l.scratch.data_ptr(), l.scratch.numel()
-        l._ops = (capi.Op * 1)(op)
-    l._ops_of = (l.output_gpu, shortcut_in, shortcut_out, l.align_bit_weights_gpu, l.biases_gpu)
+        ops = (capi.Op * 1)(op)
+    l._ops, l._conv_op, l._ops_of = ops, ops[len(ops) - 1], _named(l)
 
 
 class Sink:

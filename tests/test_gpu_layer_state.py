@@ -92,3 +92,49 @@ def test_a_captured_call_follows_the_packed_weights():
     torch.cuda.synchronize()
     assert torch.equal(out, want)
     assert_follows(l, x)
+
+
+@pytest.mark.parametrize("called_before", [False, True])
+@pytest.mark.parametrize("shape", [WORDS, PACKED], ids=["words", "packed"])
+def test_tensors_that_are_replaced(shape, called_before):
+    """Each tensor's old memory is filled with NaN (or ones) once the layer has another: a launch that still named it would show."""
+    l, x = build(shape)
+    before = assert_follows(l, x) if called_before else None
+    for name in ("mean_arr_gpu", "biases_gpu"):
+        old = getattr(l, name)
+        setattr(l, name, old * 1.5)
+        old.fill_(float("nan"))
+        before = assert_follows(l, x, before)
+        getattr(l, name).mul_(2)
+        before = assert_follows(l, x, before)
+        getattr(l, name).data = getattr(l, name) * 3
+        before = assert_follows(l, x, before)
+    old, l.scratch = l.scratch, torch.zeros_like(l.scratch)
+    old.fill_(255)
+    assert_follows(l, x)
+    assert bool((old == 255).all())
+    old, l.output_gpu = l.output_gpu, torch.empty_like(l.output_gpu)
+    old.fill_(7.0)
+    assert_follows(l, x)
+    assert bool((old == 7.0).all())
+    if shape is WORDS:
+        l.conv_words_gpu = None                        # without the copy: the packed route
+        assert_follows(l, x)
+
+
+@pytest.mark.parametrize("shape", [WORDS, PACKED], ids=["words", "packed"])
+def test_shortcuts_and_activations_that_change(shape):
+    l, x = build(shape)
+    plain = assert_follows(l, x)
+    for seed in (1, 2):
+        add = torch.from_numpy(synth.bell(seed, tuple(plain.shape))).cuda()
+        l.bin_conv_shortcut_in_gpu, l.bin_conv_shortcut_out_gpu = add, torch.empty_like(add)
+        assert torch.equal(L.forward_convolutional_layer_gpu(l, x), plain)
+        assert torch.equal(l.bin_conv_shortcut_out_gpu, add + plain)
+    total = l.bin_conv_shortcut_out_gpu
+    l.bin_conv_shortcut_out_gpu = None
+    total.zero_()
+    assert_follows(l, x)
+    assert not bool(total.any())
+    l.desc.activation = capi.LINEAR
+    assert_follows(l, x, plain)
