@@ -63,8 +63,8 @@ class ConvolutionalLayer:
         self._ops = self._conv_op = self._ops_of = None              # forward_convolutional_layer_gpu: its launches, the last of them, what they name
         self._input_floats = batch * c * h * w
 
-    # The two large buffers are made when something first asks for them: a layer inside a network that hands signs on needs neither
-    # (at batch 256 the packed operands of tiny-yolo are 1.5 GB, their allocation and zero fill most of the load time).
+    # The two large buffers are made by binary_align_weights, or when something first asks for them: a layer inside a network that hands
+    # signs on needs neither (at batch 256 the packed operands of tiny-yolo are 1.5 GB, their allocation and zero fill most of the load time).
     @property
     def output_gpu(self) -> torch.Tensor:
         if self._output is None:
@@ -85,6 +85,10 @@ class ConvolutionalLayer:
     @scratch.setter
     def scratch(self, t: torch.Tensor) -> None:
         self._scratch = t
+
+    def allocate(self) -> None:
+        """Makes both, so that no call has to (the scratch is zero-filled: under stream capture that fill would only be recorded)."""
+        self.output_gpu, self.scratch
 
     def load_weights(self, weights: torch.Tensor, biases: torch.Tensor) -> None:
         self.weights_gpu.copy_(weights.reshape(self.n, -1))
@@ -109,7 +113,7 @@ def binarize_weights(weights: torch.Tensor, n: int, size: int):
 
 def binary_align_weights(l: ConvolutionalLayer, invert: bool = False, single_calls: bool = True) -> None:
     """binary_align_weights (src-lib/convolutional_layer.cpp:1339): fills align_bit_weights_gpu and mean_arr_gpu.
-    single_calls: also what forward_convolutional_layer_gpu needs (a network that runs the layer its own way does without)."""
+    single_calls: also all that forward_convolutional_layer_gpu needs (a network that runs the layer its own way does without)."""
     l.align_bit_weights_gpu = torch.empty(l.geom.weights_bytes, dtype=torch.uint8, device=l.device)
     capi.check(capi.lib().xnor_b200_binary_align_weights(C.byref(l.desc), l.weights_gpu.data_ptr(),
                                                         l.align_bit_weights_gpu.data_ptr(), l.mean_arr_gpu.data_ptr(),
@@ -121,6 +125,9 @@ def binary_align_weights(l: ConvolutionalLayer, invert: bool = False, single_cal
             l.input_words = GridWords(l.batch, l.c, l.h, l.w, device=l.device)
     else:
         l.conv_words_gpu = None
+    if single_calls:
+        l.allocate()
+        _layer_ops(l)
 
 
 def _version(t: torch.Tensor) -> Optional[int]:

@@ -409,6 +409,10 @@ def calculate_binary_weights(net: Network, packed: Optional[Dict[int, dict]] = N
     fold_maxpools(net)
     if net.sign_chains and net.fuse_first_conv:
         net.plan = network_plan.build(net)
+    if net.plan is None:
+        for l in net.layers:
+            if l.xnor_layer is not None:
+                l.xnor_layer.allocate()                # the layer loop uses both buffers
     torch.cuda.synchronize(dev)
 
 

@@ -138,3 +138,30 @@ def test_shortcuts_and_activations_that_change(shape):
     assert not bool(total.any())
     l.desc.activation = capi.LINEAR
     assert_follows(l, x, plain)
+
+
+def allocations():
+    torch.cuda.synchronize()
+    return torch.cuda.memory_stats()["allocation.all.allocated"]
+
+
+@pytest.mark.parametrize("shape", [WORDS, PACKED], ids=["words", "packed"])
+def test_a_first_call_has_nothing_left_to_make(shape):
+    l, x = build(shape)
+    made = allocations()
+    l.output_gpu, l.scratch
+    L.forward_convolutional_layer_gpu(l, x)
+    assert allocations() == made
+
+
+def test_a_network_of_the_layer_loop_has_its_buffers_when_loaded(tmp_path):
+    from darknet_b200 import cfgs, network
+    cfg, weights = str(tmp_path / "net.cfg"), str(tmp_path / "net.weights")
+    with open(cfg, "w") as fh:
+        fh.write(cfgs.CFGS["yolov3-tiny_xnor"](96, 96))
+    network.write_synthetic_weights(network.parse_network_cfg(cfg, 1, "cpu"), weights)
+    net = network.load_network_custom(cfg, weights, 1, sign_chains=False)
+    assert net.plan is None
+    made = allocations()
+    assert len([(l.xnor_layer.scratch, l.xnor_layer.output_gpu) for l in net.layers if l.xnor_layer is not None]) == 9
+    assert allocations() == made
