@@ -28,6 +28,29 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+class _Replaced:
+    """Counts how often a weight tensor of any layer was replaced by another: what a lowered network (network_plan) looks at before it
+    looks at all of its layers."""
+
+    NAMES = frozenset(("weights_gpu", "biases_gpu", "mean_arr_gpu", "align_bit_weights_gpu", "weights_tc_gpu", "weights_blocked_gpu", "xnor_layer"))
+
+    def __init__(self) -> None:
+        self.count = 0
+
+    def watch(self, cls):
+        """Class decorator: assignments to these attributes of an instance are counted."""
+        def set_attribute(obj, name, value):
+            object.__setattr__(obj, name, value)
+            if name in self.NAMES:
+                self.count += 1
+        cls.__setattr__ = set_attribute
+        return cls
+
+
+replaced = _Replaced()
+
+
+@replaced.watch
 class ConvolutionalLayer:
     """The Darknet::Layer fields the xnor path touches (src-lib/darknet_layers.hpp:39-83, :250-261)."""
 

@@ -50,6 +50,7 @@ def read_cfg(text: str) -> List[Tuple[str, Dict[str, str]]]:
     return sections
 
 
+@L.replaced.watch
 @dataclass
 class Layer:
     type: str
@@ -353,6 +354,7 @@ def fuse_conv_batchnorm(net: Network) -> None:
             l.batch_normalize = 0
 
 
+@torch.inference_mode(False)                           # weights that count the writes to them (network_plan.Plan.current)
 def calculate_binary_weights(net: Network, packed: Optional[Dict[int, dict]] = None) -> None:
     """Packs every xnor conv through the C ABI (or takes its packed weights from `packed`, the entries of a cache file,
     where geometry and weight checksum match), drops the activation of bin_output layers and fuses a same-shape
@@ -823,7 +825,10 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
     A network that was lowered to native operations (network_plan) runs as one call; the loop below runs the others, and every
     network while xnor_b200_set_tuning pins kernels of the packed-operand route."""
     if net.plan is not None and net.plan.takes(x):
-        return net.plan.run(net, x, heads_host)
+        if not net.plan.current():
+            _lower_again(net)
+        if net.plan is not None:
+            return net.plan.run(net, x, heads_host)
     heads: List[torch.Tensor] = []
     cur = x
     side_ctx = None
@@ -927,6 +932,15 @@ def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List
     for done in joins:                                # join: the caller's stream sees both branches finished
         torch.cuda.current_stream().wait_event(done)
     return heads
+
+
+def _lower_again(net: Network) -> None:
+    """A program replaced a layer's weights, or wrote to them: the operations and the filters' copies are made again."""
+    with torch.inference_mode(False):
+        prepare_float_map_convs(net)
+        net.plan = network_plan.build(net)
+    if net.plan is not None and torch.cuda.is_current_stream_capturing():
+        net.plan.versions = None                  # its copies and zeros exist once the captured work has run: not for an ordinary call
 
 
 # ---- detections ----------------------------------------------------------------------------------

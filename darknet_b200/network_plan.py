@@ -10,12 +10,16 @@ between (xnor_b200_conv_words).  fp32 tensors exist where a float layer or a fus
 from __future__ import annotations
 
 import ctypes as C
+import operator
 from typing import Dict, List, Optional, Tuple
 
 import torch
 
 from . import capi
 from . import layer as L
+
+
+_VERSION = operator.attrgetter("_version")
 
 
 class Unsupported(Exception):
@@ -27,14 +31,45 @@ class Plan:
         self.net = net                             # while it is built: a plan that kept it would be a cycle, and its memory wait for the collector
         self.shape = (net.batch, net.c, net.h, net.w)
         self.ops: List[capi.Op] = []
-        self.keep: List = []                       # tensors the operations point at
+        self.keep: List[torch.Tensor] = []         # tensors the operations point at: their memory stays while the plan does
+        self.params: List[Tuple[object, str]] = []    # attributes the operations were made from
+        self.laid_out: List[torch.Tensor] = []     # those of which the operations read a copy in another order
         self.head_layers: List = []
         self.head_direct: List[bool] = []          # a head whose last operation may store into page-locked host memory
         self.signs: Dict[int, L.GridWords] = {}    # layer index -> its (or for a blank [shortcut] the sum's) signs
         self.floats: Dict[int, torch.Tensor] = {}  # layer index -> fp32 tensor of a float layer
         self.events: List[torch.cuda.Event] = []
 
+    def address(self, t: Optional[torch.Tensor]) -> Optional[int]:
+        if t is not None:
+            self.keep.append(t.detach())           # an alias: `t.data = ...` takes no memory away from it
+        return None if t is None else t.data_ptr()
+
+    def param(self, owner, name: str) -> int:
+        """The address of a weight tensor that a program may replace."""
+        self.params.append((owner, name))
+        return self.address(getattr(owner, name))
+
+    def reads_copy_of(self, owner, name: str) -> None:
+        self.params.append((owner, name))
+        if not getattr(owner, name).is_inference():        # made under inference_mode: counts no writes
+            self.laid_out.append(getattr(owner, name))
+
+    def _state(self) -> Tuple[List, List]:
+        return [getattr(o, n) for o, n in self.params], [t._version for t in self.laid_out]
+
+    def current(self) -> bool:
+        """Whether the operations still say what the layers say: no weight tensor was replaced, and none whose copy they read was
+        written to.  Replacing is noticed where it happens (layer.replaced), so a forward only counts the writes."""
+        if self.seen != L.replaced.count:
+            if any(now is not then for now, then in zip(self._state()[0], self.tensors)):
+                return False
+            self.seen = L.replaced.count
+        return list(map(_VERSION, self.laid_out)) == self.versions
+
     def finish(self) -> None:
+        self.seen = L.replaced.count
+        self.tensors, self.versions = self._state()
         self.array = (capi.Op * len(self.ops))(*self.ops)
         self.n_ops = len(self.ops)
         self.heads_type = C.c_void_p * max(1, len(self.head_layers))
@@ -171,7 +206,7 @@ def _build(net) -> Plan:
         elif l.type == "convolutional" and _first_conv(l):
             g = grid(k)
             plan.ops.append(capi.Op(kind=capi.OP_CONV3, arg=2 if pooled_first else 0, pitch=g.pitch, desc=_desc(net, l), input=capi.OP_INPUT,
-                                    output=g.words.data_ptr(), weights=l.weights_gpu.data_ptr(), biases=l.biases_gpu.data_ptr()))
+                                    output=g.words.data_ptr(), weights=plan.param(l, "weights_gpu"), biases=plan.param(l, "biases_gpu")))
         elif l.type == "convolutional":
             _float_conv(plan, k, float_in[k], readers.get(k) == [k + 1])
             if k in sign_read:
@@ -183,7 +218,7 @@ def _build(net) -> Plan:
             src = layers[float_in[k]]
             plan.floats[k] = torch.empty(net.batch, l.out_c, 1, 1, device=net.device)
             plan.ops.append(capi.Op(kind=capi.OP_AVGPOOL, desc=capi.ConvDesc(net.batch, src.out_c, src.out_h, src.out_w),
-                                    input=_tensor(plan, float_in[k]).data_ptr(), output=plan.floats[k].data_ptr()))
+                                    input=plan.address(_tensor(plan, float_in[k])), output=plan.floats[k].data_ptr()))
         elif l.type in ("yolo", "region", "softmax"):
             _head(plan, k, float_in[k])
         if l.branch_end:
@@ -232,7 +267,10 @@ def _xnor_conv(plan: Plan, k: int, sources: List[Source], grid, sign_read: set, 
     l = layers[k]
     xl = l.xnor_layer
     weights = L.conv_words_weights(xl)
-    plan.keep.append(weights)
+    plan.params.append((l, "xnor_layer"))
+    plan.reads_copy_of(xl, "align_bit_weights_gpu")
+    if xl.align_bit_weights_gpu.is_inference():
+        plan.ops.append(capi.Op(kind=capi.OP_FILTERS, arg=1, desc=xl.desc, weights=plan.address(xl.align_bit_weights_gpu), output=weights.data_ptr()))
     io = capi.WordsIO()
     io.n_sources = len(sources)
     for i, (s, pool_stride, pool_pad, up) in enumerate(sources):
@@ -242,41 +280,42 @@ def _xnor_conv(plan: Plan, k: int, sources: List[Source], grid, sign_read: set, 
         io.sources[i] = g.source(pool_stride, pool_pad, up)
     fused = k + 1 < len(layers) and layers[k + 1].blank
     if k in fp32_read:
-        io.output = xl.output_gpu.data_ptr()
+        io.output = plan.address(xl.output_gpu)
     out = k
     if fused:
         out = k + 1
         if k in sign_read:
             raise Unsupported("signs of a layer and of its fused shortcut")
-        io.shortcut_in = _tensor(plan, _float_layer(plan.net, layers[out].input_layers[0])).data_ptr()
+        io.shortcut_in = plan.address(_tensor(plan, _float_layer(plan.net, layers[out].input_layers[0])))
         if out in fp32_read:
-            io.shortcut_out = layers[out].output_gpu.data_ptr()
+            io.shortcut_out = plan.address(layers[out].output_gpu)
         if out in sign_read:
             io.shortcut_signs = grid(out).words.data_ptr()
     elif k in sign_read:
         io.output_signs = grid(k).words.data_ptr()
     g = plan.signs.get(out)
     io.pitch = g.pitch if g is not None else 0
-    plan.ops.append(capi.Op(kind=capi.OP_CONV_WORDS, desc=xl.desc, io=io, weights=weights.data_ptr(), mean_arr=xl.mean_arr_gpu.data_ptr(),
-                            biases=xl.biases_gpu.data_ptr()))
+    plan.ops.append(capi.Op(kind=capi.OP_CONV_WORDS, desc=xl.desc, io=io, weights=plan.address(weights), mean_arr=plan.param(xl, "mean_arr_gpu"),
+                            biases=plan.param(xl, "biases_gpu")))
 
 
 def _float_conv(plan: Plan, k: int, src: int, one_reader: bool) -> None:
     """A float convolution behind the path; in front of a [yolo] layer that alone reads it with that layer's activation, into the head."""
     net, l = plan.net, plan.net.layers[k]
     nxt = net.layers[k + 1] if k + 1 < len(net.layers) else None
-    op = capi.Op(desc=_desc(net, l), input=_tensor(plan, src).data_ptr(), biases=l.biases_gpu.data_ptr())
+    op = capi.Op(desc=_desc(net, l), input=plan.address(_tensor(plan, src)), biases=plan.param(l, "biases_gpu"))
     head = one_reader and nxt is not None and nxt.type == "yolo" and l.activation == "linear" and float(nxt.opts.get("scale_x_y", 1)) == 1.0
     entries = 5 + int(nxt.opts.get("classes", 20)) if head else 0
     head = head and l.n % entries == 0
     if l.weights_blocked_gpu is not None:
-        op.kind, op.weights = capi.OP_FLOAT_MAP, l.weights_blocked_gpu.data_ptr()
+        op.kind, op.weights = capi.OP_FLOAT_MAP, plan.param(l, "weights_blocked_gpu")
         if not l.yolo_entries:
             head = False
     elif l.weights_tc_gpu is not None:
-        op.kind, op.weights = capi.OP_FLOAT_TC, l.weights_tc_gpu.data_ptr()
+        op.kind, op.weights = capi.OP_FLOAT_TC, plan.param(l, "weights_tc_gpu")
     else:
         raise Unsupported("a float convolution of another shape")
+    plan.reads_copy_of(l, "weights_gpu")
     if head:
         op.arg = entries
         op.output = capi.OP_HEAD + len(plan.head_layers)           # the [yolo] layer behind it adds itself
@@ -295,7 +334,7 @@ def _head(plan: Plan, k: int, src: int) -> None:
         plan.head_direct.append(conv.kind == capi.OP_FLOAT_MAP)
         return
     plan.head_direct.append(False)
-    op = capi.Op(desc=capi.ConvDesc(net.batch, l.c, l.h, l.w), input=_tensor(plan, src).data_ptr(), output=slot)
+    op = capi.Op(desc=capi.ConvDesc(net.batch, l.c, l.h, l.w), input=plan.address(_tensor(plan, src)), output=slot)
     if l.type == "softmax":
         op.kind = capi.OP_SOFTMAX
     elif l.type == "yolo" and float(l.opts.get("scale_x_y", 1)) == 1.0:

@@ -70,3 +70,69 @@ def test_a_route_may_read_the_convolution_in_front_of_a_yolo_layer(batch, width,
     net, got, want = both(tmp_path, [cfgs._conv(32, 3), cfgs._conv(160, 3, xnor=1), HEAD, YOLO, "[route]\nlayers=-2\n", YOLO], batch, width, height)
     assert net.plan is not None and torch.equal(got[0], got[1])
     assert_heads_close(got, want)
+
+
+def pour(net, other, how):
+    """other's weights into net's layers."""
+    for l, o in zip(net.layers, other.layers):
+        if l.type != "convolutional":
+            continue
+        pairs = [(l, o, "biases_gpu")]
+        pairs += [(l.xnor_layer, o.xnor_layer, n) for n in ("align_bit_weights_gpu", "mean_arr_gpu", "biases_gpu")] if l.xnor else [(l, o, "weights_gpu")]
+        for to, of, name in pairs:
+            if how == "written":
+                getattr(to, name).copy_(getattr(of, name))
+            else:
+                setattr(to, name, getattr(of, name).clone())
+
+
+@pytest.mark.parametrize("how", ["written", "replaced"])
+@pytest.mark.parametrize("name,batch", [("yolov3-tiny_xnor", 1), ("yolov3-tiny_xnor", 8), ("darknet53_448_xnor", 2)])
+def test_weights_that_change_behind_the_plan(name, batch, how, tmp_path):
+    size = 160
+    cfg = tmp_path / "net.cfg"
+    cfg.write_text(cfgs.CFGS[name](size, size))
+    nets = []
+    for seed in (1, 2):
+        network.write_synthetic_weights(network.parse_network_cfg(str(cfg), 1, "cpu"), str(tmp_path / "w"), seed)
+        nets.append(network.load_network_custom(str(cfg), str(tmp_path / "w"), batch))
+    net, other = nets
+    x = image(batch, size, size)
+    first, want = ([h.clone() for h in network.forward_network_gpu(n, x)] for n in nets)
+    assert not any(torch.equal(a, b) for a, b in zip(first, want))
+    pour(net, other, how)
+    plan = net.plan
+    for _ in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(network.forward_network_gpu(net, x), want))
+    assert net.plan is not None and net.plan is not plan
+    plan = net.plan
+    network.forward_network_gpu(net, x)
+    assert net.plan is plan
+    # changed again, and the first forward behind it only captured
+    stream = torch.cuda.Stream()
+    pour(net, network.load_network_custom(str(cfg), str(tmp_path / "w"), batch), how)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        heads = network.forward_network_gpu(net, x)
+    assert all(torch.equal(a, b) for a, b in zip(network.forward_network_gpu(net, x), want))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(heads, want))
+
+
+def test_weights_made_under_inference_mode(tmp_path):
+    cfg, weights = write(tmp_path, [cfgs._conv(32, 3), cfgs._conv(160, 3, xnor=1), HEAD, YOLO], 64, 48)
+    (tmp_path / "2").mkdir()
+    _, weights2 = write(tmp_path / "2", [cfgs._conv(32, 3), cfgs._conv(160, 3, xnor=1), HEAD, YOLO], 64, 48, seed=9)
+    x = image(1, 64, 48)
+    with torch.inference_mode():
+        net, other = network.load_network_custom(cfg, weights), network.load_network_custom(cfg, weights2)
+        want = network.forward_network_gpu(other, x)[0].clone()
+        xl, ol = net.layers[1].xnor_layer, other.layers[1].xnor_layer
+        pour(net, other, "written")
+        assert torch.equal(network.forward_network_gpu(net, x)[0], want)
+        xl.align_bit_weights_gpu = torch.zeros_like(ol.align_bit_weights_gpu)       # counts no writes
+        assert not torch.equal(network.forward_network_gpu(net, x)[0], want)
+        xl.align_bit_weights_gpu.copy_(ol.align_bit_weights_gpu)
+        assert torch.equal(network.forward_network_gpu(net, x)[0], want)

@@ -28,6 +28,7 @@ def lowered(sections, tmp_path, monkeypatch, batch=2, width=64, height=64):
         l.weights_gpu, l.biases_gpu = torch.zeros(l.n, l.c, l.size, l.size), torch.zeros(l.n)
         if l.xnor:
             l.xnor_layer = L.ConvolutionalLayer(batch, l.h, l.w, l.c, l.n, l.size, l.stride, l.pad, capi.LEAKY, "cpu")
+            l.xnor_layer.align_bit_weights_gpu = torch.zeros(l.xnor_layer.geom.weights_bytes, dtype=torch.uint8)
             nxt = net.layers[l.index + 1] if l.index + 1 < len(net.layers) else None
             if nxt is not None and nxt.type == "shortcut" and nxt.activation == "linear":
                 nxt.blank, nxt.output_gpu = True, torch.zeros(batch, nxt.out_c, nxt.out_h, nxt.out_w)
@@ -76,3 +77,34 @@ def test_a_route_may_read_the_convolution_in_front_of_a_yolo_layer(tmp_path, mon
     convs, heads = [[op for op in net.plan.ops if op.kind == k] for k in (capi.OP_FLOAT_TC, capi.OP_YOLO)]
     assert len(convs) == 1 and convs[0].arg == 0 and convs[0].output not in (capi.OP_HEAD, capi.OP_HEAD + 1)
     assert [op.output for op in heads] == [capi.OP_HEAD, capi.OP_HEAD + 1] and all(op.input == convs[0].output for op in heads)
+
+
+def test_a_plan_notices_weights_that_change(tmp_path, monkeypatch):
+    net = lowered([conv(32, 3), conv(160, 3, xnor=1), head_conv(), YOLO], tmp_path, monkeypatch)
+    other = lowered([conv(32, 3), conv(160, 3, xnor=1), head_conv(), YOLO], tmp_path, monkeypatch)
+    first, xnor, last = net.layers[:3]
+    xl = xnor.xnor_layer
+    changes = [lambda: xl.align_bit_weights_gpu.fill_(3), lambda: last.weights_gpu.mul_(2)]
+    for owner, name in ((first, "weights_gpu"), (first, "biases_gpu"), (xl, "mean_arr_gpu"), (xl, "biases_gpu"), (xl, "align_bit_weights_gpu"),
+                        (last, "biases_gpu"), (last, "weights_gpu"), (last, "weights_tc_gpu")):
+        changes.append(lambda owner=owner, name=name: setattr(owner, name, getattr(owner, name).clone()))
+    changes.append(lambda: setattr(xnor, "xnor_layer", other.layers[1].xnor_layer))
+    for change in changes:
+        assert net.plan.current()
+        change()
+        assert not net.plan.current()
+        net.plan = network_plan.build(net)
+    # what the operations read in place, and other networks, change nothing
+    xl = xnor.xnor_layer
+    for t in (first.weights_gpu, first.biases_gpu, xl.mean_arr_gpu, xl.biases_gpu, last.biases_gpu):
+        t.add_(1)
+    other.layers[0].weights_gpu = torch.zeros(1)
+    assert net.plan.current() and not other.plan.current()
+
+
+def test_a_plan_keeps_the_memory_it_names(tmp_path, monkeypatch):
+    net = lowered([conv(32, 3), conv(160, 3, xnor=1), head_conv(), YOLO], tmp_path, monkeypatch)
+    named = {op.weights for op in net.plan.ops} | {op.biases for op in net.plan.ops} | {op.mean_arr for op in net.plan.ops}
+    named |= {op.input for op in net.plan.ops} | {op.io.output for op in net.plan.ops}
+    held = {t.data_ptr() for t in net.plan.keep}
+    assert named - {None, capi.OP_INPUT} <= held
