@@ -27,7 +27,7 @@ EXPORTS = (
     "xnor_b200_pack_input_pooled", "xnor_b200_conv_forward_pooled", "xnor_b200_float_conv_small", "xnor_b200_float_conv3_io", "xnor_b200_float_conv_map_weights_bytes",
     "xnor_b200_float_conv_map_prepare", "xnor_b200_float_conv_map", "xnor_b200_float_conv_map_yolo", "xnor_b200_float_conv_1x1_tc", "xnor_b200_yolo_activate", "xnor_b200_region_activate", "xnor_b200_conv_forward_io", "xnor_b200_conv_takes_masks", "xnor_b200_tap_major_weights",
     "xnor_b200_yolo_detections", "xnor_b200_nms_sort", "xnor_b200_detection_rows", "xnor_b200_detect", "xnor_b200_rows_to_host",
-    "xnor_b200_avgpool", "xnor_b200_softmax", "xnor_b200_run_ops", "xnor_b200_float_conv3_words", "xnor_b200_float_conv_tc", "xnor_b200_float_conv_tc_prepare", "xnor_b200_float_conv_tc_weights_bytes", "xnor_b200_conv_words", "xnor_b200_conv_words_weights", "xnor_b200_conv_words_weights_bytes", "xnor_b200_sign_words", "xnor_b200_grid_block_words", "xnor_b200_grid_front",
+    "xnor_b200_avgpool", "xnor_b200_softmax", "xnor_b200_run_ops", "xnor_b200_float_conv3_words", "xnor_b200_float_conv_tc", "xnor_b200_float_conv_tc_prepare", "xnor_b200_float_conv_tc_weights_bytes", "xnor_b200_conv_words", "xnor_b200_conv_words_plan", "xnor_b200_conv_words_weights", "xnor_b200_conv_words_weights_bytes", "xnor_b200_sign_words", "xnor_b200_grid_block_words", "xnor_b200_grid_front",
     "xnor_b200_measure_popc_peak", "xnor_b200_measure_bmma_peak", "xnor_b200_measure_umma_i8_peak", "xnor_b200_measure_umma_mxf4_peak",
 )
 
@@ -66,6 +66,12 @@ class WordsIO(C.Structure):
     """struct xnor_b200_words_io"""
     _fields_ = [("sources", WordsSource * 2), ("n_sources", C.c_int), ("output", C.c_void_p), ("output_signs", C.c_void_p),
                 ("shortcut_in", C.c_void_p), ("shortcut_out", C.c_void_p), ("shortcut_signs", C.c_void_p), ("pitch", C.c_int)]
+
+
+class WordsPlan(C.Structure):
+    """struct xnor_b200_words_plan"""
+    _fields_ = [(n, C.c_int) for n in ("filters", "tiles", "units", "ctas", "stages", "streamed")] + [("smem_bytes", C.c_size_t)] + \
+               [(n, C.c_int) for n in ("run_words_min", "run_words_max", "run_room")] + [("cycles", C.c_double)]
 
 
 (OP_CONV3, OP_SIGN_WORDS, OP_CONV_WORDS, OP_FLOAT_MAP, OP_FLOAT_TC, OP_YOLO, OP_REGION, OP_AVGPOOL, OP_SOFTMAX, OP_FORK,
@@ -179,6 +185,7 @@ def lib() -> C.CDLL:
     L.xnor_b200_conv_words_weights_bytes.argtypes = [dp]
     L.xnor_b200_conv_words_weights.argtypes = [dp, vp, vp, vp]
     L.xnor_b200_conv_words.argtypes = [dp, C.POINTER(WordsIO), vp, vp, vp, vp]
+    L.xnor_b200_conv_words_plan.argtypes = [dp, C.POINTER(WordsIO), C.POINTER(WordsPlan)]
     L.xnor_b200_sign_words.argtypes = [vp, ci, ci, ci, ci, ci, vp, vp]
     L.xnor_b200_grid_block_words.restype = sz
     L.xnor_b200_grid_block_words.argtypes = [ci, ci, ci]

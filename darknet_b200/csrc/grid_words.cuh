@@ -28,6 +28,13 @@ static FastDiv make_div(uint32_t d)
 	return f;
 }
 
-__device__ __forceinline__ int fdiv(int n, const FastDiv & f) { return (f.d <= 1) ? n : (int)(__umulhi((uint32_t)n, f.mul) >> f.shift); }
+__host__ __device__ __forceinline__ int fdiv(int n, const FastDiv & f)
+{
+#ifdef __CUDA_ARCH__
+	return (f.d <= 1) ? n : (int)(__umulhi((uint32_t)n, f.mul) >> f.shift);
+#else
+	return (f.d <= 1) ? n : (int)((uint32_t)(((uint64_t)(uint32_t)n * f.mul) >> 32) >> f.shift);
+#endif
+}
 
 }  // namespace xnor

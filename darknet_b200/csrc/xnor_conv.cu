@@ -256,7 +256,7 @@ struct XcRun
 	int start, words, shift;
 };
 
-__device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSource & src, int u)
+__host__ __device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSource & src, int u)
 {
 	XcRun r;
 	const int pos0 = u * p.pt * TC_PIX - p.halo;
@@ -979,10 +979,13 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 
 // ---- host side ----------------------------------------------------------------------------------------------------------
 
-// Shapes the kernel takes: 3x3 / pad 1 or 1x1 / pad 0, stride 1 or 2.
+// Shapes the kernel's indices take: 3x3 / pad 1 or 1x1 / pad 0, stride 1 or 2.  Whether a window fits is the plan's to say.
 static bool shape_taken(const xnor_b200_conv_desc & d)
 {
 	if (!((d.size == 3 && d.pad == 1) || (d.size == 1 && d.pad == 0)) || (d.stride != 1 && d.stride != 2)) { return false; }
+	const long long blocks = (d.c + 31) / 32;
+	if (blocks * d.size * d.size > 65535) { return false; }                      // grid rows of conv_words_weights_kernel
+	if (blocks * (d.batch * (d.h + 1LL) * (d.w + 1) + d.w + 64) > 0x7fff0000LL) { return false; }      // words that sign_words counts
 	// the source's grid is the larger one; a fused 2x2 max-pool doubles it again
 	return (long long)d.batch * (2LL * d.h + 2) * (4LL * d.w + 16) < 0x7ffff000LL;
 }
@@ -1118,10 +1121,9 @@ static XcPlan best_plan(const XcParams & p, int mode)
 	return best;
 }
 
-template <int MODE>
-static int launch_mode(XcParams & p, cudaStream_t stream)
+static int apply_plan(XcParams & p, int mode, XcPlan & best)
 {
-	XcPlan best = best_plan(p, MODE);
+	best = best_plan(p, mode);
 	if (best.cost >= 1e30) { return XNOR_B200_ERR_TOO_LARGE; }
 	p.pt = best.pt;
 	p.G = best.g; p.stages_k = best.stages_k; p.ring = best.ring; p.kw_full = best.kw_full;
@@ -1134,8 +1136,17 @@ static int launch_mode(XcParams & p, cudaStream_t stream)
 	p.fgroups = (p.M + best.nf - 1) / best.nf;
 	const int lanes = sm_count() / p.fgroups;
 	best.grid = p.fgroups * ((p.units < lanes) ? p.units : lanes);
+	return XNOR_B200_OK;
+}
+
+template <int MODE>
+static int launch_mode(XcParams & p, cudaStream_t stream)
+{
+	XcPlan best;
+	int rc = apply_plan(p, MODE, best);
+	if (rc != XNOR_B200_OK) { return rc; }
 	TcParams common = {};
-	const int rc = tc_fill_launch_fields(common);
+	rc = tc_fill_launch_fields(common);
 	if (rc != XNOR_B200_OK) { return rc; }
 	p.status = common.status; p.spin_limit = common.spin_limit; p.withhold = common.withhold;
 	if (best.stream) { return launch_conv<128, MODE, true>(p, best, stream); }
@@ -1184,6 +1195,14 @@ extern "C" int xnor_b200_grid_front(int pitch) { return (pitch > 1) ? grid_front
 extern "C" size_t xnor_b200_conv_words_weights_bytes(const xnor_b200_conv_desc * desc)
 {
 	if (desc == nullptr || validate_desc(desc) != XNOR_B200_OK || !shape_taken(*desc)) { return 0; }
+	alignas(16) static const uint32_t any[4] = {};
+	xnor_b200_words_io io = {};
+	io.n_sources = 1;
+	io.sources[0].words = any;
+	io.sources[0].blocks = (desc->c + 31) / 32;
+	io.sources[0].h = desc->h; io.sources[0].w = desc->w;
+	io.output = (float *)any;
+	if (xnor_b200_conv_words_plan(desc, &io, nullptr) != XNOR_B200_OK) { return 0; }
 	XcParams p = {};
 	fill_params(*desc, p, 0);
 	return (size_t)p.kwords * round_up((size_t)p.M, 128) * 4;
@@ -1197,8 +1216,7 @@ extern "C" int xnor_b200_conv_words_weights(const xnor_b200_conv_desc * desc, co
 	if (!shape_taken(*desc)) { return XNOR_B200_ERR_INVALID; }
 	if (((uintptr_t)align_bit_weights & 3u) != 0 || ((uintptr_t)conv_weights & 15u) != 0) { return XNOR_B200_ERR_ALIGNMENT; }
 	const int taps = desc->size * desc->size;
-	const long long kwords = (long long)(desc->c + 31) / 32 * taps;
-	if (kwords > 65535) { return XNOR_B200_ERR_TOO_LARGE; }
+	const int kwords = (desc->c + 31) / 32 * taps;
 	conv_words_weights_kernel<<<dim3((unsigned)((desc->n + 127) / 128), (unsigned)kwords, 1), 128, 0, (cudaStream_t)stream>>>(
 			(const uint32_t *)align_bit_weights, conv_weights, desc->n, desc->c, taps, desc->stride, aligned_lda(taps * desc->c) / 32);
 	return check_launch();
@@ -1275,4 +1293,26 @@ extern "C" int xnor_b200_conv_words(const xnor_b200_conv_desc * desc, const xnor
 	cudaStream_t s = (cudaStream_t)stream;
 	if (mode == 2) { return launch_mode<2>(p, s); }
 	return (mode == 1) ? launch_mode<1>(p, s) : launch_mode<0>(p, s);
+}
+
+extern "C" int xnor_b200_conv_words_plan(const xnor_b200_conv_desc * desc, const xnor_b200_words_io * io, xnor_b200_words_plan * plan)
+{
+	XcParams p = {};
+	int mode = 0;
+	int rc = conv_words_params(desc, io, p, &mode);
+	if (rc != XNOR_B200_OK) { return rc; }
+	XcPlan best;
+	rc = apply_plan(p, mode, best);
+	if (rc != XNOR_B200_OK || plan == nullptr) { return rc; }
+	*plan = {best.nf, best.pt, p.units, best.grid, best.ring, best.stream, best.smem, 0x7fffffff, 0, best.raw_words, best.cost};
+	for (int u = 0; u < p.units; ++u)
+	{
+		for (int i = 0; i < p.n_src; ++i)
+		{
+			const int words = run_of(p, p.src[i], u).words;
+			plan->run_words_min = min(plan->run_words_min, words);
+			plan->run_words_max = max(plan->run_words_max, words);
+		}
+	}
+	return XNOR_B200_OK;
 }

@@ -295,6 +295,8 @@ def _xnor_conv(plan: Plan, k: int, sources: List[Source], grid, sign_read: set, 
         io.output_signs = grid(k).words.data_ptr()
     g = plan.signs.get(out)
     io.pitch = g.pitch if g is not None else 0
+    if capi.lib().xnor_b200_conv_words_plan(C.byref(xl.desc), C.byref(io), None) != capi.OK:
+        raise Unsupported("a map too wide for the sign-word convolution")
     plan.ops.append(capi.Op(kind=capi.OP_CONV_WORDS, desc=xl.desc, io=io, weights=plan.address(weights), mean_arr=plan.param(xl, "mean_arr_gpu"),
                             biases=plan.param(xl, "biases_gpu")))
 

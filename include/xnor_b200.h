@@ -327,7 +327,7 @@ typedef struct xnor_b200_words_io
 } xnor_b200_words_io;
 
 /* The filters in the order this kernel reads them, made once at load time from xnor_b200_binary_align_weights(invert = 0):
- * bytes of the copy (0: a shape it does not take), and the copy itself. */
+ * bytes of the copy (0: a shape it does not take, from one source of its own size), and the copy itself. */
 XNOR_B200_API size_t xnor_b200_conv_words_weights_bytes(const xnor_b200_conv_desc * desc);
 XNOR_B200_API int xnor_b200_conv_words_weights(const xnor_b200_conv_desc * desc, const uint8_t * align_bit_weights, uint32_t * conv_weights,
 		void * stream);
@@ -338,6 +338,20 @@ XNOR_B200_API int xnor_b200_sign_words(const float * input, int batch, int c, in
 
 XNOR_B200_API int xnor_b200_conv_words(const xnor_b200_conv_desc * desc, const xnor_b200_words_io * io, const uint32_t * conv_weights,
 		const float * mean_arr, const float * biases, void * stream);
+
+/* How xnor_b200_conv_words would run this call: its return value without the launch (XNOR_B200_ERR_TOO_LARGE: rows too wide, or channels
+ * too many, for a window in shared memory; xnor_b200_conv_forward takes such a layer), and in *plan, unless NULL: filters per CTA,
+ * tiles of 128 positions per unit of work, units, CTAs, operand stages, whether filters are streamed, dynamic shared memory, and over all
+ * units and sources the smallest and largest run of sign words of a channel block that a unit copies, and the room for one.  Host only. */
+typedef struct xnor_b200_words_plan
+{
+	int filters, tiles, units, ctas, stages, streamed;
+	size_t smem_bytes;
+	int run_words_min, run_words_max, run_room;
+	double cycles;
+} xnor_b200_words_plan;
+
+XNOR_B200_API int xnor_b200_conv_words_plan(const xnor_b200_conv_desc * desc, const xnor_b200_words_io * io, xnor_b200_words_plan * plan);
 
 /* The float convolution in front of the path (3 input channels -> 16/32 filters in the xnor networks): the float
  * branch of forward_convolutional_layer_gpu (src-lib/convolutional_kernels.cu:373-434, cuDNN or im2col + sgemm) +

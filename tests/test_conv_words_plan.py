@@ -1,0 +1,55 @@
+"""Which layers xnor_b200_conv_words takes, and how it would run them (host arithmetic only)."""
+import ctypes as C
+
+import pytest
+
+pytest.importorskip("torch")
+
+from darknet_b200 import capi  # noqa: E402
+
+WORDS = (C.c_uint32 * 8)()
+ADDRESS = (C.addressof(WORDS) + 15) // 16 * 16
+
+
+def plan(batch, c, h, w, n, ks, stride, sources=None, pitch=0):
+    """(return value, plan) of a layer that writes fp32; sources: (channels, h, w, pool stride, pool pad, upsample, pitch) each."""
+    d = capi.ConvDesc(batch, c, h, w, n, ks, stride, ks // 2, capi.LINEAR)
+    io, out = capi.WordsIO(output=ADDRESS, pitch=pitch), capi.WordsPlan()
+    sources = sources or [(c, h, w, 0, 0, 0, 0)]
+    io.n_sources = len(sources)
+    for i, (sc, sh, sw, ps, pp, up, sp) in enumerate(sources):
+        io.sources[i] = capi.WordsSource(ADDRESS, (sc + 31) // 32, sh, sw, ps, pp, up, sp)
+    return capi.lib().xnor_b200_conv_words_plan(C.byref(d), C.byref(io), C.byref(out)), out
+
+
+def takes(*shape):
+    batch, c, h, w, n, ks, stride = shape
+    return capi.lib().xnor_b200_conv_words_weights_bytes(C.byref(capi.ConvDesc(batch, c, h, w, n, ks, stride, ks // 2, capi.LINEAR))) > 0
+
+
+TOO_LARGE = 6
+
+
+@pytest.mark.parametrize("shape", [
+    (1, 32, 64, 703, 64, 3, 1), (1, 1024, 13, 1408, 64, 3, 1), (1, 64, 64, 1000, 64, 3, 2), (1, 1024, 14, 400, 64, 3, 2), (1, 64, 8, 2300, 64, 1, 2),
+    (1, 32, 8, 8, 148 * 128 + 1, 1, 1), (1, 250_000, 4, 4, 32, 3, 1),
+], ids=lambda s: "b%d_c%d_%dx%d_n%d_k%d_s%d" % s)
+def test_what_has_no_plan_has_no_filters_copy(shape):
+    """The size of the filters' copy is the question that callers ask: it must not promise a launch that is then refused."""
+    assert not takes(*shape)
+    assert plan(*shape)[0] in (TOO_LARGE, 1)
+
+
+@pytest.mark.parametrize("c,n,ks,stride", [(32, 64, 3, 1), (16, 8, 3, 1), (1024, 1024, 3, 1), (64, 64, 3, 2), (512, 96, 3, 2), (1024, 64, 1, 2), (48, 48, 1, 1)])
+def test_the_two_questions_agree_at_every_width(c, n, ks, stride):
+    limits = []
+    for w in list(range(1, 40)) + list(range(40, 2500, 37)) + [702, 703]:
+        ok = plan(2, c, 20, w, n, ks, stride)[0] == capi.OK
+        assert takes(2, c, 20, w, n, ks, stride) == ok
+        limits += [w] if ok else []
+    assert limits and (max(limits) >= 321)
+
+
+def test_a_pool_in_front_narrows_what_fits():
+    assert plan(1, 256, 64, 640, 64, 3, 1)[0] == capi.OK
+    assert plan(1, 256, 64, 640, 64, 3, 1, [(256, 128, 1280, 2, 1, 0, 0)])[0] == TOO_LARGE

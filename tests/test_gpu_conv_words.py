@@ -151,3 +151,23 @@ def test_a_wait_that_runs_out_is_reported():
     L.conv_words(l, wts, [words.source()], output=out)
     capi.check(capi.lib().xnor_b200_take_device_status(capi.C.byref(status)), "status")
     assert status.value == 0 and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("case", [
+    (2, 32, 5, 702, 32, 3, 1), (2, 32, 5, 703, 32, 3, 1), (1, 64, 3, 1408, 64, 3, 1), (1, 512, 2, 700, 64, 3, 1),
+    (1, 64, 5, 850, 64, 3, 2), (1, 64, 5, 851, 64, 3, 2), (1, 64, 4, 1500, 32, 3, 2), (1, 1024, 3, 321, 32, 3, 2), (1, 1024, 3, 322, 32, 3, 2),
+    (1, 64, 3, 2246, 32, 1, 2), (1, 64, 3, 2247, 32, 1, 2), (1, 64, 2, 3000, 32, 1, 1), (1, 32, 5, 5, 148 * 128 + 32, 3, 1),
+], ids=lambda c: "b%d_c%d_%dx%d_n%d_k%d_s%d" % c)
+def test_layers_at_the_widest_maps_and_beyond(case):
+    """Where the kernel has no plan the layer keeps the packed route."""
+    l, x = build(*case, leaky=True, seed=4)
+    want = reference(l, x)
+    l.output_gpu.fill_(float("nan"))
+    assert torch.equal(L.forward_convolutional_layer_gpu(l, x), want)
+    wts = L.conv_words_weights(l)
+    assert (wts is None) == (case[3] in (703, 1408, 851, 1500, 322, 2247) or case[4] > 148 * 128)
+    if wts is not None:
+        out = torch.full_like(want, float("nan"))
+        words = L.sign_words(x)
+        L.conv_words(l, wts, [words.source()], output=out)
+        assert torch.equal(out, want)

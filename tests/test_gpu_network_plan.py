@@ -136,3 +136,13 @@ def test_weights_made_under_inference_mode(tmp_path):
         assert not torch.equal(network.forward_network_gpu(net, x)[0], want)
         xl.align_bit_weights_gpu.copy_(ol.align_bit_weights_gpu)
         assert torch.equal(network.forward_network_gpu(net, x)[0], want)
+
+
+@pytest.mark.parametrize("name", sorted(cfgs.CFGS))
+@pytest.mark.parametrize("width", [704, 1376, 1408, 1920])
+def test_wide_networks(name, width, tmp_path):
+    """Past some width the sign-word kernel has no plan for a layer and the network runs in the layer loop."""
+    sections = cfgs.CFGS[name](width, 64).split("\n[", 1)[1]
+    net, got, want = both(tmp_path, ["[" + sections], 1, width, 64)
+    assert width < 1408 or net.plan is None
+    assert_heads_close(got, want)

@@ -108,3 +108,11 @@ def test_a_plan_keeps_the_memory_it_names(tmp_path, monkeypatch):
     named |= {op.input for op in net.plan.ops} | {op.io.output for op in net.plan.ops}
     held = {t.data_ptr() for t in net.plan.keep}
     assert named - {None, capi.OP_INPUT} <= held
+
+
+@pytest.mark.parametrize("name", sorted(cfgs.CFGS))
+def test_networks_too_wide_for_the_kernel_keep_to_the_layer_loop(name, tmp_path, monkeypatch):
+    for width, fits in ((608, True), (1408, False), (1920, False)):
+        sections = cfgs.CFGS[name](width, 64).split("\n[", 1)[1]
+        net = lowered(["[" + sections], tmp_path, monkeypatch, batch=1, width=width)
+        assert (net.plan is not None) == fits, width
