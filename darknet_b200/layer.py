@@ -159,14 +159,24 @@ def _version(t: torch.Tensor) -> Optional[int]:
 
 
 def takes_words(l: ConvolutionalLayer) -> bool:
-    """Whether a single layer call runs as sign words + xnor_b200_conv_words or as packed operand + GEMM.  Measured on B200 over 44
-    shapes (7..208 pixels a side, 8..1024 channels and filters, batch 1..64): 3x3 layers 0.07 to 1.05 of the packed route's time,
+    """Whether a single layer call runs as sign words + xnor_b200_conv_words or as packed operand + GEMM.  Measured on B200 over some 700
+    shapes (7..640 pixels a side, 8..1024 channels and filters, batch 1..64): 3x3 layers 0.07 to 1.05 of the packed route's time,
     1x1 layers whose channels fill no whole words 0.07 to 1.08.  1x1 layers over whole words gain from a few million fp32 values
-    or some hundred million binary operations on (0.6 to 1.06) and lose below (1.0 to 1.4: two kernels of 3 us each do all of it)."""
-    if l.size == 1 and l.c % 32 == 0:
+    or some hundred million binary operations on (0.6 to 1.06) and lose below (1.0 to 1.4: two kernels of 3 us each do all of it),
+    or where a stride drops most of what 1024 channels had their signs taken for (1.06 to 1.49).
+    Wide maps of deep layers: a tile's window is mostly halo, and each group of filters widens it again.  3x3 at stride 2, 512 channels to
+    512 filters: 208x416 194 us against 98, 152x304 64 / 64; to 1024 filters: 80x160 b8 206 / 160, 104x208 b8 323 / 261.  At stride 1
+    512 -> 1024 120x480 382 / 277, 1024 -> 256 75x300 127 / 95; 512 -> 512 208x416 196 / 234 on the other side of the line.  Layers of
+    few operations gain at every width (512 -> 512 13x208 at stride 2 18 / 31, at stride 1 13x500 38 / 43)."""
+    if l.c % 32 != 0:
+        return True
+    binops = 2 * l.batch * l.outputs * l.c * l.size * l.size
+    if l.size == 1:
         floats = l.batch * (l.c * l.h * l.w // (l.stride * l.stride) + l.outputs)
-        return floats > 4_000_000 or 2 * l.batch * l.outputs * l.c > 250_000_000
-    return True
+        return (floats > 4_000_000 or binops > 250_000_000) and not (l.stride == 2 and l.c >= 1024)
+    if l.stride == 2:
+        return not (l.c >= 512 and l.n >= 512 and l.w >= 160 and binops > 20_000_000_000)
+    return not (l.c >= 512 and l.n >= 256 and l.c * l.w > 230_000 and l.w >= 256 and binops > 40_000_000_000)
 
 
 def pack_input(l: ConvolutionalLayer, x: torch.Tensor) -> torch.Tensor:

@@ -5,7 +5,7 @@ import pytest
 
 pytest.importorskip("torch")
 
-from darknet_b200 import capi  # noqa: E402
+from darknet_b200 import capi, layer as L  # noqa: E402
 
 WORDS = (C.c_uint32 * 8)()
 ADDRESS = (C.addressof(WORDS) + 15) // 16 * 16
@@ -53,3 +53,19 @@ def test_the_two_questions_agree_at_every_width(c, n, ks, stride):
 def test_a_pool_in_front_narrows_what_fits():
     assert plan(1, 256, 64, 640, 64, 3, 1)[0] == capi.OK
     assert plan(1, 256, 64, 640, 64, 3, 1, [(256, 128, 1280, 2, 1, 0, 0)])[0] == TOO_LARGE
+
+
+@pytest.mark.parametrize("shape,words", [
+    ((1, 512, 208, 416, 512, 3, 2), False), ((8, 512, 104, 208, 1024, 3, 2), False), ((8, 1024, 80, 160, 1024, 3, 2), False),
+    ((8, 512, 104, 208, 256, 3, 2), True), ((1, 512, 13, 208, 512, 3, 2), True), ((8, 512, 52, 104, 512, 3, 2), True), ((64, 256, 56, 56, 512, 3, 2), True),
+    ((1, 512, 120, 480, 1024, 3, 1), False), ((1, 1024, 75, 300, 256, 3, 1), False), ((1, 512, 208, 416, 512, 3, 1), True), ((1, 512, 13, 500, 512, 3, 1), True),
+    ((8, 1024, 104, 208, 1024, 3, 1), True), ((1, 75, 120, 700, 64, 3, 1), True), ((1, 1000, 75, 300, 256, 3, 1), True),
+    ((1, 1024, 13, 13, 256, 1, 1), False), ((64, 256, 56, 56, 64, 1, 1), True), ((8, 1024, 52, 104, 1024, 1, 2), False), ((8, 512, 52, 104, 512, 1, 2), True),
+], ids=str)
+def test_the_faster_route_is_taken(shape, words):
+    """Both sides of the lines, with the shapes they were measured at."""
+    batch, c, h, w, n, ks, stride = shape
+    l = L.ConvolutionalLayer.__new__(L.ConvolutionalLayer)
+    l.batch, l.c, l.h, l.w, l.n, l.size, l.stride = batch, c, h, w, n, ks, stride
+    l.outputs = n * ((h + 2 * (ks // 2) - ks) // stride + 1) * ((w + 2 * (ks // 2) - ks) // stride + 1)
+    assert L.takes_words(l) == words
