@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libxnor_b200.so")
 OK = 0
 LINEAR = 0
 LEAKY = 1
+DETECT_HEADS = 4                # XNOR_B200_DETECT_HEADS
 STATIC_SCRATCH_BYTES = 8 << 20  # XNOR_B200_STATIC_SCRATCH_BYTES
 
 # Every symbol include/xnor_b200.h declares; tests check that the library exports each one.

@@ -31,7 +31,7 @@ constexpr int DET_WARPS = DET_THREADS / 32;
 constexpr int DET_ALL_WARPS = DET_CLUSTER * DET_WARPS;
 constexpr int DET_STEP = 4;               // candidates a thread looks at between two scans
 constexpr int DET_MAX_ANCHORS = 16;
-constexpr int DET_MAX_HEADS = 4;
+constexpr int DET_MAX_HEADS = XNOR_B200_DETECT_HEADS;
 constexpr int DET_LIST_BYTES = 8;         // per candidate of one class: score, storage index, rank order
 constexpr int DET_SMEM_BUDGET = 192 * 1024;
 constexpr int DET_WARP_MAX = 64;          // candidates of one class that a warp suppresses by itself; more go to the whole CTA

@@ -1035,11 +1035,17 @@ def detection_rows(dets: DetectionBuffers) -> None:
 
 def detect(net: Network, heads: List[torch.Tensor], img_w: int, img_h: int, thresh: float, nms_thresh: float, dets: DetectionBuffers,
            relative: int = 1, letter: int = 0) -> DetectionBuffers:
-    """get_network_boxes, do_nms_sort (nms_thresh > 0) and detection_rows in one launch."""
+    """get_network_boxes, do_nms_sort (nms_thresh > 0) and detection_rows, in one launch up to capi.DETECT_HEADS heads."""
     import ctypes as C
     yolo_layers = [l for l in net.layers if l.type == "yolo"]
     if len(yolo_layers) != len(heads) or not yolo_layers:
         raise ValueError("one activated output per [yolo] layer is needed")
+    if len(heads) > capi.DETECT_HEADS:
+        get_network_boxes(net, heads, img_w, img_h, thresh, dets, relative, letter)
+        if nms_thresh > 0:
+            do_nms_sort(dets, nms_thresh)
+        detection_rows(dets)
+        return dets
     descs = (capi.YoloHead * len(heads))(*[yolo_head_desc(l, _checked_head(h)) for l, h in zip(yolo_layers, heads)])
     capi.check(capi.lib().xnor_b200_detect(descs, len(heads), net.batch, net.w, net.h, img_w, img_h, thresh, relative, letter, nms_thresh,
                                           C.byref(dets.desc), dets.rows.data_ptr(), dets.max_rows, dets.row_count.data_ptr(),

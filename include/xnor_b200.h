@@ -472,7 +472,9 @@ XNOR_B200_API int xnor_b200_nms_sort(const xnor_b200_detections * dets, int batc
 XNOR_B200_API int xnor_b200_detection_rows(const xnor_b200_detections * dets, int batch, float * rows, int max_rows, int * row_count,
 		void * stream);
 
-/* The three calls above in one launch: decode every head in order (at most 4, append = 0), suppress (nms_thresh > 0), compact. */
+#define XNOR_B200_DETECT_HEADS 4               /* most heads of one xnor_b200_detect call */
+
+/* The three calls above in one launch: decode every head in order (at most XNOR_B200_DETECT_HEADS, append = 0), suppress (nms_thresh > 0), compact. */
 XNOR_B200_API int xnor_b200_detect(const xnor_b200_yolo_head * heads, int n_heads, int batch, int netw, int neth, int img_w, int img_h,
 		float thresh, int relative, int letter, float nms_thresh, const xnor_b200_detections * dets,
 		float * rows, int max_rows, int * row_count, void * stream);

@@ -82,3 +82,24 @@ def test_rows_host_of_long_lists(counts, max_rows):
         for b, n in enumerate(counts):
             assert got[b].shape == (min(n, max_rows), 7) and (got[b] == dets.rows[b, :min(n, max_rows)].cpu().numpy()).all()
         assert min(max(counts), max_rows) <= dets.take <= max_rows
+
+
+@pytest.mark.parametrize("n_heads,nms", [(4, 0.45), (5, 0.45), (7, 0.45), (5, 0.0)])
+def test_networks_of_many_heads(tmp_path, n_heads, nms):
+    """One launch takes four heads; more go through the separate calls, in the same order."""
+    yolo = "[yolo]\nmask = 0\nanchors = 10,14\nclasses=3\nnum=1\n"
+    cfg = tmp_path / "net.cfg"
+    cfg.write_text("\n".join(["[net]\nwidth=64\nheight=64\nchannels=3\n"] + [cfgs._conv(8, 3, stride=2, bn=0, activation="linear") + "\n" + yolo] * n_heads))
+    net = network.parse_network_cfg(str(cfg), 2, "cuda:0")
+    g = torch.Generator().manual_seed(n_heads)
+    heads = [torch.rand(2, 8, l.h, l.w, generator=g).cuda() for l in net.layers if l.type == "yolo"]
+    assert len(heads) == n_heads
+    apart, joined = (network.DetectionBuffers(2, 3) for _ in range(2))
+    network.get_network_boxes(net, heads, 64, 64, 0.5, apart)
+    if nms:
+        network.do_nms_sort(apart, nms)
+    network.detection_rows(apart)
+    want = apart.rows_host()
+    network.detect(net, heads, 64, 64, 0.5, nms, joined)
+    got = joined.rows_host()
+    assert all(len(w) > 20 and np.array_equal(a, w) for a, w in zip(got, want))
