@@ -40,6 +40,7 @@ constexpr int DET_BLOCK = 128;            // ranks the CTA settles at a time
 struct YoloHeadParams
 {
 	const float * head;          // [batch][n][4 + 1 + classes][lh * lw], activated (xnor_b200_yolo_activate)
+	unsigned first;              // candidates of the heads before this one
 	int lw, lh, n, new_coords;
 	float anchor_w[DET_MAX_ANCHORS], anchor_h[DET_MAX_ANCHORS];      // biases[2 * mask[a]], biases[2 * mask[a] + 1]
 };
@@ -210,7 +211,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 	__shared__ int s_m[DET_WARPS];
 	cg::cluster_group cluster = cg::this_cluster();
 	const int rank = (int)cluster.block_rank();
-	const int b = blockIdx.y;
+	const int b = blockIdx.x / DET_CLUSTER;
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	const int all_warp = rank * DET_WARPS + warp;
@@ -220,7 +221,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 
 	if (p.n_heads > 0)
 	{
-		int * s_hit = reinterpret_cast<int *>(det_smem);         // candidate number and head of each new detection
+		unsigned * s_hit = reinterpret_cast<unsigned *>(det_smem);       // candidate number of each new detection, counted over the heads
 		const int first = found;
 		for (int hd = 0; hd < p.n_heads; ++hd)
 		{
@@ -228,16 +229,16 @@ detect_kernel(const __grid_constant__ DetectParams p)
 			const int cells = h.lw * h.lh;
 			const int entries = 4 + 1 + p.classes;
 			const float * pred = h.head + (size_t)b * h.n * entries * cells;
-			const int candidates = cells * h.n;                  // reference order: cell outer, anchor inner
-			for (int q0 = 0; q0 < candidates; q0 += DET_STEP * DET_THREADS)
+			const unsigned candidates = (unsigned)cells * h.n;   // below 2^31; reference order: cell outer, anchor inner
+			for (unsigned q0 = 0; q0 < candidates; q0 += DET_STEP * DET_THREADS)
 			{
 				unsigned hits[DET_STEP];
 				#pragma unroll
 				for (int j = 0; j < DET_STEP; ++j)
 				{
-					const int q = q0 + j * DET_THREADS + threadIdx.x;
-					const int i = q / h.n;
-					const int a = q - i * h.n;
+					const unsigned q = q0 + j * DET_THREADS + threadIdx.x;
+					const int i = (int)(q / (unsigned)h.n);
+					const int a = (int)q - i * h.n;
 					const float obj = (q < candidates) ? __ldg(pred + (size_t)(a * entries + 4) * cells + i) : 0.0f;
 					hits[j] = __ballot_sync(0xffffffffu, q < candidates && obj > p.thresh);
 				}
@@ -261,7 +262,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 					if ((hits[j] >> lane) & 1u)
 					{
 						const int slot = found + before[j] + __popc(hits[j] & ((1u << lane) - 1u));
-						if (slot < p.max_dets) { s_hit[slot - first] = (hd << 28) | (q0 + j * DET_THREADS + (int)threadIdx.x); }
+						if (slot < p.max_dets) { s_hit[slot - first] = h.first + q0 + j * DET_THREADS + threadIdx.x; }
 					}
 				}
 				found += total;
@@ -280,8 +281,11 @@ detect_kernel(const __grid_constant__ DetectParams p)
 		const int stored = min(found, p.max_dets);
 		for (int slot = first + all_warp; slot < stored; slot += DET_ALL_WARPS)
 		{
-			const YoloHeadParams & h = p.heads[s_hit[slot - first] >> 28];
-			const int q = s_hit[slot - first] & 0x0fffffff;
+			const unsigned hit = s_hit[slot - first];
+			int hd = 0;
+			while (hd + 1 < p.n_heads && hit >= p.heads[hd + 1].first) { ++hd; }
+			const YoloHeadParams & h = p.heads[hd];
+			const int q = (int)(hit - h.first);
 			const int cells = h.lw * h.lh;
 			const int entries = 4 + 1 + p.classes;
 			const int i = q / h.n;
@@ -468,8 +472,12 @@ static int add_head(const xnor_b200_yolo_head & head, int classes, DetectParams 
 {
 	if (head.output == nullptr) { return XNOR_B200_ERR_NULL; }
 	if (head.w <= 0 || head.h <= 0 || head.n <= 0 || head.n > DET_MAX_ANCHORS || head.classes != classes) { return XNOR_B200_ERR_INVALID; }
-	if ((long long)head.w * head.h * head.n >= (1 << 28)) { return XNOR_B200_ERR_TOO_LARGE; }
+	const long long candidates = (long long)head.w * head.h * head.n;
+	long long first = 0;
+	for (int i = 0; i < p.n_heads; ++i) { first += (long long)p.heads[i].lw * p.heads[i].lh * p.heads[i].n; }
+	if (candidates > 0x7fffffffLL || first + candidates > 0xffffffffLL) { return XNOR_B200_ERR_TOO_LARGE; }
 	YoloHeadParams & h = p.heads[p.n_heads++];
+	h.first = (unsigned)first;
 	h.head = head.output;
 	h.lw = head.w; h.lh = head.h; h.n = head.n; h.new_coords = head.new_coords;
 	for (int a = 0; a < DET_MAX_ANCHORS; ++a)
@@ -498,7 +506,7 @@ static int set_rows(DetectParams & p, float * rows, int max_rows, int * row_coun
 
 static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int batch, void * stream)
 {
-	if (batch > 65535) { return XNOR_B200_ERR_TOO_LARGE; }
+	if (batch > (p.nms ? 65535 : 0x7fffffff / DET_CLUSTER)) { return XNOR_B200_ERR_TOO_LARGE; }
 	p.boxes = d->boxes; p.objectness = d->objectness; p.probs = d->probs; p.count = d->count;
 	p.max_dets = d->max_dets; p.classes = d->classes;
 	// shared memory: the hit list, then the candidate lists (as many as the classes of a CTA and the budget ask for), then two
@@ -510,7 +518,7 @@ static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int b
 	const size_t smem = p.nms ? round_up((size_t)p.lists * list_bytes, 16) + (size_t)p.lists * box_bytes : (size_t)list_bytes;
 	const int rc = ensure_dynamic_smem((const void *)detect_kernel, smem);
 	if (rc != XNOR_B200_OK) { return rc; }
-	detect_kernel<<<dim3(DET_CLUSTER, (unsigned)batch, 1), DET_THREADS, smem, (cudaStream_t)stream>>>(p);
+	detect_kernel<<<(unsigned)batch * DET_CLUSTER, DET_THREADS, smem, (cudaStream_t)stream>>>(p);
 	return check_launch();
 }
 

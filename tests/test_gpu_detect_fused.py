@@ -6,7 +6,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from darknet_b200 import cfgs, network  # noqa: E402
+from darknet_b200 import capi, cfgs, network  # noqa: E402
 
 
 def iou(a, b):
@@ -103,3 +103,44 @@ def test_networks_of_many_heads(tmp_path, n_heads, nms):
     network.detect(net, heads, 64, 64, 0.5, nms, joined)
     got = joined.rows_host()
     assert all(len(w) > 20 and np.array_equal(a, w) for a, w in zip(got, want))
+
+
+def head_of(output, w, h, n, classes):
+    head = capi.YoloHead(output=output.data_ptr(), w=w, h=h, n=n, classes=classes)
+    for a in range(2 * n):
+        head.anchors[a] = 10.0
+    return head
+
+
+def test_more_images_than_a_grid_has_rows():
+    batch = 70_000
+    head = torch.zeros(batch, 1, 6, 1, device="cuda")
+    head[::3, 0, 4:] = 0.9
+    dets = network.DetectionBuffers(batch, 1, max_dets=1, max_rows=1)
+    stream = torch.cuda.current_stream().cuda_stream
+    capi.check(capi.lib().xnor_b200_yolo_detections(capi.C.byref(head_of(head, 1, 1, 1, 1)), batch, 32, 32, 32, 32, 0.5, 1, 0, 0,
+                                                    capi.C.byref(dets.desc), stream), "xnor_b200_yolo_detections")
+    network.detection_rows(dets)
+    want = torch.zeros(batch, dtype=torch.int32, device="cuda")
+    want[::3] = 1
+    assert torch.equal(dets.count, want) and torch.equal(dets.row_count, want)
+    assert bool((dets.rows[::3, 0, 4] == head[0, 0, 4, 0]).all())
+
+
+def test_a_head_of_very_many_cells():
+    """Candidate numbers past 2^28 (a head of 6.4 GB): the last cells are found, in order, at their places."""
+    w = h = 16384
+    head = torch.zeros(1, 6, h, w, device="cuda")
+    cells = [0, 12345, w * h - 2, w * h - 1]
+    for k, cell in enumerate(cells):
+        head.view(6, -1)[4:, cell] = 0.9 + 0.01 * k
+    dets = network.DetectionBuffers(1, 1, max_dets=8, max_rows=8)
+    two = torch.zeros(1, 6, 2, 2, device="cuda")
+    two[0, 4:, 1, 0] = 0.8
+    heads = (capi.YoloHead * 2)(head_of(head, w, h, 1, 1), head_of(two, 2, 2, 1, 1))
+    capi.check(capi.lib().xnor_b200_detect(heads, 2, 1, w, h, w, h, 0.5, 1, 0, 0.0, capi.C.byref(dets.desc), dets.rows.data_ptr(), 8,
+                                           dets.row_count.data_ptr(), torch.cuda.current_stream().cuda_stream), "xnor_b200_detect")
+    rows = dets.rows_host()[0]
+    assert rows[:, 4].tolist() == [np.float32(v) for v in (0.9, 0.91, 0.92, 0.93, 0.8)]
+    want = [((c % w) / w, (c // w) / h) for c in cells] + [(0.0, 0.5)]
+    assert np.allclose(rows[:, :2], want, atol=1e-6)
