@@ -38,7 +38,7 @@ constexpr int F3_MAX_PT = 8;                  // tiles of 128 blocks per unit
 constexpr int F3_MAX_UNITS_AHEAD = 16;        // entries of the ring of unit maxima: stages + accumulators + 1 are under way
 constexpr int F3_QUEUE = 64;                  // values of a warp that wait to be formed exactly
 constexpr int F3_HALVES = 12;                 // 16-byte pieces of K: four patch rows x three pairs
-constexpr int F3_SMEM_MAX = 200 * 1024;
+constexpr int F3_SMEM_MAX = 190 * 1024;      // dynamic; with the kernel's static part (37 KB for 32 filters) what a block may have
 
 struct F3Params
 {
@@ -138,6 +138,8 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	__shared__ float s_xmax[F3_MAX_UNITS_AHEAD][CONV_WARPS];
 	__shared__ uint2 s_queue[EPI_WARPS][F3_QUEUE];
 	__shared__ uint64_t st_full[F3_STAGES], st_empty[F3_STAGES], acc_full[ACC], acc_empty[ACC], drain_bar;
+	static_assert(sizeof(s_b) + sizeof(s_w) + sizeof(s_bias) + sizeof(s_xmax) + sizeof(s_queue) + sizeof(st_full) + sizeof(st_empty) + sizeof(acc_full)
+			+ sizeof(acc_empty) + 256 + F3_SMEM_MAX <= 227 * 1024, "static and dynamic shared memory of a block");
 	__shared__ uint32_t tmem_base_slot;
 	__shared__ int s_failed_storage;
 	volatile int * s_failed = &s_failed_storage;

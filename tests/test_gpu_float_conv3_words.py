@@ -64,3 +64,29 @@ def test_signs_at_every_scale(x_scale, w_scale, pool, n):
     front = capi.lib().xnor_b200_grid_front(ow + 1)
     body = grid.words[0, front:front + 2 * (oh + 1) * (ow + 1)].view(2, oh + 1, ow + 1)[:, :oh, :ow].to(torch.int64) & 0xFFFFFFFF
     assert torch.equal(body, sum(masks[..., i].to(torch.int64) << (8 * i) for i in range(n // 8)))
+
+
+@pytest.mark.parametrize("batch,h,w,n,pool", [
+    (1, 2048, 2048, 32, 0), (1, 2048, 2112, 17, 0), (1, 2048, 2048, 32, 2), (1, 2048, 2200, 24, 2), (1, 512, 3000, 32, 0),     # the widest windows
+    (1, 33, 35, 32, 0), (2, 17, 64, 16, 0), (3, 40, 41, 20, 0), (1, 1, 7, 8, 0), (1, 5, 3, 32, 0), (2, 101, 1999, 32, 0),      # odd rows and columns
+])
+def test_signs_at_the_widest_and_at_odd_sizes(batch, h, w, n, pool):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(h + w)
+    x = torch.randn(batch, 3, h, w, generator=g, device="cuda")
+    wt, b = torch.randn(n, 27, generator=g, device="cuda"), torch.randn(n, generator=g, device="cuda")
+    desc = capi.ConvDesc(batch, 3, h, w, n, 3, 1, 1, capi.LINEAR)
+    oh, ow = (h // 2, w // 2) if pool else (h, w)
+    grid = L.GridWords(batch, n, oh, ow)
+    masks = torch.zeros(batch, oh, ow, (n + 7) // 8, dtype=torch.uint8, device="cuda")
+    capi.check(capi.lib().xnor_b200_float_conv3_words(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), grid.words.data_ptr(), 0, None), "words")
+    capi.check(capi.lib().xnor_b200_float_conv3_io(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), None, None, masks.data_ptr(), None), "io")
+    front = capi.lib().xnor_b200_grid_front(ow + 1)
+    body = grid.words[0, front:front + batch * (oh + 1) * (ow + 1)].view(batch, oh + 1, ow + 1).to(torch.int64) & 0xFFFFFFFF
+    assert torch.equal(body[:, :oh, :ow], sum(masks[..., i].to(torch.int64) << (8 * i) for i in range(masks.shape[-1])))
+    assert int(body[:, oh].sum()) == 0 and int(body[:, :, ow:].sum()) == 0
+    y = F.conv2d(x.double(), wt.double().view(n, 3, 3, 3), b.double(), 1, 1)
+    y = F.max_pool2d(y, 2, 2) if pool else y
+    sure = y.abs() > 1e-4                                      # 27 fp32 products of magnitude a few
+    bits = (body[:, None, :oh, :ow] >> torch.arange(n, device="cuda").view(1, n, 1, 1)) & 1
+    assert torch.equal(bits.bool()[sure], (y > 0)[sure])
