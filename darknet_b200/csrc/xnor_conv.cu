@@ -275,7 +275,8 @@ __host__ __device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSou
 			const int y = fdiv(pos - img * (int)p.d_img.d, p.d_pitch);
 			return img * (src.h + 1) + ((src.scale == 2) ? 2 * y : (src.scale == 1) ? y : y >> 1);
 		};
-		const int a = row_of(max(pos0, 0));
+		// (a unit that begins in the padding behind the last image needs no row; it copies the last one)
+		const int a = min(row_of(max(pos0, 0)), p.batch * (src.h + 1) - 1);
 		const int b = row_of(min(pos0 + p.slots_plane - 1, p.total_pos - 1)) + ((src.scale != 0) ? 1 : 0);
 		lo = src.front + a * src.pitch;
 		hi = src.front + (b + 1) * src.pitch;

@@ -69,3 +69,30 @@ def test_the_faster_route_is_taken(shape, words):
     l.batch, l.c, l.h, l.w, l.n, l.size, l.stride = batch, c, h, w, n, ks, stride
     l.outputs = n * ((h + 2 * (ks // 2) - ks) // stride + 1) * ((w + 2 * (ks // 2) - ks) // stride + 1)
     assert L.takes_words(l) == words
+
+
+def test_every_unit_copies_a_run_that_exists_and_fits():
+    """A unit may begin in the padding behind the last image: its run must not begin past the source's end (an empty copy), and no run may
+    be longer than its place in shared memory."""
+    seen = 0
+    for ks, stride in ((1, 1), (1, 2), (3, 1), (3, 2)):
+        for c in (16, 40, 96):
+            for h in list(range(1, 34)) + [52, 53, 101]:
+                for w in list(range(1, 70, 3)) + [51, 104, 207, 301]:
+                    for batch in (1, 2, 5):
+                        rc, p = plan(batch, c, h, w, 32, ks, stride)
+                        assert rc == capi.OK
+                        assert 0 < p.run_words_min <= p.run_words_max <= p.run_room, (ks, stride, c, h, w, batch)
+                        seen += 1
+    for ks in (1, 3):
+        for h in range(2, 40):
+            for w in (2, 5, 13, 26, 51, 104, 208):
+                for ps, pp in ((1, 0), (1, 1), (2, 0), (2, 1)):
+                    oh, ow = (h + pp - 2) // ps + 1, (w + pp - 2) // ps + 1
+                    for batch in (1, 3):
+                        rc, p = plan(batch, 64, oh, ow, 32, ks, 1, [(64, h, w, ps, pp, 0, 0)])
+                        assert rc == capi.OK and 0 < p.run_words_min <= p.run_words_max <= p.run_room, (ks, h, w, ps, pp, batch)
+                        rc, p = plan(batch, 64, 2 * h, 2 * w, 32, ks, 1, [(32, h, w, 0, 0, 2, 0), (32, 2 * h, 2 * w, 0, 0, 0, 0)])
+                        assert rc == capi.OK and 0 < p.run_words_min <= p.run_words_max <= p.run_room, (ks, h, w, "up", batch)
+                        seen += 2
+    assert seen > 20_000
