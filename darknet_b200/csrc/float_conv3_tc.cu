@@ -150,7 +150,6 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	const uint32_t limit = p.spin_limit;
 	const uint32_t a_base = smem_u32(f3_smem);
 	const int my_units = (p.units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-	pdl_trigger();
 
 	if (tid == 0)
 	{
@@ -175,6 +174,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	}
 	for (int i = tid; i < NF * 27; i += F3_THREADS) { s_w[i] = (i < p.N * 27) ? __ldg(p.weights + i) : 0.0f; }
 	__syncthreads();
+	pdl_trigger();                                              // this CTA has its tensor memory
 	if (tid < NF)
 	{
 		float sum = 0.0f;

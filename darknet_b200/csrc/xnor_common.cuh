@@ -96,7 +96,8 @@ extern thread_local bool g_behind_kernel;
 // The kernel's prologue may run before the previous kernel on the stream has finished; everything from here on runs behind it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next kernel on the stream may be launched once every CTA of this one has come here.  Only behind pdl_wait (or in a kernel
-// that is never launched through launch_behind), so that what a prologue reads is finished: it lies two kernels back.
+// that is never launched through launch_behind), so that what a prologue reads is finished: it lies two kernels back.  And only
+// once the CTA has its tensor memory: a dependent CTA on the same SM may take all of it and keeps it until this kernel ends.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class Kernel, class Params>
