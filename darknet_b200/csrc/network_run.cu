@@ -85,8 +85,17 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 {
 	if (ops == nullptr || input == nullptr || (n_heads > 0 && heads == nullptr)) { return XNOR_B200_ERR_NULL; }
 	void * at = stream;
-	bool forked = false;
 	struct Reset { ~Reset() { g_behind_kernel = false; } } reset;
+	// Behind a fork the caller's stream waits for the side stream before this call returns, whether or not all was issued: what the caller
+	// queues next may read, or overwrite, what the side stream works on.
+	bool forked = false;
+	auto join = [&](int rc)
+	{
+		if (!forked) { return rc; }
+		cudaError_t e = cudaEventRecord((cudaEvent_t)join_event, (cudaStream_t)side_stream);
+		if (e == cudaSuccess) { e = cudaStreamWaitEvent((cudaStream_t)stream, (cudaEvent_t)join_event, 0); }
+		return (rc == XNOR_B200_OK && e != cudaSuccess) ? cuda_fail(e) : rc;
+	};
 	for (int i = 0; i < n_ops; ++i)
 	{
 		const xnor_b200_op & op = ops[i];
@@ -117,7 +126,7 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 				if (op.arg == 0)
 				{
 					const cudaError_t e = cudaStreamIsCapturing((cudaStream_t)at, &capture);
-					if (e != cudaSuccess) { return cuda_fail(e); }
+					if (e != cudaSuccess) { return join(cuda_fail(e)); }
 				}
 				if (op.arg != 0 || capture != cudaStreamCaptureStatusNone) { rc = xnor_b200_conv_words_weights(&d, (const uint8_t *)op.weights, (uint32_t *)out, at); }
 				break;
@@ -125,29 +134,18 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 			case XNOR_B200_OP_FORK:
 			{
 				// what follows runs on the side stream, behind everything issued so far
-				if (side_stream == nullptr || fork_event == nullptr || join_event == nullptr) { return XNOR_B200_ERR_NULL; }
+				if (side_stream == nullptr || fork_event == nullptr || join_event == nullptr) { return join(XNOR_B200_ERR_NULL); }
 				cudaError_t e = cudaEventRecord((cudaEvent_t)fork_event, (cudaStream_t)stream);
 				if (e == cudaSuccess) { e = cudaStreamWaitEvent((cudaStream_t)side_stream, (cudaEvent_t)fork_event, 0); }
-				if (e != cudaSuccess) { return cuda_fail(e); }
+				if (e != cudaSuccess) { return join(cuda_fail(e)); }
 				at = side_stream;
 				forked = true;
 				break;
 			}
-			case XNOR_B200_OP_BACK:
-			{
-				const cudaError_t e = cudaEventRecord((cudaEvent_t)join_event, (cudaStream_t)side_stream);
-				if (e != cudaSuccess) { return cuda_fail(e); }
-				at = stream;
-				break;
-			}
-			default: return XNOR_B200_ERR_INVALID;
+			case XNOR_B200_OP_BACK: at = stream; break;
+			default: return join(XNOR_B200_ERR_INVALID);
 		}
-		if (rc != XNOR_B200_OK) { return rc; }
+		if (rc != XNOR_B200_OK) { return join(rc); }
 	}
-	if (forked)
-	{
-		const cudaError_t e = cudaStreamWaitEvent((cudaStream_t)stream, (cudaEvent_t)join_event, 0);
-		if (e != cudaSuccess) { return cuda_fail(e); }
-	}
-	return XNOR_B200_OK;
+	return join(XNOR_B200_OK);
 }

@@ -146,3 +146,24 @@ def test_wide_networks(name, width, tmp_path):
     net, got, want = both(tmp_path, ["[" + sections], 1, width, 64)
     assert width < 1408 or net.plan is None
     assert_heads_close(got, want)
+
+
+def test_a_call_that_fails_behind_a_fork_leaves_nothing_running_beside_the_caller():
+    """An operation of an unknown kind behind a long one on the side stream: the call reports it, and what the caller queues next still
+    comes behind the long one."""
+    from darknet_b200 import layer as L
+    x = torch.randn(8, 256, 416, 416, device="cuda")
+    words = L.GridWords(8, 256, 416, 416)
+    want = L.sign_words(x).words
+    signs = capi.Op(kind=capi.OP_SIGN_WORDS, desc=capi.ConvDesc(8, 256, 416, 416), input=capi.OP_INPUT, output=words.words.data_ptr(), pitch=417)
+    ops = (capi.Op * 3)(capi.Op(kind=capi.OP_FORK), signs, capi.Op(kind=99))
+    side, events = torch.cuda.Stream(), [torch.cuda.Event() for _ in range(2)]
+    for e in events:
+        e.record(side)
+    for _ in range(3):
+        words.words.zero_()
+        torch.cuda.synchronize()
+        rc = capi.lib().xnor_b200_run_ops(ops, 3, x.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream, side.cuda_stream,
+                                          *(e.cuda_event for e in events))
+        got = words.words.clone()
+        assert rc == 1 and torch.equal(got, want)
