@@ -76,7 +76,7 @@ class WordsPlan(C.Structure):
 
 
 (OP_CONV3, OP_SIGN_WORDS, OP_CONV_WORDS, OP_FLOAT_MAP, OP_FLOAT_TC, OP_YOLO, OP_REGION, OP_AVGPOOL, OP_SOFTMAX, OP_FORK,
- OP_BACK, OP_CONV, OP_FILTERS) = range(1, 14)
+ OP_BACK, OP_CONV, OP_FILTERS, OP_MARK) = range(1, 15)
 OP_INPUT, OP_HEAD = 1, 2
 
 

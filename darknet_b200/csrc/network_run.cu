@@ -89,6 +89,7 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 	// Behind a fork the caller's stream waits for the side stream before this call returns, whether or not all was issued: what the caller
 	// queues next may read, or overwrite, what the side stream works on.
 	bool forked = false;
+	bool behind = false;                                       // the stream's last entry is a kernel of this call
 	auto join = [&](int rc)
 	{
 		if (!forked) { return rc; }
@@ -103,8 +104,9 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 		float * out = (float *)resolve(op.output, input, heads, n_heads);
 		const xnor_b200_conv_desc & d = op.desc;
 		int rc = XNOR_B200_OK;
-		// behind a fork, a return or filters (seldom made again) the stream's last entry may be no kernel of this call
-		g_behind_kernel = (i > 0 && ops[i - 1].kind != XNOR_B200_OP_FORK && ops[i - 1].kind != XNOR_B200_OP_BACK && ops[i - 1].kind != XNOR_B200_OP_FILTERS);
+		g_behind_kernel = behind;
+		const bool was_behind = behind;
+		behind = true;
 		switch (op.kind)
 		{
 			case XNOR_B200_OP_CONV3: rc = xnor_b200_float_conv3_words(&d, op.arg, in, (const float *)op.weights, op.biases, (uint32_t *)out, op.pitch, at); break;
@@ -122,6 +124,7 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 				break;
 			case XNOR_B200_OP_FILTERS:
 			{
+				behind = false;                                  // seldom made again, and the kernel that reads them does so before it waits
 				cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
 				if (op.arg == 0)
 				{
@@ -140,9 +143,20 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 				if (e != cudaSuccess) { return join(cuda_fail(e)); }
 				at = side_stream;
 				forked = true;
+				behind = false;
 				break;
 			}
-			case XNOR_B200_OP_BACK: at = stream; break;
+			case XNOR_B200_OP_BACK: at = stream; behind = false; break;
+			case XNOR_B200_OP_MARK:
+			{
+				behind = was_behind && out == nullptr;
+				if (out != nullptr)
+				{
+					const cudaError_t e = cudaEventRecord((cudaEvent_t)(void *)out, (cudaStream_t)at);
+					if (e != cudaSuccess) { return join(cuda_fail(e)); }
+				}
+				break;
+			}
 			default: return join(XNOR_B200_ERR_INVALID);
 		}
 		if (rc != XNOR_B200_OK) { return join(rc); }

@@ -136,6 +136,7 @@ class Network:
     heads_direct_to_host: bool = True      # with heads_host: a fused head convolution stores into the pinned host tensor itself
     side_branches: bool = True             # a head branch that nothing later reads runs on a second stream
     side_stream: Optional[torch.cuda.Stream] = None
+    copy_stream: Optional[torch.cuda.Stream] = None    # on which finished heads cross to the host
     packed_from_cache: int = 0             # xnor layers whose packed weights came from the cache file beside the .weights file
     sink_max_batch: int = 1 << 30          # batch up to which direct sign sinks are linked (measured: a gain at every batch for yolov3-tiny, within 2% either way for the other two networks at batch 32-256)
     sink_links: int = 0
@@ -820,8 +821,8 @@ def _region(x: torch.Tensor, l: Layer) -> torch.Tensor:
 def forward_network_gpu(net: Network, x: torch.Tensor, heads_host: Optional[List[torch.Tensor]] = None) -> List[torch.Tensor]:
     """The layer loop of forward_network_gpu (src-lib/network_kernels.cu:30-65).  Returns the outputs of the
     network's head layers (yolo / region / softmax).  heads_host: pinned host tensors, one per head; each head is
-    copied there as soon as it exists, on the stream that made it (Darknet's yolo layer pulls its output to the host
-    in every forward, src-lib/yolo_layer.cpp:1439-1489), so the copy of an early head overlaps the rest of the network.
+    copied there as soon as it exists, beside the rest of the network (Darknet's yolo layer pulls its output to the host
+    in every forward, src-lib/yolo_layer.cpp:1439-1489).
     A network that was lowered to native operations (network_plan) runs as one call; the loop below runs the others, and every
     network while xnor_b200_set_tuning pins kernels of the packed-operand route."""
     if net.plan is not None and net.plan.takes(x):
@@ -1103,7 +1104,7 @@ def load_network_custom(cfg: str, weights: str, batch: int = 1, device: str = "c
 def own_launches_per_forward(net: Network) -> int:
     """Kernels of libxnor_b200.so that one forward launches, after every fusion that load_network_custom set up."""
     if net.plan is not None:
-        return sum(1 for op in net.plan.ops if op.kind not in (capi.OP_FORK, capi.OP_BACK))
+        return sum(1 for op in net.plan.ops if op.kind not in (capi.OP_FORK, capi.OP_BACK, capi.OP_MARK))
     n = 0
     for l in net.layers:
         if l.type == "convolutional":

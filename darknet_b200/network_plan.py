@@ -35,9 +35,11 @@ class Plan:
         self.params: List[Tuple[object, str]] = []    # attributes the operations were made from
         self.laid_out: List[torch.Tensor] = []     # those of which the operations read a copy in another order
         self.head_layers: List = []
+        self.finished: List[int] = []              # per head: operations up to and with the one that makes it
         self.head_direct: List[bool] = []          # a head whose last operation may store into page-locked host memory
         self.signs: Dict[int, L.GridWords] = {}    # layer index -> its (or for a blank [shortcut] the sum's) signs
         self.floats: Dict[int, torch.Tensor] = {}  # layer index -> fp32 tensor of a float layer
+        self.marks: List[Optional[torch.cuda.Event]] = []    # per head: recorded where it is finished, None for the last thing a forward makes
         self.events: List[torch.cuda.Event] = []
 
     def address(self, t: Optional[torch.Tensor]) -> Optional[int]:
@@ -70,10 +72,23 @@ class Plan:
     def finish(self) -> None:
         self.seen = L.replaced.count
         self.tensors, self.versions = self._state()
+        # a head is marked unless nothing of the forward comes behind it
+        self.marked = [self.finished[i] < len(self.ops) for i in range(len(self.head_layers))]
+        for i in reversed(range(len(self.head_layers))):
+            if self.marked[i]:
+                self.ops.insert(self.finished[i], capi.Op(kind=capi.OP_MARK, output=capi.OP_HEAD + len(self.head_layers) + i))
         self.array = (capi.Op * len(self.ops))(*self.ops)
         self.n_ops = len(self.ops)
-        self.heads_type = C.c_void_p * max(1, len(self.head_layers))
+        # the tensors of the heads, then the events behind them
+        self.heads_type = C.c_void_p * (2 * max(1, len(self.head_layers)))
         self.head_shapes = [(self.net.batch, l.out_c, l.out_h, l.out_w) for l in self.head_layers]
+        if any(self.marked) and self.net.device.type == "cuda":
+            if self.net.copy_stream is None:
+                self.net.copy_stream = torch.cuda.Stream(self.net.device)
+            self.marks = [torch.cuda.Event() if marked else None for marked in self.marked]
+            for e in self.marks:
+                if e is not None:
+                    e.record(self.net.copy_stream)     # a torch event exists from its first record on
         self.side = self.fork = self.join = None
         if any(op.kind == capi.OP_FORK for op in self.ops):
             if self.net.side_stream is None:
@@ -93,15 +108,27 @@ class Plan:
         heads = [heads_host[i] if direct and self.head_direct[i] else torch.empty(s, dtype=torch.float32, device=x.device)
                  for i, s in enumerate(self.head_shapes)]
         pointers = self.heads_type(*[h.data_ptr() for h in heads])
-        capi.check(capi.lib().xnor_b200_run_ops(self.array, self.n_ops, x.data_ptr(), pointers, len(heads),
+        copied = [i for i, h in enumerate(heads) if heads_host is not None and h is not heads_host[i]]
+        early = [i for i in copied if self.marked[i]]
+        if early:
+            for i in early:
+                pointers[len(heads) + i] = self.marks[i].cuda_event
+        capi.check(capi.lib().xnor_b200_run_ops(self.array, self.n_ops, x.data_ptr(), pointers, 2 * len(heads),
                                                torch._C._cuda_getCurrentRawStream(x.device.index), self.side, self.fork, self.join),
                    "xnor_b200_run_ops")
         for l, h in zip(self.head_layers, heads):
             l.output_gpu = h
-        if heads_host is not None:
-            for h, host in zip(heads, heads_host):
-                if h is not host:
-                    host.copy_(h, non_blocking=True)
+        if early:
+            # each head crosses as soon as it exists, beside the rest of the network
+            with torch.cuda.stream(net.copy_stream):
+                for i in early:
+                    net.copy_stream.wait_event(self.marks[i])
+                    heads_host[i].copy_(heads[i], non_blocking=True)
+        for i in copied:
+            if i not in early:
+                heads_host[i].copy_(heads[i], non_blocking=True)
+        if early:
+            torch.cuda.current_stream(x.device).wait_stream(net.copy_stream)
         return heads
 
 
@@ -221,6 +248,7 @@ def _build(net) -> Plan:
                                     input=plan.address(_tensor(plan, float_in[k])), output=plan.floats[k].data_ptr()))
         elif l.type in ("yolo", "region", "softmax"):
             _head(plan, k, float_in[k])
+            plan.finished.append(len(plan.ops))
         if l.branch_end:
             plan.ops.append(capi.Op(kind=capi.OP_BACK))
     if not plan.head_layers:

@@ -506,6 +506,7 @@ XNOR_B200_API int xnor_b200_softmax(const float * input, float * output, int bat
 #define XNOR_B200_OP_CONV       12   /* xnor_b200_conv_forward(desc, input, weights, mean_arr, biases, output, io.shortcut_in, io.shortcut_out, scratch) */
 #define XNOR_B200_OP_FILTERS    13   /* xnor_b200_conv_words_weights(desc, weights, output), where arg != 0 or the stream is being captured
                                       * (a captured forward then follows later changes of the packed weights)                         */
+#define XNOR_B200_OP_MARK       14   /* records the cudaEvent_t that `output` stands for (an entry of heads; NULL: nothing) where it stands */
 
 /* Values of input / output that stand for the run's own tensors. */
 #define XNOR_B200_OP_INPUT       1   /* the network's input                 */
@@ -525,8 +526,8 @@ typedef struct xnor_b200_op
 	size_t scratch_bytes;
 } xnor_b200_op;
 
-/* heads: n_heads tensors the operations write (device memory, or page-locked host memory for the head convolutions).  side_stream
- * and the two events (cudaEvent_t) are needed when the operations fork, at most once; the caller's stream has joined the side
+/* heads: n_heads tensors the operations write (device memory, or page-locked host memory for the head convolutions) and events they mark.  side_stream
+ * and the two events (cudaEvent_t) are needed when the operations fork; the caller's stream has joined the side
  * stream when the call returns. */
 XNOR_B200_API int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const float * input, void * const * heads, int n_heads, void * stream,
 		void * side_stream, void * fork_event, void * join_event);

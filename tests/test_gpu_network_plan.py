@@ -167,3 +167,34 @@ def test_a_call_that_fails_behind_a_fork_leaves_nothing_running_beside_the_calle
                                           *(e.cuda_event for e in events))
         got = words.words.clone()
         assert rc == 1 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("name,batch", [("yolov3-tiny_xnor", 1), ("yolov3-tiny_xnor", 8), ("tiny-yolo_xnor", 8), ("darknet53_448_xnor", 2)])
+def test_heads_that_cross_to_the_host(name, batch, tmp_path):
+    """Page-locked tensors, and others that a plain copy takes; as ordinary calls and captured."""
+    size = 160
+    cfg = tmp_path / "net.cfg"
+    cfg.write_text(cfgs.CFGS[name](size, size))
+    network.write_synthetic_weights(network.parse_network_cfg(str(cfg), 1, "cpu"), str(tmp_path / "w"))
+    net = network.load_network_custom(str(cfg), str(tmp_path / "w"), batch)
+    want = [h.cpu() for h in network.forward_network_gpu(net, image(batch, size, size))]
+    pinned = [torch.empty_like(h).pin_memory() for h in want]
+    doubles = [torch.empty(h.shape, dtype=torch.float64) for h in want]
+    strided = [torch.empty(*h.shape[:-1], 2 * h.shape[-1]).pin_memory()[..., ::2] for h in want]
+    for hosts in (pinned, strided, doubles):
+        direct = net.heads_direct_to_host
+        net.heads_direct_to_host = hosts is pinned
+        for seed in (2, 1):
+            network.forward_network_gpu(net, image(batch, size, size, seed), heads_host=hosts)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a.float(), b) for a, b in zip(hosts, want))
+        net.heads_direct_to_host = direct
+    x, stream, graph = image(batch, size, size), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        network.forward_network_gpu(net, x, heads_host=pinned)
+    for h in pinned:
+        h.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(pinned, want))

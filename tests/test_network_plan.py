@@ -116,3 +116,11 @@ def test_networks_too_wide_for_the_kernel_keep_to_the_layer_loop(name, tmp_path,
         sections = cfgs.CFGS[name](width, 64).split("\n[", 1)[1]
         net = lowered(["[" + sections], tmp_path, monkeypatch, batch=1, width=width)
         assert (net.plan is not None) == fits, width
+
+
+def test_heads_are_marked_where_they_are_finished(tmp_path, monkeypatch):
+    net = lowered([conv(32, 3), conv(160, 3, xnor=1), head_conv(), YOLO, "[route]\nlayers=-3\n", conv(160, 3, xnor=1), head_conv(), YOLO], tmp_path, monkeypatch)
+    marks = [i for i, op in enumerate(net.plan.ops) if op.kind == capi.OP_MARK]
+    assert net.plan.marked == [True, False] and len(marks) == 1
+    assert net.plan.ops[marks[0] - 1].output == capi.OP_HEAD and net.plan.ops[marks[0]].output == capi.OP_HEAD + 2
+    assert network.own_launches_per_forward(net) == len(net.plan.ops) - 1
