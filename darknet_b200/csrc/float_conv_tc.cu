@@ -6,15 +6,21 @@
 // Replaces, for those layers, the float branch of forward_convolutional_layer_gpu (src-lib/convolutional_kernels.cu:373-434:
 // a cuBLAS/cuDNN GEMM per image) + add_bias_gpu + activate_array_ongpu.  out[b][f][p] = bias[f] + sum_c w[f][c] * x[b][c][p].
 //
-// The tensor core multiplies tf32 (10 mantissa bits).  Every fp32 operand value v is therefore split into hi = v with the low
-// 13 mantissa bits cleared (exactly a tf32) and lo = v - hi (exact in fp32, magnitude <= 2^-10 |v|), and three products are
-// accumulated per pair: hi*hi + lo*hi + hi*lo.  What is dropped (lo*lo and the bits of lo below tf32) is below 2^-20 of each
-// product.  The tensor core adds into its fp32 accumulator without rounding to nearest (measured: the error of a sum grows
-// linearly with the number of accumulating instructions, ~1e-7 of the sum per instruction), so consecutive K blocks go to four
-// accumulators in turn (all 512 tensor-memory columns) and the epilogue adds the four partial sums with ordinary fp32
-// additions: 1024 channels come out within 2e-5 of an fp64 convolution for results of magnitude 1 -- far inside what the
-// reference's own GPU path does (it asks cuDNN for tensor-op math, i.e. single tf32 products, on every convolution:
-// src-lib/convolutional_layer.cpp:350).
+// The tensor core multiplies tf32 (11 significant bits).  Every fp32 operand value v is therefore split into hi, of 11 bits, and lo = v - hi
+// (exact in fp32), and three products are accumulated per pair: hi*hi + lo*hi + hi*lo.  The tensor core adds into its fp32 accumulator
+// without rounding to nearest: a sum is off by about 2e-8 of itself per accumulating instruction (the small products count for nothing in
+// an accumulator of their own).  What decides the accuracy is thus how many instructions one accumulator takes and how the operands are
+// split: to the nearest hi, which leaves lo one bit fewer and either sign, or cut off.  Where this kernel stands in for one in plain fp32
+// it is no less accurate (2-norm error against fp64, leaky inputs; launch_float_tc has the rule):
+//   up to 1024 pixels    every K block's sum taken out of tensor memory: 1.2e-7 .. 1.4e-7 (float_conv_map.cu 1.2e-7 .. 3.0e-7); about
+//                        650 cycles a block: 3x3 256 -> 512, 4 images of 13x13, 33 us, 27 with 1.3e-6
+//   3x3, more pixels     small products apart, large ones in three accumulators, nearest split: 1.7e-6 at 72 K blocks (cuDNN's fp32
+//                        convolution 2.7e-6; its largest errors are seven times as large): 64 images 171 us, 162 with 4.1e-6; tiles
+//                        of more blocks in groups of eight, 6.4e-7 (190 us)
+//   1x1, more pixels     all products in four accumulators, cut off: 5.6e-7 at 256 channels, 1.9e-6 at 1024 -- far inside what the
+//                        reference's own GPU path does (it asks cuDNN for tensor-op math, i.e. single tf32 products, on every
+//                        convolution: src-lib/convolutional_layer.cpp:350)
+// Results that the split cannot form (infinite, NaN or nearly infinite factors) are formed again by fp32 multiply-adds, but for the last kind.
 //
 // One tile of 128 pixels (TMEM lanes; the batch is folded into the pixel index) x 128 filters (TMEM columns) per CTA.  Warp 0 issues
 // (converged, one elected lane: a divergent lane takes longer to bring an instruction's operands to the uniform registers than the
@@ -25,8 +31,8 @@
 // sums meet in the first one's shared memory and are added in order.  The epilogue adds the bias, applies leaky or the [yolo]
 // layer's logistic and stores 32 consecutive pixels of one filter per warp-store.  Every barrier wait is bounded (status word
 // shared with the xnor tensor-core kernels).
-// Measured: 3x3 256 -> 512 on 13x13 at batch 64 162 us (one block in flight and the filters split on the way: 300), at batch 8 30 us
-// (101 without the cluster); 1x1 1024 -> 425 on 13x13 at batch 256 269 us (475).  Bound by the tensor pipe (880 cycles per K block) and
+// Measured: 3x3 256 -> 512 on 13x13 at batch 64 171 us (one block in flight and the filters split on the way: 300), at batch 8 33 us
+// (101 without the cluster); 1x1 1024 -> 425 on 13x13 at batch 256 270 us (475).  Bound by the tensor pipe (880 cycles per K block) and
 // by shared-memory bandwidth (64 KB written and 96 KB read per K block: 1280 cycles).
 #include "tc_common.cuh"
 
@@ -39,6 +45,7 @@ namespace cg = cooperative_groups;
 
 constexpr int FT_NF = 128;                                 // filters per tile
 constexpr int FT_ACCS = 4;                                 // accumulators that take the K blocks in turn
+constexpr int FT_BUFFERS = 2;                              // groups of K blocks whose sums can be in tensor memory: two accumulators each
 constexpr int FT_STAGES = 3;
 constexpr int FT_TILE_BYTES = 128 * 128;                   // 128 rows x 32 tf32
 constexpr int FT_STAGE_BYTES = 4 * FT_TILE_BYTES;          // pixel hi, pixel lo, filter hi, filter lo
@@ -69,9 +76,18 @@ struct FtParams
 	uint32_t spin_limit;
 };
 
+// v = hi + lo exactly: hi the nearest value of 11 significant bits (halves away from zero), so that lo, of either sign, fits 12.  An infinity
+// or NaN leaves NaN in lo, and so does a value that rounds past the largest: those results are formed again (plain_sum).
+__device__ __forceinline__ void split_nearest(float v, float & hi, float & lo)
+{
+	hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
+	lo = __fsub_rn(v, hi);
+}
+
 // A thread's part of one operand row of one K block: FT_CH fp32 values -> their 16-byte chunks in the row of the hi tile and
 // of the lo tile (chunk c of row r at chunk position c ^ (r % 8); row_swz has the row's swizzle term and the part's first
 // chunk folded in).
+template <bool NEAREST>
 __device__ __forceinline__ void split_row(uint32_t row_swz_hi, uint32_t lo_offset, const float (&v)[FT_CH])
 {
 	#pragma unroll
@@ -82,7 +98,7 @@ __device__ __forceinline__ void split_row(uint32_t row_swz_hi, uint32_t lo_offse
 		for (int j = 0; j < 4; ++j)
 		{
 			const uint32_t bits = __float_as_uint(v[4 * c + j]);
-			hi[j] = bits & 0xFFFFE000u;
+			hi[j] = (NEAREST ? bits + 0x1000u : bits) & 0xFFFFE000u;          // split_nearest, or cut off
 			lo[j] = __float_as_uint(__fsub_rn(v[4 * c + j], __uint_as_float(hi[j])));
 		}
 		const uint32_t addr = row_swz_hi ^ (uint32_t)(c << 4);
@@ -107,15 +123,65 @@ __device__ __forceinline__ void tile_sums(uint32_t tmem, int used, float (&acc)[
 	}
 }
 
+// Adds a group's two accumulators (32 columns of this warp's lanes) to the sums, in fp32.  Eight columns at a time: the loop around it
+// keeps the sums and the next K blocks in registers as well.
+__device__ __forceinline__ void add_group(uint32_t tmem, float (&sums)[32])
+{
+	#pragma unroll
+	for (int h = 0; h < 32; h += 8)
+	{
+		uint32_t a[8], b[8];
+		asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+			: "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]) : "r"(tmem + (uint32_t)h) : "memory");
+		asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+			: "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]) : "r"(tmem + (uint32_t)(FT_NF + h)) : "memory");
+		// nothing uses the registers before the loads have returned
+		asm volatile("tcgen05.wait::ld.sync.aligned;"
+			: "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+			  "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]) :: "memory");
+		#pragma unroll
+		for (int j = 0; j < 8; ++j) { sums[h + j] = __fadd_rn(sums[h + j], __fadd_rn(__uint_as_float(a[j]), __uint_as_float(b[j]))); }
+	}
+}
+
+// One result by fp32 multiply-adds from the prepared filters, for those that the split products cannot form: a factor that is infinite,
+// NaN or next to the largest value.
+__device__ __forceinline__ float plain_sum(const FtParams & p, int img, int pix, int f)
+{
+	const int py = pix / p.W, px = pix - py * p.W, row = f % FT_NF;
+	const float * base = p.x + (size_t)img * p.C * p.HW + pix;
+	float acc = 0.0f;
+	for (int tap = 0; tap < p.taps; ++tap)
+	{
+		const int dy = (p.taps == 9) ? tap / 3 - 1 : 0, dx = (p.taps == 9) ? tap % 3 - 1 : 0;
+		const bool inside = (py + dy >= 0 && py + dy < p.H && px + dx >= 0 && px + dx < p.W);       // else zeros, as im2col has them
+		for (int c = 0; c < p.C; ++c)
+		{
+			const float * tile = p.w + ((size_t)(f / FT_NF) * p.kblocks + tap * p.cblocks + (c >> 5)) * (2 * FT_TILE_BYTES / 4);
+			const int at = row * 32 + ((((c & 31) >> 2) ^ (row & 7)) << 2) + (c & 3);
+			acc = fmaf(inside ? __ldg(base + dy * p.W + dx + (size_t)c * p.HW) : 0.0f, __ldg(tile + at) + __ldg(tile + FT_TILE_BYTES / 4 + at), acc);
+		}
+	}
+	return acc;
+}
+
 // RAW: the filters come as Darknet keeps them and are split by the producers as well (callers without a prepared copy, 1x1 only).
-template <bool RAW>
+// Where the sums are formed (see launch_float_tc).  GROUP > 0: that many K blocks (a power of two) meet in tensor memory before their sum
+// is taken out and added in fp32.  Whole tiles: FT_TURNS, K blocks take the FT_ACCS accumulators in turn; FT_APART, their small products
+// share the first and the large ones take the others in turn.  All but FT_TURNS split to nearest and form again what did not come out.
+constexpr int FT_TURNS = 0, FT_APART = -1;
+
+template <bool RAW, int GROUP>
 __global__ void __launch_bounds__(FT_THREADS, 1)
 float_conv_tc_kernel(const FtParams p)
 {
+	constexpr bool WHOLE = (GROUP <= 0), FINE = (GROUP != FT_TURNS);
+	constexpr int BLOCKS = WHOLE ? 1 : GROUP;
 	extern __shared__ uint8_t ft_smem_raw[];
 	__shared__ uint64_t bar_full[FT_STAGES];
 	__shared__ uint64_t bar_empty[FT_STAGES];
-	__shared__ uint64_t bar_done;
+	__shared__ uint64_t bar_done;                              // the whole tile, or (groups) what was issued before a failure
+	__shared__ uint64_t acc_full[FT_BUFFERS], acc_empty[FT_BUFFERS];
 	__shared__ uint32_t tmem_base_slot;
 	__shared__ float s_bias[FT_NF];
 	__shared__ int s_failed_storage;
@@ -144,6 +210,11 @@ float_conv_tc_kernel(const FtParams p)
 			mbar_init(&bar_empty[s], 1);
 		}
 		mbar_init(&bar_done, 1);
+		for (int a = 0; a < (WHOLE ? 0 : FT_BUFFERS); ++a)
+		{
+			mbar_init(&acc_full[a], 1);
+			mbar_init(&acc_empty[a], FT_PRODUCER_WARPS);
+		}
 		s_failed_storage = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -158,6 +229,9 @@ float_conv_tc_kernel(const FtParams p)
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
 
+	// producers: sums of pixel quarter * 32 + lane, filters of the chunk
+	const int quarter = warp & 3, chunk = (warp - 1) >> 2;
+	float sums[32];
 	if (warp == 0)
 	{
 		{
@@ -170,34 +244,75 @@ float_conv_tc_kernel(const FtParams p)
 				const int s = kb % FT_STAGES;
 				ok = __all_sync(0xffffffffu, mbar_wait(&bar_full[s], (uint32_t)((kb / FT_STAGES) & 1), s_failed, p.spin_limit));
 				if (!ok) { break; }
+				const int buffer = (kb / BLOCKS) % FT_BUFFERS;
+				if (!WHOLE && kb % BLOCKS == 0 && kb / BLOCKS >= FT_BUFFERS)
+				{
+					ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buffer], (uint32_t)((kb / BLOCKS / FT_BUFFERS - 1) & 1), s_failed, p.spin_limit));
+					if (!ok) { break; }
+				}
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 				const uint32_t a_hi = ring + (uint32_t)s * FT_STAGE_BYTES;
 				const uint32_t a_lo = a_hi + FT_TILE_BYTES;
 				const uint32_t b_hi = a_hi + 2 * FT_TILE_BYTES;
 				const uint32_t b_lo = a_hi + 3 * FT_TILE_BYTES;
-				#pragma unroll
-				for (int k = 0; k < 4; ++k)                       // 8 tf32 = 32 bytes of every row per instruction
+				if constexpr (WHOLE)
 				{
 					#pragma unroll
-					for (int term = 0; term < 3; ++term)          // the two small terms first, the large one last
+					for (int k = 0; k < 4; ++k)                       // 8 tf32 = 32 bytes of every row per instruction
 					{
+						#pragma unroll
+						for (int term = 0; term < 3; ++term)          // the two small terms first, the large one last
+						{
+							const uint64_t adesc = make_smem_desc((term == 0 ? a_lo : a_hi) + k * 32);
+							const uint64_t bdesc = make_smem_desc((term == 1 ? b_lo : b_hi) + k * 32);
+							const bool small = (GROUP == FT_APART && term < 2);
+							const int turn = (GROUP == FT_TURNS) ? kb % FT_ACCS : small ? 0 : 1 + kb % (FT_ACCS - 1);
+							const bool begun = (GROUP == FT_TURNS) ? (kb >= FT_ACCS || k > 0 || term > 0) : small ? (kb > 0 || k > 0 || term > 0) : (kb >= FT_ACCS - 1 || k > 0);
+							const uint32_t accumulate = begun ? 1u : 0u;
+							if (leader) asm volatile(
+								"{\n\t.reg .pred p;\n\t"
+								"setp.ne.b32 p, %4, 0;\n\t"
+								"tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+								:: "r"(tmem_base + (uint32_t)(turn * FT_NF)), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+						}
+					}
+				}
+				else
+				{
+					// the small products in the first accumulator, the large ones in the second; of a single block, the large ones of the first 16
+					// channels behind the small ones, so that no sum of large ones takes more than two instructions
+					constexpr int FIRST = (GROUP == 1) ? 2 : 0;
+					#pragma unroll
+					for (int i = 0; i < 12; ++i)
+					{
+						const int term = i / 4, k = i % 4;
+						const bool second = (term == 2 && k >= FIRST);
 						const uint64_t adesc = make_smem_desc((term == 0 ? a_lo : a_hi) + k * 32);
 						const uint64_t bdesc = make_smem_desc((term == 1 ? b_lo : b_hi) + k * 32);
-						const uint32_t accumulate = (kb >= FT_ACCS || k > 0 || term > 0) ? 1u : 0u;
+						const uint32_t accumulate = (kb % BLOCKS > 0 || (i > 0 && !(second && k == FIRST))) ? 1u : 0u;
 						if (leader) asm volatile(
 							"{\n\t.reg .pred p;\n\t"
 							"setp.ne.b32 p, %4, 0;\n\t"
 							"tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-							:: "r"(tmem_base + (uint32_t)((kb % FT_ACCS) * FT_NF)), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+							:: "r"(tmem_base + (uint32_t)((2 * buffer + (second ? 1 : 0)) * FT_NF)), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 					}
 				}
 				if (leader) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
 						:: "r"(smem_u32(&bar_empty[s])) : "memory");
+				if (!WHOLE && leader && (kb % BLOCKS == BLOCKS - 1 || kb == kbn - 1))
+				{
+					asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&acc_full[buffer])) : "memory");
+				}
 			}
-			if (ok && leader)
+			if (WHOLE ? ok : !ok)
 			{
-				asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-						:: "r"(smem_u32(&bar_done)) : "memory");
+				if (leader)
+				{
+					asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+							:: "r"(smem_u32(&bar_done)) : "memory");
+				}
+				// leaving early: what was issued must have finished before the tensor memory is released
+				if (!WHOLE) { mbar_wait_plain(&bar_done, 0, p.spin_limit); }
 			}
 		}
 		__syncwarp();
@@ -240,6 +355,22 @@ float_conv_tc_kernel(const FtParams p)
 				for (int k = 0; k < FT_CH; ++k) { w[k] = (f < p.N && c0 + k < p.C) ? __ldg(p.w + (size_t)f * p.C + c0 + k) : 0.0f; }
 			}
 		};
+		// the sums of the next group of K blocks, from tensor memory into this thread's
+		int n_group = 0;
+		#pragma unroll
+		for (int j = 0; j < (WHOLE ? 0 : 32); ++j) { sums[j] = 0.0f; }
+		auto collect = [&]()
+		{
+			const int buffer = n_group % FT_BUFFERS;
+			if (!__all_sync(0xffffffffu, mbar_wait<64>(&acc_full[buffer], (uint32_t)((n_group / FT_BUFFERS) & 1), s_failed, p.spin_limit))) { return false; }
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			add_group(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buffer * 2 * FT_NF + chunk * 32), sums);
+			++n_group;
+			asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+			__syncwarp();
+			if (lane == 0) { mbar_arrive(&acc_empty[buffer]); }
+			return true;
+		};
 		if (kbn > 0) { fetch(buf[0], fil[0]); }
 		if (kbn > 1) { fetch(buf[1], fil[1]); }
 		bool ok = true;
@@ -253,17 +384,25 @@ float_conv_tc_kernel(const FtParams p)
 				if (kb + u >= FT_STAGES)
 				{
 					ok = mbar_wait(&bar_empty[s], (uint32_t)(((kb + u) / FT_STAGES - 1) & 1), s_failed, p.spin_limit);
+					if (!WHOLE) { ok = __all_sync(0xffffffffu, ok); }
 					if (!ok) { break; }
 				}
-				split_row(row_swz0 + (uint32_t)s * FT_STAGE_BYTES, (uint32_t)FT_TILE_BYTES, buf[u]);
-				if constexpr (RAW) { split_row(row_swz0 + (uint32_t)s * FT_STAGE_BYTES + 2u * FT_TILE_BYTES, (uint32_t)FT_TILE_BYTES, fil[u]); }
+				split_row<FINE>(row_swz0 + (uint32_t)s * FT_STAGE_BYTES, (uint32_t)FT_TILE_BYTES, buf[u]);
+				if constexpr (RAW) { split_row<false>(row_swz0 + (uint32_t)s * FT_STAGE_BYTES + 2u * FT_TILE_BYTES, (uint32_t)FT_TILE_BYTES, fil[u]); }
 				if (kb + u + 2 < kbn) { fetch(buf[u], fil[u]); }
 				asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 				__syncwarp();
 				if (lane == 0) { mbar_arrive(&bar_full[s]); }
+				if constexpr (!WHOLE)
+				{
+					// a group is taken out while the next is added up: two blocks, which are in flight, behind its last one
+					if (kb + u >= (n_group + 1) * GROUP + 1) { ok = collect(); }
+					if (!ok) { break; }
+				}
 			}
 		}
 		if (part == 0) { s_bias[row] = (f < p.N && p.bias != nullptr) ? __ldg(p.bias + f) : 0.0f; }
+		if constexpr (!WHOLE) { while (n_group * GROUP < kbn && ok) { ok = collect(); } }
 	}
 	else if (!RAW)
 	{
@@ -289,19 +428,19 @@ float_conv_tc_kernel(const FtParams p)
 			++issued;
 			__syncwarp();
 		}
-		// no copy may be in flight when the CTA leaves: bar_done covers it unless something failed
+		// no copy may be in flight when the CTA leaves: the tile's sums cover it unless something failed
 		if (!ok)
 		{
 			for (int s = 0; s < FT_STAGES && s < issued; ++s) { mbar_wait_plain(&bar_full[s], (uint32_t)(((issued - 1 - s) / FT_STAGES) & 1), p.spin_limit); }
 		}
 	}
 
-	if (tid == 0) { mbar_wait<64>(&bar_done, 0, s_failed, p.spin_limit); }
+	if (WHOLE && tid == 0) { mbar_wait<64>(&bar_done, 0, s_failed, p.spin_limit); }
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const bool failed = (*s_failed != 0);
-	const int used = min(FT_ACCS, kbn);
+	const int used = (GROUP == FT_TURNS) ? min(FT_ACCS, kbn) : min(FT_ACCS, kbn + 1);
 	cg::cluster_group cluster = cg::this_cluster();
 	if (p.split > 1)
 	{
@@ -310,12 +449,9 @@ float_conv_tc_kernel(const FtParams p)
 		if (rank > 0 && warp >= 1 && warp <= FT_PRODUCER_WARPS)
 		{
 			float * theirs = cluster.map_shared_rank(reinterpret_cast<float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))), 0) + (size_t)(rank - 1) * FT_NF * TC_PIX;
-			const int quarter = warp & 3;
-			const int chunk = (warp - 1) >> 2;
-			float acc[32];
-			tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, acc);
+			if constexpr (WHOLE) { tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, sums); }
 			#pragma unroll
-			for (int j = 0; j < 32; ++j) { theirs[(chunk * 32 + j) * TC_PIX + quarter * 32 + lane] = acc[j]; }
+			for (int j = 0; j < 32; ++j) { theirs[(chunk * 32 + j) * TC_PIX + quarter * 32 + lane] = sums[j]; }
 		}
 		cluster.sync();
 	}
@@ -323,27 +459,27 @@ float_conv_tc_kernel(const FtParams p)
 	if (!failed && rank == 0 && warp >= 1 && warp <= FT_PRODUCER_WARPS)
 	{
 		// warp w reads the TMEM lanes of quarter w % 4 and one of the four 32-filter chunks
-		const int quarter = warp & 3;
-		const int chunk = (warp - 1) >> 2;
 		const int g = g0 + quarter * 32 + lane;
 		const bool col_ok = g < p.total;
 		const int img = col_ok ? g / p.HW : 0;
 		const int pix = col_ok ? g - img * p.HW : 0;
 		float * out_pix = p.out + ((size_t)img * p.N + f0 + chunk * 32) * p.HW + pix;
 		const float slope = p.leaky ? 0.1f : 1.0f;
-		float acc[32];
-		tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, acc);
-		const float * sums = reinterpret_cast<const float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))) + (size_t)chunk * 32 * TC_PIX + quarter * 32 + lane;
-		for (int r = 1; r < p.split; ++r, sums += FT_NF * TC_PIX)
+		if constexpr (WHOLE) { tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, sums); }
+		const float * others = reinterpret_cast<const float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))) + (size_t)chunk * 32 * TC_PIX + quarter * 32 + lane;
+		for (int r = 1; r < p.split; ++r, others += FT_NF * TC_PIX)
 		{
 			#pragma unroll
-			for (int j = 0; j < 32; ++j) { acc[j] = __fadd_rn(acc[j], sums[j * TC_PIX]); }
+			for (int j = 0; j < 32; ++j) { sums[j] = __fadd_rn(sums[j], others[j * TC_PIX]); }
 		}
-		int e = (p.yolo_entries > 0) ? (f0 + chunk * 32) % p.yolo_entries : 0;
+		const int e0 = (p.yolo_entries > 0) ? (f0 + chunk * 32) % p.yolo_entries : 0;
+		int e = e0;
+		uint32_t again = 0;
 		#pragma unroll
 		for (int j = 0; j < 32; ++j)
 		{
-			float v = __fadd_rn(acc[j], s_bias[chunk * 32 + j]);
+			if (FINE && !(fabsf(sums[j]) <= 3.0e38f)) { again |= 1u << j; }
+			float v = __fadd_rn(sums[j], s_bias[chunk * 32 + j]);
 			v = fmaxf(v, __fmul_rn(v, slope));
 			if (p.yolo_entries > 0)
 			{
@@ -352,6 +488,18 @@ float_conv_tc_kernel(const FtParams p)
 				if (++e == p.yolo_entries) { e = 0; }
 			}
 			if (col_ok && f0 + chunk * 32 + j < p.N) { out_pix[(size_t)j * p.HW] = v; }
+		}
+		if constexpr (FINE)
+		{
+			for (int j = 0; j < 32; ++j)
+			{
+				if (((again >> j) & 1u) == 0 || !col_ok || f0 + chunk * 32 + j >= p.N) { continue; }
+				float v = __fadd_rn(plain_sum(p, img, pix, f0 + chunk * 32 + j), s_bias[chunk * 32 + j]);
+				v = fmaxf(v, __fmul_rn(v, slope));
+				const int entry = (p.yolo_entries > 0) ? (e0 + j) % p.yolo_entries : 2;
+				if (entry != 2 && entry != 3) { v = 1.0f / (1.0f + expf(-v)); }
+				out_pix[(size_t)j * p.HW] = v;
+			}
 		}
 	}
 	else if (failed && tid == 0)
@@ -378,10 +526,18 @@ __global__ void float_conv_tc_weights_kernel(const float * __restrict__ w, float
 		const int row = i >> 5, k = i & 31;
 		const int f = tile_f * FT_NF + row, c = c0 + k;
 		const float v = (f < n && c < C) ? w[((size_t)f * C + c) * taps + tap] : 0.0f;
-		const float hi = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
+		float hi, lo;
+		split_nearest(v, hi, lo);
+		if (!(fabsf(v) <= 3.0e38f))
+		{
+			// parts that still add up to v: an infinity or NaN stays in the first
+			const bool finite = fabsf(v) <= 3.4028235e38f;
+			hi = finite ? __uint_as_float(__float_as_uint(v) & 0xFFFFE000u) : v;
+			lo = finite ? __fsub_rn(v, hi) : 0.0f;
+		}
 		const int at = row * 32 + (((k >> 2) ^ (row & 7)) << 2) + (k & 3);
 		dst[at] = hi;
-		dst[FT_TILE_BYTES / 4 + at] = __fsub_rn(v, hi);
+		dst[FT_TILE_BYTES / 4 + at] = lo;
 	}
 }
 
@@ -423,7 +579,15 @@ static int launch_float_tc(const xnor_b200_conv_desc * desc, const float * input
 	// as many CTAs per tile as leave the grid one wave and each of them a few K blocks (about 3 us go into joining the sums)
 	p.split = 1;
 	for (int s = 2; s <= FT_MAX_SPLIT; ++s) { if (tiles * s <= sm_count() && p.kblocks >= 4 * s) { p.split = s; } }
-	rc = ensure_dynamic_smem((const void *)float_conv_tc_kernel<RAW>, FT_SMEM_BYTES);
+	// Which sums: no less accurate than the fp32 kernel that would do it otherwise (figures above).  An accumulator of FT_APART takes 96
+	// instructions of large products at 72 K blocks; the error grows with their number.
+	auto kernel = float_conv_tc_kernel<RAW, FT_TURNS>;
+	if constexpr (!RAW)
+	{
+		if (total <= 1024) { kernel = float_conv_tc_kernel<false, 1>; }
+		else if (p.taps == 9) { kernel = (p.kblocks <= 72 * p.split) ? float_conv_tc_kernel<false, FT_APART> : float_conv_tc_kernel<false, 8>; }
+	}
+	rc = ensure_dynamic_smem((const void *)kernel, FT_SMEM_BYTES);
 	if (rc != XNOR_B200_OK) { return rc; }
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3((unsigned)(tiles * p.split), 1, 1);
@@ -437,7 +601,7 @@ static int launch_float_tc(const xnor_b200_conv_desc * desc, const float * input
 	attr[0].val.clusterDim.z = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
-	const cudaError_t e = cudaLaunchKernelEx(&cfg, float_conv_tc_kernel<RAW>, p);
+	const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
 	return (e == cudaSuccess) ? check_launch() : cuda_fail(e);
 }
 

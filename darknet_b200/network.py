@@ -687,14 +687,16 @@ def _map_conv_desc(net: Network, l: Layer) -> capi.ConvDesc:
 
 
 def _map_conv_wins(net: Network, l: Layer) -> bool:
-    """Whether a float convolution runs on the small-map kernel rather than as a tensor-core GEMM.  Measured on B200 (us, map / GEMM):
-    3x3 256 -> 512: 21 / 25 at 169 pixels, 31 / 25 at 338, 101 / 30 at 1352; 1x1 512 -> 255: 7 / 15 at 169, 16 / 15 at 627;
-    1x1 256 -> 255: 9 / 13 at 676, 22 / 13 at 2508; 1x1 1024 -> 512: 27 / 18 at 196.  The map kernels work in runs of 32 pixels of
-    one image (1x1 512 -> 1000 on 64 maps of one pixel: 116 / 21)."""
+    """Whether a float convolution runs on the small-map kernel rather than as a tensor-core GEMM; both are as accurate there.  Measured
+    on B200 (us, map / GEMM): 3x3 256 -> 512: 23 / 33 at 169 pixels, 32 / 33 at 338, 56 / 35 at 676; 1x1 512 -> 255: 9 / 18 at 169, 18 / 18
+    at 676, 21 / 18 at 1014; 1x1 256 -> 255: 10 / 16 at 784; 1x1 1024 -> 425: 19 / 23 at 169, 29 / 23 at 338; 1024 -> 1000: 25 / 23 at one
+    pixel, 51 / 23 at 196.  The map kernels work in runs of 32 pixels of one image (1x1 1024 -> 1000 on 64 maps of one pixel: 977 / 30)."""
     pixels = net.batch * (-(-l.out_h * l.out_w // 32) * 32)
     if net.batch * l.out_h * l.out_w > net.float_map_max_pixels:
         return False
-    return pixels <= 256 if l.size == 3 else (l.c <= 512 and pixels <= 704)
+    if l.size == 3:
+        return pixels <= 384
+    return pixels <= 800 if l.c <= 512 else pixels <= 192 and l.c * l.n <= 450_000
 
 
 def prepare_float_map_convs(net: Network) -> None:

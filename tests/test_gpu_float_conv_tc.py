@@ -20,6 +20,9 @@ from darknet_b200 import capi  # noqa: E402
     (1, 32, 11, 19, 40, 3, 1, 0),       # 9 K blocks: split 2
     (3, 64, 7, 9, 129, 3, 1, 0),        # 18 K blocks: split 4, halo rows of neighbouring images
     (40, 64, 16, 33, 16, 3, 0, 8),      # one wave full: no split
+    (64, 512, 13, 13, 64, 3, 1, 0),     # more K blocks a tile than two accumulators may take: groups of eight
+    (1, 32, 32, 32, 130, 3, 0, 0), (1, 32, 25, 41, 130, 3, 0, 0),      # 1024 pixels and one more
+    (2, 300, 23, 22, 33, 1, 1, 11), (3, 300, 19, 18, 33, 1, 1, 11),    # 1012 and 1026, K blocks that are not whole
 ])
 def test_prepared_filters_match_fp64(batch, c, h, w, n, size, leaky, entries):
     seed = batch + c + h + n
@@ -42,3 +45,65 @@ def test_prepared_filters_match_fp64(batch, c, h, w, n, size, leaky, entries):
     st = C.c_int(-1)
     capi.check(lib.xnor_b200_take_device_status(C.byref(st)), "xnor_b200_take_device_status")
     assert st.value == 0
+
+
+def prepared_conv(kind, desc, x, wt, b):
+    lib, stream = capi.lib(), torch.cuda.current_stream().cuda_stream
+    call = {"tc": lambda *a: lib.xnor_b200_float_conv_tc(*a[:-1], 0, a[-1]), "map": lib.xnor_b200_float_conv_map}[kind]
+    nbytes = getattr(lib, f"xnor_b200_float_conv_{kind}_weights_bytes")(C.byref(desc))
+    assert nbytes
+    prepared = torch.empty(nbytes // 4, device="cuda")
+    capi.check(getattr(lib, f"xnor_b200_float_conv_{kind}_prepare")(C.byref(desc), wt.data_ptr(), prepared.data_ptr(), stream), "prepare")
+    out = torch.full((desc.batch, desc.n, desc.h, desc.w), float("nan"), device="cuda")
+    capi.check(call(C.byref(desc), x.data_ptr(), prepared.data_ptr(), b.data_ptr(), out.data_ptr(), stream), "conv")
+    return out
+
+
+def fp64(x, wt, b):
+    """The convolution as one matrix product an image, in 64 bits."""
+    n, c, size, _ = wt.shape
+    cols = F.unfold(x, size, padding=size // 2).double()
+    return (wt.double().view(n, -1) @ cols + b.double().view(1, n, 1)).view(x.shape[0], n, *x.shape[2:])
+
+
+@pytest.mark.parametrize("batch,c,h,w,n,size", [
+    (2, 256, 13, 13, 512, 3), (3, 256, 11, 19, 512, 3), (16, 256, 7, 7, 512, 3), (1, 256, 19, 19, 512, 3), (4, 512, 13, 13, 255, 1), (1, 512, 28, 28, 255, 1),
+    (1, 1024, 13, 13, 425, 1), (6, 1024, 13, 13, 425, 1), (1, 1024, 14, 14, 1000, 1), (8, 1024, 1, 1, 1000, 1),
+    (8, 256, 13, 13, 512, 3), (64, 256, 13, 13, 512, 3), (9, 256, 11, 19, 512, 3), (32, 256, 7, 7, 512, 3), (16, 512, 13, 13, 128, 3),
+])
+def test_no_less_accurate_than_the_fp32_kernels(batch, c, h, w, n, size):
+    """Against the small-map kernel where that one would run (up to 1024 pixels), against cuDNN's fp32 convolution beyond.  A tenth of
+    the rounding of a single fp32 result (2^-24, 6e-8) is left for the draw of the values."""
+    torch.backends.cudnn.allow_tf32 = False
+    g = torch.Generator(device="cuda").manual_seed(batch + c + n)
+    x = F.leaky_relu(torch.randn(batch, c, h, w, generator=g, device="cuda") * 3, 0.1)
+    wt = torch.randn(n, c, size, size, generator=g, device="cuda") * (c * size * size) ** -0.5
+    b = torch.randn(n, generator=g, device="cuda") * 0.01
+    want = fp64(x, wt, b)
+
+    def error(y):
+        return float((y.double() - want).norm() / want.norm())
+    desc = capi.ConvDesc(batch, c, h, w, n, size, 1, size // 2, capi.LINEAR)
+    other = prepared_conv("map", desc, x, wt, b) if batch * h * w <= 1024 else F.conv2d(x, wt, b, 1, size // 2)
+    assert error(prepared_conv("tc", desc, x, wt, b)) <= error(other) + 6e-9
+
+
+@pytest.mark.parametrize("batch,c,h,w,n,size", [(2, 64, 9, 7, 140, 3), (9, 64, 13, 13, 33, 3), (2, 96, 9, 7, 140, 1), (64, 512, 13, 13, 32, 3)])
+@pytest.mark.parametrize("leaky", [0, 1])
+def test_infinite_and_huge_values(batch, c, h, w, n, size, leaky):
+    """Infinities and NaN come out where plain arithmetic puts them, and values next to the largest lose nothing."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(batch, c, h, w, generator=g, device="cuda")
+    wt = torch.randn(n, c, size, size, generator=g, device="cuda") * 0.05
+    b = torch.randn(n, generator=g, device="cuda")
+    x[:, 0].clamp_(-0.9, 0.9)                                  # no overflow of fp32 that 64 bits would not have
+    x[0, 3, 1, 2], x[0, 5, 6, 6], x[1, 0, 0, 0], x[1, 7, 4, 3] = float("inf"), float("-inf"), float("nan"), 3.4e38
+    wt[1, 2, 0, 0], wt[2, 1, size - 1, 0], wt[4, 0, 0, size - 1] = float("inf"), float("nan"), -3.4e38
+    want = fp64(x, wt, b)
+    want = torch.where(want > 0, want, want * 0.1) if leaky else want
+    want32 = want.float()
+    got = prepared_conv("tc", capi.ConvDesc(batch, c, h, w, n, size, 1, size // 2, capi.LEAKY if leaky else capi.LINEAR), x, wt, b)
+    assert torch.equal(got.isnan(), want32.isnan()) and torch.equal(got.isinf(), want32.isinf())
+    assert torch.equal(got[got.isinf()], want32[want32.isinf()])
+    fine = want32.isfinite()
+    assert bool(((got[fine] - want32[fine]).abs() <= 2e-5 + 2e-5 * want32[fine].abs()).all())
