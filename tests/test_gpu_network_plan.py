@@ -198,3 +198,20 @@ def test_heads_that_cross_to_the_host(name, batch, tmp_path):
     graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(pinned, want))
+
+
+@pytest.mark.parametrize("name,batch", [("yolov3-tiny_xnor", 1), ("yolov3-tiny_xnor", 4), ("tiny-yolo_xnor", 4), ("darknet53_448_xnor", 1), ("darknet53_448_xnor", 4)])
+def test_the_layer_loop_still_hands_signs_on(name, batch, tmp_path):
+    """The linked layers (sign sinks, sign words, shortcut sums, folded pools) that run a network without a plan, against the plan."""
+    size = 160
+    cfg = tmp_path / "net.cfg"
+    cfg.write_text(cfgs.CFGS[name](size, size))
+    network.write_synthetic_weights(network.parse_network_cfg(str(cfg), 1, "cpu"), str(tmp_path / "w"), exact_first_conv=True)
+    net = network.load_network_custom(str(cfg), str(tmp_path / "w"), batch)
+    assert net.plan is not None and net.sink_links > 0 and any(l.emit_masks or l.emit_planes for l in net.layers)
+    assert (net.sum_sign_links > 0) == (name == "darknet53_448_xnor" and batch >= net.sum_signs_min_batch)
+    x = image(batch, size, size)
+    want = [h.clone() for h in network.forward_network_gpu(net, x)]
+    net.plan = None
+    for _ in range(2):
+        assert_heads_close(network.forward_network_gpu(net, x), want)
