@@ -448,10 +448,11 @@ def run_gpu_arm(args) -> None:
             "vs_baseline": None, "dtype": "u32", "data": "synthetic",
             "config": {"workload": workload_text(args.workload, net.h, batch_text), "global_batch": images_per_forward,
                        "forwards_per_step": fps, "images_per_step": images_per_forward * fps,
-                       "folded_maxpools": net.folded_maxpools, "sign_sinks": net.sink_links, "sign_links": net.sign_links,
+                       "forward": (f"one native call of {network.own_launches_per_forward(net)} kernels, signs handed over as grid words" if net.plan is not None else
+                                   f"layer loop, {net.sink_links} sign sinks, {net.sign_links} sign links, {net.folded_maxpools} folded maxpools"),
                        "side_branch": any(l.branch_start for l in net.layers), "parallelism": f"replicas x{world} (no collective)",
                        "l2": "256 MiB buffer written between timed forwards", "timing": "per-forward CUDA events on the launch stream, CUDA graph replay",
-                       "float_layers": "this library's fp32 kernels at small batch (first conv + pool + sign, small-map convs with the yolo activation), cuDNN/ATen otherwise",
+                       "float_layers": "this library's kernels: first conv + pool as exact signs, small-map fp32 convs and three-product tf32 GEMMs with the head activations",
                        "xnor_binops_per_image": binops_per_image},
             "xnor_gemm_tops": roofline["achieved"] if roofline else None,
             "roofline": roofline, **extra,
@@ -560,7 +561,7 @@ def kernel_rooflines(net, batch, binops_per_image, stream, flush, dev):
     achieved = binops_per_image * batch / (ms_gemm * 1e-3) / 1e12
     traffic, traffic_source = captured_traffic("xnor_gemm_b1_yolov3_tiny_set") if batch == 1 else (None, None)
     roofline = {
-        "kernel": "xnor GEMM kernels of one forward (9 launches = the xnor layers of yolov3-tiny_xnor, stand-alone calls with fp32 epilogue)",
+        "kernel": "packed-operand xnor GEMMs of the nine xnor layers of yolov3-tiny_xnor (stand-alone calls with fp32 epilogue; what xnor_b200_conv_forward launches -- a lowered forward runs xnor_conv_kernel instead)",
         "bound": "int_popc", "achieved": achieved, "peak": popc_peak_tops, "unit": "TOP/s (binary ops, 2*M*N*K)",
         "frac": achieved / popc_peak_tops, "traffic": traffic, "traffic_source": traffic_source,
         "algorithmic_bytes": sum((xl.n + batch * xl.geom.n_out) * xl.geom.new_lda // 8 + 4 * xl.n * batch * xl.geom.n_out for xl in xl_layers),

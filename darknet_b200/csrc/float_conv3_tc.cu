@@ -9,7 +9,9 @@
 //   |approximate - exact| <= (xmax + 1e-4) * 1.03e-3
 //
 // (compared in fp16, hence 1.032e-3 + 1.2e-7) for a filter scaled to sum|w| = 1 and xmax the largest input of the unit: 2^-10 for the
-// two fp16 roundings of a product, 2^-25 each for subnormal operands, the rest for the scaling and the accumulation here and there.
+// two fp16 roundings of a product, 2^-25 each for subnormal operands, and 5.3e-5 for the rest: 2e-6 for the scaling and the fp32 sum
+// there, and for the sum here six instructions of 17 terms that lose up to 2^-23 of the largest each, twice over where the bias is as large
+// as the products (2.4e-5).  That loss per term is how fp32 accumulation is taken to be, not something the hardware states.
 // Inputs or filters that fp16 cannot hold make the bound infinite or the value NaN, and every value is formed again.
 //
 // One MMA row is a 2x2 block of pixels, its columns the block's four values of every filter, K the patch of pixels around it: with

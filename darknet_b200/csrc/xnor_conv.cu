@@ -856,7 +856,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					{
 						const int down = 2 - p.src[si].scale, src_pitch = p.src[si].pitch, src_rows = p.src[si].h + 1;
 						const int base = p.src[si].front - (si ? run1.start : run0.start);
-						// a division per entry: four independent ones at a time beat one chain of steps of 32 positions (104x104 83 / 115 us)
+						// a division per entry: two independent ones at a time beat four, and one chain of steps of 32 positions (104x104 83 / 115 us)
 						#pragma unroll 2
 						for (int s = lane; s < slots_plane; s += 32)
 						{
@@ -1048,7 +1048,8 @@ static bool plan_sizes(const XcParams & p, int nf, int pt, int stream, XcPlan * 
 }
 
 // Estimated cycles of the busiest SM, fitted to clock traces of the roles.  Per tile: MMAs (73 / 56 / 47 cycles per 64 bits for 128 /
-// 64 / 32 filters), epilogue (about 130 issue slots per sign word, 450 with fp32 values, over four schedulers); per stage the
+// 64 / 32 filters), epilogue (about 130 issue slots per sign word; 450 with fp32 values, some more than it takes since values go in pairs, which
+// ranks the plans as well and is kept); per stage the
 // expanders: 350 cycles of hand-overs and 110 per round of words (170 through the table with a pool, 350 for four parity planes).
 // The slowest role sets the pace, the others take issue slots and shared-memory bandwidth from it.
 static double plan_cost(const XcParams & p, const XcPlan & q, int mode)

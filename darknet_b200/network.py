@@ -1072,8 +1072,8 @@ def load_network_custom(cfg: str, weights: str, batch: int = 1, device: str = "c
                         sum_signs_min_batch: Optional[int] = None, sink_max_batch: Optional[int] = None,
                         packed_cache: bool = False) -> Network:
     """load_network_custom (src-lib/weights.cpp:665-691): parse, load, fold batch-norm, pack binary weights.
-    float_map_max_pixels, sum_signs_min_batch and sink_max_batch override the measured hand-over thresholds of the Network
-    (tuning runs).  packed_cache: read the packed weights from <weights>.xnorpack where it matches, and (re)write that file
+    float_map_max_pixels, sum_signs_min_batch and sink_max_batch override the measured thresholds of the Network (tuning runs); the last
+    two are of the layer loop, which runs what network_plan does not lower.  packed_cache: read the packed weights from <weights>.xnorpack where it matches, and (re)write that file
     when any layer had to be packed afresh."""
     torch.backends.cudnn.allow_tf32 = False
     torch.backends.cuda.matmul.allow_tf32 = False
