@@ -688,15 +688,16 @@ def _map_conv_desc(net: Network, l: Layer) -> capi.ConvDesc:
 
 def _map_conv_wins(net: Network, l: Layer) -> bool:
     """Whether a float convolution runs on the small-map kernel rather than as a tensor-core GEMM; both are as accurate there.  Measured
-    on B200 (us, map / GEMM): 3x3 256 -> 512: 23 / 33 at 169 pixels, 32 / 33 at 338, 56 / 35 at 676; 1x1 512 -> 255: 9 / 18 at 169, 18 / 18
-    at 676, 21 / 18 at 1014; 1x1 256 -> 255: 10 / 16 at 784; 1x1 1024 -> 425: 19 / 23 at 169, 29 / 23 at 338; 1024 -> 1000: 25 / 23 at one
-    pixel, 51 / 23 at 196.  The map kernels work in runs of 32 pixels of one image (1x1 1024 -> 1000 on 64 maps of one pixel: 977 / 30)."""
+    on B200 (us, map / GEMM): 3x3 256 -> 512, one image: 23..27 / 33 up to 190 pixels, 35 / 33 from 204 on; two of 7x7 23 / 33, three
+    35 / 33, five 62 / 33; 1x1 512 -> 255: 9 / 19 at 169, 19 / 19 from 676 on, 21 / 18 at 1014; 1x1 256 -> 255: 10 / 17 at 784;
+    1x1 1024 -> 425: 19 / 23 at 190, three of 7x7 41 / 23, two of 13x13 29 / 23; 1024 -> 1000: 25 / 23 at one pixel, 51 / 23 at 196.
+    The map kernels work in runs of 32 pixels of one image (1x1 1024 -> 1000 on 64 maps of one pixel: 977 / 30)."""
     pixels = net.batch * (-(-l.out_h * l.out_w // 32) * 32)
     if net.batch * l.out_h * l.out_w > net.float_map_max_pixels:
         return False
     if l.size == 3:
-        return pixels <= 384
-    return pixels <= 800 if l.c <= 512 else pixels <= 192 and l.c * l.n <= 450_000
+        return net.batch <= 2 and pixels <= 192
+    return pixels <= 800 if l.c <= 512 else net.batch == 1 and pixels <= 192 and l.c * l.n <= 450_000
 
 
 def prepare_float_map_convs(net: Network) -> None:

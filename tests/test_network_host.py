@@ -96,3 +96,15 @@ def test_maxpool_follows_darknet_padding_rule():
     l = network.Layer("maxpool", 0, 1, 6, 6, size=2, stride=2, pad=1, out_c=1, out_h=3, out_w=3)
     y = network._maxpool(torch.arange(36.0).reshape(1, 1, 6, 6), l)
     assert y.flatten().tolist() == [7, 9, 11, 19, 21, 23, 31, 33, 35]
+
+
+@pytest.mark.parametrize("batch,c,h,w,n,size,small_map", [
+    (1, 256, 13, 13, 512, 3, True), (1, 256, 12, 17, 512, 3, False), (2, 256, 7, 7, 512, 3, True), (5, 256, 7, 7, 512, 3, False), (1, 512, 19, 19, 255, 1, True),
+    (4, 512, 13, 13, 255, 1, True), (6, 512, 13, 13, 255, 1, False), (1, 256, 28, 28, 255, 1, True), (1, 1024, 13, 13, 425, 1, True),
+    (3, 1024, 7, 7, 425, 1, False), (1, 1024, 1, 1, 1000, 1, False), (64, 1024, 1, 1, 1000, 1, False),
+])
+def test_float_convolutions_take_the_faster_kernel(batch, c, h, w, n, size, small_map):
+    """Both sides of the lines between the small-map kernel and the GEMM, with the shapes they were measured at."""
+    net = network.Network(batch, 3, 32, 32, [], "cpu")
+    l = network.Layer("convolutional", 0, c, h, w, n, h, w, n=n, size=size)
+    assert network._map_conv_wins(net, l) == small_map
