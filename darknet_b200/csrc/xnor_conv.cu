@@ -35,8 +35,8 @@
 //
 // Measured (B200, 64 images, before and after the shortcut operand's loads lost their conditions and values went in pairs): 128 -> 256
 // 3x3 56x56 with a shortcut 153 -> 88 us (63 at the copy rate), 256 -> 512 28x28 88 -> 59; 128 -> 256 104x104 to fp32 188 -> 172
-// (108 at the copy rate).  Bound by the SM's issue slots, 55 to 70 % busy, beside operand reads that take half of the shared-memory
-// pipe.  Twice the expanders (188 us), half the epilogue warps (225), scales kept in registers (172): no gain.
+// (108 at the copy rate).  Bound by the SM's issue slots, 53 % busy for the last of these, and the shared-memory pipe (68 %); with a
+// shortcut and both tensors written, by memory latency (issue slots 26 %, DRAM 41 %).  Twice the expanders (188 us), half the epilogue warps (225), scales kept in registers (172): no gain.
 #include "grid_words.cuh"
 #include "tc_common.cuh"
 
