@@ -29,12 +29,15 @@ constexpr int DET_CLUSTER = 8;            // CTAs per image
 constexpr int DET_THREADS = 512;
 constexpr int DET_WARPS = DET_THREADS / 32;
 constexpr int DET_ALL_WARPS = DET_CLUSTER * DET_WARPS;
-constexpr int DET_STEP = 4;               // candidates a thread looks at between two scans
+constexpr int DET_STEP = 8;               // candidates a thread looks at between two scans
 constexpr int DET_MAX_ANCHORS = 16;
 constexpr int DET_MAX_HEADS = XNOR_B200_DETECT_HEADS;
 constexpr int DET_LIST_BYTES = 8;         // per candidate of one class: score, storage index, rank order
 constexpr int DET_SMEM_BUDGET = 192 * 1024;
-constexpr int DET_WARP_MAX = 64;          // candidates of one class that a warp suppresses by itself; more go to the whole CTA
+constexpr int DET_MATRIX_MAX = 768;       // detections whose overlaps are kept as a bit matrix (72 KB of shared memory)
+constexpr int DET_MATRIX_WORDS = DET_MATRIX_MAX / 32;
+constexpr int DET_RANK_MAX = 128;         // candidates of one class that a warp ranks by itself; more go to the whole CTA
+constexpr int DET_WARP_MAX = 64;          // without the matrix: candidates of one class that a warp suppresses by itself
 constexpr int DET_BLOCK = 128;            // ranks the CTA settles at a time
 
 struct YoloHeadParams
@@ -61,7 +64,8 @@ struct DetectParams
 	// suppression
 	int nms;
 	float nms_thresh;
-	int lists;                   // per-class candidate lists that fit a CTA's shared memory (at most one per warp)
+	int matrix_max;              // detections up to which the overlap matrix is used: min(max_dets, DET_MATRIX_MAX)
+	int lists, matrix_lists;     // per-class candidate lists that fit a CTA's shared memory (at most one per warp), without and with the matrix
 	// compaction (rows != nullptr)
 	float * rows;                // [batch][max_rows][7]
 	int * row_count;             // [batch]: pairs found (may exceed max_rows: the surplus is not stored)
@@ -71,8 +75,10 @@ struct DetectParams
 // box_iou of src-lib/box.cpp:68-113, :310-344, operation for operation (no contraction into FMAs)
 __device__ __forceinline__ float overlap_1d(float x1, float w1, float x2, float w2)
 {
-	const float l1 = __fsub_rn(x1, __fdiv_rn(w1, 2.0f)), l2 = __fsub_rn(x2, __fdiv_rn(w2, 2.0f));
-	const float r1 = __fadd_rn(x1, __fdiv_rn(w1, 2.0f)), r2 = __fadd_rn(x2, __fdiv_rn(w2, 2.0f));
+	// (half of a value is the same by a division and by a product)
+	const float h1 = __fmul_rn(w1, 0.5f), h2 = __fmul_rn(w2, 0.5f);
+	const float l1 = __fsub_rn(x1, h1), l2 = __fsub_rn(x2, h2);
+	const float r1 = __fadd_rn(x1, h1), r2 = __fadd_rn(x2, h2);
 	return __fsub_rn(fminf(r1, r2), fmaxf(l1, l2));
 }
 
@@ -102,7 +108,7 @@ __device__ __forceinline__ int score_rank(const float * s_score, int m, int c)
 	return rank;
 }
 
-// Greedy suppression of one class's m <= DET_WARP_MAX candidates by one warp.  The boxes go to shared memory in rank order, lane l
+// Lists of more than DET_MATRIX_MAX detections: greedy suppression of one class's m <= DET_WARP_MAX candidates by one warp.  The boxes go to shared memory in rank order, lane l
 // decides about ranks l, l + 32, ...; its verdicts stay in a register, so a step is one shuffle, one broadcast read and the
 // overlaps (reading order, score and box per step from memory took 600 cycles a candidate, this takes about 150).
 __device__ __forceinline__ void suppress_warp(const DetectParams & p, int m, const float * s_score, const uint16_t * s_idx, uint16_t * s_order,
@@ -134,7 +140,7 @@ __device__ __forceinline__ void suppress_warp(const DetectParams & p, int m, con
 	}
 }
 
-// The same for a crowded class, by the whole CTA, DET_BLOCK ranks at a time: every overlap inside the block at once as a bit
+// The same for a crowded class of such a list, by the whole CTA, DET_BLOCK ranks at a time: every overlap inside the block at once as a bit
 // matrix, one warp walks the matrix in rank order (a step costs a shuffle), then the block's survivors are held against all later
 // ranks at once.  Step by step over the list, as a warp does it, 170 candidates took 45 us.
 __device__ __forceinline__ void suppress_cta(const DetectParams & p, int m, float * s_score, const uint16_t * s_idx, uint16_t * s_order,
@@ -197,6 +203,65 @@ __device__ __forceinline__ void suppress_cta(const DetectParams & p, int m, floa
 	}
 }
 
+// The detections of class k that a warp has to deal with: their scores and numbers, in storage order.  Returns how many.
+__device__ __forceinline__ int gather_class(const DetectParams & p, int n, const float * probs, int k, float * s_score, uint16_t * s_idx)
+{
+	const int lane = threadIdx.x & 31;
+	int m = 0;
+	for (int d0 = 0; d0 < n; d0 += 8 * 32)
+	{
+		float s[8];
+		#pragma unroll
+		for (int j = 0; j < 8; ++j)
+		{
+			const int d = d0 + j * 32 + lane;
+			s[j] = (d < n) ? __ldcg(probs + (size_t)d * p.classes + k) : 0.0f;
+		}
+		#pragma unroll
+		for (int j = 0; j < 8; ++j)
+		{
+			const unsigned mask = __ballot_sync(0xffffffffu, s[j] > 0.0f);
+			if (s[j] > 0.0f)
+			{
+				const int at = m + __popc(mask & ((1u << lane) - 1u));
+				s_score[at] = s[j];
+				s_idx[at] = (uint16_t)(d0 + j * 32 + lane);
+			}
+			m += __popc(mask);
+		}
+	}
+	__syncwarp();
+	return m;
+}
+
+// Greedy suppression of one class by one warp: its m detections in rank order, each looked up in the bits of those that a kept one has
+// overlapped, and its own row of the overlap matrix added where it is kept.  Lane l holds the bits of detections 32 l ...; returns them.
+// Overlaps are symmetric and a kept detection overlaps no kept one before it, so a row marks nothing that was kept.  The rows of four
+// ranks are read ahead: a step is a shuffle and a few logical operations, about 40 cycles.
+__device__ __forceinline__ uint32_t walk_class(int m, int words, const uint16_t * s_order, const uint32_t * s_over)
+{
+	const int lane = threadIdx.x & 31;
+	uint32_t dead = 0;
+	for (int r0 = 0; r0 < m; r0 += 4)
+	{
+		int d[4];
+		uint32_t row[4];
+		#pragma unroll
+		for (int j = 0; j < 4; ++j)
+		{
+			d[j] = s_order[min(r0 + j, m - 1)];
+			row[j] = (lane < words) ? s_over[d[j] * DET_MATRIX_WORDS + lane] : 0u;
+		}
+		#pragma unroll
+		for (int j = 0; j < 4; ++j)
+		{
+			const uint32_t word = __shfl_sync(0xffffffffu, dead, d[j] >> 5);
+			if (r0 + j < m && ((word >> (d[j] & 31)) & 1u) == 0) { dead |= row[j]; }
+		}
+	}
+	return dead;
+}
+
 // One cluster of DET_CLUSTER CTAs per image runs decode, suppression and compaction back to back: a frame has some tens of
 // detections, so each step is a few microseconds of latency and the launches between them would cost as much again.  Work is
 // dealt to warps (a warp per detection, per class, per detection again), the scans that fix the order are short enough for every
@@ -223,51 +288,63 @@ detect_kernel(const __grid_constant__ DetectParams p)
 	{
 		unsigned * s_hit = reinterpret_cast<unsigned *>(det_smem);       // candidate number of each new detection, counted over the heads
 		const int first = found;
-		for (int hd = 0; hd < p.n_heads; ++hd)
+		const int entries = 4 + 1 + p.classes;
+		const YoloHeadParams & last = p.heads[p.n_heads - 1];
+		const unsigned candidates = last.first + (unsigned)(last.lw * last.lh) * (unsigned)last.n;     // of all heads: below 2^32
+		auto head_of = [&](unsigned c)
 		{
-			const YoloHeadParams & h = p.heads[hd];
-			const int cells = h.lw * h.lh;
-			const int entries = 4 + 1 + p.classes;
-			const float * pred = h.head + (size_t)b * h.n * entries * cells;
-			const unsigned candidates = (unsigned)cells * h.n;   // below 2^31; reference order: cell outer, anchor inner
-			for (unsigned q0 = 0; q0 < candidates; q0 += DET_STEP * DET_THREADS)
+			int hd = 0;
+			while (hd + 1 < p.n_heads && c >= p.heads[hd + 1].first) { ++hd; }
+			return hd;
+		};
+		for (unsigned long long q0 = 0; q0 < candidates; q0 += DET_STEP * DET_THREADS)
+		{
+			// reference order: heads, cells, anchors from outer to inner
+			float obj[DET_STEP];
+			#pragma unroll
+			for (int j = 0; j < DET_STEP; ++j)
 			{
-				unsigned hits[DET_STEP];
-				#pragma unroll
-				for (int j = 0; j < DET_STEP; ++j)
+				const unsigned long long c = q0 + j * DET_THREADS + threadIdx.x;
+				obj[j] = -INFINITY;
+				if (c < candidates)
 				{
-					const unsigned q = q0 + j * DET_THREADS + threadIdx.x;
-					const int i = (int)(q / (unsigned)h.n);
-					const int a = (int)q - i * h.n;
-					const float obj = (q < candidates) ? __ldg(pred + (size_t)(a * entries + 4) * cells + i) : 0.0f;
-					hits[j] = __ballot_sync(0xffffffffu, q < candidates && obj > p.thresh);
+					const YoloHeadParams & h = p.heads[head_of((unsigned)c)];
+					const unsigned q = (unsigned)c - h.first;
+					const unsigned i = q / (unsigned)h.n, a = q - i * (unsigned)h.n;
+					const size_t cells = (size_t)(h.lw * h.lh);
+					obj[j] = __ldg(h.head + (((size_t)b * h.n + a) * entries + 4) * cells + i);
 				}
-				#pragma unroll
-				for (int j = 0; j < DET_STEP; ++j) { if (lane == 0) { s_cnt[j * DET_WARPS + warp] = __popc(hits[j]); } }
-				__syncthreads();
-				int total = 0, before[DET_STEP];
-				#pragma unroll
-				for (int j = 0; j < DET_STEP; ++j)
-				{
-					#pragma unroll
-					for (int w = 0; w < DET_WARPS; ++w)
-					{
-						if (w == warp) { before[j] = total; }
-						total += s_cnt[j * DET_WARPS + w];
-					}
-				}
-				#pragma unroll
-				for (int j = 0; j < DET_STEP; ++j)
-				{
-					if ((hits[j] >> lane) & 1u)
-					{
-						const int slot = found + before[j] + __popc(hits[j] & ((1u << lane) - 1u));
-						if (slot < p.max_dets) { s_hit[slot - first] = h.first + q0 + j * DET_THREADS + threadIdx.x; }
-					}
-				}
-				found += total;
-				__syncthreads();
 			}
+			unsigned hits[DET_STEP];
+			#pragma unroll
+			for (int j = 0; j < DET_STEP; ++j)
+			{
+				const bool in = q0 + j * DET_THREADS + threadIdx.x < candidates;
+				hits[j] = __ballot_sync(0xffffffffu, in && obj[j] > p.thresh);
+				if (lane == 0) { s_cnt[j * DET_WARPS + warp] = __popc(hits[j]); }
+			}
+			__syncthreads();
+			// prefix sums over (j, warp): four counts a lane
+			static_assert(DET_STEP * DET_WARPS == 128, "four counts per lane");
+			const int4 c4 = *reinterpret_cast<const int4 *>(s_cnt + 4 * lane);
+			int incl = c4.x + c4.y + c4.z + c4.w;
+			const int own = incl;
+			#pragma unroll
+			for (int o = 1; o < 32; o <<= 1)
+			{
+				const int u = __shfl_up_sync(0xffffffffu, incl, o);
+				if (lane >= o) { incl += u; }
+			}
+			const int part = warp & 3;                            // of a lane's four counts, those before this warp's
+			const int before = incl - own + ((part > 0) ? c4.x : 0) + ((part > 1) ? c4.y : 0) + ((part > 2) ? c4.z : 0);
+			#pragma unroll
+			for (int j = 0; j < DET_STEP; ++j)
+			{
+				const int slot = found + __shfl_sync(0xffffffffu, before, j * (DET_WARPS / 4) + warp / 4) + __popc(hits[j] & ((1u << lane) - 1u));
+				if (((hits[j] >> lane) & 1u) && slot < p.max_dets) { s_hit[slot - first] = (unsigned)(q0 + j * DET_THREADS + threadIdx.x); }
+			}
+			found += __shfl_sync(0xffffffffu, incl, 31);
+			__syncthreads();
 		}
 		// correct_yolo_boxes: the network-to-image mapping, in double as the reference computes it
 		int new_w = p.netw, new_h = p.neth;
@@ -278,32 +355,53 @@ detect_kernel(const __grid_constant__ DetectParams p)
 		}
 		const float deltaw = (float)(p.netw - new_w), deltah = (float)(p.neth - new_h);
 		const float ratiow = (float)new_w / p.netw, ratioh = (float)new_h / p.neth;
+		const bool whole = (new_w == p.netw && new_h == p.neth);  // the mapping takes 0 off and divides by 1
 		const int stored = min(found, p.max_dets);
-		for (int slot = first + all_warp; slot < stored; slot += DET_ALL_WARPS)
+		// a warp per detection; its first three entries a lane are asked for while the one before is worked on
+		constexpr int AHEAD = 3;
+		auto entries_of = [&](int slot)
 		{
 			const unsigned hit = s_hit[slot - first];
-			int hd = 0;
-			while (hd + 1 < p.n_heads && hit >= p.heads[hd + 1].first) { ++hd; }
-			const YoloHeadParams & h = p.heads[hd];
+			const YoloHeadParams & h = p.heads[head_of(hit)];
+			const unsigned q = hit - h.first, i = q / (unsigned)h.n, a = q - i * (unsigned)h.n;
+			return h.head + ((size_t)b * h.n + a) * entries * (size_t)(h.lw * h.lh) + i;
+		};
+		auto fetch = [&](int slot, float (&v)[AHEAD])
+		{
+			if (slot >= stored) { return; }
+			const float * e = entries_of(slot);
+			const YoloHeadParams & h = p.heads[head_of(s_hit[slot - first])];
+			#pragma unroll
+			for (int j = 0; j < AHEAD; ++j) { v[j] = (lane + 32 * j < entries) ? __ldg(e + (size_t)(lane + 32 * j) * (h.lw * h.lh)) : 0.0f; }
+		};
+		float next[AHEAD] = {};
+		fetch(first + all_warp, next);
+		for (int slot = first + all_warp; slot < stored; slot += DET_ALL_WARPS)
+		{
+			float now[AHEAD];
+			#pragma unroll
+			for (int j = 0; j < AHEAD; ++j) { now[j] = next[j]; }
+			fetch(slot + DET_ALL_WARPS, next);
+			const unsigned hit = s_hit[slot - first];
+			const YoloHeadParams & h = p.heads[head_of(hit)];
 			const int q = (int)(hit - h.first);
-			const int cells = h.lw * h.lh;
-			const int entries = 4 + 1 + p.classes;
 			const int i = q / h.n;
 			const int a = q - i * h.n;
-			const float * e = h.head + ((size_t)b * h.n + a) * entries * cells + i;
-			const float v = (lane < entries) ? __ldg(e + (size_t)lane * cells) : 0.0f;
-			const float tx = __shfl_sync(0xffffffffu, v, 0), ty = __shfl_sync(0xffffffffu, v, 1);
-			const float tw = __shfl_sync(0xffffffffu, v, 2), th = __shfl_sync(0xffffffffu, v, 3);
-			const float obj = __shfl_sync(0xffffffffu, v, 4);
+			const float tx = __shfl_sync(0xffffffffu, now[0], 0), ty = __shfl_sync(0xffffffffu, now[0], 1);
+			const float tw = __shfl_sync(0xffffffffu, now[0], 2), th = __shfl_sync(0xffffffffu, now[0], 3);
+			const float obj = __shfl_sync(0xffffffffu, now[0], 4);
 			float * pr = probs + (size_t)slot * p.classes;
-			if (lane >= 5 && lane < entries)
+			#pragma unroll
+			for (int j = 0; j < AHEAD; ++j)
 			{
-				const float prob = __fmul_rn(obj, v);
-				pr[lane - 5] = (prob > p.thresh) ? prob : 0.0f;
+				const int at = lane + 32 * j;
+				const float prob = __fmul_rn(obj, now[j]);
+				if (at >= 5 && at < entries) { pr[at - 5] = (prob > p.thresh) ? prob : 0.0f; }
 			}
-			for (int j = lane + 32; j < entries; j += 32)
+			const float * e = entries_of(slot);
+			for (int j = lane + 32 * AHEAD; j < entries; j += 32)
 			{
-				const float prob = __fmul_rn(obj, __ldg(e + (size_t)j * cells));
+				const float prob = __fmul_rn(obj, __ldg(e + (size_t)j * (h.lw * h.lh)));
 				pr[j - 5] = (prob > p.thresh) ? prob : 0.0f;
 			}
 			const int row = i / h.lw, col = i - row * h.lw;
@@ -320,10 +418,13 @@ detect_kernel(const __grid_constant__ DetectParams p)
 				bw = __fdiv_rn(__fmul_rn(expf(tw), h.anchor_w[a]), (float)p.netw);
 				bh = __fdiv_rn(__fmul_rn(expf(th), h.anchor_h[a]), (float)p.neth);
 			}
-			bx = (float)(((double)bx - (double)deltaw / 2. / p.netw) / (double)ratiow);
-			by = (float)(((double)by - (double)deltah / 2. / p.neth) / (double)ratioh);
-			bw = __fmul_rn(bw, __fdiv_rn(1.0f, ratiow));
-			bh = __fmul_rn(bh, __fdiv_rn(1.0f, ratioh));
+			if (!whole)
+			{
+				bx = (float)(((double)bx - (double)deltaw / 2. / p.netw) / (double)ratiow);
+				by = (float)(((double)by - (double)deltah / 2. / p.neth) / (double)ratioh);
+				bw = __fmul_rn(bw, __fdiv_rn(1.0f, ratiow));
+				bh = __fmul_rn(bh, __fdiv_rn(1.0f, ratioh));
+			}
 			if (!p.relative)
 			{
 				bx = __fmul_rn(bx, (float)p.img_w); bw = __fmul_rn(bw, (float)p.img_w);
@@ -339,9 +440,79 @@ detect_kernel(const __grid_constant__ DetectParams p)
 		cluster.sync();                                          // the lists are complete; every CTA has read the old count
 		if (rank == 0 && threadIdx.x == 0) { p.count[b] = found; }
 	}
+	else { cluster.sync(); }                                     // every CTA runs: its shared memory may be written to
 	const int n = min(found, p.max_dets);
 
-	if (p.nms)
+	// With the matrix the counts and first rows of the detections need no pass of their own: the suppression counts what it leaves.
+	const bool matrix = (p.nms && n <= p.matrix_max);
+	int * const s_rows = reinterpret_cast<int *>(det_smem);      // rows of a detection
+	if (matrix)
+	{
+		float4 * s_box = reinterpret_cast<float4 *>(s_rows + ((p.matrix_max + 3) & ~3));
+		uint32_t * s_over = reinterpret_cast<uint32_t *>(s_box + p.matrix_max);
+		float * s_lists = reinterpret_cast<float *>(s_over + p.matrix_max * DET_MATRIX_WORDS);
+		for (int d = threadIdx.x; d < n; d += DET_THREADS)
+		{
+			s_rows[d] = 0;
+			s_box[d] = __ldcg(boxes + d);
+		}
+		float * s_score = s_lists + (size_t)warp * p.matrix_max * (DET_LIST_BYTES / 4);
+		uint16_t * s_idx = reinterpret_cast<uint16_t *>(s_score + p.matrix_max);
+		uint16_t * s_order = s_idx + p.matrix_max;
+		const int words = (n + 31) / 32;
+		for (int k0 = 0; k0 < p.classes; k0 += DET_CLUSTER * p.matrix_lists)
+		{
+			// warps 0 .. lists-1 of every CTA: one class each
+			const int k = k0 + warp * DET_CLUSTER + rank;
+			const int m = (warp < p.matrix_lists && k < p.classes) ? gather_class(p, n, probs, k, s_score, s_idx) : 0;
+			if (lane == 0) { s_m[warp] = m; }
+			__syncthreads();
+			if (k0 == 0)
+			{
+				for (int i = all_warp; i < n * words; i += DET_ALL_WARPS)
+				{
+					const int r = i / words, w = i - r * words, c = w * 32 + lane;
+					const bool over = (c < n && c != r) && box_iou_dev(s_box[r], s_box[c]) > p.nms_thresh;
+					const uint32_t bits = __ballot_sync(0xffffffffu, over);
+					if (lane < DET_CLUSTER) { *cluster.map_shared_rank(s_over + r * DET_MATRIX_WORDS + w, lane) = bits; }
+				}
+			}
+			if (m <= DET_RANK_MAX)
+			{
+				for (int c = lane; c < m; c += 32) { s_order[score_rank(s_score, m, c)] = s_idx[c]; }
+			}
+			for (int w = 0; w < p.matrix_lists; ++w)             // crowded classes: ranked by the whole CTA
+			{
+				const int mw = s_m[w];
+				if (mw <= DET_RANK_MAX) { continue; }
+				const float * score = s_lists + (size_t)w * p.matrix_max * (DET_LIST_BYTES / 4);
+				const uint16_t * idx = reinterpret_cast<const uint16_t *>(score + p.matrix_max);
+				uint16_t * order = const_cast<uint16_t *>(idx) + p.matrix_max;
+				for (int c = threadIdx.x; c < mw; c += DET_THREADS) { order[score_rank(score, mw, c)] = idx[c]; }
+			}
+			if (k0 == 0) { cluster.sync(); }                      // the matrix is complete, everybody's counts are zero
+			else { __syncthreads(); }
+			if (m > 0)
+			{
+				const uint32_t dead = walk_class(m, words, s_order, s_over);
+				for (int c0 = 0; c0 < m; c0 += 32)
+				{
+					const int d = s_idx[min(c0 + lane, m - 1)];
+					const uint32_t word = __shfl_sync(0xffffffffu, dead, d >> 5);
+					if (c0 + lane >= m) { continue; }
+					if ((word >> (d & 31)) & 1u) { probs[(size_t)d * p.classes + k] = 0.0f; }
+					else
+					{
+						#pragma unroll
+						for (int r = 0; r < DET_CLUSTER; ++r) { atomicAdd(cluster.map_shared_rank(s_rows + d, r), 1); }
+					}
+				}
+			}
+			__syncthreads();
+		}
+		cluster.sync();
+	}
+	else if (p.nms)
 	{
 		const int warp_max = min(DET_WARP_MAX, p.max_dets);
 		float4 * s_boxes = reinterpret_cast<float4 *>(det_smem + (((size_t)p.lists * p.max_dets * DET_LIST_BYTES + 15) & ~(size_t)15));
@@ -355,29 +526,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 			int m = 0;
 			if (warp < p.lists && k < p.classes)
 			{
-				for (int d0 = 0; d0 < n; d0 += 4 * 32)
-				{
-					float s[4];
-					#pragma unroll
-					for (int j = 0; j < 4; ++j)
-					{
-						const int d = d0 + j * 32 + lane;
-						s[j] = (d < n) ? __ldcg(probs + (size_t)d * p.classes + k) : 0.0f;
-					}
-					#pragma unroll
-					for (int j = 0; j < 4; ++j)
-					{
-						const unsigned mask = __ballot_sync(0xffffffffu, s[j] > 0.0f);
-						if (s[j] > 0.0f)
-						{
-							const int at = m + __popc(mask & ((1u << lane) - 1u));
-							s_score[at] = s[j];
-							s_idx[at] = (uint16_t)(d0 + j * 32 + lane);
-						}
-						m += __popc(mask);
-					}
-				}
-				__syncwarp();
+				m = gather_class(p, n, probs, k, s_score, s_idx);
 				if (m > 1 && m <= DET_WARP_MAX) { suppress_warp(p, m, s_score, s_idx, s_order, s_boxes + warp * warp_max, boxes, probs, k); }
 			}
 			if (lane == 0) { s_m[warp] = m; }
@@ -398,22 +547,24 @@ detect_kernel(const __grid_constant__ DetectParams p)
 	if (p.rows != nullptr)
 	{
 		// rows per detection, then the prefix sums every CTA needs for its own detections
-		int * s_rows = reinterpret_cast<int *>(det_smem);        // rows of detection d: kept by the CTA whose warp counts it
-		int * s_start = s_rows + p.max_dets;
-		for (int d = all_warp; d < n; d += DET_ALL_WARPS)
+		int * s_start = s_rows + (matrix ? p.matrix_max : p.max_dets);
+		if (!matrix)
 		{
-			int c = 0;
-			for (int k = lane; k < p.classes; k += 32) { c += (__ldcg(probs + (size_t)d * p.classes + k) > 0.0f) ? 1 : 0; }
-			c = __reduce_add_sync(0xffffffffu, c);
-			if (lane == 0) { s_rows[d] = c; }
+			for (int d = all_warp; d < n; d += DET_ALL_WARPS)
+			{
+				int c = 0;
+				for (int k = lane; k < p.classes; k += 32) { c += (__ldcg(probs + (size_t)d * p.classes + k) > 0.0f) ? 1 : 0; }
+				c = __reduce_add_sync(0xffffffffu, c);
+				if (lane < DET_CLUSTER) { cluster.map_shared_rank(s_rows, lane)[d] = c; }
+			}
+			cluster.sync();
 		}
-		cluster.sync();
 		int base = 0;
 		for (int d0 = 0; d0 < n; d0 += DET_THREADS)
 		{
 			const int d = d0 + threadIdx.x;
 			int c = 0;
-			if (d < n) { c = cluster.map_shared_rank(s_rows, (d % DET_ALL_WARPS) / DET_WARPS)[d]; }
+			if (d < n) { c = s_rows[d]; }
 			int incl = c;
 			#pragma unroll
 			for (int o = 1; o < 32; o <<= 1)
@@ -440,23 +591,55 @@ detect_kernel(const __grid_constant__ DetectParams p)
 			const size_t dd = (size_t)b * p.max_dets + d;
 			const float4 box = __ldcg(boxes + d);
 			const float obj = __ldcg(p.objectness + dd);
-			for (int k0 = 0; k0 < p.classes; k0 += 32)
+			for (int k0 = 0; k0 < p.classes; k0 += 4 * 32)
 			{
-				const int k = k0 + lane;
-				const float s = (k < p.classes) ? __ldcg(probs + (size_t)d * p.classes + k) : 0.0f;
-				const unsigned mask = __ballot_sync(0xffffffffu, s > 0.0f);
-				const int at = slot + __popc(mask & ((1u << lane) - 1u));
-				if (s > 0.0f && at < p.max_rows)
+				float s[4];
+				#pragma unroll
+				for (int j = 0; j < 4; ++j)
 				{
-					float * r = p.rows + ((size_t)b * p.max_rows + at) * 7;
-					r[0] = box.x; r[1] = box.y; r[2] = box.z; r[3] = box.w; r[4] = obj; r[5] = (float)k; r[6] = s;
+					const int k = k0 + j * 32 + lane;
+					s[j] = (k < p.classes) ? __ldcg(probs + (size_t)d * p.classes + k) : 0.0f;
 				}
-				slot += __popc(mask);
+				#pragma unroll
+				for (int j = 0; j < 4; ++j)
+				{
+					const unsigned mask = __ballot_sync(0xffffffffu, s[j] > 0.0f);
+					const int at = slot + __popc(mask & ((1u << lane) - 1u));
+					if (s[j] > 0.0f && at < p.max_rows)
+					{
+						float * r = p.rows + ((size_t)b * p.max_rows + at) * 7;
+						r[0] = box.x; r[1] = box.y; r[2] = box.z; r[3] = box.w; r[4] = obj; r[5] = (float)(k0 + j * 32 + lane); r[6] = s[j];
+					}
+					slot += __popc(mask);
+				}
 			}
 		}
 		if (rank == 0 && threadIdx.x == 0) { p.row_count[b] = base; }
-		cluster.sync();                                          // nobody's counts may go while another CTA still reads them
 	}
+}
+
+// The counts and first rows of every image, stored straight into page-locked host memory; a CTA column per image
+__global__ void __launch_bounds__(256)
+rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __restrict__ row_count, int take, float * __restrict__ host_rows, int * __restrict__ host_count)
+{
+	const size_t b = blockIdx.y;
+	const size_t floats = (size_t)take * 7;
+	const float * from = rows + b * max_rows * 7;
+	float * to = host_rows + b * floats;
+	for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < floats; i += (size_t)gridDim.x * 256) { to[i] = __ldg(from + i); }
+	if (blockIdx.x == 0 && threadIdx.x == 0) { host_count[b] = __ldg(row_count + b); }
+}
+
+// The address at which a kernel may write host memory, or nullptr for memory that is not page-locked
+static void * device_view(void * host)
+{
+	cudaPointerAttributes a = {};
+	if (cudaPointerGetAttributes(&a, host) != cudaSuccess)
+	{
+		cudaGetLastError();
+		return nullptr;
+	}
+	return (a.type == cudaMemoryTypeHost) ? a.devicePointer : nullptr;
 }
 
 static int check_dets(const xnor_b200_detections * d, int batch)
@@ -509,13 +692,18 @@ static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int b
 	if (batch > (p.nms ? 65535 : 0x7fffffff / DET_CLUSTER)) { return XNOR_B200_ERR_TOO_LARGE; }
 	p.boxes = d->boxes; p.objectness = d->objectness; p.probs = d->probs; p.count = d->count;
 	p.max_dets = d->max_dets; p.classes = d->classes;
-	// shared memory: the hit list, then the candidate lists (as many as the classes of a CTA and the budget ask for), then two
-	// ints per detection
+	// shared memory: the hit list; then, with the overlap matrix, counts, boxes, the matrix and candidate lists (as many as the classes of a
+	// CTA ask for), or without it candidate lists of max_dets (as many as the budget allows) and the boxes of a warp; then two ints per detection
 	const int want = min(DET_WARPS, (p.classes + DET_CLUSTER - 1) / DET_CLUSTER);
 	const int list_bytes = p.max_dets * DET_LIST_BYTES;
 	const int box_bytes = min(DET_WARP_MAX, p.max_dets) * (int)sizeof(float4);
 	p.lists = max(1, min(want, DET_SMEM_BUDGET / (list_bytes + box_bytes)));
-	const size_t smem = p.nms ? round_up((size_t)p.lists * list_bytes, 16) + (size_t)p.lists * box_bytes : (size_t)list_bytes;
+	p.matrix_max = min(p.max_dets, DET_MATRIX_MAX);
+	p.matrix_lists = want;
+	const size_t matrix_bytes = round_up((size_t)p.matrix_max, 4) * 4 + (size_t)p.matrix_max * (sizeof(float4) + DET_MATRIX_WORDS * 4 + (size_t)want * DET_LIST_BYTES);
+	size_t smem = (size_t)list_bytes;
+	if (p.nms && p.max_dets > p.matrix_max) { smem = round_up((size_t)p.lists * list_bytes, 16) + (size_t)p.lists * box_bytes; }
+	if (p.nms && matrix_bytes > smem) { smem = matrix_bytes; }
 	const int rc = ensure_dynamic_smem((const void *)detect_kernel, smem);
 	if (rc != XNOR_B200_OK) { return rc; }
 	detect_kernel<<<(unsigned)batch * DET_CLUSTER, DET_THREADS, smem, (cudaStream_t)stream>>>(p);
@@ -587,6 +775,14 @@ extern "C" int xnor_b200_rows_to_host(const float * rows, int max_rows, const in
 {
 	if (rows == nullptr || row_count == nullptr || host_rows == nullptr || host_count == nullptr) { return XNOR_B200_ERR_NULL; }
 	if (batch <= 0 || take <= 0 || take > max_rows) { return XNOR_B200_ERR_INVALID; }
+	float * rows_at = (float *)device_view(host_rows);
+	int * count_at = (int *)device_view(host_count);
+	if (rows_at != nullptr && count_at != nullptr && batch <= 65535 && (((uintptr_t)rows_at | (uintptr_t)count_at) & 3u) == 0)
+	{
+		// one launch for two copies of 3 to 8 us each and the gap between them
+		rows_host_kernel<<<dim3((unsigned)((take * 7LL + 1023) / 1024), (unsigned)batch, 1), 256, 0, (cudaStream_t)stream>>>(rows, max_rows, row_count, take, rows_at, count_at);
+		return check_launch();
+	}
 	cudaError_t e = cudaMemcpyAsync(host_count, row_count, (size_t)batch * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
 	if (e != cudaSuccess) { return cuda_fail(e); }
 	const size_t row = 7 * sizeof(float);

@@ -71,6 +71,70 @@ def test_detect_equals_the_restatement(tmp_path, share, size, max_dets, favourit
         assert np.array_equal(fused.probs[b, :n].cpu().numpy(), kept)
 
 
+def overlaps(b, thresh):
+    """iou() of every pair at once, fp32 operation for operation."""
+    f = np.float32
+    lo, hi = b[:, :2] - b[:, 2:] * f(0.5), b[:, :2] + b[:, 2:] * f(0.5)
+    side = np.minimum(hi[:, None], hi[None]) - np.maximum(lo[:, None], lo[None])
+    inter = side[..., 0] * side[..., 1]
+    area = b[:, 2] * b[:, 3]
+    return (side > 0).all(2) & (inter / ((area[:, None] + area[None]) - inter) > f(thresh))
+
+
+@pytest.mark.parametrize("found", [1, 32, 33, 128, 129, 767, 768, 769])
+def test_detect_at_the_lines_of_the_overlap_matrix(tmp_path, found):
+    """Up to 768 detections the overlaps are kept as bits, beyond they are formed on the way; up to 128 of a class a warp ranks them."""
+    size, max_dets = 256, 1024
+    cfg = tmp_path / "net.cfg"
+    cfg.write_text(cfgs.yolov3_tiny_xnor_cfg(size, size))
+    net = network.parse_network_cfg(str(cfg), 1, "cuda:0")
+    g = torch.Generator().manual_seed(found)
+    yolo = [l for l in net.layers if l.type == "yolo"]
+    heads = [torch.rand(1, 3, 85, l.h * l.w, generator=g) * 0.3 for l in yolo]
+    cells = sum(3 * l.h * l.w for l in yolo)
+    chosen = torch.zeros(cells, dtype=torch.bool)
+    chosen[torch.randperm(cells, generator=g)[:found]] = True
+    parts = chosen.split([3 * l.h * l.w for l in yolo])
+    for h, c, l in zip(heads, parts, yolo):
+        h[:, :, 4] = torch.where(c.view(1, 3, -1), 0.9 + 0.1 * h[:, :, 4], 0.1 * h[:, :, 4])
+        h[:, :, 5:] = torch.where(torch.rand(1, 3, 80, l.h * l.w, generator=g) < 0.02, h[:, :, 5:] + 0.6, h[:, :, 5:])
+        h[:, :, 5 + 17] += 0.65                                     # a class that every detection belongs to
+    heads = [h.reshape(1, 255, l.h, l.w).cuda().contiguous() for h, l in zip(heads, yolo)]
+    apart = network.DetectionBuffers(1, 80, max_dets=max_dets, max_rows=20000)
+    network.get_network_boxes(net, heads, size, size, 0.5, apart)
+    torch.cuda.synchronize()
+    assert int(apart.count.cpu()[0]) == found
+    boxes, obj, probs = (t.cpu().numpy()[0, :found].copy() for t in (apart.boxes, apart.objectness, apart.probs))
+    over = overlaps(boxes, 0.45)
+    for k in range(80):
+        order = [d for d in np.argsort(-probs[:, k], kind="stable") if probs[d, k] > 0]
+        for r, i in enumerate(order):
+            if probs[i, k] > 0:
+                later = np.array(order[r + 1:], int)
+                probs[later[over[i, later]], k] = 0
+    d, k = np.nonzero(probs > 0)
+    want = np.concatenate([boxes[d], obj[d, None], k[:, None].astype(np.float32), probs[d, k][:, None]], 1)
+    fused = network.DetectionBuffers(1, 80, max_dets=max_dets, max_rows=20000)
+    network.detect(net, heads, size, size, 0.5, 0.45, fused)
+    network.do_nms_sort(apart, 0.45)
+    network.detection_rows(apart)
+    for dets in (fused, apart):
+        assert np.array_equal(dets.rows_host()[0], want)
+        assert np.array_equal(dets.probs[0, :found].cpu().numpy(), probs)
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_rows_to_host_into_either_kind_of_memory(pinned):
+    """Page-locked memory is written by a kernel, any other through the copies."""
+    rows, count = torch.randn(3, 40, 7, device="cuda"), torch.tensor([5, 40, 0], dtype=torch.int32, device="cuda")
+    host = torch.full((3, 33, 7), -1.0, pin_memory=pinned)
+    host_count = torch.full((3,), -1, dtype=torch.int32, pin_memory=pinned)
+    capi.check(capi.lib().xnor_b200_rows_to_host(rows.data_ptr(), 40, count.data_ptr(), 3, 33, host.data_ptr(), host_count.data_ptr(),
+                                                 torch.cuda.current_stream().cuda_stream), "xnor_b200_rows_to_host")
+    torch.cuda.synchronize()
+    assert torch.equal(host, rows[:, :33].cpu()) and torch.equal(host_count, count.cpu())
+
+
 @pytest.mark.parametrize("counts,max_rows", [([0, 512], 4096), ([513, 3], 4096), ([2049, 700], 4096), ([900, 901], 900)])
 def test_rows_host_of_long_lists(counts, max_rows):
     """Lists longer than the first copy: whole the first time, and from then on in one copy."""
