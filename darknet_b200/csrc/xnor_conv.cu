@@ -303,8 +303,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	__shared__ uint64_t acc_full[ACC];
 	__shared__ uint64_t acc_empty[ACC];
 	__shared__ uint64_t drain_bar;
+	__shared__ uint64_t ready_bar;                              // filters and scale factors are in place
 	__shared__ uint32_t tmem_base_slot;
-	__shared__ uint32_t s_koff[XC_MAX_KW / 2];                 // per instruction of a stage: start | LBO << 16 of the pixel operand
 	__shared__ __align__(16) float s_thr[NF];                  // MODE 0: smallest accumulator whose output is > 0
 	__shared__ __align__(16) float s_mean[NF];
 	__shared__ __align__(16) float s_bias[NF];
@@ -328,8 +328,10 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	// this filter group's words: [K word][128]
 	const uint32_t * my_filters = p.weights + (size_t)(f0 >> 7) * p.kwords * 128 + (f0 & 127);
 
-	// What this prologue reads (filters, means, biases) was written long before the previous kernel; behind a kernel of the same
-	// forward it runs while that one finishes (griddepcontrol.wait below).
+	// What runs in front of pdl_wait reads filters, means and biases only, which were written long before the previous kernel; behind a
+	// kernel of the same forward it runs while that one finishes.  The roles part as soon as barriers and tensor memory exist: the first
+	// bits are on their way while the epilogue warps, which have nothing to do yet, widen the filters (all in one prologue in front of the
+	// copies a layer at batch 1 took about 2 us longer wherever its CTAs had to wait for SMs).
 	if (warp == XC_COPY_WARP)
 	{
 		if (lane < XC_RAW_STAGES)
@@ -350,6 +352,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		if (lane == 31)
 		{
 			mbar_init(&drain_bar, 1);
+			mbar_init(&ready_bar, XC_EPI_WARPS);
 			s_failed_storage = 0;
 		}
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -359,93 +362,80 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
 				:: "r"(smem_u32(&tmem_base_slot)), "r"((uint32_t)XC_TMEM_COLS) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-		for (int i = lane; i < p.kw_full / 2; i += 32)
-		{
-			const int j0 = 2 * i, j1 = 2 * i + 1;
-			const int g0 = block_of(j0, p.taps), g1 = block_of(j1, p.taps);
-			const int o0 = g0 * p.slots + tap_offset(p, tap_of(j0 - g0 * p.taps, p.stride, p.taps));
-			// the word past an odd number meets zero filters: any finite operand will do
-			const int o1 = (g1 < p.G) ? g1 * p.slots + tap_offset(p, tap_of(j1 - g1 * p.taps, p.stride, p.taps)) : o0;
-			s_koff[i] = (uint32_t)o0 | ((uint32_t)(o1 - o0) << 16);
-		}
-	}
-	float mean = 0.0f, bias = -0.0f;                               // v + -0.0 is v
-	if (tid < NF && f0 + tid < p.M)
-	{
-		mean = __ldg(p.mean_arr + f0 + tid);
-		if (p.bias != nullptr) { bias = __ldg(p.bias + f0 + tid); }
-	}
-	if (!STREAM)
-	{
-		// a warp takes 32 filters of every STEP-th K word, eight loads in flight per thread
-		constexpr int STEP = XC_THREADS / NF;
-		const int f = tid % NF;
-		const int total = p.stages_k * p.kw_full;
-		const int g_words = p.G * p.taps;
-		for (int k0 = tid / NF; k0 < total; k0 += 8 * STEP)
-		{
-			uint32_t bits[8];
-			int at[8];                                            // stage and word of the stage
-			#pragma unroll
-			for (int q = 0; q < 8; ++q)
-			{
-				bits[q] = 0;
-				const int kk = k0 + q * STEP;
-				const int st = fdiv(kk, p.d_kw);
-				at[q] = kk - st * p.kw_full | (st << 8);
-				const int k = st * g_words + (at[q] & 255);
-				if (kk < total && (at[q] & 255) < g_words && k < p.kwords) { bits[q] = __ldg(my_filters + (size_t)k * 128 + f); }
-			}
-			#pragma unroll
-			for (int q = 0; q < 8; ++q)
-			{
-				if (k0 + q * STEP < total) { put_filter<NF>(p, b_base + (uint32_t)((at[q] >> 8) * p.b_stage_bytes), at[q] >> 8, at[q] & 255, f, bits[q]); }
-			}
-		}
-		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-	}
-	if (tid < NF)
-	{
-		s_mean[tid] = mean;
-		s_bias[tid] = bias;
-		if (MODE == 0)
-		{
-			// fl(fl(d * mean) + bias) grows with d, so its sign is one comparison with the smallest d that makes it positive
-			auto positive = [&](int d) { return __fadd_rn(__fmul_rn((float)d, mean), bias) > 0.0f; };
-			int lo = -p.K - 1, hi = p.K + 1;                     // positive(hi) assumed, positive(lo) assumed not
-			while (hi - lo > 1)
-			{
-				const int mid = lo + ((hi - lo) >> 1);
-				if (positive(mid)) { hi = mid; } else { lo = mid; }
-			}
-			s_thr[tid] = (f0 + tid < p.M) ? (float)hi : 3.0e38f;
-		}
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
-	if (warp < 4)
-	{
-		const uint32_t taddr = tmem_base + (uint32_t)XC_SF_COL + ((uint32_t)(warp * 32) << 16);
-		asm volatile(
-			"tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
-			:: "r"(taddr), "r"(0x7F7F7F7Fu) : "memory");
-		asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-	}
-	if (warp < 4 || warp == XC_MMA_WARP)
-	{
-		// the scale factors are in place: only the issuer has to know
-		asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-		asm volatile("bar.sync 1, 160;" ::: "memory");
-		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-	}
-	// Everything the previous kernel wrote, and everything it read and this one overwrites, from here on.
-	pdl_wait();
-	if (tid == 0) { pdl_trigger(); }
-
 	if (warp < XC_EPI_WARPS)
 	{
+		// ---- epilogue warps, first: what the tiles need besides the bits ---------------------------------------------------
+		float mean = 0.0f, bias = -0.0f;                           // v + -0.0 is v
+		if (tid < NF && f0 + tid < p.M)
+		{
+			mean = __ldg(p.mean_arr + f0 + tid);
+			if (p.bias != nullptr) { bias = __ldg(p.bias + f0 + tid); }
+		}
+		if (warp < 4)
+		{
+			// the block scale factors, all 2^0
+			const uint32_t taddr = tmem_base + (uint32_t)XC_SF_COL + ((uint32_t)(warp * 32) << 16);
+			asm volatile(
+				"tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
+				:: "r"(taddr), "r"(0x7F7F7F7Fu) : "memory");
+			asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+			asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+		}
+		if (!STREAM)
+		{
+			// a warp takes 32 filters of every STEP-th K word, eight loads in flight per thread
+			constexpr int STEP = XC_EPI_WARPS * 32 / NF;
+			const int f = tid % NF;
+			const int total = p.stages_k * p.kw_full;
+			const int g_words = p.G * p.taps;
+			for (int k0 = tid / NF; k0 < total; k0 += 8 * STEP)
+			{
+				uint32_t bits[8];
+				int at[8];                                            // stage and word of the stage
+				#pragma unroll
+				for (int q = 0; q < 8; ++q)
+				{
+					bits[q] = 0;
+					const int kk = k0 + q * STEP;
+					const int st = fdiv(kk, p.d_kw);
+					at[q] = kk - st * p.kw_full | (st << 8);
+					const int k = st * g_words + (at[q] & 255);
+					if (kk < total && (at[q] & 255) < g_words && k < p.kwords) { bits[q] = __ldg(my_filters + (size_t)k * 128 + f); }
+				}
+				#pragma unroll
+				for (int q = 0; q < 8; ++q)
+				{
+					if (k0 + q * STEP < total) { put_filter<NF>(p, b_base + (uint32_t)((at[q] >> 8) * p.b_stage_bytes), at[q] >> 8, at[q] & 255, f, bits[q]); }
+				}
+			}
+			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+		}
+		__syncwarp();
+		if (lane == 0) { mbar_arrive(&ready_bar); }
+		if (tid < NF)
+		{
+			s_mean[tid] = mean;
+			s_bias[tid] = bias;
+			if (MODE == 0)
+			{
+				// fl(fl(d * mean) + bias) grows with d, so its sign is one comparison with the smallest d that makes it positive
+				auto positive = [&](int d) { return __fadd_rn(__fmul_rn((float)d, mean), bias) > 0.0f; };
+				int lo = -p.K - 1, hi = p.K + 1;                     // positive(hi) assumed, positive(lo) assumed not
+				while (hi - lo > 1)
+				{
+					const int mid = lo + ((hi - lo) >> 1);
+					if (positive(mid)) { hi = mid; } else { lo = mid; }
+				}
+				s_thr[tid] = (f0 + tid < p.M) ? (float)hi : 3.0e38f;
+			}
+		}
+		asm volatile("bar.sync 1, %0;" :: "n"(XC_EPI_WARPS * 32) : "memory");
+
 		// ---- epilogue: a warp takes every fourth (tile, 32-filter chunk) of its lane quarter -----------------------------
 		// Parameters in registers, whole groups of filters without per-filter checks: about 11 instructions a value with a shortcut.
 		const int quarter = warp & 3;
@@ -515,9 +505,11 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			}
 		};
 		Item it = Item{false, 0, 0};
+		if (tile < my_tiles) { it = locate(pos_of()); }
+		// everything the previous kernel wrote, and everything it read and this one overwrites, from here on
+		pdl_wait();
 		if (tile < my_tiles)
 		{
-			it = locate(pos_of());
 			if (left > 0)
 			{
 				#pragma unroll
@@ -809,15 +801,46 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 	{
 		// ---- bulk copies ------------------------------------------------------------------------------------------------------
 		const bool leader = elect_one();
-		asm volatile("fence.proxy.async.global;" ::: "memory");            // the previous kernel's stores -> this one's bulk copies
 		int rs = 0;
 		uint32_t rs_phase = 1, k = 0;
 		bool ok = true;
 		int n_unit = 0;
+		// which word of the run each position of unit u's window is (-1: padding)
+		auto fill_table = [&](int u, const XcRun & run0, const XcRun & run1)
+		{
+			int * tab = s_table + (n_unit % XC_TABLES) * (p.n_src * p.slots_plane);
+			const int slots_plane = p.slots_plane, pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos;
+			const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
+			const int pos0 = u * p.pt * TC_PIX - p.halo;
+			for (int si = 0; si < p.n_src; ++si, tab += slots_plane)
+			{
+				const int down = 2 - p.src[si].scale, src_pitch = p.src[si].pitch, src_rows = p.src[si].h + 1;
+				const int base = p.src[si].front - (si ? run1.start : run0.start);
+				// a division per entry: two independent ones at a time beat four, and one chain of steps of 32 positions (104x104 83 / 115 us)
+				#pragma unroll 2
+				for (int s = lane; s < slots_plane; s += 32)
+				{
+					const int pos = pos0 + s;
+					const int img = fdiv(pos, d_img);
+					const int r = pos - img * (int)d_img.d;
+					const int y = fdiv(r, d_pitch);
+					const int x = r - y * pitch;
+					const int sy = (2 * y) >> down, sx = (2 * x) >> down;
+					tab[s] = (pos >= 0 && pos < total_pos && y < OH && x < OW) ? base + (img * src_rows + sy) * src_pitch + sx : -1;
+				}
+			}
+		};
 		for (int u = unit0; u < p.units && ok; u += unit_step, ++n_unit)
 		{
 			const XcRun run0 = run_of(p, p.src[0], u);
 			const XcRun run1 = (p.n_src > 1) ? run_of(p, p.src[1], u) : run0;
+			if (n_unit == 0)
+			{
+				// the first table while the previous kernel finishes; then its stores -> this one's bulk copies
+				if (p.tabled) { fill_table(u, run0, run1); }
+				pdl_wait();
+				asm volatile("fence.proxy.async.global;" ::: "memory");
+			}
 			for (int st = 0; st < p.stages_k; ++st, ++k)
 			{
 				if (k >= XC_RAW_STAGES)
@@ -844,32 +867,10 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					{
 						bulk_load(dst + (uint32_t)(p.G * p.raw_words * 4), my_filters + (size_t)cb0 * p.taps * 128, (uint32_t)fil_words * 4u, &raw_full[rs]);
 					}
+					if (k == 0) { pdl_trigger(); }
 				}
-				if (st == 0 && p.tabled)
-				{
-					// which word of the run each position of the window is (-1: padding); the copies are on their way meanwhile
-					int * tab = s_table + (n_unit % XC_TABLES) * (p.n_src * p.slots_plane);
-					const int slots_plane = p.slots_plane, pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos;
-					const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
-					const int pos0 = u * p.pt * TC_PIX - p.halo;
-					for (int si = 0; si < p.n_src; ++si, tab += slots_plane)
-					{
-						const int down = 2 - p.src[si].scale, src_pitch = p.src[si].pitch, src_rows = p.src[si].h + 1;
-						const int base = p.src[si].front - (si ? run1.start : run0.start);
-						// a division per entry: two independent ones at a time beat four, and one chain of steps of 32 positions (104x104 83 / 115 us)
-						#pragma unroll 2
-						for (int s = lane; s < slots_plane; s += 32)
-						{
-							const int pos = pos0 + s;
-							const int img = fdiv(pos, d_img);
-							const int r = pos - img * (int)d_img.d;
-							const int y = fdiv(r, d_pitch);
-							const int x = r - y * pitch;
-							const int sy = (2 * y) >> down, sx = (2 * x) >> down;
-							tab[s] = (pos >= 0 && pos < total_pos && y < OH && x < OW) ? base + (img * src_rows + sy) * src_pitch + sx : -1;
-						}
-					}
-				}
+				// the copies are on their way meanwhile
+				if (st == 0 && n_unit > 0 && p.tabled) { fill_table(u, run0, run1); }
 				__syncwarp();
 				if (lane == 0) { mbar_arrive(&raw_full[rs]); }
 				if (++rs == XC_RAW_STAGES) { rs = 0; rs_phase ^= 1u; }
@@ -890,15 +891,26 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(NF >> 3) << 17) | (1u << 23) | ((uint32_t)(TC_PIX >> 4) << 24);
 		const uint32_t sfa = tmem_base + (uint32_t)XC_SF_COL;
 		const uint32_t sfb = sfa + 8u;
-		// the pixel operand's offsets are the same in every stage
+		// the pixel operand's offsets, the same in every stage: lane k makes those of instruction k, start | LBO << 16
+		uint32_t koff = 0;
+		if (lane < p.kw_full / 2)
+		{
+			const int j0 = 2 * lane, j1 = 2 * lane + 1;
+			const int g0 = block_of(j0, p.taps), g1 = block_of(j1, p.taps);
+			const int o0 = g0 * p.slots + tap_offset(p, tap_of(j0 - g0 * p.taps, p.stride, p.taps));
+			// the word past an odd number meets zero filters: any finite operand will do
+			const int o1 = (g1 < p.G) ? g1 * p.slots + tap_offset(p, tap_of(j1 - g1 * p.taps, p.stride, p.taps)) : o0;
+			koff = (uint32_t)o0 | ((uint32_t)(o1 - o0) << 16);
+		}
 		uint32_t ko[XC_MAX_KW / 2];
 		#pragma unroll
-		for (int k = 0; k < XC_MAX_KW / 2; ++k) { ko[k] = __shfl_sync(0xffffffffu, (2 * k < p.kw_full) ? s_koff[k] : 0u, 0); }
+		for (int k = 0; k < XC_MAX_KW / 2; ++k) { ko[k] = __shfl_sync(0xffffffffu, koff, k); }
 		int es = 0;
 		uint32_t es_phase = 0;
 		int a_unit = 0, used = 0;                                // accumulator of the unit's first tile; tiles started so far, up to ACC
 		uint32_t a_phase = 1;                                    // parity of the wait for an emptied accumulator, for a_unit
-		bool ok = true;
+		// filters and scale factors
+		bool ok = __all_sync(0xffffffffu, mbar_wait<0>(&ready_bar, 0, s_failed, limit));
 		for (int u = unit0; u < p.units && ok; u += unit_step)
 		{
 			for (int st = 0; st < p.stages_k && ok; ++st)
