@@ -7,6 +7,7 @@ namespace xnor
 {
 
 thread_local bool g_behind_kernel = false;
+thread_local int g_walk = WALK_ALONE;
 
 // A pointer of an operation: an address, or (small values) the network's input or one of its heads.
 static const void * resolve(const void * at, const void * input, void * const * heads, int n_heads)
@@ -85,7 +86,11 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 {
 	if (ops == nullptr || input == nullptr || (n_heads > 0 && heads == nullptr)) { return XNOR_B200_ERR_NULL; }
 	void * at = stream;
-	struct Reset { ~Reset() { g_behind_kernel = false; } } reset;
+	struct Reset { ~Reset() { g_behind_kernel = false; g_walk = WALK_ALONE; } } reset;
+	int layers = 0;                                            // xnor convolutions that write fp32
+	auto writes_fp32 = [](const xnor_b200_op & op) { return op.kind == XNOR_B200_OP_CONV_WORDS && (op.io.output != nullptr || op.io.shortcut_in != nullptr); };
+	for (int i = 0; i < n_ops; ++i) { layers += writes_fp32(ops[i]) ? 1 : 0; }
+	int walk = WALK_FORWARDS;
 	// Behind a fork the caller's stream waits for the side stream before this call returns, whether or not all was issued: what the caller
 	// queues next may read, or overwrite, what the side stream works on.
 	bool forked = false;
@@ -111,7 +116,15 @@ extern "C" int xnor_b200_run_ops(const xnor_b200_op * ops, int n_ops, const floa
 		{
 			case XNOR_B200_OP_CONV3: rc = xnor_b200_float_conv3_words(&d, op.arg, in, (const float *)op.weights, op.biases, (uint32_t *)out, op.pitch, at); break;
 			case XNOR_B200_OP_SIGN_WORDS: rc = xnor_b200_sign_words(in, d.batch, d.c, d.h, d.w, op.pitch, (uint32_t *)out, at); break;
-			case XNOR_B200_OP_CONV_WORDS: rc = xnor_b200_conv_words(&d, &op.io, (const uint32_t *)op.weights, op.mean_arr, op.biases, at); break;
+			case XNOR_B200_OP_CONV_WORDS:
+				if (layers > 1 && writes_fp32(op))
+				{
+					g_walk = walk;
+					walk = (walk == WALK_FORWARDS) ? WALK_BACKWARDS : WALK_FORWARDS;
+				}
+				rc = xnor_b200_conv_words(&d, &op.io, (const uint32_t *)op.weights, op.mean_arr, op.biases, at);
+				g_walk = WALK_ALONE;
+				break;
 			case XNOR_B200_OP_FLOAT_MAP: rc = xnor_b200_float_conv_map_yolo(&d, in, (const float *)op.weights, op.biases, out, op.arg, at); break;
 			case XNOR_B200_OP_FLOAT_TC: rc = xnor_b200_float_conv_tc(&d, in, (const float *)op.weights, op.biases, out, op.arg, at); break;
 			case XNOR_B200_OP_YOLO: rc = xnor_b200_yolo_activate(in, out, d.batch, d.n, op.arg, d.h * d.w, at); break;

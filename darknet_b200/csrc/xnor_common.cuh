@@ -92,6 +92,10 @@ bool gemm_takes_planes(int M, int n_total, int c, int size, int stride, int pad)
 // know how (launch_behind) then start while that one finishes.
 extern thread_local bool g_behind_kernel;
 
+// How xnor_b200_conv_words goes through a batch whose fp32 tensors do not fit the L2 (set by xnor_b200_run_ops for the layers of a network)
+enum { WALK_ALONE = 0, WALK_FORWARDS, WALK_BACKWARDS };
+extern thread_local int g_walk;
+
 #ifdef __CUDACC__
 // The kernel's prologue may run before the previous kernel on the stream has finished; everything from here on runs behind it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

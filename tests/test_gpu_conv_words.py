@@ -173,3 +173,35 @@ def test_layers_at_the_widest_maps_and_beyond(case):
         words = L.sign_words(x)
         L.conv_words(l, wts, [words.source()], output=out)
         assert torch.equal(out, want)
+
+
+def test_layers_of_a_network_walk_a_large_batch_in_turn():
+    """Inside one xnor_b200_run_ops call every second layer that writes large fp32 tensors begins at the batch's end: the same values,
+    with a plain window, through the window table (stride 2, a pool) and with a shortcut, over a batch that ends within a unit."""
+    batch, n, h, w = 5, 128, 100, 151
+    ops, checks = [], []
+    sc = torch.randn(batch, n, h, w, device="cuda")
+    for i, (c, ks, stride, pool, shortcut) in enumerate([(32, 3, 1, 0, False), (32, 3, 1, 0, True), (64, 3, 2, 0, False), (32, 3, 1, 2, True), (40, 1, 1, 0, False), (32, 3, 2, 0, True)]):
+        l, _ = build(batch, c, h * stride, w * stride, n, ks, stride, True, 20 + i)
+        src = L.sign_words(torch.randn(batch, c, h * stride * max(pool, 1), w * stride * max(pool, 1), device="cuda"))
+        wts = L.conv_words_weights(l)
+        got, want = (torch.full((batch, n, h, w), float("nan"), device="cuda") for _ in range(2))
+        signs, want_signs = L.GridWords(batch, n, h, w), L.GridWords(batch, n, h, w)
+        assert got.numel() * 4 > 32 << 20
+        kw = dict(shortcut_in=sc, shortcut_out=want) if shortcut else dict(output=want)
+        L.conv_words(l, wts, [src.source(pool, 1 if pool else 0)], signs=want_signs, **kw)
+        op = capi.Op(kind=capi.OP_CONV_WORDS, desc=l.desc, weights=wts.data_ptr(), mean_arr=l.mean_arr_gpu.data_ptr(), biases=l.biases_gpu.data_ptr())
+        op.io.n_sources, op.io.sources[0], op.io.pitch = 1, src.source(pool, 1 if pool else 0), signs.pitch
+        if shortcut:
+            op.io.shortcut_in, op.io.shortcut_out, op.io.shortcut_signs = sc.data_ptr(), got.data_ptr(), signs.words.data_ptr()
+        else:
+            op.io.output, op.io.output_signs = got.data_ptr(), signs.words.data_ptr()
+        ops.append(op)
+        checks.append((l, src, wts, got, want, signs, want_signs))
+    array = (capi.Op * len(ops))(*ops)
+    capi.check(capi.lib().xnor_b200_run_ops(array, len(ops), sc.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream, None, None, None), "run_ops")
+    for l, src, wts, got, want, signs, want_signs in checks:
+        assert torch.equal(got, want) and torch.equal(signs.words, want_signs.words)
+    status = capi.C.c_int(-1)
+    capi.check(capi.lib().xnor_b200_take_device_status(capi.C.byref(status)), "status")
+    assert status.value == 0
