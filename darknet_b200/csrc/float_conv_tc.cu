@@ -1,5 +1,5 @@
-// Float 1x1 and 3x3 stride-1 convolutions at batch (the layers behind the xnor path: yolo and region heads, 255..1024 filters
-// over 256..1024 channels and tens of thousands of pixels, and the 3x3 layer in front of a head) on the tcgen05 tensor cores, at
+// Float 1x1 and 3x3 stride-1 convolutions (the layers behind the xnor path: yolo and region heads, 255..1024 filters over 256..1024
+// channels, and the 3x3 layer in front of a head) on the tcgen05 tensor cores, at
 // fp32 accuracy.  A 3x3 layer is the same GEMM with K = (tap, channel): a K block of 32 channels lies in one tap, so its pixel
 // rows are the 1x1 layer's, shifted, with zeros where the tap leaves the map.
 //
@@ -12,14 +12,12 @@
 // an accumulator of their own).  What decides the accuracy is thus how many instructions one accumulator takes and how the operands are
 // split: to the nearest hi, which leaves lo one bit fewer and either sign, or cut off.  Where this kernel stands in for one in plain fp32
 // it is no less accurate (2-norm error against fp64, leaky inputs; launch_float_tc has the rule):
-//   up to 1024 pixels    every K block's sum taken out of tensor memory: 1.2e-7 .. 1.4e-7 (float_conv_map.cu 1.2e-7 .. 3.0e-7); about
+//   prepared filters     every K block's sum taken out of tensor memory: 1.2e-7 .. 1.4e-7 (float_conv_map.cu 1.2e-7 .. 3.0e-7); about
 //                        650 cycles a block: 3x3 256 -> 512, 4 images of 13x13, 33 us, 27 with 1.3e-6
-//   3x3, more pixels     small products apart, large ones in three accumulators, nearest split: 1.7e-6 at 72 K blocks (cuDNN's fp32
-//                        convolution 2.7e-6; its largest errors are seven times as large): 64 images 171 us, 162 with 4.1e-6; tiles
-//                        of more blocks in groups of eight, 6.4e-7 (190 us)
-//   1x1, more pixels     all products in four accumulators, cut off: 5.6e-7 at 256 channels, 1.9e-6 at 1024 -- far inside what the
+//   unprepared, 1x1      all products in four accumulators, cut off: 5.6e-7 at 256 channels, 1.9e-6 at 1024 -- far inside what the
 //                        reference's own GPU path does (it asks cuDNN for tensor-op math, i.e. single tf32 products, on every
 //                        convolution: src-lib/convolutional_layer.cpp:350)
+// More than 1024 pixels of a layer with prepared filters: float_conv_tcp.cu.
 // Results that the split cannot form (infinite, NaN or nearly infinite factors) are formed again by fp32 multiply-adds, but for the last kind.
 //
 // One tile of 128 pixels (TMEM lanes; the batch is folded into the pixel index) x 128 filters (TMEM columns) per CTA.  Warp 0 issues
@@ -31,10 +29,9 @@
 // sums meet in the first one's shared memory and are added in order.  The epilogue adds the bias, applies leaky or the [yolo]
 // layer's logistic and stores 32 consecutive pixels of one filter per warp-store.  Every barrier wait is bounded (status word
 // shared with the xnor tensor-core kernels).
-// Measured: 3x3 256 -> 512 on 13x13 at batch 64 171 us (one block in flight and the filters split on the way: 300), at batch 8 33 us
-// (101 without the cluster); 1x1 1024 -> 425 on 13x13 at batch 256 270 us (475).  Bound by the tensor pipe (880 cycles per K block) and
-// by shared-memory bandwidth (64 KB written and 96 KB read per K block: 1280 cycles).
-#include "tc_common.cuh"
+// Measured: 3x3 256 -> 512 on 4 images of 13x13 33 us (101 without the cluster).  Bound by the tensor pipe and by shared-memory bandwidth
+// (64 KB written and 96 KB read per K block: 1280 cycles).
+#include "float_tc.cuh"
 
 #include <cooperative_groups.h>
 
@@ -43,11 +40,9 @@ namespace xnor
 
 namespace cg = cooperative_groups;
 
-constexpr int FT_NF = 128;                                 // filters per tile
 constexpr int FT_ACCS = 4;                                 // accumulators that take the K blocks in turn
-constexpr int FT_BUFFERS = 2;                              // groups of K blocks whose sums can be in tensor memory: two accumulators each
+constexpr int FT_BUFFERS = 2;                              // K blocks whose sums can be in tensor memory: two accumulators each
 constexpr int FT_STAGES = 3;
-constexpr int FT_TILE_BYTES = 128 * 128;                   // 128 rows x 32 tf32
 constexpr int FT_STAGE_BYTES = 4 * FT_TILE_BYTES;          // pixel hi, pixel lo, filter hi, filter lo
 constexpr int FT_SMEM_BYTES = FT_STAGES * FT_STAGE_BYTES + 1024;
 constexpr int FT_PARTS = 4;                                // producer threads per pixel row: each takes 8 channels of a K block
@@ -55,34 +50,6 @@ constexpr int FT_CH = 32 / FT_PARTS;
 constexpr int FT_PRODUCER_WARPS = 4 * FT_PARTS;
 constexpr int FT_COPY_WARP = FT_PRODUCER_WARPS + 1;
 constexpr int FT_THREADS = 32 * (FT_COPY_WARP + 1);
-constexpr int FT_MAX_SPLIT = 4;                            // CTAs that share a tile's K blocks: their sums fill the first one's stages
-
-struct FtParams
-{
-	const float * x;      // [batch][C][HW]
-	const float * w;      // RAW: [N][C] (1x1); else [filter tile][K block][hi, lo][128 rows x 32 channels, swizzled]
-	const float * bias;   // [N] or nullptr
-	float * out;          // [batch][N][HW]
-	int C, HW, N;
-	int total;            // batch * HW
-	int H, W, taps;       // taps 1 or 9
-	int cblocks;          // ceil(C / 32): K blocks per tap
-	int kblocks;          // taps * cblocks
-	int yolo_entries;     // > 0: the [yolo] layer's activation step is applied to the result (xnor_b200_yolo_activate)
-	int leaky;
-	int tiles_f;
-	int split;            // CTAs per tile
-	int * status;
-	uint32_t spin_limit;
-};
-
-// v = hi + lo exactly: hi the nearest value of 11 significant bits (halves away from zero), so that lo, of either sign, fits 12.  An infinity
-// or NaN leaves NaN in lo, and so does a value that rounds past the largest: those results are formed again (plain_sum).
-__device__ __forceinline__ void split_nearest(float v, float & hi, float & lo)
-{
-	hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
-	lo = __fsub_rn(v, hi);
-}
 
 // A thread's part of one operand row of one K block: FT_CH fp32 values -> their 16-byte chunks in the row of the hi tile and
 // of the lo tile (chunk c of row r at chunk position c ^ (r % 8); row_swz has the row's swizzle term and the part's first
@@ -144,43 +111,16 @@ __device__ __forceinline__ void add_group(uint32_t tmem, float (&sums)[32])
 	}
 }
 
-// One result by fp32 multiply-adds from the prepared filters, for those that the split products cannot form: a factor that is infinite,
-// NaN or next to the largest value.
-__device__ __forceinline__ float plain_sum(const FtParams & p, int img, int pix, int f)
-{
-	const int py = pix / p.W, px = pix - py * p.W, row = f % FT_NF;
-	const float * base = p.x + (size_t)img * p.C * p.HW + pix;
-	float acc = 0.0f;
-	for (int tap = 0; tap < p.taps; ++tap)
-	{
-		const int dy = (p.taps == 9) ? tap / 3 - 1 : 0, dx = (p.taps == 9) ? tap % 3 - 1 : 0;
-		const bool inside = (py + dy >= 0 && py + dy < p.H && px + dx >= 0 && px + dx < p.W);       // else zeros, as im2col has them
-		for (int c = 0; c < p.C; ++c)
-		{
-			const float * tile = p.w + ((size_t)(f / FT_NF) * p.kblocks + tap * p.cblocks + (c >> 5)) * (2 * FT_TILE_BYTES / 4);
-			const int at = row * 32 + ((((c & 31) >> 2) ^ (row & 7)) << 2) + (c & 3);
-			acc = fmaf(inside ? __ldg(base + dy * p.W + dx + (size_t)c * p.HW) : 0.0f, __ldg(tile + at) + __ldg(tile + FT_TILE_BYTES / 4 + at), acc);
-		}
-	}
-	return acc;
-}
-
-// RAW: the filters come as Darknet keeps them and are split by the producers as well (callers without a prepared copy, 1x1 only).
-// Where the sums are formed (see launch_float_tc).  GROUP > 0: that many K blocks (a power of two) meet in tensor memory before their sum
-// is taken out and added in fp32.  Whole tiles: FT_TURNS, K blocks take the FT_ACCS accumulators in turn; FT_APART, their small products
-// share the first and the large ones take the others in turn.  All but FT_TURNS split to nearest and form again what did not come out.
-constexpr int FT_TURNS = 0, FT_APART = -1;
-
-template <bool RAW, int GROUP>
+// RAW: the filters come as Darknet keeps them and are split by the producers as well (callers without a prepared copy, 1x1 only); the K
+// blocks then take the accumulators in turn.  Prepared filters: every K block's sum is taken out of tensor memory and added in fp32.
+template <bool RAW>
 __global__ void __launch_bounds__(FT_THREADS, 1)
 float_conv_tc_kernel(const FtParams p)
 {
-	constexpr bool WHOLE = (GROUP <= 0), FINE = (GROUP != FT_TURNS);
-	constexpr int BLOCKS = WHOLE ? 1 : GROUP;
 	extern __shared__ uint8_t ft_smem_raw[];
 	__shared__ uint64_t bar_full[FT_STAGES];
 	__shared__ uint64_t bar_empty[FT_STAGES];
-	__shared__ uint64_t bar_done;                              // the whole tile, or (groups) what was issued before a failure
+	__shared__ uint64_t bar_done;                              // RAW: the whole tile; else what was issued before a failure
 	__shared__ uint64_t acc_full[FT_BUFFERS], acc_empty[FT_BUFFERS];
 	__shared__ uint32_t tmem_base_slot;
 	__shared__ float s_bias[FT_NF];
@@ -210,7 +150,7 @@ float_conv_tc_kernel(const FtParams p)
 			mbar_init(&bar_empty[s], 1);
 		}
 		mbar_init(&bar_done, 1);
-		for (int a = 0; a < (WHOLE ? 0 : FT_BUFFERS); ++a)
+		for (int a = 0; a < (RAW ? 0 : FT_BUFFERS); ++a)
 		{
 			mbar_init(&acc_full[a], 1);
 			mbar_init(&acc_empty[a], FT_PRODUCER_WARPS);
@@ -244,10 +184,10 @@ float_conv_tc_kernel(const FtParams p)
 				const int s = kb % FT_STAGES;
 				ok = __all_sync(0xffffffffu, mbar_wait(&bar_full[s], (uint32_t)((kb / FT_STAGES) & 1), s_failed, p.spin_limit));
 				if (!ok) { break; }
-				const int buffer = (kb / BLOCKS) % FT_BUFFERS;
-				if (!WHOLE && kb % BLOCKS == 0 && kb / BLOCKS >= FT_BUFFERS)
+				const int buffer = kb % FT_BUFFERS;
+				if (!RAW && kb >= FT_BUFFERS)
 				{
-					ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buffer], (uint32_t)((kb / BLOCKS / FT_BUFFERS - 1) & 1), s_failed, p.spin_limit));
+					ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buffer], (uint32_t)((kb / FT_BUFFERS - 1) & 1), s_failed, p.spin_limit));
 					if (!ok) { break; }
 				}
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -255,7 +195,7 @@ float_conv_tc_kernel(const FtParams p)
 				const uint32_t a_lo = a_hi + FT_TILE_BYTES;
 				const uint32_t b_hi = a_hi + 2 * FT_TILE_BYTES;
 				const uint32_t b_lo = a_hi + 3 * FT_TILE_BYTES;
-				if constexpr (WHOLE)
+				if constexpr (RAW)
 				{
 					#pragma unroll
 					for (int k = 0; k < 4; ++k)                       // 8 tf32 = 32 bytes of every row per instruction
@@ -265,10 +205,8 @@ float_conv_tc_kernel(const FtParams p)
 						{
 							const uint64_t adesc = make_smem_desc((term == 0 ? a_lo : a_hi) + k * 32);
 							const uint64_t bdesc = make_smem_desc((term == 1 ? b_lo : b_hi) + k * 32);
-							const bool small = (GROUP == FT_APART && term < 2);
-							const int turn = (GROUP == FT_TURNS) ? kb % FT_ACCS : small ? 0 : 1 + kb % (FT_ACCS - 1);
-							const bool begun = (GROUP == FT_TURNS) ? (kb >= FT_ACCS || k > 0 || term > 0) : small ? (kb > 0 || k > 0 || term > 0) : (kb >= FT_ACCS - 1 || k > 0);
-							const uint32_t accumulate = begun ? 1u : 0u;
+							const int turn = kb % FT_ACCS;
+							const uint32_t accumulate = (kb >= FT_ACCS || k > 0 || term > 0) ? 1u : 0u;
 							if (leader) asm volatile(
 								"{\n\t.reg .pred p;\n\t"
 								"setp.ne.b32 p, %4, 0;\n\t"
@@ -279,9 +217,9 @@ float_conv_tc_kernel(const FtParams p)
 				}
 				else
 				{
-					// the small products in the first accumulator, the large ones in the second; of a single block, the large ones of the first 16
-					// channels behind the small ones, so that no sum of large ones takes more than two instructions
-					constexpr int FIRST = (GROUP == 1) ? 2 : 0;
+					// the small products and the large ones of the first 16 channels in the first accumulator, the other large ones in the second: no
+					// sum of large ones takes more than two instructions
+					constexpr int FIRST = 2;
 					#pragma unroll
 					for (int i = 0; i < 12; ++i)
 					{
@@ -289,7 +227,7 @@ float_conv_tc_kernel(const FtParams p)
 						const bool second = (term == 2 && k >= FIRST);
 						const uint64_t adesc = make_smem_desc((term == 0 ? a_lo : a_hi) + k * 32);
 						const uint64_t bdesc = make_smem_desc((term == 1 ? b_lo : b_hi) + k * 32);
-						const uint32_t accumulate = (kb % BLOCKS > 0 || (i > 0 && !(second && k == FIRST))) ? 1u : 0u;
+						const uint32_t accumulate = (i > 0 && !(second && k == FIRST)) ? 1u : 0u;
 						if (leader) asm volatile(
 							"{\n\t.reg .pred p;\n\t"
 							"setp.ne.b32 p, %4, 0;\n\t"
@@ -299,12 +237,12 @@ float_conv_tc_kernel(const FtParams p)
 				}
 				if (leader) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
 						:: "r"(smem_u32(&bar_empty[s])) : "memory");
-				if (!WHOLE && leader && (kb % BLOCKS == BLOCKS - 1 || kb == kbn - 1))
+				if (!RAW && leader)
 				{
 					asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&acc_full[buffer])) : "memory");
 				}
 			}
-			if (WHOLE ? ok : !ok)
+			if (RAW ? ok : !ok)
 			{
 				if (leader)
 				{
@@ -312,7 +250,7 @@ float_conv_tc_kernel(const FtParams p)
 							:: "r"(smem_u32(&bar_done)) : "memory");
 				}
 				// leaving early: what was issued must have finished before the tensor memory is released
-				if (!WHOLE) { mbar_wait_plain(&bar_done, 0, p.spin_limit); }
+				if (!RAW) { mbar_wait_plain(&bar_done, 0, p.spin_limit); }
 			}
 		}
 		__syncwarp();
@@ -358,7 +296,7 @@ float_conv_tc_kernel(const FtParams p)
 		// the sums of the next group of K blocks, from tensor memory into this thread's
 		int n_group = 0;
 		#pragma unroll
-		for (int j = 0; j < (WHOLE ? 0 : 32); ++j) { sums[j] = 0.0f; }
+		for (int j = 0; j < (RAW ? 0 : 32); ++j) { sums[j] = 0.0f; }
 		auto collect = [&]()
 		{
 			const int buffer = n_group % FT_BUFFERS;
@@ -384,25 +322,25 @@ float_conv_tc_kernel(const FtParams p)
 				if (kb + u >= FT_STAGES)
 				{
 					ok = mbar_wait(&bar_empty[s], (uint32_t)(((kb + u) / FT_STAGES - 1) & 1), s_failed, p.spin_limit);
-					if (!WHOLE) { ok = __all_sync(0xffffffffu, ok); }
+					if (!RAW) { ok = __all_sync(0xffffffffu, ok); }
 					if (!ok) { break; }
 				}
-				split_row<FINE>(row_swz0 + (uint32_t)s * FT_STAGE_BYTES, (uint32_t)FT_TILE_BYTES, buf[u]);
+				split_row<!RAW>(row_swz0 + (uint32_t)s * FT_STAGE_BYTES, (uint32_t)FT_TILE_BYTES, buf[u]);
 				if constexpr (RAW) { split_row<false>(row_swz0 + (uint32_t)s * FT_STAGE_BYTES + 2u * FT_TILE_BYTES, (uint32_t)FT_TILE_BYTES, fil[u]); }
 				if (kb + u + 2 < kbn) { fetch(buf[u], fil[u]); }
 				asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 				__syncwarp();
 				if (lane == 0) { mbar_arrive(&bar_full[s]); }
-				if constexpr (!WHOLE)
+				if constexpr (!RAW)
 				{
 					// a group is taken out while the next is added up: two blocks, which are in flight, behind its last one
-					if (kb + u >= (n_group + 1) * GROUP + 1) { ok = collect(); }
+					if (kb + u >= n_group + 2) { ok = collect(); }
 					if (!ok) { break; }
 				}
 			}
 		}
 		if (part == 0) { s_bias[row] = (f < p.N && p.bias != nullptr) ? __ldg(p.bias + f) : 0.0f; }
-		if constexpr (!WHOLE) { while (n_group * GROUP < kbn && ok) { ok = collect(); } }
+		if constexpr (!RAW) { while (n_group < kbn && ok) { ok = collect(); } }
 	}
 	else if (!RAW)
 	{
@@ -435,12 +373,12 @@ float_conv_tc_kernel(const FtParams p)
 		}
 	}
 
-	if (WHOLE && tid == 0) { mbar_wait<64>(&bar_done, 0, s_failed, p.spin_limit); }
+	if (RAW && tid == 0) { mbar_wait<64>(&bar_done, 0, s_failed, p.spin_limit); }
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const bool failed = (*s_failed != 0);
-	const int used = (GROUP == FT_TURNS) ? min(FT_ACCS, kbn) : min(FT_ACCS, kbn + 1);
+	const int used = min(FT_ACCS, kbn);
 	cg::cluster_group cluster = cg::this_cluster();
 	if (p.split > 1)
 	{
@@ -449,7 +387,7 @@ float_conv_tc_kernel(const FtParams p)
 		if (rank > 0 && warp >= 1 && warp <= FT_PRODUCER_WARPS)
 		{
 			float * theirs = cluster.map_shared_rank(reinterpret_cast<float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))), 0) + (size_t)(rank - 1) * FT_NF * TC_PIX;
-			if constexpr (WHOLE) { tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, sums); }
+			if constexpr (RAW) { tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, sums); }
 			#pragma unroll
 			for (int j = 0; j < 32; ++j) { theirs[(chunk * 32 + j) * TC_PIX + quarter * 32 + lane] = sums[j]; }
 		}
@@ -465,7 +403,7 @@ float_conv_tc_kernel(const FtParams p)
 		const int pix = col_ok ? g - img * p.HW : 0;
 		float * out_pix = p.out + ((size_t)img * p.N + f0 + chunk * 32) * p.HW + pix;
 		const float slope = p.leaky ? 0.1f : 1.0f;
-		if constexpr (WHOLE) { tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, sums); }
+		if constexpr (RAW) { tile_sums(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chunk * 32), used, sums); }
 		const float * others = reinterpret_cast<const float *>(ft_smem_raw + (ring - smem_u32(ft_smem_raw))) + (size_t)chunk * 32 * TC_PIX + quarter * 32 + lane;
 		for (int r = 1; r < p.split; ++r, others += FT_NF * TC_PIX)
 		{
@@ -478,7 +416,7 @@ float_conv_tc_kernel(const FtParams p)
 		#pragma unroll
 		for (int j = 0; j < 32; ++j)
 		{
-			if (FINE && !(fabsf(sums[j]) <= 3.0e38f)) { again |= 1u << j; }
+			if (!RAW && !(fabsf(sums[j]) <= 3.0e38f)) { again |= 1u << j; }
 			float v = __fadd_rn(sums[j], s_bias[chunk * 32 + j]);
 			v = fmaxf(v, __fmul_rn(v, slope));
 			if (p.yolo_entries > 0)
@@ -489,7 +427,7 @@ float_conv_tc_kernel(const FtParams p)
 			}
 			if (col_ok && f0 + chunk * 32 + j < p.N) { out_pix[(size_t)j * p.HW] = v; }
 		}
-		if constexpr (FINE)
+		if constexpr (!RAW)
 		{
 			for (int j = 0; j < 32; ++j)
 			{
@@ -579,14 +517,8 @@ static int launch_float_tc(const xnor_b200_conv_desc * desc, const float * input
 	// as many CTAs per tile as leave the grid one wave and each of them a few K blocks (about 3 us go into joining the sums)
 	p.split = 1;
 	for (int s = 2; s <= FT_MAX_SPLIT; ++s) { if (tiles * s <= sm_count() && p.kblocks >= 4 * s) { p.split = s; } }
-	// Which sums: no less accurate than the fp32 kernel that would do it otherwise (figures above).  An accumulator of FT_APART takes 96
-	// instructions of large products at 72 K blocks; the error grows with their number.
-	auto kernel = float_conv_tc_kernel<RAW, FT_TURNS>;
-	if constexpr (!RAW)
-	{
-		if (total <= 1024) { kernel = float_conv_tc_kernel<false, 1>; }
-		else if (p.taps == 9) { kernel = (p.kblocks <= 72 * p.split) ? float_conv_tc_kernel<false, FT_APART> : float_conv_tc_kernel<false, 8>; }
-	}
+	if (!RAW && total > 1024) { return launch_float_tcp(p, stream); }
+	const auto kernel = float_conv_tc_kernel<RAW>;
 	rc = ensure_dynamic_smem((const void *)kernel, FT_SMEM_BYTES);
 	if (rc != XNOR_B200_OK) { return rc; }
 	cudaLaunchConfig_t cfg = {};

@@ -20,7 +20,10 @@ from darknet_b200 import capi  # noqa: E402
     (1, 32, 11, 19, 40, 3, 1, 0),       # 9 K blocks: split 2
     (3, 64, 7, 9, 129, 3, 1, 0),        # 18 K blocks: split 4, halo rows of neighbouring images
     (40, 64, 16, 33, 16, 3, 0, 8),      # one wave full: no split
-    (64, 512, 13, 13, 64, 3, 1, 0),     # more K blocks a tile than two accumulators may take: groups of eight
+    (64, 512, 13, 13, 64, 3, 1, 0),     # 144 K blocks a tile, fewer tiles than SMs
+    (113, 512, 13, 13, 40, 3, 1, 0),    # 150 tiles: a round of the SMs, and two whose K blocks go to clusters of four
+    (150, 416, 13, 13, 130, 1, 0, 65), (64, 96, 31, 33, 33, 1, 1, 11), (9, 128, 40, 41, 129, 1, 1, 0), (9, 129, 40, 41, 129, 1, 0, 0),
+                                        # several tiles an SM; 3 and 4 K blocks (each taken out by itself) and 5
     (1, 32, 32, 32, 130, 3, 0, 0), (1, 32, 25, 41, 130, 3, 0, 0),      # 1024 pixels and one more
     (2, 300, 23, 22, 33, 1, 1, 11), (3, 300, 19, 18, 33, 1, 1, 11),    # 1012 and 1026, K blocks that are not whole
 ])
