@@ -3,15 +3,18 @@
 // What the layer behind it wants is one bit per value: fl(sum) + bias > 0, the sum formed by fmaf over (channel, ky, kx) from zero.
 // 27 multiply-adds a value on the FMA pipe are 620 us for 16 filters at 416x416 and 256 images (1070 us with everything around
 // them).  Here the values are first formed approximately, as fp16 products with fp32 accumulation, together with a bound on how far
-// off they can be; wherever the value is farther from zero than that, the sign is known, and the rest -- about half a percent --
+// off they can be; wherever the value is farther from zero than that, the sign is known, and the rest -- about a quarter of a percent --
 // are formed again in fp32, in the order above.  Every bit is therefore the exact one.
 //
-//   |approximate - exact| <= (xmax + 1e-4) * 1.03e-3
+//   |approximate - exact| <= ulp(xmax) / 2 + xmax * (d + 5.3e-5) + 1.1e-7
 //
-// (compared in fp16, hence 1.032e-3 + 1.2e-7) for a filter scaled to sum|w| = 1 and xmax the largest input of the unit: 2^-10 for the
-// two fp16 roundings of a product, 2^-25 each for subnormal operands, and 5.3e-5 for the rest: 2e-6 for the scaling and the fp32 sum
-// there, and for the sum here six instructions of 17 terms that lose up to 2^-23 of the largest each, twice over where the bias is as large
-// as the products (2.4e-5).  That loss per term is how fp32 accumulation is taken to be, not something the hardware states.
+// for a filter scaled to sum|w| = 1 and xmax the largest input of the unit: ulp(xmax) / 2 = 2^-12 of the power of two above xmax, what
+// rounding an input to fp16 takes at most; d the sum of what rounding took of the weights, the largest of the filters (about 2e-4, 2^-11
+// at most); 2^-25 each for subnormal operands; and 5.3e-5 for the rest: 2e-6 for the scaling and the fp32 sum there, and for the sum
+// here six instructions of 17 terms that lose up to 2^-23 of the largest each, twice over where the bias is as large as the products
+// (2.4e-5).  That loss per term is how fp32 accumulation is taken to be, not something the hardware states.  (Compared in fp16, hence a
+// factor of 1.002 and 1.2e-7 more.)  For 8-bit images half of the bound that takes 2^-10 for the two roundings of every product, and half
+// as many values to form again.
 // Inputs or filters that fp16 cannot hold make the bound infinite or the value NaN, and every value is formed again.
 //
 // One MMA row is a 2x2 block of pixels, its columns the block's four values of every filter, K the patch of pixels around it: with
@@ -21,7 +24,7 @@
 // bx, the pair behind a row is zero).  The ones carry the bias, as three fp16 parts in the filter operand.
 //
 // Roles (one CTA per SM): warps 0..11 (unpooled 0..15) epilogue, then converters (global fp32 -> planes), 23 issuer.
-// Measured at 416x416, 16 filters, pooled, 64 images: 90 us; 350 with every load followed by its use, 104 with unaligned pairs
+// Measured at 416x416, 16 filters, pooled, 64 images: 82 us, 90 with the bound of two roundings a product; 350 with every load followed by its use, 104 with unaligned pairs
 // (2q - 1, 2q), a shuffle for each, and bias and bound per filter in the epilogue.  Clock traces: converters and epilogue, bound by
 // issue slots and by the latency of the doubtful values, take turns as the bound; HBM would be 22 us.
 #include "grid_words.cuh"
@@ -67,11 +70,11 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi)
 	return r;
 }
 
-// Largest magnitude so far of the two halves each, NaN if one is
-__device__ __forceinline__ uint32_t max_half2(uint32_t a, uint32_t b)
+// Largest magnitude of the three, NaN if one is
+__device__ __forceinline__ float max_abs3(float a, float b, float c)
 {
-	uint32_t r;
-	asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b & 0x7fff7fffu));
+	float r;
+	asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
 	return r;
 }
 
@@ -137,10 +140,11 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	__shared__ __align__(128) uint4 s_b[F3_HALVES * NN];                // filter operand [16-byte half of K][column]
 	__shared__ float s_w[NF * 27];
 	__shared__ float s_bias[NF];                                // as given
+	__shared__ float s_dev[NF];
 	__shared__ float s_xmax[F3_MAX_UNITS_AHEAD][CONV_WARPS];
 	__shared__ uint2 s_queue[EPI_WARPS][F3_QUEUE];
 	__shared__ uint64_t st_full[F3_STAGES], st_empty[F3_STAGES], acc_full[ACC], acc_empty[ACC], drain_bar;
-	static_assert(sizeof(s_b) + sizeof(s_w) + sizeof(s_bias) + sizeof(s_xmax) + sizeof(s_queue) + sizeof(st_full) + sizeof(st_empty) + sizeof(acc_full)
+	static_assert(sizeof(s_b) + sizeof(s_w) + sizeof(s_bias) + sizeof(s_dev) + sizeof(s_xmax) + sizeof(s_queue) + sizeof(st_full) + sizeof(st_empty) + sizeof(acc_full)
 			+ sizeof(acc_empty) + 256 + F3_SMEM_MAX <= 227 * 1024, "static and dynamic shared memory of a block");
 	__shared__ uint32_t tmem_base_slot;
 	__shared__ int s_failed_storage;
@@ -186,6 +190,9 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 		// a filter of zeros stays as it is; one whose scale fp32 cannot hold, or whose bias fp16 cannot, gets a bias of NaN
 		const float scale = (sum > 0.0f) ? 1.0f / sum : 1.0f;
 		const bool fits = (sum < 1e30f) && (scale < 1e30f) && (fabsf(bias * scale) < 60000.0f);
+		float lost = 0.0f;
+		for (int k = 0; k < 27; ++k) { lost += fabsf(s_w[tid * 27 + k] * scale - half_of(s_w[tid * 27 + k] * scale)); }
+		s_dev[tid] = fits ? lost : 0.0f;                         // (a bias of NaN leaves no value sure)
 		float part[3];
 		part[0] = fits ? bias * scale : NAN;
 		part[1] = part[0] - half_of(part[0]);
@@ -223,6 +230,9 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 		while (t >= p.pt) { t -= p.pt; ++nu; }
 		int a = tile % ACC;
 		uint32_t phase = (uint32_t)((tile / ACC) & 1);
+		float dev = (lane < NF) ? s_dev[lane] : 0.0f;            // what rounding took of the weights
+		#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) { dev = fmaxf(dev, __shfl_xor_sync(0xffffffffu, dev, o)); }
 		int have_unit = -1;
 		uint32_t limit2 = 0;                                     // the bound of the unit, in both halves
 		int q_head = 0, q_count = 0;                             // this warp's ring of values to be formed exactly
@@ -279,8 +289,11 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 				float xmax = (lane < CONV_WARPS) ? s_xmax[nu % F3_MAX_UNITS_AHEAD][lane] : 0.0f;
 				#pragma unroll
 				for (int o = 8; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
+				xmax = __shfl_sync(0xffffffffu, xmax, 0);
+				// the power of two that xmax does not pass
+				const float above = __uint_as_float((__float_as_uint(xmax) + 0x7fffffu) & 0xff800000u);
 				// values are compared as fp16, so a little more for their rounding; infinity stays infinity
-				const float bound = (__shfl_sync(0xffffffffu, xmax, 0) + 1e-4f) * 1.032e-3f + 1.2e-7f;
+				const float bound = (above * 2.4439e-4f + xmax * (dev * 1.001f + 5.3e-5f) + 1.1e-7f) * 1.002f + 1.2e-7f;
 				limit2 = pack_half2(bound, bound);
 			}
 			const int pos = (((int)blockIdx.x + nu * (int)gridDim.x) * p.pt + t) * TC_PIX + quarter * 32 + lane;
@@ -395,7 +408,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 			const int pos0 = ((int)blockIdx.x + nu * (int)gridDim.x) * p.pt * TC_PIX - 1;
 			const uint32_t odd = a_base + (uint32_t)(es * p.stage_bytes);
 			const uint32_t even = odd + (uint32_t)(plane_slots * 16);
-			uint32_t top = 0;                                     // largest magnitudes, two halves
+			float top = 0.0f;                                     // largest magnitude
 			if (nu >= F3_STAGES)
 			{
 				ok = __all_sync(0xffffffffu, mbar_wait<32>(&st_empty[es], es_phase, s_failed, limit));
@@ -445,9 +458,9 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 					{
 						const float2 c0 = v[i][3 * k], c1 = v[i][3 * k + 1], c2 = v[i][3 * k + 2];
 						const uint32_t left = pack_half2(c0.x, c1.x), right = pack_half2(c0.y, c1.y), third = pack_half2(c2.x, c2.y);
-						top = max_half2(top, left);
-						top = max_half2(top, right);
-						top = max_half2(top, third);
+						top = max_abs3(top, c0.x, c0.y);
+						top = max_abs3(top, c1.x, c1.y);
+						top = max_abs3(top, c2.x, c2.y);
 						if (s < plane_slots)
 						{
 							constexpr uint32_t ONE = 0x3c00u;
@@ -457,13 +470,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 					}
 				}
 			}
-			float xmax;
-			{
-				// (a little more than the fp16 maximum for what its rounding may have taken; NaN counts as infinity)
-				float lo, hi;
-				asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, h;\n\t}" : "=f"(lo), "=f"(hi) : "r"(top));
-				xmax = (lo <= 65504.0f && hi <= 65504.0f) ? fmaxf(lo, hi) * 1.001f : INFINITY;
-			}
+			float xmax = (top <= 65504.0f) ? top : INFINITY;       // NaN counts as infinity
 			#pragma unroll
 			for (int o = 16; o > 0; o >>= 1) { xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o)); }
 			if (lane == 0) { s_xmax[nu % F3_MAX_UNITS_AHEAD][cw] = xmax; }

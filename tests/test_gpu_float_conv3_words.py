@@ -90,3 +90,31 @@ def test_signs_at_the_widest_and_at_odd_sizes(batch, h, w, n, pool):
     sure = y.abs() > 1e-4                                      # 27 fp32 products of magnitude a few
     bits = (body[:, None, :oh, :ow] >> torch.arange(n, device="cuda").view(1, n, 1, 1)) & 1
     assert torch.equal(bits.bool()[sure], (y > 0)[sure])
+
+
+@pytest.mark.parametrize("pool,n", [(2, 16), (0, 32)])
+@pytest.mark.parametrize("value,top", [(0.5 + 2 ** -12, 0.9), (0.5 + 2 ** -12, 1.0), (0.75 + 2 ** -12 - 2 ** -24, 0.75 + 2 ** -12 - 2 ** -24), (1.0 + 2 ** -11, 1.5), (1.0 + 2 ** -11, 1.0 + 2 ** -11),
+                                       (1.0 + 2 ** -11 - 2 ** -23, 1.0), (1.998, 2.0), (2.0 + 2 ** -10, 2.0), (0.3, 3.0e4)])
+def test_signs_where_rounding_takes_as_much_as_it_can(value, top, pool, n):
+    """Every input off by about half an fp16 unit the same way, and biases that leave next to nothing of the sum, on either side of zero."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    h, w = 40, 44
+    x = torch.full((1, 3, h, w), value, device="cuda")
+    x[0, 1, 7, 9] = top
+    wt = (torch.rand(n, 27, generator=g, device="cuda") + 0.5) * torch.tensor([1.0, -1.0], device="cuda").repeat(n // 2)[:, None]
+    desc = capi.ConvDesc(1, 3, h, w, n, 3, 1, 1, capi.LINEAR)
+    lib, stream = capi.lib(), torch.cuda.current_stream().cuda_stream
+    y = torch.empty(1, n, h, w, device="cuda")
+    zero = torch.zeros(n, device="cuda")
+    capi.check(lib.xnor_b200_float_conv3_io(C.byref(desc), 0, x.data_ptr(), wt.data_ptr(), zero.data_ptr(), y.data_ptr(), None, None, stream), "io")
+    oh, ow = (h // 2, w // 2) if pool else (h, w)
+    for off in (1e-6, -1e-6, 3e-5, -3e-5, 2e-4, -2e-4, 4e-4, -4e-4):
+        b = -y[0, :, 20, 20] * (1.0 + off)
+        grid = L.GridWords(1, n, oh, ow)
+        masks = torch.zeros(1, oh, ow, n // 8, dtype=torch.uint8, device="cuda")
+        capi.check(lib.xnor_b200_float_conv3_words(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), grid.words.data_ptr(), 0, stream), "words")
+        capi.check(lib.xnor_b200_float_conv3_io(C.byref(desc), pool, x.data_ptr(), wt.data_ptr(), b.data_ptr(), None, None, masks.data_ptr(), stream), "io")
+        front = lib.xnor_b200_grid_front(ow + 1)
+        body = grid.words[0, front:front + (oh + 1) * (ow + 1)].view(1, oh + 1, ow + 1)[:, :oh, :ow].to(torch.int64) & 0xFFFFFFFF
+        assert torch.equal(body, sum(masks[..., i].to(torch.int64) << (8 * i) for i in range(n // 8))), off
