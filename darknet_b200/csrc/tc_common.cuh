@@ -192,8 +192,13 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr)
 template <int G>
 __device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&d)[G])
 {
-	static_assert(G == 16 || G == 32, "16 or 32 columns");
-	if constexpr (G == 16)
+	static_assert(G == 8 || G == 16 || G == 32, "8, 16 or 32 columns");
+	if constexpr (G == 8)
+	{
+		asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+			: "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]) : "r"(taddr) : "memory");
+	}
+	else if constexpr (G == 16)
 	{
 		asm volatile(
 			"tcgen05.ld.sync.aligned.32x32b.x16.b32 "

@@ -190,8 +190,12 @@ template <int G>
 __device__ __forceinline__ void tmem_wait(uint32_t (&d)[G])
 {
 	asm volatile("tcgen05.wait::ld.sync.aligned;"
-			: "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]),
-			  "+r"(d[8]), "+r"(d[9]), "+r"(d[10]), "+r"(d[11]), "+r"(d[12]), "+r"(d[13]), "+r"(d[14]), "+r"(d[15]));
+			: "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]));
+	if constexpr (G >= 16)
+	{
+		asm volatile(""
+				: "+r"(d[8]), "+r"(d[9]), "+r"(d[10]), "+r"(d[11]), "+r"(d[12]), "+r"(d[13]), "+r"(d[14]), "+r"(d[15]));
+	}
 	if constexpr (G == 32)
 	{
 		asm volatile(""
@@ -290,13 +294,17 @@ __host__ __device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSou
 }
 
 // MODE 0: sign words only.  1: fp32 output (and its sign words).  2: fp32 sum with a shortcut operand (its sign words, and the
-// layer's own output if asked for).  STREAM: the filters come through the stages instead of staying in shared memory.
-template <int NF, int MODE, bool STREAM>
+// layer's own output if asked for).  STREAM: the filters come through the stages instead of staying in shared memory.  SPLIT: the epilogue
+// warps that would take different tiles share one, a part of its filters each.
+template <int NF, int MODE, bool STREAM, bool SPLIT>
 __global__ void __launch_bounds__(XC_THREADS, 1)
 xnor_conv_kernel(const __grid_constant__ XcParams p)
 {
 	constexpr int ACC = (XC_SF_COL / NF < XC_MAX_ACC) ? XC_SF_COL / NF : XC_MAX_ACC;
 	constexpr int CHUNKS = NF / 32;
+	constexpr int SHARES = 4 / CHUNKS;                         // epilogue warps of a lane quarter that are at a chunk of 32 filters
+	constexpr int COLS = SPLIT ? 32 / SHARES : 32;             // filters of a warp
+	constexpr int TILE_STEP = SPLIT ? 1 : SHARES;
 	extern __shared__ __align__(128) uint8_t xc_smem[];
 	__shared__ uint64_t raw_full[XC_RAW_STAGES];
 	__shared__ uint64_t raw_empty[XC_RAW_STAGES];
@@ -350,7 +358,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		if (lane < ACC)
 		{
 			mbar_init(&acc_full[lane], 1);
-			mbar_init(&acc_empty[lane], 4 * CHUNKS);
+			mbar_init(&acc_empty[lane], 4 * CHUNKS * (SPLIT ? SHARES : 1));
 		}
 		if (lane == 31)
 		{
@@ -445,8 +453,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const int share = warp >> 2;
 		// items of this warp: CHUNKS of 1, 2 or 4 divide the four shares, so the chunk is always the same
 		const int chunk = share % CHUNKS;
-		const int fb = chunk * 32;
-		constexpr int TILE_STEP = 4 / CHUNKS;
+		const int part = SPLIT ? share / CHUNKS : 0;
+		const int fb = chunk * 32 + part * COLS;
 		const FastDiv d_img = p.d_img, d_pitch = p.d_pitch;
 		const int pitch = p.pitch, OH = p.OH, OW = p.OW, total_pos = p.total_pos, pt = p.pt, batch = p.batch;
 		const size_t n_pix = (size_t)p.n_pix;
@@ -478,7 +486,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const float * const sc_in = p.sc_in;
 		const uint64_t policy = stream_policy(p.stream_values != 0), out_policy = stream_policy(p.stream_out != 0);
 		const int my_tiles = my_units * pt;
-		int tile = share / CHUNKS;                               // tiles of this CTA, counted over its units
+		int tile = SPLIT ? 0 : share / CHUNKS;                   // tiles of this CTA, counted over its units
 		int u = unit0, t = tile;                                 // ... as unit and tile of the unit
 		while (t >= pt) { t -= pt; u += unit_step; }
 		int a = tile % ACC;                                      // accumulator, and the parity of its phase
@@ -486,7 +494,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		auto pos_of = [&]() { return (place(u) * pt + t) * TC_PIX + quarter * 32 + lane; };
 		// The shortcut operand: a ring of four groups of eight filters, each asked for again, for the next item, as soon as it has
 		// been used, so that a thread always has 24 to 32 loads in flight.
-		float sc[MODE == 2 ? 32 : 1];
+		float sc[MODE == 2 ? COLS : 1];
 		auto load8 = [&](const Item & it, int h)
 		{
 			if constexpr (MODE == 2)
@@ -494,7 +502,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				// No condition per value: a load behind one was waited for on the spot, four times the latency per 32 values.  Filters
 				// that do not exist read the last one that does.
 				const char * at = reinterpret_cast<const char *>(sc_in + it.elem);
-				if (left >= 32)
+				if (left >= COLS)
 				{
 					at += (size_t)step * (uint32_t)h;
 					#pragma unroll
@@ -516,7 +524,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			if (left > 0)
 			{
 				#pragma unroll
-				for (int h = 0; h < 32; h += 8) { load8(it, h); }
+				for (int h = 0; h < COLS; h += 8) { load8(it, h); }
 			}
 		}
 		while (tile < my_tiles)
@@ -560,20 +568,21 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				char * const dst = reinterpret_cast<char *>(((MODE == 2) ? sc_out : out) + it.elem);
 				char * const own = reinterpret_cast<char *>((MODE == 2 && out != nullptr) ? out + it.elem : nullptr);
 				const bool store = it.ok && (MODE == 1 || sc_out != nullptr);       // else only the sum's signs are wanted
+				constexpr int W = (COLS < 16) ? COLS : 16;
 				#pragma unroll
-				for (int h = 0; h < 32; h += 16)
+				for (int h = 0; h < COLS; h += W)
 				{
-					uint32_t d[16];
-					tmem_load<16>(tacc + (uint32_t)h, d);
-					tmem_wait<16>(d);
-					if (h == 16)
+					uint32_t d[W];
+					tmem_load<W>(tacc + (uint32_t)h, d);
+					tmem_wait<W>(d);
+					if (h + W == COLS)
 					{
 						asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 						__syncwarp();
 						if (lane == 0) { mbar_arrive(&acc_empty[a_now]); }
 					}
 					#pragma unroll
-					for (int u0 = 0; u0 < 16; u0 += 8)
+					for (int u0 = 0; u0 < W; u0 += 8)
 					{
 						const int j0 = h + u0;
 						uint64_t w[4];                           // eight values, in pairs
@@ -607,7 +616,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 							for (int i = 0; i < 8; ++i) { v[i] = __fadd_rn(sc[MODE == 2 ? j0 + i : 0], v[i]); }
 							if (more) { load8(next, j0); }
 						}
-						if (store && left >= 32)
+						if (store && left >= COLS)
 						{
 							#pragma unroll
 							for (int i = 0; i < 8; ++i) { st_policy(reinterpret_cast<float *>(dst + (size_t)step * (uint32_t)(j0 + i)), v[i], out_policy); }
@@ -625,9 +634,14 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 						}
 					}
 				}
-				word = __brev(word);
+				word = __brev(word) >> (32 - COLS);
 			}
-			if (words != nullptr && it.ok) { words[it.pos] = word; }
+			if (words != nullptr && it.ok)
+			{
+				if constexpr (COLS == 32) { words[it.pos] = word; }
+				else if constexpr (COLS == 16) { reinterpret_cast<uint16_t *>(words + it.pos)[part] = (uint16_t)word; }
+				else { reinterpret_cast<uint8_t *>(words + it.pos)[part] = (uint8_t)word; }
+			}
 			it = next;
 		}
 	}
@@ -1067,11 +1081,11 @@ static bool plan_sizes(const XcParams & p, int nf, int pt, int stream, XcPlan * 
 // ranks the plans as well and is kept); per stage the
 // expanders: 350 cycles of hand-overs and 110 per round of words (170 through the table with a pool, 350 for four parity planes).
 // The slowest role sets the pace, the others take issue slots and shared-memory bandwidth from it.
-static double plan_cost(const XcParams & p, const XcPlan & q, int mode)
+static double plan_cost(const XcParams & p, const XcPlan & q, int mode, int sms)
 {
 	const int fgroups = (p.M + q.nf - 1) / q.nf;
 	const int units = (int)((p.total_pos + (long long)q.pt * TC_PIX - 1) / (q.pt * TC_PIX));
-	const int lanes = sm_count() / fgroups;                                      // CTAs per filter group
+	const int lanes = sms / fgroups;                                             // CTAs per filter group
 	if (lanes < 1) { return 1e30; }
 	const double waves = (double)((units + lanes - 1) / lanes);
 	const double steps = 0.5 * q.kw_full * q.stages_k;
@@ -1108,18 +1122,19 @@ static void fill_params(const xnor_b200_conv_desc & d, XcParams & p, int pitch)
 	p.out_block_words = grid_block_words(d.batch, p.OH, p.pitch);
 }
 
-template <int NF, int MODE, bool STREAM>
+template <int NF, int MODE, bool STREAM, bool SPLIT>
 static int launch_conv(XcParams & p, const XcPlan & q, cudaStream_t stream)
 {
-	int rc = ensure_dynamic_smem((const void *)xnor_conv_kernel<NF, MODE, STREAM>, q.smem);
+	int rc = ensure_dynamic_smem((const void *)xnor_conv_kernel<NF, MODE, STREAM, SPLIT>, q.smem);
 	if (rc != XNOR_B200_OK) { return rc; }
-	return launch_behind(xnor_conv_kernel<NF, MODE, STREAM>, (unsigned)q.grid, XC_THREADS, q.smem, stream, p);
+	return launch_behind(xnor_conv_kernel<NF, MODE, STREAM, SPLIT>, (unsigned)q.grid, XC_THREADS, q.smem, stream, p);
 }
 
 static XcPlan best_plan(const XcParams & p, int mode)
 {
 	XcPlan best = {};
 	best.cost = 1e30;
+	const int sms = sm_count();
 	for (int nf = 32; nf <= 128; nf *= 2)
 	{
 		for (int pt = 1; pt <= 4; pt *= 2)
@@ -1130,7 +1145,7 @@ static XcPlan best_plan(const XcParams & p, int mode)
 				if (st ? (nf != 128 || pt > 2) : (nf == 128 && pt > 1)) { continue; }
 				XcPlan q;
 				if (!plan_sizes(p, nf, pt, st, &q)) { continue; }
-				q.cost = plan_cost(p, q, mode);
+				q.cost = plan_cost(p, q, mode, sms);
 				if (q.cost < best.cost) { best = q; }
 			}
 		}
@@ -1166,10 +1181,17 @@ static int launch_mode(XcParams & p, cudaStream_t stream)
 	rc = tc_fill_launch_fields(common);
 	if (rc != XNOR_B200_OK) { return rc; }
 	p.status = common.status; p.spin_limit = common.spin_limit; p.withhold = common.withhold;
-	if (best.stream) { return launch_conv<128, MODE, true>(p, best, stream); }
-	if (best.nf == 128) { return launch_conv<128, MODE, false>(p, best, stream); }
-	if (best.nf == 64) { return launch_conv<64, MODE, false>(p, best, stream); }
-	return launch_conv<32, MODE, false>(p, best, stream);
+	if (best.stream) { return launch_conv<128, MODE, true, false>(p, best, stream); }
+	if (best.nf == 128) { return launch_conv<128, MODE, false, false>(p, best, stream); }
+	if constexpr (MODE != 0)
+	{
+		// Fewer tiles a CTA than epilogue warps of a lane quarter that would take one each: at batch 1 a quarter or half of the warps did
+		// all of a sum with its shortcut, 2 us of a layer's 7 (darknet53 at batch 1: 382 us, 360 with the filters shared).
+		const int tiles = (p.units * p.fgroups + best.grid - 1) / best.grid * p.pt;
+		if (tiles < 128 / best.nf) { return (best.nf == 64) ? launch_conv<64, MODE, false, true>(p, best, stream) : launch_conv<32, MODE, false, true>(p, best, stream); }
+	}
+	if (best.nf == 64) { return launch_conv<64, MODE, false, false>(p, best, stream); }
+	return launch_conv<32, MODE, false, false>(p, best, stream);
 }
 
 // [filter][K in the layout of xnor_b200_binary_align_weights] -> [filters / 128][channel block * taps + tap, in the order the stages
