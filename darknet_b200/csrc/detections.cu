@@ -94,6 +94,22 @@ __device__ __forceinline__ float box_iou_dev(const float4 a, const float4 b)
 	return __fdiv_rn(inter, uni);
 }
 
+// Whether box_iou_dev(a, b) > thresh: by a product where the two are farther apart than rounding can take them, else by that division.
+__device__ __forceinline__ bool overlap_exceeds(const float4 a, const float4 b, float thresh)
+{
+	const float w = overlap_1d(a.x, a.z, b.x, b.z), h = overlap_1d(a.y, a.w, b.y, b.w);
+	const float inter = __fmul_rn(w, h);
+	if (w <= 0.0f || h <= 0.0f || inter == 0.0f) { return 0.0f > thresh; }
+	const float uni = __fsub_rn(__fadd_rn(__fmul_rn(a.z, a.w), __fmul_rn(b.z, b.w)), inter);
+	const float line = thresh * uni;
+	if (line > 1e-30f)
+	{
+		if (inter > line * 1.000001f) { return true; }
+		if (inter < line * 0.999999f) { return false; }
+	}
+	return __fdiv_rn(inter, uni) > thresh;
+}
+
 // Rank of candidate c by score, highest first; equal scores keep their storage order.
 __device__ __forceinline__ int score_rank(const float * s_score, int m, int c)
 {
@@ -359,49 +375,44 @@ detect_kernel(const __grid_constant__ DetectParams p)
 		const int stored = min(found, p.max_dets);
 		// a warp per detection; its first three entries a lane are asked for while the one before is worked on
 		constexpr int AHEAD = 3;
-		auto entries_of = [&](int slot)
+		struct Found { const float * e; int hd, i, a; float v[AHEAD]; };          // a detection's first entry, head, cell, anchor
+		auto fetch = [&](int slot)
 		{
+			Found f = {};
+			if (slot >= stored) { return f; }
 			const unsigned hit = s_hit[slot - first];
-			const YoloHeadParams & h = p.heads[head_of(hit)];
+			f.hd = head_of(hit);
+			const YoloHeadParams & h = p.heads[f.hd];
 			const unsigned q = hit - h.first, i = q / (unsigned)h.n, a = q - i * (unsigned)h.n;
-			return h.head + ((size_t)b * h.n + a) * entries * (size_t)(h.lw * h.lh) + i;
-		};
-		auto fetch = [&](int slot, float (&v)[AHEAD])
-		{
-			if (slot >= stored) { return; }
-			const float * e = entries_of(slot);
-			const YoloHeadParams & h = p.heads[head_of(s_hit[slot - first])];
+			const size_t cells = (size_t)(h.lw * h.lh);
+			f.i = (int)i;
+			f.a = (int)a;
+			f.e = h.head + ((size_t)b * h.n + a) * entries * cells + i;
 			#pragma unroll
-			for (int j = 0; j < AHEAD; ++j) { v[j] = (lane + 32 * j < entries) ? __ldg(e + (size_t)(lane + 32 * j) * (h.lw * h.lh)) : 0.0f; }
+			for (int j = 0; j < AHEAD; ++j) { f.v[j] = (lane + 32 * j < entries) ? __ldg(f.e + (lane + 32 * j) * cells) : 0.0f; }
+			return f;
 		};
-		float next[AHEAD] = {};
-		fetch(first + all_warp, next);
+		Found next = fetch(first + all_warp);
 		for (int slot = first + all_warp; slot < stored; slot += DET_ALL_WARPS)
 		{
-			float now[AHEAD];
-			#pragma unroll
-			for (int j = 0; j < AHEAD; ++j) { now[j] = next[j]; }
-			fetch(slot + DET_ALL_WARPS, next);
-			const unsigned hit = s_hit[slot - first];
-			const YoloHeadParams & h = p.heads[head_of(hit)];
-			const int q = (int)(hit - h.first);
-			const int i = q / h.n;
-			const int a = q - i * h.n;
-			const float tx = __shfl_sync(0xffffffffu, now[0], 0), ty = __shfl_sync(0xffffffffu, now[0], 1);
-			const float tw = __shfl_sync(0xffffffffu, now[0], 2), th = __shfl_sync(0xffffffffu, now[0], 3);
-			const float obj = __shfl_sync(0xffffffffu, now[0], 4);
+			const Found now = next;
+			next = fetch(slot + DET_ALL_WARPS);
+			const YoloHeadParams & h = p.heads[now.hd];
+			const int i = now.i, a = now.a;
+			const float tx = __shfl_sync(0xffffffffu, now.v[0], 0), ty = __shfl_sync(0xffffffffu, now.v[0], 1);
+			const float tw = __shfl_sync(0xffffffffu, now.v[0], 2), th = __shfl_sync(0xffffffffu, now.v[0], 3);
+			const float obj = __shfl_sync(0xffffffffu, now.v[0], 4);
 			float * pr = probs + (size_t)slot * p.classes;
 			#pragma unroll
 			for (int j = 0; j < AHEAD; ++j)
 			{
 				const int at = lane + 32 * j;
-				const float prob = __fmul_rn(obj, now[j]);
+				const float prob = __fmul_rn(obj, now.v[j]);
 				if (at >= 5 && at < entries) { pr[at - 5] = (prob > p.thresh) ? prob : 0.0f; }
 			}
-			const float * e = entries_of(slot);
 			for (int j = lane + 32 * AHEAD; j < entries; j += 32)
 			{
-				const float prob = __fmul_rn(obj, __ldg(e + (size_t)j * (h.lw * h.lh)));
+				const float prob = __fmul_rn(obj, __ldg(now.e + (size_t)j * (h.lw * h.lh)));
 				pr[j - 5] = (prob > p.thresh) ? prob : 0.0f;
 			}
 			const int row = i / h.lw, col = i - row * h.lw;
@@ -451,10 +462,13 @@ detect_kernel(const __grid_constant__ DetectParams p)
 		float4 * s_box = reinterpret_cast<float4 *>(s_rows + ((p.matrix_max + 3) & ~3));
 		uint32_t * s_over = reinterpret_cast<uint32_t *>(s_box + p.matrix_max);
 		float * s_lists = reinterpret_cast<float *>(s_over + p.matrix_max * DET_MATRIX_WORDS);
-		for (int d = threadIdx.x; d < n; d += DET_THREADS)
+		static_assert(DET_MATRIX_MAX <= 2 * DET_THREADS, "two boxes a thread");
+		float4 box[2];                                           // (stored behind the first gathering, whose loads wait beside these)
+		#pragma unroll
+		for (int q = 0; q < 2; ++q)
 		{
-			s_rows[d] = 0;
-			s_box[d] = __ldcg(boxes + d);
+			const int d = threadIdx.x + q * DET_THREADS;
+			if (d < n) { box[q] = __ldcg(boxes + d); }
 		}
 		float * s_score = s_lists + (size_t)warp * p.matrix_max * (DET_LIST_BYTES / 4);
 		uint16_t * s_idx = reinterpret_cast<uint16_t *>(s_score + p.matrix_max);
@@ -466,13 +480,27 @@ detect_kernel(const __grid_constant__ DetectParams p)
 			const int k = k0 + warp * DET_CLUSTER + rank;
 			const int m = (warp < p.matrix_lists && k < p.classes) ? gather_class(p, n, probs, k, s_score, s_idx) : 0;
 			if (lane == 0) { s_m[warp] = m; }
+			if (k0 == 0)
+			{
+				#pragma unroll
+				for (int q = 0; q < 2; ++q)
+				{
+					const int d = threadIdx.x + q * DET_THREADS;
+					if (d < n)
+					{
+						s_rows[d] = 0;
+						s_box[d] = box[q];
+					}
+				}
+			}
 			__syncthreads();
 			if (k0 == 0)
 			{
+				#pragma unroll 2
 				for (int i = all_warp; i < n * words; i += DET_ALL_WARPS)
 				{
 					const int r = i / words, w = i - r * words, c = w * 32 + lane;
-					const bool over = (c < n && c != r) && box_iou_dev(s_box[r], s_box[c]) > p.nms_thresh;
+					const bool over = (c < n && c != r) && overlap_exceeds(s_box[r], s_box[c], p.nms_thresh);
 					const uint32_t bits = __ballot_sync(0xffffffffu, over);
 					if (lane < DET_CLUSTER) { *cluster.map_shared_rank(s_over + r * DET_MATRIX_WORDS + w, lane) = bits; }
 				}
