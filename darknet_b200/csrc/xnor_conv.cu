@@ -295,8 +295,10 @@ __host__ __device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSou
 
 // MODE 0: sign words only.  1: fp32 output (and its sign words).  2: fp32 sum with a shortcut operand (its sign words, and the
 // layer's own output if asked for).  STREAM: the filters come through the stages instead of staying in shared memory.  SPLIT: the epilogue
-// warps that would take different tiles share one, a part of its filters each.
-template <int NF, int MODE, bool STREAM, bool SPLIT>
+// warps that would take different tiles share one, a part of its filters each.  TABLED: the window is found through the table.
+// (A kernel holds only the code it runs: layers wait for their instructions as well.  With the table's code in every kernel darknet53 took
+// 349 us at batch 1, 337 without, tiny-yolo at batch 256 1342 and 1279.)
+template <int NF, int MODE, bool STREAM, bool SPLIT, bool TABLED>
 __global__ void __launch_bounds__(XC_THREADS, 1)
 xnor_conv_kernel(const __grid_constant__ XcParams p)
 {
@@ -656,7 +658,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const int table_len = p.n_src * slots_plane;
 		const int blocks0 = p.src[0].blocks;
 		const int mode = p.src[0].mode;                          // OR4 and SINGLE may meet in one layer (a route); both work as OR4
-		const bool tabled = (mode != XC_LINEAR);
+		constexpr bool tabled = TABLED;
 		const uint32_t down0 = (p.src[0].mode == XC_SINGLE) ? 0u : (uint32_t)p.src[0].pitch * 4u;
 		const uint32_t down1 = (p.src[1].mode == XC_SINGLE) ? 0u : (uint32_t)p.src[1].pitch * 4u;
 		const uint32_t raw_bytes = (uint32_t)p.raw_words * 4u, raw_stage = (uint32_t)p.raw_stage_bytes;
@@ -692,8 +694,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		for (int u = unit0; u < units && ok; u += unit_step, ++n_unit)
 		{
 			const uint32_t table_addr = smem_u32(s_table + (n_unit % XC_TABLES) * table_len);
-			const uint32_t shift0 = tabled ? 0u : (uint32_t)run_of(p, p.src[0], place(u)).shift * 4u;
-			const uint32_t shift1 = (tabled || p.n_src == 1) ? 0u : (uint32_t)run_of(p, p.src[1], place(u)).shift * 4u;
+			const uint32_t shift0 = TABLED ? 0u : (uint32_t)run_of(p, p.src[0], place(u)).shift * 4u;
+			const uint32_t shift1 = (TABLED || p.n_src == 1) ? 0u : (uint32_t)run_of(p, p.src[1], place(u)).shift * 4u;
 			for (int st = 0; st < stages_k; ++st, ++k)
 			{
 				const int cb0 = st * G;
@@ -710,7 +712,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				const bool second = (cb0 >= blocks0);            // the blocks of a stage come from one source
 				// item j of this thread exists: always but for the last round
 				auto has = [&](int j) { return j < full_items || (j == full_items && has_last); };
-				if (!tabled)
+				if constexpr (!TABLED)
 				{
 					const uint32_t src = raw + (second ? shift1 : shift0);
 					#pragma unroll
@@ -854,7 +856,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 			if (n_unit == 0)
 			{
 				// the first table while the previous kernel finishes; then its stores -> this one's bulk copies
-				if (p.tabled) { fill_table(u, run0, run1); }
+				if (TABLED) { fill_table(u, run0, run1); }
 				pdl_wait();
 				asm volatile("fence.proxy.async.global;" ::: "memory");
 			}
@@ -887,7 +889,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					if (k == 0) { pdl_trigger(); }
 				}
 				// the copies are on their way meanwhile
-				if (st == 0 && n_unit > 0 && p.tabled) { fill_table(u, run0, run1); }
+				if (TABLED && st == 0 && n_unit > 0) { fill_table(u, run0, run1); }
 				__syncwarp();
 				if (lane == 0) { mbar_arrive(&raw_full[rs]); }
 				if (++rs == XC_RAW_STAGES) { rs = 0; rs_phase ^= 1u; }
@@ -1125,9 +1127,10 @@ static void fill_params(const xnor_b200_conv_desc & d, XcParams & p, int pitch)
 template <int NF, int MODE, bool STREAM, bool SPLIT>
 static int launch_conv(XcParams & p, const XcPlan & q, cudaStream_t stream)
 {
-	int rc = ensure_dynamic_smem((const void *)xnor_conv_kernel<NF, MODE, STREAM, SPLIT>, q.smem);
+	const auto kernel = p.tabled ? xnor_conv_kernel<NF, MODE, STREAM, SPLIT, true> : xnor_conv_kernel<NF, MODE, STREAM, SPLIT, false>;
+	int rc = ensure_dynamic_smem((const void *)kernel, q.smem);
 	if (rc != XNOR_B200_OK) { return rc; }
-	return launch_behind(xnor_conv_kernel<NF, MODE, STREAM, SPLIT>, (unsigned)q.grid, XC_THREADS, q.smem, stream, p);
+	return launch_behind(kernel, (unsigned)q.grid, XC_THREADS, q.smem, stream, p);
 }
 
 static XcPlan best_plan(const XcParams & p, int mode)
