@@ -140,11 +140,11 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 	__shared__ __align__(128) uint4 s_b[F3_HALVES * NN];                // filter operand [16-byte half of K][column]
 	__shared__ float s_w[NF * 27];
 	__shared__ float s_bias[NF];                                // as given
-	__shared__ float s_dev[NF];
+	__shared__ float s_dev[NF], s_scale[NF], s_part[NF][3];
 	__shared__ float s_xmax[F3_MAX_UNITS_AHEAD][CONV_WARPS];
 	__shared__ uint2 s_queue[EPI_WARPS][F3_QUEUE];
-	__shared__ uint64_t st_full[F3_STAGES], st_empty[F3_STAGES], acc_full[ACC], acc_empty[ACC], drain_bar;
-	static_assert(sizeof(s_b) + sizeof(s_w) + sizeof(s_bias) + sizeof(s_dev) + sizeof(s_xmax) + sizeof(s_queue) + sizeof(st_full) + sizeof(st_empty) + sizeof(acc_full)
+	__shared__ uint64_t st_full[F3_STAGES], st_empty[F3_STAGES], acc_full[ACC], acc_empty[ACC], drain_bar, ready_bar;
+	static_assert(sizeof(s_b) + sizeof(s_w) + sizeof(s_bias) + sizeof(s_dev) + sizeof(s_scale) + sizeof(s_part) + sizeof(s_xmax) + sizeof(s_queue) + sizeof(st_full) + sizeof(st_empty) + sizeof(acc_full)
 			+ sizeof(acc_empty) + 256 + F3_SMEM_MAX <= 227 * 1024, "static and dynamic shared memory of a block");
 	__shared__ uint32_t tmem_base_slot;
 	__shared__ int s_failed_storage;
@@ -170,6 +170,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 			mbar_init(&acc_empty[a], 4);
 		}
 		mbar_init(&drain_bar, 1);
+		mbar_init(&ready_bar, EPI_WARPS);
 		s_failed_storage = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -178,50 +179,65 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
-	for (int i = tid; i < NF * 27; i += F3_THREADS) { s_w[i] = (i < p.N * 27) ? __ldg(p.weights + i) : 0.0f; }
-	__syncthreads();
-	pdl_trigger();                                              // this CTA has its tensor memory
-	if (tid < NF)
-	{
-		float sum = 0.0f;
-		for (int k = 0; k < 27; ++k) { sum += fabsf(s_w[tid * 27 + k]); }
-		const float bias = (p.biases != nullptr && tid < p.N) ? __ldg(p.biases + tid) : 0.0f;
-		s_bias[tid] = bias;
-		// a filter of zeros stays as it is; one whose scale fp32 cannot hold, or whose bias fp16 cannot, gets a bias of NaN
-		const float scale = (sum > 0.0f) ? 1.0f / sum : 1.0f;
-		const bool fits = (sum < 1e30f) && (scale < 1e30f) && (fabsf(bias * scale) < 60000.0f);
-		float lost = 0.0f;
-		for (int k = 0; k < 27; ++k) { lost += fabsf(s_w[tid * 27 + k] * scale - half_of(s_w[tid * 27 + k] * scale)); }
-		s_dev[tid] = fits ? lost : 0.0f;                         // (a bias of NaN leaves no value sure)
-		float part[3];
-		part[0] = fits ? bias * scale : NAN;
-		part[1] = part[0] - half_of(part[0]);
-		part[2] = part[1] - half_of(part[1]);
-		for (int h = 0; h < F3_HALVES; ++h)
-		{
-			// half h: patch rows 0, 2 (odd pixel rows), 1, 3 (even ones), three pairs each
-			const int row = (h / 6) + 2 * ((h / 3) & 1), pair = h % 3;
-			for (int s = 0; s < 4; ++s)
-			{
-				float v[8];
-				for (int q = 0; q < 8; ++q)
-				{
-					const int ky = row - (s >> 1), kx = 2 * (pair - 1) + (q >> 2) - (s & 1) + 1, c = q & 3;
-					v[q] = (fits && c < 3 && ky >= 0 && ky < 3 && kx >= 0 && kx < 3) ? s_w[tid * 27 + (c * 3 + ky) * 3 + kx] * scale : 0.0f;
-				}
-				if (h < 3) { v[3] = part[h]; }
-				s_b[h * NN + (POOL ? tid * 4 + s : s * NF + tid)] = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
-			}
-		}
-	}
-	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
+	pdl_trigger();                                              // this CTA has its tensor memory
 
 	if (warp < EPI_WARPS)
 	{
+		// ---- epilogue warps, first: the filter operand, while the converters begin.  A warp per filter for its scale and what rounding
+		// takes, then an operand entry a thread (a thread per filter, in front of all roles, took a third of the layer at batch 1).
+		auto epilogue_warps = [&]() { asm volatile("bar.sync 1, %0;" :: "n"(EPI_WARPS * 32) : "memory"); };
+		for (int i = tid; i < NF * 27; i += EPI_WARPS * 32) { s_w[i] = (i < p.N * 27) ? __ldg(p.weights + i) : 0.0f; }
+		epilogue_warps();
+		for (int f = warp; f < NF; f += EPI_WARPS)
+		{
+			const float w = (lane < 27) ? s_w[f * 27 + lane] : 0.0f;
+			float sum = fabsf(w);
+			#pragma unroll
+			for (int o = 16; o > 0; o >>= 1) { sum += __shfl_xor_sync(0xffffffffu, sum, o); }
+			const float bias = (p.biases != nullptr && f < p.N) ? __ldg(p.biases + f) : 0.0f;
+			// a filter of zeros stays as it is; one whose scale fp32 cannot hold, or whose bias fp16 cannot, gets a bias of NaN
+			const float scale = (sum > 0.0f) ? 1.0f / sum : 1.0f;
+			const bool fits = (sum < 1e30f) && (scale < 1e30f) && (fabsf(bias * scale) < 60000.0f);
+			float lost = fabsf(w * scale - half_of(w * scale));
+			#pragma unroll
+			for (int o = 16; o > 0; o >>= 1) { lost += __shfl_xor_sync(0xffffffffu, lost, o); }
+			if (lane == 0)
+			{
+				s_bias[f] = bias;
+				s_dev[f] = fits ? lost : 0.0f;                          // (a bias of NaN leaves no value sure)
+				s_scale[f] = fits ? scale : 0.0f;
+				const float first = fits ? bias * scale : NAN, second = first - half_of(first);
+				s_part[f][0] = first;
+				s_part[f][1] = second;
+				s_part[f][2] = second - half_of(second);
+			}
+		}
+		epilogue_warps();
+		for (int i = tid; i < NF * F3_HALVES * 4; i += EPI_WARPS * 32)
+		{
+			const int f = i % NF, s = i / NF % 4, h = i / (NF * 4);
+			// half h: patch rows 0, 2 (odd pixel rows), 1, 3 (even ones), three pairs each
+			const int row = (h / 6) + 2 * ((h / 3) & 1), pair = h % 3;
+			const int ky = row - (s >> 1);
+			const float scale = s_scale[f];
+			float v[8];
+			#pragma unroll
+			for (int q = 0; q < 8; ++q)
+			{
+				const int kx = 2 * (pair - 1) + (q >> 2) - (s & 1) + 1, c = q & 3;
+				v[q] = (scale > 0.0f && c < 3 && ky >= 0 && ky < 3 && kx >= 0 && kx < 3) ? s_w[f * 27 + (c * 3 + ky) * 3 + kx] * scale : 0.0f;
+			}
+			if (h < 3) { v[3] = s_part[f][h]; }
+			s_b[h * NN + (POOL ? f * 4 + s : s * NF + f)] = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
+		}
+		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+		__syncwarp();
+		if (lane == 0) { mbar_arrive(&ready_bar); }
+
 		// ---- epilogue: warp w takes the tiles w / 4, w / 4 + 4, ... of this CTA, lane quarter w % 4 -----------------------------
 		const int quarter = warp & 3;
 		const int my_tiles = my_units * p.pt;
@@ -489,7 +505,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 		const uint32_t b16 = smem_u32(s_b) >> 4;
 		int es = 0, a = 0, used = 0;
 		uint32_t es_phase = 0, a_phase = 1;
-		bool ok = true;
+		bool ok = __all_sync(0xffffffffu, mbar_wait<0>(&ready_bar, 0, s_failed, limit));          // the filter operand
 		for (int nu = 0; nu < my_units && ok; ++nu)
 		{
 			ok = __all_sync(0xffffffffu, mbar_wait<0>(&st_full[es], es_phase, s_failed, limit));
