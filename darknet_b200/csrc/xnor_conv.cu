@@ -159,22 +159,22 @@ __device__ __forceinline__ int tap_of(int j, int stride, int taps)
 }
 
 // Where tap t of a stage's first channel block starts, in 16-byte units from the start of that block's planes.
-__device__ __forceinline__ int tap_offset(const XcParams & p, int t)
+__device__ __forceinline__ int tap_offset(const XcParams & p, int t, int stride, int taps)
 {
-	if (p.taps == 1) { return 0; }
+	if (taps == 1) { return 0; }
 	const int ky = t / 3, kx = t - ky * 3;
-	if (p.stride == 1) { return ky * p.pitch + kx; }
+	if (stride == 1) { return ky * p.pitch + kx; }
 	const int plane = ((ky == 1) ? 0 : 2) + ((kx == 1) ? 0 : 1);
 	return plane * p.slots_plane + p.halo + ((ky == 0) ? -p.pitch : 0) + ((kx == 0) ? -1 : 0);
 }
 
 // K word j of stage st, widened into its place in the filter operand; what does not exist is +0.0.
 template <int NF>
-__device__ __forceinline__ void put_filter(const XcParams & p, uint32_t dst, int st, int j, int f, uint32_t bits)
+__device__ __forceinline__ void put_filter(const XcParams & p, int taps, uint32_t dst, int st, int j, int f, uint32_t bits)
 {
-	const int k = st * p.G * p.taps + j;
+	const int k = st * p.G * taps + j;
 	uint4 v = make_uint4(0, 0, 0, 0);
-	if (k < p.kwords && j < p.G * p.taps) { v = expand_filter(bits, (k >= p.kwords - p.taps) ? p.last_mask : 0xffffffffu); }
+	if (k < p.kwords && j < p.G * taps) { v = expand_filter(bits, (k >= p.kwords - taps) ? p.last_mask : 0xffffffffu); }
 	st_shared_v4(dst + (uint32_t)(j * NF + f) * 16u, v);
 }
 
@@ -262,12 +262,14 @@ struct XcRun
 	int start, words, shift;
 };
 
+// KNOWN: 0 linear, 1 not, -1 either.
+template <int KNOWN>
 __host__ __device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSource & src, int u)
 {
 	XcRun r;
 	const int pos0 = u * p.pt * TC_PIX - p.halo;
 	int lo, hi;
-	if (src.mode == XC_LINEAR)
+	if (KNOWN == 0 || (KNOWN < 0 && src.mode == XC_LINEAR))
 	{
 		lo = src.front + pos0;
 		hi = lo + p.slots_plane;
@@ -295,14 +297,23 @@ __host__ __device__ __forceinline__ XcRun run_of(const XcParams & p, const XcSou
 
 // MODE 0: sign words only.  1: fp32 output (and its sign words).  2: fp32 sum with a shortcut operand (its sign words, and the
 // layer's own output if asked for).  STREAM: the filters come through the stages instead of staying in shared memory.  SPLIT: the epilogue
-// warps that would take different tiles share one, a part of its filters each.  TABLED: the window is found through the table.
+// warps that would take different tiles share one, a part of its filters each.  KIND: where the window comes from and how many taps it has.
+// PLAIN: whole words of filters, and (mode 2) the layer's own output is not asked for.
 // (A kernel holds only the code it runs: layers wait for their instructions as well.  With the table's code in every kernel darknet53 took
-// 349 us at batch 1, 337 without, tiny-yolo at batch 256 1342 and 1279.)
-template <int NF, int MODE, bool STREAM, bool SPLIT, bool TABLED>
+// 349 us at batch 1, 337 without, 326 with 1x1 layers apart and 317 without what partial words of filters and a sum's own tensor need;
+// tiny-yolo at batch 256 1342 and 1279.  Nine taps stay a parameter: known to the compiler they cost 16 -> 32 on 208x208 217 us, 199 so.)
+enum { XC_ROWS = 0, XC_POINTS = 1, XC_TABLE = 2 };          // 3x3 and 1x1 of stride 1 from a run of words; any layer through the table
+
+template <int NF, int MODE, bool STREAM, bool SPLIT, int KIND, bool PLAIN>
 __global__ void __launch_bounds__(XC_THREADS, 1)
 xnor_conv_kernel(const __grid_constant__ XcParams p)
 {
 	constexpr int ACC = (XC_SF_COL / NF < XC_MAX_ACC) ? XC_SF_COL / NF : XC_MAX_ACC;
+	constexpr bool TABLED = (KIND == XC_TABLE);
+	constexpr int RUN = TABLED ? 1 : STREAM ? -1 : 0;            // (streamed filters: no difference but in the compiler's order, 211 / 201 us)
+	const int taps = (KIND == XC_POINTS) ? 1 : p.taps;
+	const int stride = TABLED ? p.stride : 1;
+	constexpr int MAX_STEPS = (KIND == XC_POINTS) ? 4 : XC_MAX_KW / 2;          // instructions of a stage: 64 K bits each
 	constexpr int CHUNKS = NF / 32;
 	constexpr int SHARES = 4 / CHUNKS;                         // epilogue warps of a lane quarter that are at a chunk of 32 filters
 	constexpr int COLS = SPLIT ? 32 / SHARES : 32;             // filters of a warp
@@ -401,17 +412,18 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		}
 		if (!STREAM)
 		{
-			// a warp takes 32 filters of every STEP-th K word, eight loads in flight per thread
+			// a warp takes 32 filters of every STEP-th K word, four loads in flight per thread (eight are more
+			// code, which every launch fetches anew: darknet53 at batch 1 333 us, 329 with four)
 			constexpr int STEP = XC_EPI_WARPS * 32 / NF;
 			const int f = tid % NF;
 			const int total = p.stages_k * p.kw_full;
-			const int g_words = p.G * p.taps;
-			for (int k0 = tid / NF; k0 < total; k0 += 8 * STEP)
+			const int g_words = p.G * taps;
+			for (int k0 = tid / NF; k0 < total; k0 += 4 * STEP)
 			{
-				uint32_t bits[8];
-				int at[8];                                            // stage and word of the stage
+				uint32_t bits[4];
+				int at[4];                                            // stage and word of the stage
 				#pragma unroll
-				for (int q = 0; q < 8; ++q)
+				for (int q = 0; q < 4; ++q)
 				{
 					bits[q] = 0;
 					const int kk = k0 + q * STEP;
@@ -421,9 +433,9 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					if (kk < total && (at[q] & 255) < g_words && k < p.kwords) { bits[q] = __ldg(my_filters + (size_t)k * 128 + f); }
 				}
 				#pragma unroll
-				for (int q = 0; q < 8; ++q)
+				for (int q = 0; q < 4; ++q)
 				{
-					if (k0 + q * STEP < total) { put_filter<NF>(p, b_base + (uint32_t)((at[q] >> 8) * p.b_stage_bytes), at[q] >> 8, at[q] & 255, f, bits[q]); }
+					if (k0 + q * STEP < total) { put_filter<NF>(p, taps, b_base + (uint32_t)((at[q] >> 8) * p.b_stage_bytes), at[q] >> 8, at[q] & 255, f, bits[q]); }
 				}
 			}
 			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -504,7 +516,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				// No condition per value: a load behind one was waited for on the spot, four times the latency per 32 values.  Filters
 				// that do not exist read the last one that does.
 				const char * at = reinterpret_cast<const char *>(sc_in + it.elem);
-				if (left >= COLS)
+				if (PLAIN || left >= COLS)
 				{
 					at += (size_t)step * (uint32_t)h;
 					#pragma unroll
@@ -609,7 +621,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 						}
 						if (MODE == 2)
 						{
-							if (own != nullptr && it.ok)
+							if (!PLAIN && own != nullptr && it.ok)
 							{
 								#pragma unroll
 								for (int i = 0; i < 8; ++i) { if (j0 + i < left) { st_policy(reinterpret_cast<float *>(own + (size_t)step * (uint32_t)(j0 + i)), v[i], out_policy); } }
@@ -618,12 +630,12 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 							for (int i = 0; i < 8; ++i) { v[i] = __fadd_rn(sc[MODE == 2 ? j0 + i : 0], v[i]); }
 							if (more) { load8(next, j0); }
 						}
-						if (store && left >= COLS)
+						if (store && (PLAIN || left >= COLS))
 						{
 							#pragma unroll
 							for (int i = 0; i < 8; ++i) { st_policy(reinterpret_cast<float *>(dst + (size_t)step * (uint32_t)(j0 + i)), v[i], out_policy); }
 						}
-						else if (store)
+						else if (!PLAIN && store)
 						{
 							#pragma unroll
 							for (int i = 0; i < 8; ++i) { if (j0 + i < left) { st_policy(reinterpret_cast<float *>(dst + (size_t)step * (uint32_t)(j0 + i)), v[i], out_policy); } }
@@ -665,7 +677,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		const uint32_t a_stage = (uint32_t)p.a_stage_bytes, b_stage = (uint32_t)p.b_stage_bytes;
 		const uint32_t block_bytes = (uint32_t)p.slots * 16u, plane_bytes = (uint32_t)slots_plane * 16u;
 		const bool withhold = (p.withhold != 0 && ew == 0);
-		const int g_words = G * p.taps, kw_full = p.kw_full;
+		const int g_words = G * taps, kw_full = p.kw_full;
 		const uint32_t last_mask = p.last_mask;
 		// The words this thread widens lie at the same places in every stage (a last stage with fewer channel blocks is widened whole:
 		// no filter reads what lies behind its blocks).  The loops over them are straight-line code: with the dealing done by
@@ -694,8 +706,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		for (int u = unit0; u < units && ok; u += unit_step, ++n_unit)
 		{
 			const uint32_t table_addr = smem_u32(s_table + (n_unit % XC_TABLES) * table_len);
-			const uint32_t shift0 = TABLED ? 0u : (uint32_t)run_of(p, p.src[0], place(u)).shift * 4u;
-			const uint32_t shift1 = (TABLED || p.n_src == 1) ? 0u : (uint32_t)run_of(p, p.src[1], place(u)).shift * 4u;
+			const uint32_t shift0 = TABLED ? 0u : (uint32_t)run_of<RUN>(p, p.src[0], place(u)).shift * 4u;
+			const uint32_t shift1 = (TABLED || p.n_src == 1) ? 0u : (uint32_t)run_of<RUN>(p, p.src[1], place(u)).shift * 4u;
 			for (int st = 0; st < stages_k; ++st, ++k)
 			{
 				const int cb0 = st * G;
@@ -798,7 +810,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 							for (int q = 0; q < 6; ++q)
 							{
 								const int i = et + (i0 + q) * XC_EXP_THREADS;
-								if (i < n) { put_filter<NF>(p, b_dst - (uint32_t)et * 16u, st, i / NF, i % NF, w[q]); }
+								if (i < n) { put_filter<NF>(p, taps, b_dst - (uint32_t)et * 16u, st, i / NF, i % NF, w[q]); }
 							}
 						}
 					}
@@ -851,8 +863,8 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		};
 		for (int u = unit0; u < p.units && ok; u += unit_step, ++n_unit)
 		{
-			const XcRun run0 = run_of(p, p.src[0], place(u));
-			const XcRun run1 = (p.n_src > 1) ? run_of(p, p.src[1], place(u)) : run0;
+			const XcRun run0 = run_of<RUN>(p, p.src[0], place(u));
+			const XcRun run1 = (p.n_src > 1) ? run_of<RUN>(p, p.src[1], place(u)) : run0;
 			if (n_unit == 0)
 			{
 				// the first table while the previous kernel finishes; then its stores -> this one's bulk copies
@@ -876,7 +888,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					const XcSource & src = p.src[second ? 1 : 0];
 					const XcRun run = second ? run1 : run0;
 					const uint32_t * words = src.words + (size_t)(second ? cb0 - p.src[0].blocks : cb0) * src.block_words + run.start;
-					const int fil_words = STREAM ? min(p.G * p.taps, p.kwords - cb0 * p.taps) * NF : 0;
+					const int fil_words = STREAM ? min(p.G * taps, p.kwords - cb0 * taps) * NF : 0;
 					mbar_expect_tx(&raw_full[rs], (uint32_t)(blocks * run.words + fil_words) * 4u);
 					for (int g = 0; g < blocks; ++g)
 					{
@@ -884,7 +896,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					}
 					if (STREAM)
 					{
-						bulk_load(dst + (uint32_t)(p.G * p.raw_words * 4), my_filters + (size_t)cb0 * p.taps * 128, (uint32_t)fil_words * 4u, &raw_full[rs]);
+						bulk_load(dst + (uint32_t)(p.G * p.raw_words * 4), my_filters + (size_t)cb0 * taps * 128, (uint32_t)fil_words * 4u, &raw_full[rs]);
 					}
 					if (k == 0) { pdl_trigger(); }
 				}
@@ -915,15 +927,15 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 		if (lane < p.kw_full / 2)
 		{
 			const int j0 = 2 * lane, j1 = 2 * lane + 1;
-			const int g0 = block_of(j0, p.taps), g1 = block_of(j1, p.taps);
-			const int o0 = g0 * p.slots + tap_offset(p, tap_of(j0 - g0 * p.taps, p.stride, p.taps));
+			const int g0 = block_of(j0, taps), g1 = block_of(j1, taps);
+			const int o0 = g0 * p.slots + tap_offset(p, tap_of(j0 - g0 * taps, stride, taps), stride, taps);
 			// the word past an odd number meets zero filters: any finite operand will do
-			const int o1 = (g1 < p.G) ? g1 * p.slots + tap_offset(p, tap_of(j1 - g1 * p.taps, p.stride, p.taps)) : o0;
+			const int o1 = (g1 < p.G) ? g1 * p.slots + tap_offset(p, tap_of(j1 - g1 * taps, stride, taps), stride, taps) : o0;
 			koff = (uint32_t)o0 | ((uint32_t)(o1 - o0) << 16);
 		}
-		uint32_t ko[XC_MAX_KW / 2];
+		uint32_t ko[MAX_STEPS];
 		#pragma unroll
-		for (int k = 0; k < XC_MAX_KW / 2; ++k) { ko[k] = __shfl_sync(0xffffffffu, koff, k); }
+		for (int k = 0; k < MAX_STEPS; ++k) { ko[k] = __shfl_sync(0xffffffffu, koff, k); }
 		int es = 0;
 		uint32_t es_phase = 0;
 		int a_unit = 0, used = 0;                                // accumulator of the unit's first tile; tiles started so far, up to ACC
@@ -938,7 +950,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 				if (!ok) { break; }
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 				const int blocks = min(p.G, p.nb - st * p.G);
-				const int steps = (blocks * p.taps + 1) / 2;
+				const int steps = (blocks * taps + 1) / 2;
 				uint32_t at = (a_base + (uint32_t)(es * p.a_stage_bytes)) >> 4;
 				const uint32_t b16 = ((b_base + (uint32_t)((STREAM ? es : st) * p.b_stage_bytes)) >> 4) | ((uint32_t)NF << 16);
 				int a = a_unit;
@@ -957,7 +969,7 @@ xnor_conv_kernel(const __grid_constant__ XcParams p)
 					}
 					const uint32_t acc = tmem_base + (uint32_t)(a * NF);
 					#pragma unroll
-					for (int k = 0; k < XC_MAX_KW / 2; ++k)
+					for (int k = 0; k < MAX_STEPS; ++k)
 					{
 						if (k >= steps) { break; }
 						if (leader)
@@ -1127,7 +1139,16 @@ static void fill_params(const xnor_b200_conv_desc & d, XcParams & p, int pitch)
 template <int NF, int MODE, bool STREAM, bool SPLIT>
 static int launch_conv(XcParams & p, const XcPlan & q, cudaStream_t stream)
 {
-	const auto kernel = p.tabled ? xnor_conv_kernel<NF, MODE, STREAM, SPLIT, true> : xnor_conv_kernel<NF, MODE, STREAM, SPLIT, false>;
+	auto kernel = p.tabled ? xnor_conv_kernel<NF, MODE, STREAM, SPLIT, XC_TABLE, true>
+			: (p.taps == 1) ? xnor_conv_kernel<NF, MODE, STREAM, SPLIT, XC_POINTS, true> : xnor_conv_kernel<NF, MODE, STREAM, SPLIT, XC_ROWS, true>;
+	if constexpr (MODE != 0)
+	{
+		if (p.M % 32 != 0 || (MODE == 2 && p.out != nullptr))
+		{
+			kernel = p.tabled ? xnor_conv_kernel<NF, MODE, STREAM, SPLIT, XC_TABLE, false>
+					: (p.taps == 1) ? xnor_conv_kernel<NF, MODE, STREAM, SPLIT, XC_POINTS, false> : xnor_conv_kernel<NF, MODE, STREAM, SPLIT, XC_ROWS, false>;
+		}
+	}
 	int rc = ensure_dynamic_smem((const void *)kernel, q.smem);
 	if (rc != XNOR_B200_OK) { return rc; }
 	return launch_behind(kernel, (unsigned)q.grid, XC_THREADS, q.smem, stream, p);
@@ -1355,7 +1376,7 @@ extern "C" int xnor_b200_conv_words_plan(const xnor_b200_conv_desc * desc, const
 	{
 		for (int i = 0; i < p.n_src; ++i)
 		{
-			const int words = run_of(p, p.src[i], u).words;
+			const int words = run_of<-1>(p, p.src[i], u).words;
 			plan->run_words_min = min(plan->run_words_min, words);
 			plan->run_words_max = max(plan->run_words_max, words);
 		}
