@@ -8,7 +8,8 @@ import synth  # noqa: E402
 from darknet_b200 import capi  # noqa: E402
 
 
-@pytest.mark.parametrize("batch,anchors,classes,hw", [(1, 1, 1, 1), (2, 3, 127, 33), (1, 2, 150, 165), (1, 2, 150, 166), (2, 1, 1000, 50), (70, 5, 3, 169)])
+@pytest.mark.parametrize("batch,anchors,classes,hw", [(1, 1, 1, 1), (2, 3, 127, 33), (1, 2, 150, 165), (1, 2, 150, 166), (2, 1, 1000, 50), (70, 5, 3, 169),
+                                                      (3, 5, 80, 169), (2, 2, 7, 256), (1, 2, 9, 257), (1, 1, 30, 512), (1, 1, 30, 513), (2, 1, 2, 64)])
 def test_class_softmax(batch, anchors, classes, hw):
     x = torch.from_numpy(synth.bell(classes + hw, (batch, anchors, 5 + classes, hw), 3.0)).cuda()
     out = torch.full_like(x, float("nan"))
