@@ -291,6 +291,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 	__shared__ __align__(16) int s_cnt[DET_STEP * DET_WARPS];
 	__shared__ int s_m[DET_WARPS];
 	cg::cluster_group cluster = cg::this_cluster();
+	pdl_trigger();                                               // (rows_host_kernel; it reads nothing before this one has finished)
 	const int rank = (int)cluster.block_rank();
 	const int b = blockIdx.x / DET_CLUSTER;
 	const int lane = threadIdx.x & 31;
@@ -650,24 +651,26 @@ detect_kernel(const __grid_constant__ DetectParams p)
 __global__ void __launch_bounds__(256)
 rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __restrict__ row_count, int take, float * __restrict__ host_rows, int * __restrict__ host_count)
 {
+	pdl_wait();                                                  // launched while the kernel in front of it, detect_kernel as a rule, finishes
 	const size_t b = blockIdx.y;
 	const size_t floats = (size_t)take * 7;
 	const float * from = rows + b * max_rows * 7;
 	float * to = host_rows + b * floats;
-	for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < floats; i += (size_t)gridDim.x * 256) { to[i] = __ldg(from + i); }
-	if (blockIdx.x == 0 && threadIdx.x == 0) { host_count[b] = __ldg(row_count + b); }
+	for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < floats; i += (size_t)gridDim.x * 256) { to[i] = __ldcg(from + i); }
+	if (blockIdx.x == 0 && threadIdx.x == 0) { host_count[b] = __ldcg(row_count + b); }
 }
 
-// The address at which a kernel may write host memory, or nullptr for memory that is not page-locked
-static void * device_view(void * host)
+// The address at which a kernel may write the given bytes of host memory, or nullptr unless first and last of them are page-locked together
+static void * device_view(void * host, size_t bytes)
 {
-	cudaPointerAttributes a = {};
-	if (cudaPointerGetAttributes(&a, host) != cudaSuccess)
+	cudaPointerAttributes a = {}, z = {};
+	if (cudaPointerGetAttributes(&a, host) != cudaSuccess || cudaPointerGetAttributes(&z, (char *)host + bytes - 1) != cudaSuccess)
 	{
 		cudaGetLastError();
 		return nullptr;
 	}
-	return (a.type == cudaMemoryTypeHost) ? a.devicePointer : nullptr;
+	const bool whole = a.type == cudaMemoryTypeHost && z.type == cudaMemoryTypeHost && (char *)a.devicePointer + (bytes - 1) == (char *)z.devicePointer;
+	return whole ? a.devicePointer : nullptr;
 }
 
 static int check_dets(const xnor_b200_detections * d, int batch)
@@ -803,13 +806,22 @@ extern "C" int xnor_b200_rows_to_host(const float * rows, int max_rows, const in
 {
 	if (rows == nullptr || row_count == nullptr || host_rows == nullptr || host_count == nullptr) { return XNOR_B200_ERR_NULL; }
 	if (batch <= 0 || take <= 0 || take > max_rows) { return XNOR_B200_ERR_INVALID; }
-	float * rows_at = (float *)device_view(host_rows);
-	int * count_at = (int *)device_view(host_count);
+	float * rows_at = (float *)device_view(host_rows, (size_t)batch * take * 7 * sizeof(float));
+	int * count_at = (int *)device_view(host_count, (size_t)batch * sizeof(int));
 	if (rows_at != nullptr && count_at != nullptr && batch <= 65535 && (((uintptr_t)rows_at | (uintptr_t)count_at) & 3u) == 0)
 	{
 		// one launch for two copies of 3 to 8 us each and the gap between them
-		rows_host_kernel<<<dim3((unsigned)((take * 7LL + 1023) / 1024), (unsigned)batch, 1), 256, 0, (cudaStream_t)stream>>>(rows, max_rows, row_count, take, rows_at, count_at);
-		return check_launch();
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3((unsigned)((take * 7LL + 1023) / 1024), (unsigned)batch, 1);
+		cfg.blockDim = dim3(256, 1, 1);
+		cfg.stream = (cudaStream_t)stream;
+		cudaLaunchAttribute attr[1];
+		attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+		attr[0].val.programmaticStreamSerializationAllowed = 1;
+		cfg.attrs = attr;
+		cfg.numAttrs = 1;
+		const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_host_kernel, rows, max_rows, row_count, take, rows_at, count_at);
+		return (e == cudaSuccess) ? check_launch() : cuda_fail(e);
 	}
 	cudaError_t e = cudaMemcpyAsync(host_count, row_count, (size_t)batch * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
 	if (e != cudaSuccess) { return cuda_fail(e); }

@@ -479,8 +479,8 @@ XNOR_B200_API int xnor_b200_detect(const xnor_b200_yolo_head * heads, int n_head
 		float thresh, int relative, int letter, float nms_thresh, const xnor_b200_detections * dets,
 		float * rows, int max_rows, int * row_count, void * stream);
 
-/* Queues the copies of row_count [batch] and of each image's first `take` rows to host memory (page-locked for the copies to be
- * asynchronous): host_count [batch], host_rows [batch][take][7]. */
+/* Queues the copies of row_count [batch] and of each image's first `take` rows to host memory: host_count [batch], host_rows
+ * [batch][take][7].  Page-locked memory is written by one kernel; other memory by two copies, which then are not asynchronous. */
 XNOR_B200_API int xnor_b200_rows_to_host(const float * rows, int max_rows, const int * row_count, int batch, int take, float * host_rows,
 		int * host_count, void * stream);
 
