@@ -25,6 +25,8 @@ from darknet_b200 import capi  # noqa: E402
     (150, 416, 13, 13, 130, 1, 0, 65), (64, 96, 31, 33, 33, 1, 1, 11), (9, 128, 40, 41, 129, 1, 1, 0), (9, 129, 40, 41, 129, 1, 0, 0),
                                         # several tiles an SM; 3 and 4 K blocks (each taken out by itself) and 5
     (1, 32, 32, 32, 130, 3, 0, 0), (1, 32, 25, 41, 130, 3, 0, 0),      # 1024 pixels and one more
+    (9, 96, 13, 13, 425, 1, 0, 0), (150, 64, 13, 13, 240, 1, 1, 8), (150, 64, 13, 13, 241, 1, 1, 0), (150, 64, 13, 13, 257, 3, 1, 0),
+    (113, 512, 13, 13, 144, 3, 1, 0),   # a last filter tile of 41, 112, 113, 1 and 16, the last with its K blocks dealt to clusters
     (2, 300, 23, 22, 33, 1, 1, 11), (3, 300, 19, 18, 33, 1, 1, 11),    # 1012 and 1026, K blocks that are not whole
 ])
 def test_prepared_filters_match_fp64(batch, c, h, w, n, size, leaky, entries):
