@@ -15,8 +15,8 @@
 // Roles: warp 0 issues, 1 copies filters, 4..11 produce the pixel operand (a pixel and 16 of the 32 channels each, two K blocks in flight),
 // 12..27 collect (a pixel and 32 filters each).  Tensor memory: two buffers of 128 columns for groups of K blocks, four stages of 64
 // columns of pixels.  Every wait is bounded.
-// Measured, us before and after: 3x3 256 -> 512 on 64 maps of 13x13 170 -> 139, 1x1 256 -> 255 with the yolo step on 64 of 26x26 76 -> 53,
-// 512 -> 255 on 64 of 13x13 41 -> 35, 1024 -> 425 on 256 of 13x13 271 -> 240.  Bound by the tensor pipe (about 1100 cycles a K block; 1400
+// Measured, us before and after: 3x3 256 -> 512 on 64 maps of 13x13 170 -> 138, 1x1 256 -> 255 with the yolo step on 64 of 26x26 76 -> 53,
+// 512 -> 255 on 64 of 13x13 41 -> 35, 1024 -> 425 on 256 of 13x13 271 -> 232.  Bound by the tensor pipe (about 1100 cycles a K block; 1400
 // in all where sums are long) and, in a head of 8 K blocks, by the way out of a tile's values.  With the shared memory's load halved
 // twice the producers (148) or half the collectors (137; heads 65 instead of 53) give nothing.
 #include "float_tc.cuh"
@@ -36,7 +36,9 @@ constexpr int FP_CH = 16;                      // channels of a K block that a p
 constexpr int FP_PRODUCERS = 8, FP_COLLECTORS = 16;
 constexpr int FP_COPY_WARP = 1, FP_FIRST_PRODUCER = 4, FP_FIRST_COLLECTOR = FP_FIRST_PRODUCER + FP_PRODUCERS;
 constexpr int FP_THREADS = 32 * (FP_FIRST_COLLECTOR + FP_COLLECTORS);
-constexpr int FP_REST_KBLOCKS = 48;            // tiles beyond whole rounds are split from so many K blocks on: a launch costs about 12 us
+// Tiles beyond whole rounds are split from so many K blocks on.  A launch for them that starts as SMs become free costs a few us: at 32 K blocks
+// (1x1 1024 -> 425 on 256 of 13x13) 240 without, 232 with it; at 16 (512 -> 255 on 64) 33 without.
+constexpr int FP_REST_KBLOCKS = 24;
 constexpr int FP_COLS = FT_NF / (FP_COLLECTORS / 4);                    // filters of a collector thread
 constexpr int FP_STAGE_BYTES = 2 * FT_TILE_BYTES;                       // filters' heads and remainders
 constexpr int FP_SUMS_BYTES = FP_COLLECTORS * 32 * FP_COLS * 4;         // a tile's sums on their way out
@@ -107,6 +109,9 @@ float_conv_tcp_kernel(const __grid_constant__ FtParams p)
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
+	// The launch of the tiles that are left over reads nothing of this one's: it starts as SMs become free, and waits for this one's end only so as
+	// to end behind it.
+	if (p.more) { pdl_trigger(); }
 	// producers and collectors: a warp reaches the 32 tensor-memory lanes (pixels) of its number modulo 4
 	const int quarter = warp & 3;
 	// what every role does at its end: nobody's shared or tensor memory goes while another still works on it
@@ -441,9 +446,10 @@ float_conv_tcp_kernel(const __grid_constant__ FtParams p)
 		}
 		meet();
 	}
+	pdl_wait();
 }
 
-static int launch_tiles(const FtParams & p, cudaStream_t stream)
+static int launch_tiles(const FtParams & p, cudaStream_t stream, bool behind = false)
 {
 	const int rc = ensure_dynamic_smem((const void *)float_conv_tcp_kernel, FP_SMEM_BYTES);
 	if (rc != XNOR_B200_OK) { return rc; }
@@ -452,13 +458,15 @@ static int launch_tiles(const FtParams & p, cudaStream_t stream)
 	cfg.blockDim = dim3(FP_THREADS, 1, 1);
 	cfg.dynamicSmemBytes = FP_SMEM_BYTES;
 	cfg.stream = stream;
-	cudaLaunchAttribute attr[1];
+	cudaLaunchAttribute attr[2];
 	attr[0].id = cudaLaunchAttributeClusterDimension;
 	attr[0].val.clusterDim.x = (unsigned)p.split;
 	attr[0].val.clusterDim.y = 1;
 	attr[0].val.clusterDim.z = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = 1;
+	attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[1].val.programmaticStreamSerializationAllowed = 1;
+	cfg.numAttrs = behind ? 2 : 1;
 	const cudaError_t e = cudaLaunchKernelEx(&cfg, float_conv_tcp_kernel, p);
 	return (e == cudaSuccess) ? check_launch() : cuda_fail(e);
 }
@@ -475,6 +483,7 @@ int launch_float_tcp(FtParams & p, cudaStream_t stream)
 	if (all > rest && p.kblocks < FP_REST_KBLOCKS) { split = 1; }
 	p.tile0 = 0;
 	p.split = 1;
+	p.more = 0;
 	// Where every CTA would take the same filter tile each time (four of them, 148 SMs), the order moves on by one after every round: the last
 	// filter tile may be narrower, and those that had no other would finish early (3x3 512 -> 144 on 128 of 13x13 252 -> 240 us, 1x1 1024 -> 425 on
 	// 256 of them 244 -> 240; narrow tiles all at the end instead: 244 and 254, a tile's pixels then come from memory twice).
@@ -485,6 +494,7 @@ int launch_float_tcp(FtParams & p, cudaStream_t stream)
 		return launch_tiles(p, stream);
 	}
 	p.tiles = all - rest;
+	p.more = 1;
 	if (p.tiles > 0)
 	{
 		const int rc = launch_tiles(p, stream);
@@ -493,7 +503,8 @@ int launch_float_tcp(FtParams & p, cudaStream_t stream)
 	p.tile0 = all - rest;
 	p.tiles = rest;
 	p.split = split;
-	return launch_tiles(p, stream);
+	p.more = 0;
+	return launch_tiles(p, stream, all > rest);
 }
 
 }  // namespace xnor

@@ -26,6 +26,7 @@ struct FtParams
 	int tiles_f;
 	int split;            // CTAs per tile
 	int tile0, tiles;     // first tile of the launch, tiles
+	int more;             // float_conv_tcp.cu: another launch with the rest of the tiles follows
 	int turn;             // float_conv_tcp.cu: tiles after which the order of the filter tiles moves on by one
 	int * status;
 	uint32_t spin_limit;
