@@ -1105,7 +1105,8 @@ def load_network_custom(cfg: str, weights: str, batch: int = 1, device: str = "c
 
 
 def own_launches_per_forward(net: Network) -> int:
-    """Kernels of libxnor_b200.so that one forward launches, after every fusion that load_network_custom set up."""
+    """Kernels of libxnor_b200.so that one forward launches, after every fusion that load_network_custom set up (a float convolution counts
+    once, also where the last tiles of a batch are a launch of their own)."""
     if net.plan is not None:
         return sum(1 for op in net.plan.ops if op.kind not in (capi.OP_FORK, capi.OP_BACK, capi.OP_MARK))
     n = 0
