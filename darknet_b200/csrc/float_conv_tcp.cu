@@ -8,9 +8,10 @@
 //   * a CTA stays on its SM and takes tile after tile: producers fetch the next tile's pixels while the epilogue of the last one runs;
 //   * tiles that do not fill a round of the SMs are a launch of their own whose K blocks are dealt to clusters of two to four CTAs.
 // The tensor core adds into its accumulator without rounding to nearest, an error that grows with the number of instructions one takes
-// (float_conv_tc.cu).  So the sum is taken out after every two K blocks, or after each where there are at most four (FP_FEW), and added in
-// fp32 by warps that do nothing else: 2-norm error against fp64, leaky inputs, 3.4e-7 to 3.8e-7 at any number of channels, where
-// accumulators of whole sums left 3.4e-7 (up to 4 K blocks) to 1.9e-6 (32) and 1.7e-6 (72, of 3x3 layers).
+// (float_conv_tc.cu).  So the sum is taken out after every two K blocks, or after each where a CTA has few (FP_FEW, FP_FEW_3X3), and added in
+// fp32 by warps that do nothing else.  2-norm error against fp64, leaky inputs: 3.3e-7 to 4.0e-7 by pairs, up to 144 K blocks, and 0.9e-7 to
+// 1.6e-7 one by one.  Accumulators of whole sums left, 1x1, 3.3e-7 (up to 4 K blocks a CTA) to 1.9e-6 (32), and 3x3, where the small products had
+// one of their own, 1.8e-7 (3), 2.7e-7 (9), 3.3e-7 (12), 3.8e-7 (14), 4.7e-7 (18) and 1.7e-6 (72).
 //
 // Roles: warp 0 issues, 1 copies filters, 4..11 produce the pixel operand (a pixel and 16 of the 32 channels each, two K blocks in flight),
 // 12..27 collect (a pixel and 32 filters each).  Tensor memory: two buffers of 128 columns for groups of K blocks, four stages of 64
@@ -28,7 +29,9 @@ namespace xnor
 
 namespace cg = cooperative_groups;
 
-constexpr int FP_FEW = 4;                      // K blocks of a sum up to which each is taken out by itself
+// K blocks of a CTA's sum up to which each is taken out by itself: where pairs would be less accurate than whole sums were (above), in 3x3
+// layers, or where it takes no time.  3x3 with 9 K blocks on 64 maps of 13x13, 512 filters: 35.0 us, 30.9 by pairs, 45 by whole sums.
+constexpr int FP_FEW = 4, FP_FEW_3X3 = 12;
 constexpr int FP_BUFFERS = 2;
 constexpr int FP_STAGES = 4;
 constexpr int FP_A_COL = FP_BUFFERS * FT_NF;   // tensor-memory column of the first pixel stage: 32 heads, 32 remainders
@@ -77,7 +80,7 @@ float_conv_tcp_kernel(const __grid_constant__ FtParams p)
 	const int kbn = max(0, min(p.kblocks - kb0, per));                 // this CTA's K blocks of a tile
 	const int my_tiles = (end_tile - first_tile + tile_step - 1) / tile_step;
 	const int total = my_tiles * kbn;
-	const int group_blocks = (per <= FP_FEW) ? 1 : 2;                  // K blocks whose products meet in tensor memory
+	const int group_blocks = (per <= ((p.taps == 9) ? FP_FEW_3X3 : FP_FEW)) ? 1 : 2;                  // K blocks whose products meet in tensor memory
 	auto filters_of = [&](int tile) { return (tile + tile / p.turn) % p.tiles_f; };                                // filter tile of a tile
 	// Filters that its products are formed for: an instruction takes any multiple of 16, in time that goes with it (1x1 256 -> 18 on 64 of 26x26
 	// 24.9 -> 22.7 us, 512 -> 75 on 64 of 13x13 18.7 -> 17.8)

@@ -93,6 +93,26 @@ def test_no_less_accurate_than_the_fp32_kernels(batch, c, h, w, n, size):
     assert error(prepared_conv("tc", desc, x, wt, b)) <= error(other) + 6e-9
 
 
+@pytest.mark.parametrize("batch,c,h,w,n,size,bound", [
+    # K blocks of a CTA, each sum taken out by itself: up to 4 of a 1x1 layer, up to 12 of a 3x3 one (9, 5, 12 of 36, 12 of 45)
+    (9, 8, 13, 13, 128, 1, 2e-7), (9, 128, 40, 41, 129, 1, 2e-7), (24, 256, 13, 13, 128, 1, 2e-7),
+    (64, 32, 13, 13, 512, 3, 2e-7), (9, 64, 13, 13, 128, 3, 2e-7), (24, 128, 13, 13, 128, 3, 2e-7), (9, 160, 13, 13, 128, 3, 2e-7),
+    # by pairs: 5, 8 and 32, the last with its left-over tiles dealt to clusters of three; 18, 72 and 144
+    (24, 160, 26, 26, 128, 1, 4.5e-7), (24, 256, 26, 26, 128, 1, 4.5e-7), (64, 1024, 13, 13, 425, 1, 4.5e-7),
+    (64, 64, 13, 13, 512, 3, 4.5e-7), (64, 256, 13, 13, 512, 3, 4.5e-7), (113, 512, 13, 13, 40, 3, 4.5e-7),
+])
+def test_error_of_batches(batch, c, h, w, n, size, bound):
+    """More than 1024 pixels.  One K block is twelve instructions into one accumulator: about 1.4e-7; two leave 3.3e-7 to 4.0e-7; sums that
+    stay there whole 4.3e-7 at 5 (1x1), 5.5e-7 at 8 and 1.9e-6 at 32.  The bounds lie between."""
+    g = torch.Generator(device="cuda").manual_seed(batch + c + n)
+    x = F.leaky_relu(torch.randn(batch, c, h, w, generator=g, device="cuda") * 3, 0.1)
+    wt = torch.randn(n, c, size, size, generator=g, device="cuda") * (c * size * size) ** -0.5
+    b = torch.randn(n, generator=g, device="cuda") * 0.01
+    want = torch.cat([fp64(x[i:i + 1], wt, b) for i in range(batch)])
+    got = prepared_conv("tc", capi.ConvDesc(batch, c, h, w, n, size, 1, size // 2, capi.LINEAR), x, wt, b)
+    assert float((got.double() - want).norm() / want.norm()) <= bound
+
+
 @pytest.mark.parametrize("batch,c,h,w,n,size", [(2, 64, 9, 7, 140, 3), (9, 64, 13, 13, 33, 3), (2, 96, 9, 7, 140, 1), (64, 512, 13, 13, 32, 3)])
 @pytest.mark.parametrize("leaky", [0, 1])
 def test_infinite_and_huge_values(batch, c, h, w, n, size, leaky):
