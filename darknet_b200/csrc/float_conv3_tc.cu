@@ -328,7 +328,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 				{
 					uint32_t d[32];
 					tmem_load<32>(tacc + (uint32_t)(h * 32), d);
-					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					tmem_wait<32>(d);
 					if (h == NN / 32 - 1)
 					{
 						asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -368,7 +368,7 @@ float_conv3_signs_kernel(const __grid_constant__ F3Params p)
 				{
 					uint32_t d[NF];
 					tmem_load<NF>(tacc + (uint32_t)(s * NF), d);
-					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					tmem_wait<NF>(d);
 					if (s == 3)
 					{
 						asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -84,7 +84,7 @@ __device__ __forceinline__ void tile_sums(uint32_t tmem, int used, float (&acc)[
 	{
 		uint32_t d[32];
 		tmem_load<32>(tmem + (uint32_t)(a * FT_NF), d);
-		asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+		tmem_wait<32>(d);
 		#pragma unroll
 		for (int j = 0; j < 32; ++j) { acc[j] = (a == 0) ? __uint_as_float(d[j]) : __fadd_rn(acc[j], __uint_as_float(d[j])); }
 	}

@@ -410,7 +410,7 @@ float_conv_tcp_kernel(const __grid_constant__ FtParams p)
 				{
 					uint32_t d[16];
 					tmem_load<16>(from + (uint32_t)(buffer * FT_NF + h), d);
-					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					tmem_wait<16>(d);
 					#pragma unroll
 					for (int j = 0; j < 16; ++j) { sums[h + j] = __fadd_rn(sums[h + j], __uint_as_float(d[j])); }
 				}

@@ -221,6 +221,26 @@ __device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&d)[G])
 	}
 }
 
+// Waits for this thread's tensor-memory loads; the loaded registers pass through it, so nothing can use them before:
+// what is computed from them is no memory access, which a clobber of memory would hold back.
+template <int G>
+__device__ __forceinline__ void tmem_wait(uint32_t (&d)[G])
+{
+	asm volatile("tcgen05.wait::ld.sync.aligned;"
+			: "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]));
+	if constexpr (G >= 16)
+	{
+		asm volatile(""
+				: "+r"(d[8]), "+r"(d[9]), "+r"(d[10]), "+r"(d[11]), "+r"(d[12]), "+r"(d[13]), "+r"(d[14]), "+r"(d[15]));
+	}
+	if constexpr (G == 32)
+	{
+		asm volatile(""
+				: "+r"(d[16]), "+r"(d[17]), "+r"(d[18]), "+r"(d[19]), "+r"(d[20]), "+r"(d[21]), "+r"(d[22]), "+r"(d[23]),
+				  "+r"(d[24]), "+r"(d[25]), "+r"(d[26]), "+r"(d[27]), "+r"(d[28]), "+r"(d[29]), "+r"(d[30]), "+r"(d[31]));
+	}
+}
+
 // 2 * agreeing - K of one output, as a float, from its raw accumulator.
 //   ACCF == false (kind::i8, operands 0 / -1, s32 accumulator d = popc(a & b)):  (K - 2 popc(b)) - 2 popc(a) + 4 d = k_b + fx + 4 d
 //   ACCF == true  (kind::mxf4, operands +1 / -1 over the zero-padded rows, f32 accumulator): every position the K blocks cover
@@ -306,7 +326,7 @@ __device__ __forceinline__ void epilogue_values(const TcParams & p, const Filter
 				for (int u = 0; u < G; ++u) { if (f0 + fbn + u < p.M) { scn[u] = ld_stream(sc_in + (size_t)(fbn + u) * p.ldc); } }
 			}
 		}
-		asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+		tmem_wait<G>(d);
 		if (col_ok)
 		{
 			uint32_t bits = 0;
@@ -449,7 +469,7 @@ __device__ __forceinline__ void epilogue_tile(const TcParams & p, const int * s_
 	{
 		uint32_t d[32];
 		tmem_load<32>(tlane + (uint32_t)(chunk * 32), d);
-		asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+		tmem_wait<32>(d);
 		const int fbase = chunk * 32;
 		if (p.signs != nullptr || p.x.n_sinks > 0)
 		{

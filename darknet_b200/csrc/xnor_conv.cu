@@ -185,25 +185,6 @@ __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr)
 	return v;
 }
 
-// Waits for this thread's tensor-memory loads; the loaded registers pass through it, so nothing can use them before.
-template <int G>
-__device__ __forceinline__ void tmem_wait(uint32_t (&d)[G])
-{
-	asm volatile("tcgen05.wait::ld.sync.aligned;"
-			: "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]));
-	if constexpr (G >= 16)
-	{
-		asm volatile(""
-				: "+r"(d[8]), "+r"(d[9]), "+r"(d[10]), "+r"(d[11]), "+r"(d[12]), "+r"(d[13]), "+r"(d[14]), "+r"(d[15]));
-	}
-	if constexpr (G == 32)
-	{
-		asm volatile(""
-				: "+r"(d[16]), "+r"(d[17]), "+r"(d[18]), "+r"(d[19]), "+r"(d[20]), "+r"(d[21]), "+r"(d[22]), "+r"(d[23]),
-				  "+r"(d[24]), "+r"(d[25]), "+r"(d[26]), "+r"(d[27]), "+r"(d[28]), "+r"(d[29]), "+r"(d[30]), "+r"(d[31]));
-	}
-}
-
 __device__ __forceinline__ void bulk_load(uint32_t dst, const uint32_t * src, uint32_t bytes, uint64_t * bar)
 {
 	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"

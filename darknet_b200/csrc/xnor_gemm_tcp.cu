@@ -255,7 +255,7 @@ xnor_gemm_tcp_kernel(const TcParams p, const __grid_constant__ CUtensorMap map_p
 					}
 					uint32_t d[32];
 					tmem_load<32>(tlane + (uint32_t)(chunk * 32), d);
-					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					tmem_wait<32>(d);
 					if (half == 1)
 					{
 						// the accumulator is read: the issuer may fill it again

@@ -19,3 +19,13 @@ def test_dependents_start_once_a_cta_has_its_tensor_memory(path):
             continue
         between = kernel[kernel.index("tcgen05.alloc"):kernel.index("pdl_trigger()")]
         assert kernel.index("tcgen05.alloc") < kernel.index("pdl_trigger()") and "__syncthreads();" in between
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cu*"))), ids=os.path.basename)
+def test_waits_for_tensor_memory_loads_hold_the_registers(path):
+    """A load from tensor memory fills its registers some time after the instruction.  The wait takes them as operands: without, only the
+    compiler's order of instructions keeps arithmetic on them behind it (a clobber of memory holds back accesses, not arithmetic)."""
+    with open(path) as fh:
+        text = re.sub(r"//[^\n]*", "", fh.read())
+    for rest in text.split('"tcgen05.wait::ld')[1:]:
+        assert re.match(r'[^"]*"\s*:\s*"\+r"', rest), rest[:120]
