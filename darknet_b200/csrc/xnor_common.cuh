@@ -13,9 +13,11 @@ namespace xnor
 // Last failing CUDA status seen by this library on the calling thread.
 extern thread_local int g_last_cuda_error;
 
+// The runtime keeps the error of a failed call: taken out with the report, or the next launch, which asks for it, would report it again.
 inline int cuda_fail(cudaError_t e)
 {
 	g_last_cuda_error = (int)e;
+	cudaGetLastError();
 	return XNOR_B200_ERR_CUDA;
 }
 

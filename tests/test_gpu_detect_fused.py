@@ -1,5 +1,8 @@
 """xnor_b200_detect (decode, suppress and compact in one launch) against a plain CPU restatement, at list lengths around the
 kernel's own limits: none, one scan step, a class crowded past what one warp ranks, more detections than slots."""
+import ctypes as C
+import mmap
+
 import numpy as np
 import pytest
 
@@ -133,6 +136,46 @@ def test_rows_to_host_into_either_kind_of_memory(pinned):
                                                  torch.cuda.current_stream().cuda_stream), "xnor_b200_rows_to_host")
     torch.cuda.synchronize()
     assert torch.equal(host, rows[:, :33].cpu()) and torch.equal(host_count, count.cpu())
+
+
+def recorded_kernels(call):
+    """Kernels that `call(stream)` records into a graph, which is not run."""
+    cu, n, graph, stream = C.CDLL("libcuda.so.1"), C.c_size_t(0), C.c_void_p(), torch.cuda.Stream()
+    handle = C.c_void_p(stream.cuda_stream)
+    assert cu.cuStreamBeginCapture_v2(handle, 2) == 0
+    call(stream.cuda_stream)
+    if cu.cuStreamEndCapture(handle, C.byref(graph)) != 0:          # what the call did cannot be recorded: no kernel, then
+        return 0
+    assert cu.cuGraphGetNodes(graph, None, C.byref(n)) == 0
+    nodes, kernels, kind = (C.c_void_p * n.value)(), 0, C.c_int(-1)
+    assert n.value == 0 or cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0
+    for node in nodes:
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        kernels += kind.value == 0
+    assert cu.cuGraphDestroy(graph) == 0
+    return kernels
+
+
+def test_a_failed_call_is_reported_once():
+    """What a call reported is not the next one's: here counts that would go over the end of a registration, refused when they are recorded."""
+    rt, page = torch.cuda.cudart(), mmap.PAGESIZE
+    rows, count = torch.randn(2, 40, 7, device="cuda"), torch.tensor([3, 40], dtype=torch.int32, device="cuda")
+    host, host_count = torch.zeros(2, 40, 7, pin_memory=True), torch.zeros(2, dtype=torch.int32, pin_memory=True)
+    memory = mmap.mmap(-1, 2 * page)
+    base = C.addressof(C.c_char.from_buffer(memory))
+    codes = []
+
+    def call(at, stream):
+        codes.append(capi.lib().xnor_b200_rows_to_host(rows.data_ptr(), 40, count.data_ptr(), 2, 40, host.data_ptr(), at, stream))
+    assert int(rt.cudaHostRegister(base, page, 0)) == 0
+    try:
+        recorded_kernels(lambda stream: call(base + page - 4, stream))
+    finally:
+        assert int(rt.cudaHostUnregister(base)) == 0
+    call(host_count.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert codes[0] != capi.OK and codes[1] == capi.OK
+    assert torch.equal(host, rows.cpu()) and torch.equal(host_count, count.cpu())
 
 
 @pytest.mark.parametrize("counts,max_rows", [([0, 512], 4096), ([513, 3], 4096), ([2049, 700], 4096), ([900, 901], 900)])
