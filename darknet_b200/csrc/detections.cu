@@ -19,6 +19,9 @@
 #include "xnor_common.cuh"
 
 #include <cooperative_groups.h>
+#include <cuda.h>       // pointer attributes; the query itself is fetched through cudaGetDriverEntryPoint
+
+#include <mutex>
 
 namespace xnor
 {
@@ -660,17 +663,37 @@ rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __re
 	if (blockIdx.x == 0 && threadIdx.x == 0) { host_count[b] = __ldcg(row_count + b); }
 }
 
-// The address at which a kernel may write the given bytes of host memory, or nullptr unless first and last of them are page-locked together
+typedef CUresult (*PointerQuery)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+
+static PointerQuery pointer_query()
+{
+	static std::once_flag once;
+	static PointerQuery fn = nullptr;
+	std::call_once(once, []()
+	{
+		void * sym = nullptr;
+		cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+		if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess) { fn = (PointerQuery)sym; }
+	});
+	return fn;
+}
+
+// The address at which a kernel may write the given bytes of host memory; nullptr unless they lie in one page-locked allocation or
+// registration, which the device may write to.  (Where first and last byte are says nothing: two registrations keep the distance of their
+// host addresses, with memory between them that the device does not have.)
 static void * device_view(void * host, size_t bytes)
 {
-	cudaPointerAttributes a = {}, z = {};
-	if (cudaPointerGetAttributes(&a, host) != cudaSuccess || cudaPointerGetAttributes(&z, (char *)host + bytes - 1) != cudaSuccess)
-	{
-		cudaGetLastError();
-		return nullptr;
-	}
-	const bool whole = a.type == cudaMemoryTypeHost && z.type == cudaMemoryTypeHost && (char *)a.devicePointer + (bytes - 1) == (char *)z.devicePointer;
-	return whole ? a.devicePointer : nullptr;
+	const PointerQuery query = pointer_query();
+	CUpointer_attribute which[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+			CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+	unsigned type = 0, access = 0;
+	CUdeviceptr at = 0, start = 0;
+	size_t size = 0;
+	void * out[5] = {&type, &at, &start, &size, &access};
+	if (query == nullptr || query(5, which, out, (CUdeviceptr)host) != CUDA_SUCCESS) { return nullptr; }        // (pageable memory: all zero)
+	const CUdeviceptr first = (CUdeviceptr)host;
+	const bool whole = type == CU_MEMORYTYPE_HOST && at != 0 && start <= first && first - start <= size && bytes <= size - (first - start);
+	return (whole && access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE) ? (void *)at : nullptr;
 }
 
 static int check_dets(const xnor_b200_detections * d, int batch)

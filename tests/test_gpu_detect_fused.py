@@ -156,6 +156,35 @@ def recorded_kernels(call):
     return kernels
 
 
+def test_rows_go_by_a_kernel_into_one_page_locked_range_only():
+    """Two registrations with a gap between them, one behind the other, one that ends too early, one the device may only read: copies, which
+    leave the range to the runtime.  Recorded only: a kernel that stored there would write to addresses that the device does not have."""
+    rt, page = torch.cuda.cudart(), mmap.PAGESIZE
+    rows, count = torch.zeros(2, 512, 7, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda")
+    memory = mmap.mmap(-1, 24 * page)
+    base = C.addressof(C.c_char.from_buffer(memory))
+    pinned_rows, pinned_count = torch.empty(2, 512, 7, pin_memory=True), torch.empty(2, dtype=torch.int32, pin_memory=True)
+
+    def kernels(host_rows, host_count, take):
+        return recorded_kernels(lambda stream: capi.lib().xnor_b200_rows_to_host(rows.data_ptr(), 512, count.data_ptr(), 2, take, host_rows, host_count, stream))
+    ranges = [(0, 2, 0), (4, 2, 0), (8, 2, 0), (10, 2, 0), (14, 4, 0), (20, 4, 8)]       # first page, pages, flags (8: read-only)
+    for first, pages, flags in ranges:
+        assert int(rt.cudaHostRegister(base + first * page, pages * page, flags)) == 0
+    try:
+        take = 6 * page // 56                                       # rows of two images that fill six pages, all but a few bytes
+        assert kernels(base, pinned_count.data_ptr(), take) == 0    # pages 0..5, 2 and 3 not registered
+        assert kernels(base + 8 * page, pinned_count.data_ptr(), 4 * page // 56) == 0
+        assert kernels(base + 15 * page, pinned_count.data_ptr(), 4 * page // 56) == 0
+        assert kernels(base + 20 * page, pinned_count.data_ptr(), page // 56) == 0
+        assert kernels(pinned_rows.data_ptr(), base + 16 * page - 4, take) == 1      # counts across two pages of one registration
+        assert kernels(pinned_rows.data_ptr(), base + 18 * page - 4, take) == 0      # ... and over the end of it
+        assert kernels(base + 15 * page + 8, pinned_count.data_ptr(), 2 * page // 56) == 1
+        assert kernels(pinned_rows.data_ptr(), pinned_count.data_ptr(), 512) == 1
+    finally:
+        for first, _, _ in ranges:
+            assert int(rt.cudaHostUnregister(base + first * page)) == 0
+
+
 def test_a_failed_call_is_reported_once():
     """What a call reported is not the next one's: here counts that would go over the end of a registration, refused when they are recorded."""
     rt, page = torch.cuda.cudart(), mmap.PAGESIZE
