@@ -19,9 +19,11 @@
 #include "xnor_common.cuh"
 
 #include <cooperative_groups.h>
-#include <cuda.h>       // pointer attributes; the query itself is fetched through cudaGetDriverEntryPoint
+#include <cuda.h>       // pointer attributes and contexts; the calls themselves are fetched by name
+#include <cudaTypedefs.h>
 
 #include <mutex>
+#include <type_traits>
 
 namespace xnor
 {
@@ -663,19 +665,34 @@ rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __re
 	if (blockIdx.x == 0 && threadIdx.x == 0) { host_count[b] = __ldcg(row_count + b); }
 }
 
-typedef CUresult (*PointerQuery)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+struct DriverCalls
+{
+	PFN_cuPointerGetAttributes_v7000 attributes;
+	PFN_cuStreamGetCtx_v9020 stream_context;
+	PFN_cuCtxGetCurrent_v4000 context;
+};
 
-static PointerQuery pointer_query()
+// nullptr: not to be had
+static const DriverCalls * driver()
 {
 	static std::once_flag once;
-	static PointerQuery fn = nullptr;
+	static DriverCalls calls = {};
+	static bool all = false;
 	std::call_once(once, []()
 	{
-		void * sym = nullptr;
-		cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-		if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess) { fn = (PointerQuery)sym; }
+		// each in the version of its type: the newest cuStreamGetCtx has another parameter
+		auto find = [](const char * name, unsigned version, auto & fn)
+		{
+			void * sym = nullptr;
+			cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+			if (cudaGetDriverEntryPointByVersion(name, &sym, version, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) { return false; }
+			fn = (std::remove_reference_t<decltype(fn)>)sym;
+			return true;
+		};
+		all = find("cuPointerGetAttributes", 7000, calls.attributes) && find("cuStreamGetCtx", 9020, calls.stream_context)
+				&& find("cuCtxGetCurrent", 4000, calls.context);
 	});
-	return fn;
+	return all ? &calls : nullptr;
 }
 
 // The address at which a kernel may write the given bytes of host memory; nullptr unless they lie in one page-locked allocation or
@@ -683,17 +700,37 @@ static PointerQuery pointer_query()
 // host addresses, with memory between them that the device does not have.)
 static void * device_view(void * host, size_t bytes)
 {
-	const PointerQuery query = pointer_query();
+	const DriverCalls * const calls = driver();
 	CUpointer_attribute which[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
 			CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
 	unsigned type = 0, access = 0;
 	CUdeviceptr at = 0, start = 0;
 	size_t size = 0;
 	void * out[5] = {&type, &at, &start, &size, &access};
-	if (query == nullptr || query(5, which, out, (CUdeviceptr)host) != CUDA_SUCCESS) { return nullptr; }        // (pageable memory: all zero)
+	if (calls == nullptr || calls->attributes(5, which, out, (CUdeviceptr)host) != CUDA_SUCCESS) { return nullptr; }        // (pageable memory: all zero)
 	const CUdeviceptr first = (CUdeviceptr)host;
 	const bool whole = type == CU_MEMORYTYPE_HOST && at != 0 && start <= first && first - start <= size && bytes <= size - (first - start);
 	return (whole && access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE) ? (void *)at : nullptr;
+}
+
+// Whether the stream and what a kernel on it would read belong to the current device (copies take any)
+static bool of_this_device(const float * rows, const int * row_count, cudaStream_t stream)
+{
+	// (the stream's context: asking for its device would end a capture)
+	const DriverCalls * const calls = driver();
+	int device = -1;
+	CUcontext current = nullptr, streams = nullptr;
+	if (calls == nullptr || cudaGetDevice(&device) != cudaSuccess || calls->context(&current) != CUDA_SUCCESS
+			|| calls->stream_context((CUstream)stream, &streams) != CUDA_SUCCESS || streams != current) { return false; }
+	for (const void * at : {(const void *)rows, (const void *)row_count})
+	{
+		CUpointer_attribute which[2] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL};
+		unsigned type = 0;
+		int owner = -1;
+		void * out[2] = {&type, &owner};
+		if (calls->attributes(2, which, out, (CUdeviceptr)at) != CUDA_SUCCESS || type != CU_MEMORYTYPE_DEVICE || owner != device) { return false; }
+	}
+	return true;
 }
 
 static int check_dets(const xnor_b200_detections * d, int batch)
@@ -831,7 +868,7 @@ extern "C" int xnor_b200_rows_to_host(const float * rows, int max_rows, const in
 	if (batch <= 0 || take <= 0 || take > max_rows) { return XNOR_B200_ERR_INVALID; }
 	float * rows_at = (float *)device_view(host_rows, (size_t)batch * take * 7 * sizeof(float));
 	int * count_at = (int *)device_view(host_count, (size_t)batch * sizeof(int));
-	if (rows_at != nullptr && count_at != nullptr && batch <= 65535 && (((uintptr_t)rows_at | (uintptr_t)count_at) & 3u) == 0)
+	if (rows_at != nullptr && count_at != nullptr && of_this_device(rows, row_count, (cudaStream_t)stream) && batch <= 65535 && (((uintptr_t)rows_at | (uintptr_t)count_at) & 3u) == 0)
 	{
 		// one launch for two copies of 3 to 8 us each and the gap between them
 		cudaLaunchConfig_t cfg = {};

@@ -185,6 +185,24 @@ def test_rows_go_by_a_kernel_into_one_page_locked_range_only():
             assert int(rt.cudaHostUnregister(base + first * page)) == 0
 
 
+@pytest.mark.parametrize("side", [False, True])
+def test_rows_that_are_not_the_current_devices_go_by_copies(side):
+    """Copies take rows from anywhere the runtime knows, here page-locked memory of the host; a kernel is for device memory and streams of the
+    current device alone."""
+    stream = torch.cuda.Stream() if side else torch.cuda.default_stream()
+    rows, count = torch.randn(3, 40, 7), torch.tensor([5, 40, 0], dtype=torch.int32)
+    host, host_count = torch.zeros(3, 40, 7, pin_memory=True), torch.zeros(3, dtype=torch.int32, pin_memory=True)
+    for r, c, kernels in ((rows.cuda(), count.cuda(), 1), (rows.pin_memory(), count.cuda(), 0), (rows.cuda(), count.pin_memory(), 0)):
+        def call(handle):
+            return capi.lib().xnor_b200_rows_to_host(r.data_ptr(), 40, c.data_ptr(), 3, 40, host.data_ptr(), host_count.data_ptr(), handle)
+        torch.cuda.synchronize()
+        assert recorded_kernels(call) == kernels
+        if kernels:
+            capi.check(call(stream.cuda_stream), "xnor_b200_rows_to_host")
+            torch.cuda.synchronize()
+            assert torch.equal(host, rows) and torch.equal(host_count, count)
+
+
 def test_a_failed_call_is_reported_once():
     """What a call reported is not the next one's: here counts that would go over the end of a registration, refused when they are recorded."""
     rt, page = torch.cuda.cudart(), mmap.PAGESIZE
