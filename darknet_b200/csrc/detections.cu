@@ -652,7 +652,12 @@ detect_kernel(const __grid_constant__ DetectParams p)
 	}
 }
 
-// The counts and first rows of every image, stored straight into page-locked host memory; a CTA column per image
+// The counts and first rows of every image, stored straight into page-locked host memory; a CTA column per image.
+// Its stores hold the SMs while they cross, and cross no faster than the copy engine's: us issued / alone / a 512 MB pass on another stream
+// beside it, by the kernel and by two copies: 14 KB 6.2 / 13.9 / - and 6.9 / 15.3 / -, 112 KB 6.2 / 17.7 / 161 and 8.9 / 17.4 / 159, 224 KB
+// 8.2 / 19.1 / 161 and 10.8 / 18.9 / 159, 448 KB 13.2 / 23.9 / 163 and 14.6 / 23.1 / 159, 3.5 MB 74 / 84 / 212 and 71 / 79 / 161.
+constexpr size_t ROWS_KERNEL_BYTES = 256 << 10;
+
 __global__ void __launch_bounds__(256)
 rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __restrict__ row_count, int take, float * __restrict__ host_rows, int * __restrict__ host_count)
 {
@@ -866,9 +871,15 @@ extern "C" int xnor_b200_rows_to_host(const float * rows, int max_rows, const in
 {
 	if (rows == nullptr || row_count == nullptr || host_rows == nullptr || host_count == nullptr) { return XNOR_B200_ERR_NULL; }
 	if (batch <= 0 || take <= 0 || take > max_rows) { return XNOR_B200_ERR_INVALID; }
-	float * rows_at = (float *)device_view(host_rows, (size_t)batch * take * 7 * sizeof(float));
-	int * count_at = (int *)device_view(host_count, (size_t)batch * sizeof(int));
-	if (rows_at != nullptr && count_at != nullptr && of_this_device(rows, row_count, (cudaStream_t)stream) && batch <= 65535 && (((uintptr_t)rows_at | (uintptr_t)count_at) & 3u) == 0)
+	const size_t bytes = (size_t)batch * take * 7 * sizeof(float);
+	float * rows_at = nullptr;
+	int * count_at = nullptr;
+	if (bytes <= ROWS_KERNEL_BYTES && batch <= 65535 && of_this_device(rows, row_count, (cudaStream_t)stream))
+	{
+		rows_at = (float *)device_view(host_rows, bytes);
+		count_at = (int *)device_view(host_count, (size_t)batch * sizeof(int));
+	}
+	if (rows_at != nullptr && count_at != nullptr && (((uintptr_t)rows_at | (uintptr_t)count_at) & 3u) == 0)
 	{
 		// one launch for two copies of 3 to 8 us each and the gap between them
 		cudaLaunchConfig_t cfg = {};

@@ -480,8 +480,8 @@ XNOR_B200_API int xnor_b200_detect(const xnor_b200_yolo_head * heads, int n_head
 		float * rows, int max_rows, int * row_count, void * stream);
 
 /* Queues the copies of row_count [batch] and of each image's first `take` rows to host memory: host_count [batch], host_rows
- * [batch][take][7].  Where each of the two lies within one page-locked allocation or registration one kernel writes them; else two copies
- * do, which are not asynchronous in pageable memory. */
+ * [batch][take][7].  Up to 256 KB of rows are written by one kernel where each of the two lies within one page-locked allocation or
+ * registration; else by two copies, which are not asynchronous in pageable memory. */
 XNOR_B200_API int xnor_b200_rows_to_host(const float * rows, int max_rows, const int * row_count, int batch, int take, float * host_rows,
 		int * host_count, void * stream);
 

@@ -128,7 +128,7 @@ def test_detect_at_the_lines_of_the_overlap_matrix(tmp_path, found):
 
 @pytest.mark.parametrize("pinned", [True, False])
 def test_rows_to_host_into_either_kind_of_memory(pinned):
-    """Page-locked memory is written by a kernel, any other through the copies."""
+    """A short list in page-locked memory is written by a kernel, any other through the copies."""
     rows, count = torch.randn(3, 40, 7, device="cuda"), torch.tensor([5, 40, 0], dtype=torch.int32, device="cuda")
     host = torch.full((3, 33, 7), -1.0, pin_memory=pinned)
     host_count = torch.full((3,), -1, dtype=torch.int32, pin_memory=pinned)
@@ -201,6 +201,20 @@ def test_rows_that_are_not_the_current_devices_go_by_copies(side):
             capi.check(call(stream.cuda_stream), "xnor_b200_rows_to_host")
             torch.cuda.synchronize()
             assert torch.equal(host, rows) and torch.equal(host_count, count)
+
+
+@pytest.mark.parametrize("batch,take,kernels", [(1, 4096, 1), (16, 585, 1), (16, 586, 0), (64, 512, 0)])
+def test_long_lists_go_by_copies(batch, take, kernels):
+    """Up to 256 KB (16 images of 585 rows: 262080 bytes) by a kernel; beyond, by the copy engine, beside which the SMs are free."""
+    rows, count = torch.randn(batch, 4096, 7, device="cuda"), torch.arange(batch, dtype=torch.int32, device="cuda")
+    host, host_count = torch.zeros(batch, take, 7, pin_memory=True), torch.zeros(batch, dtype=torch.int32, pin_memory=True)
+
+    def call(stream):
+        return capi.lib().xnor_b200_rows_to_host(rows.data_ptr(), 4096, count.data_ptr(), batch, take, host.data_ptr(), host_count.data_ptr(), stream)
+    assert recorded_kernels(call) == kernels
+    capi.check(call(torch.cuda.current_stream().cuda_stream), "xnor_b200_rows_to_host")
+    torch.cuda.synchronize()
+    assert torch.equal(host, rows[:, :take].cpu()) and torch.equal(host_count, count.cpu())
 
 
 def test_a_failed_call_is_reported_once():
