@@ -107,7 +107,8 @@ __device__ __forceinline__ bool overlap_exceeds(const float4 a, const float4 b, 
 	if (w <= 0.0f || h <= 0.0f || inter == 0.0f) { return 0.0f > thresh; }
 	const float uni = __fsub_rn(__fadd_rn(__fmul_rn(a.z, a.w), __fmul_rn(b.z, b.w)), inter);
 	const float line = thresh * uni;
-	if (line > 1e-30f)
+	// (a quotient near a threshold that is nearly subnormal rounds by more than the margin; thresholds and unions below zero meet as a line above it)
+	if (thresh > 1e-30f && line > 1e-30f)
 	{
 		if (inter > line * 1.000001f) { return true; }
 		if (inter < line * 0.999999f) { return false; }

@@ -126,6 +126,24 @@ def test_detect_at_the_lines_of_the_overlap_matrix(tmp_path, found):
         assert np.array_equal(dets.probs[0, :found].cpu().numpy(), probs)
 
 
+@pytest.mark.parametrize("boxes,thresh", [
+    ([(1e6, 1e6, 0.07, 0.07)] * 2, -0.5),                                   # far out: the intersection rounds to more than both, their union below 0
+    ([(1e6, 1e6, 0.07, 0.07), (5, 5, 1, 1), (5.2, 5, 1, 1)], -3.0),
+    ([(0, 0, 1e8, 1e8), (0, 0, 1e-14, 1e-14)], 7 * 2.0 ** -149),            # 7.1 units of the smallest value, which rounds to seven
+    ([(5, 5, 1, 1), (5.2, 5, 1, 1), (5.9, 5, 1, 1), (9, 9, 1, 1)], 0.0),
+])
+def test_suppression_at_odd_thresholds(boxes, thresh):
+    n = len(boxes)
+    dets = network.DetectionBuffers(1, 1, max_dets=8, max_rows=8)
+    dets.boxes[0, :n], dets.objectness[0, :n] = torch.tensor(boxes), 1.0
+    dets.probs[0, :n, 0] = torch.linspace(0.9, 0.5, n)
+    dets.count.fill_(n)
+    want, _ = expected_rows(*(t[0, :n].cpu().numpy() for t in (dets.boxes, dets.objectness, dets.probs)), np.float32(thresh))
+    network.do_nms_sort(dets, float(np.float32(thresh)))
+    network.detection_rows(dets)
+    assert np.array_equal(dets.rows_host()[0], want)
+
+
 @pytest.mark.parametrize("pinned", [True, False])
 def test_rows_to_host_into_either_kind_of_memory(pinned):
     """A short list in page-locked memory is written by a kernel, any other through the copies."""
