@@ -144,6 +144,76 @@ def test_suppression_at_odd_thresholds(boxes, thresh):
     assert np.array_equal(dets.rows_host()[0], want)
 
 
+def sparse_heads(found, size, crowd=0, classes=80, at=17):
+    """Activated heads of one image with `found` detections of about one class each, and `crowd` of them of class `at` too."""
+    g = torch.Generator().manual_seed(found + crowd)
+    heads = [torch.rand(1, 3, 5 + classes, hw, hw, generator=g) * 0.3 for hw in (size // 32, size // 16)]
+    places = torch.randperm(sum(h[:, :, 4].numel() for h in heads), generator=g)[:found]
+    obj, extra = (torch.zeros(sum(h[:, :, 4].numel() for h in heads)) for _ in range(2))
+    obj[places], extra[places[:crowd]] = 0.9, 0.6
+    parts = [h[:, :, 4].numel() for h in heads]
+    for h, o, e in zip(heads, obj.split(parts), extra.split(parts)):
+        h[:, :, 4] = o.view_as(h[:, :, 4]) + 0.1 * torch.rand(h[:, :, 4].shape, generator=g)
+        h[:, :, 5:] += 0.6 * (torch.rand(h[:, :, 5:].shape, generator=g) < 1 / classes)
+        h[:, :, 5 + at] = 0.3 * torch.rand(h[:, :, 4].shape, generator=g) + e.view_as(h[:, :, 4])
+    return [h.reshape(1, -1, *h.shape[3:]).cuda().contiguous() for h in heads]
+
+
+def class_cfg(tmp_path, size, classes):
+    cfg = tmp_path / f"net{classes}.cfg"
+    cfg.write_text(cfgs.yolov3_tiny_xnor_cfg(size, size).replace("classes=80", f"classes={classes}").replace("filters=255", f"filters={3 * (5 + classes)}"))
+    return network.parse_network_cfg(str(cfg), 1, "cuda:0")
+
+
+@pytest.mark.parametrize("classes", [80, 140])
+@pytest.mark.parametrize("found,crowd", [(256, 2), (257, 2), (300, 31), (300, 32), (300, 33), (300, 34), (700, 32), (700, 200), (768, 30)])
+def test_detect_of_classes_with_few_candidates(tmp_path, found, crowd, classes):
+    """More than 256 detections: up to 32 candidates in every class the overlaps are those of each class, else of all pairs; more than 128
+    classes come in rounds, of which the first may be without and the next with the matrix."""
+    size, max_dets = 256, 768
+    net = class_cfg(tmp_path, size, classes)
+    at = 17 if classes == 80 else 135                               # of 140 in the second round
+    heads = sparse_heads(found, size, crowd, classes, at)
+    apart = network.DetectionBuffers(1, classes, max_dets=max_dets, max_rows=20000)
+    network.get_network_boxes(net, heads, size, size, 0.5, apart)
+    torch.cuda.synchronize()
+    assert int(apart.count.cpu()[0]) == found
+    boxes, obj, probs = (t.cpu().numpy()[0, :found].copy() for t in (apart.boxes, apart.objectness, apart.probs))
+    members = (probs > 0).sum(0)
+    assert members[at] == crowd and np.delete(members, at).max() <= 32
+    want, kept = expected_rows(boxes, obj, probs, 0.45)
+    fused = network.DetectionBuffers(1, classes, max_dets=max_dets, max_rows=20000)
+    network.detect(net, heads, size, size, 0.5, 0.45, fused)
+    network.do_nms_sort(apart, 0.45)
+    network.detection_rows(apart)
+    for dets in (fused, apart):
+        assert np.array_equal(dets.rows_host()[0], want)
+        assert np.array_equal(dets.probs[0, :found].cpu().numpy(), kept)
+
+
+def test_few_candidates_a_class_take_no_longer_with_a_list_that_fits_the_matrix(tmp_path):
+    """760 detections of one class each: no slower than by the lists that serve 776 of them (with all pairs formed it was 1.6 times)."""
+    net = class_cfg(tmp_path, 416, 80)
+    times = []
+    for found in (760, 776):
+        heads, dets = sparse_heads(found, 416), network.DetectionBuffers(1, 80)
+        network.detect(net, heads, 416, 416, 0.5, 0.45, dets)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                network.detect(net, heads, 416, 416, 0.5, 0.45, dets)
+        best = float("inf")
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[0] <= 1.15 * times[1], times
+
+
 @pytest.mark.parametrize("pinned", [True, False])
 def test_rows_to_host_into_either_kind_of_memory(pinned):
     """A short list in page-locked memory is written by a kernel, any other through the copies."""
