@@ -42,6 +42,7 @@ constexpr int DET_SMEM_BUDGET = 192 * 1024;
 constexpr int DET_SMEM_HALF = 104 * 1024; // two CTAs on an SM, as many as their registers allow,
 constexpr int DET_SMEM_SHARED = 72 * 1024; // and the matrix of one of them: what it takes more is missing as cache
 constexpr int DET_MATRIX_MAX = 768;       // detections whose overlaps are kept as a bit matrix (72 KB of shared memory)
+constexpr int DET_MATRIX_WORDS = DET_MATRIX_MAX / 32;    // of a row, also of fewer (a length that is a parameter costs 3 to 5 % of a crowded list)
 // Up to so many detections the matrix costs less than asking whether it is worth it; beyond, only where a class has more than DET_FEW candidates
 constexpr int DET_MATRIX_SURE = 256;
 constexpr int DET_FEW = 32;
@@ -74,7 +75,6 @@ struct DetectParams
 	int nms;
 	float nms_thresh;
 	int matrix_max;              // detections up to which the overlap matrix is used: at most min(max_dets, DET_MATRIX_MAX)
-	int matrix_words;            // of a row of it
 	int lists, matrix_lists;     // per-class candidate lists that fit a CTA's shared memory (at most one per warp), without and with the matrix
 	// compaction (rows != nullptr)
 	float * rows;                // [batch][max_rows][7]
@@ -265,7 +265,7 @@ __device__ __forceinline__ int gather_class(const DetectParams & p, int n, const
 // overlapped, and its own row of the overlap matrix added where it is kept.  Lane l holds the bits of detections 32 l ...; returns them.
 // Overlaps are symmetric and a kept detection overlaps no kept one before it, so a row marks nothing that was kept.  The rows of four
 // ranks are read ahead: a step is a shuffle and a few logical operations, about 40 cycles.
-__device__ __forceinline__ uint32_t walk_class(int m, int words, int row_words, const uint16_t * s_order, const uint32_t * s_over)
+__device__ __forceinline__ uint32_t walk_class(int m, int words, const uint16_t * s_order, const uint32_t * s_over)
 {
 	const int lane = threadIdx.x & 31;
 	uint32_t dead = 0;
@@ -277,7 +277,7 @@ __device__ __forceinline__ uint32_t walk_class(int m, int words, int row_words, 
 		for (int j = 0; j < 4; ++j)
 		{
 			d[j] = s_order[min(r0 + j, m - 1)];
-			row[j] = (lane < words) ? s_over[d[j] * row_words + lane] : 0u;
+			row[j] = (lane < words) ? s_over[d[j] * DET_MATRIX_WORDS + lane] : 0u;
 		}
 		#pragma unroll
 		for (int j = 0; j < 4; ++j)
@@ -493,7 +493,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 	{
 		float4 * s_box = reinterpret_cast<float4 *>(s_rows + ((p.matrix_max + 3) & ~3));
 		uint32_t * s_over = reinterpret_cast<uint32_t *>(s_box + p.matrix_max);
-		float * s_lists = reinterpret_cast<float *>(s_over + p.matrix_max * p.matrix_words);
+		float * s_lists = reinterpret_cast<float *>(s_over + p.matrix_max * DET_MATRIX_WORDS);
 		static_assert(DET_MATRIX_MAX <= 2 * DET_THREADS, "two boxes a thread");
 		float4 box[2];                                           // (stored behind the first gathering, whose loads wait beside these)
 		#pragma unroll
@@ -567,7 +567,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 					const int r = i / words, w = i - r * words, c = w * 32 + lane;
 					const bool over = (c < n && c != r) && overlap_exceeds(s_box[r], s_box[c], p.nms_thresh);
 					const uint32_t bits = __ballot_sync(0xffffffffu, over);
-					if (lane < DET_CLUSTER) { *cluster.map_shared_rank(s_over + r * p.matrix_words + w, lane) = bits; }
+					if (lane < DET_CLUSTER) { *cluster.map_shared_rank(s_over + r * DET_MATRIX_WORDS + w, lane) = bits; }
 				}
 			}
 			if (m <= DET_RANK_MAX)
@@ -588,7 +588,7 @@ detect_kernel(const __grid_constant__ DetectParams p)
 			formed = true;
 			if (m > 0)
 			{
-				const uint32_t dead = walk_class(m, words, p.matrix_words, s_order, s_over);
+				const uint32_t dead = walk_class(m, words, s_order, s_over);
 				for (int c0 = 0; c0 < m; c0 += 32)
 				{
 					const int d = s_idx[min(c0 + lane, m - 1)];
@@ -864,10 +864,9 @@ static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int b
 		// half an SM has, 30 / 37 / 47 so; 33 / 39 / 49 before there was a matrix)
 		const bool shared = (long long)batch * DET_CLUSTER > sm_count() && smem <= DET_SMEM_HALF;
 		const size_t room = shared ? max(smem, (size_t)DET_SMEM_SHARED) : DET_SMEM_BUDGET;
-		auto matrix_bytes = [&](int max) { return round_up((size_t)max, 4) * 4 + (size_t)max * (sizeof(float4) + (max + 31) / 32 * 4 + (size_t)want * DET_LIST_BYTES); };
+		auto matrix_bytes = [&](int max) { return round_up((size_t)max, 4) * 4 + (size_t)max * (sizeof(float4) + DET_MATRIX_WORDS * 4 + (size_t)want * DET_LIST_BYTES); };
 		p.matrix_max = min(p.max_dets, DET_MATRIX_MAX);
 		while (matrix_bytes(p.matrix_max) > room) { p.matrix_max = (p.matrix_max - 1) & ~31; }
-		p.matrix_words = (p.matrix_max + 31) / 32;
 		if (p.matrix_max >= p.max_dets) { smem = (size_t)list_bytes; }             // no list goes without it
 		smem = max(smem, matrix_bytes(p.matrix_max));
 	}

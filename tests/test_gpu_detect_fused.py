@@ -268,7 +268,7 @@ def test_many_images_share_the_sms(tmp_path, batch, max_dets, ctas):
     assert ctas * (kernel.shared + static + reserved) <= 228 * 1024
 
 
-@pytest.mark.parametrize("found", [416, 447, 448, 449, 480, 700])
+@pytest.mark.parametrize("found", [256, 351, 352, 353, 384, 700])
 def test_detect_at_the_lines_of_many_images(tmp_path, found):
     """Where the matrix is smaller, since two CTAs share an SM: the list of each image is what it is alone."""
     size, batch, max_dets = 256, 19, 700
