@@ -45,7 +45,7 @@ constexpr int DET_MATRIX_MAX = 768;       // detections whose overlaps are kept 
 constexpr int DET_MATRIX_WORDS = DET_MATRIX_MAX / 32;    // of a row, also of fewer (a length that is a parameter costs 3 to 5 % of a crowded list)
 // Up to so many detections the matrix costs less than asking whether it is worth it; beyond, only where a class has more than DET_FEW candidates
 constexpr int DET_MATRIX_SURE = 256;
-constexpr int DET_FEW = 32;
+constexpr int DET_FEW = 96;
 constexpr int DET_RANK_MAX = 128;         // candidates of one class that a warp ranks by itself; more go to the whole CTA
 constexpr int DET_WARP_MAX = 64;          // without the matrix: candidates of one class that a warp suppresses by itself
 constexpr int DET_BLOCK = 128;            // ranks the CTA settles at a time
@@ -289,21 +289,31 @@ __device__ __forceinline__ uint32_t walk_class(int m, int words, const uint16_t 
 	return dead;
 }
 
-// The same for a class of at most DET_FEW candidates without the matrix: lane l holds the box of rank l.  Returns the bits of the ranks to go;
-// s_order has the detections in rank order.
+// The same for a class of at most DET_FEW candidates without the matrix: lane l holds the boxes of ranks l, l + 32, l + 64 and returns, as bits,
+// which of them go; s_order has the detections in rank order.
+constexpr int DET_FEW_LANE = DET_FEW / 32;
+
 __device__ __forceinline__ uint32_t suppress_few(int m, const float * s_score, const uint16_t * s_idx, uint16_t * s_order, const float4 * s_box, float thresh)
 {
 	const int lane = threadIdx.x & 31;
-	if (lane < m) { s_order[score_rank(s_score, m, lane)] = s_idx[lane]; }
+	for (int c = lane; c < m; c += 32) { s_order[score_rank(s_score, m, c)] = s_idx[c]; }
 	__syncwarp();
-	const float4 box = s_box[s_order[min(lane, m - 1)]];
+	float4 box[DET_FEW_LANE];
+	#pragma unroll
+	for (int j = 0; j < DET_FEW_LANE; ++j) { box[j] = s_box[s_order[min(j * 32 + lane, m - 1)]]; }
 	uint32_t gone = 0;
 	for (int r = 0; r < m - 1; ++r)
 	{
-		if ((gone >> r) & 1u) { continue; }
-		const float4 a = make_float4(__shfl_sync(0xffffffffu, box.x, r), __shfl_sync(0xffffffffu, box.y, r), __shfl_sync(0xffffffffu, box.z, r),
-				__shfl_sync(0xffffffffu, box.w, r));
-		gone |= __ballot_sync(0xffffffffu, lane > r && lane < m && overlap_exceeds(a, box, thresh));
+		const uint32_t owner = __shfl_sync(0xffffffffu, gone, r & 31);
+		if ((owner >> (r >> 5)) & 1u) { continue; }
+		const float4 a = s_box[s_order[r]];
+		#pragma unroll
+		for (int j = 0; j < DET_FEW_LANE; ++j)
+		{
+			if (j * 32 >= m) { break; }
+			const int r2 = j * 32 + lane;
+			if (r2 > r && r2 < m && overlap_exceeds(a, box[j], thresh)) { gone |= 1u << j; }
+		}
 	}
 	return gone;
 }
@@ -545,10 +555,10 @@ detect_kernel(const __grid_constant__ DetectParams p)
 				if (m > 0)
 				{
 					const uint32_t gone = suppress_few(m, s_score, s_idx, s_order, s_box, p.nms_thresh);
-					if (lane < m)
+					for (int j = 0; j * 32 + lane < m; ++j)
 					{
-						const int d = s_order[lane];
-						if ((gone >> lane) & 1u) { probs[(size_t)d * p.classes + k] = 0.0f; }
+						const int d = s_order[j * 32 + lane];
+						if ((gone >> j) & 1u) { probs[(size_t)d * p.classes + k] = 0.0f; }
 						else
 						{
 							#pragma unroll

@@ -166,9 +166,9 @@ def class_cfg(tmp_path, size, classes):
 
 
 @pytest.mark.parametrize("classes", [80, 140])
-@pytest.mark.parametrize("found,crowd", [(256, 2), (257, 2), (300, 31), (300, 32), (300, 33), (300, 34), (700, 32), (700, 200), (768, 30)])
+@pytest.mark.parametrize("found,crowd", [(256, 2), (257, 2), (300, 32), (300, 33), (300, 64), (300, 65), (300, 95), (300, 96), (300, 97), (700, 96), (700, 200), (768, 30)])
 def test_detect_of_classes_with_few_candidates(tmp_path, found, crowd, classes):
-    """More than 256 detections: up to 32 candidates in every class the overlaps are those of each class, else of all pairs; more than 128
+    """More than 256 detections: up to 96 candidates in every class the overlaps are those of each class, else of all pairs; more than 128
     classes come in rounds, of which the first may be without and the next with the matrix."""
     size, max_dets = 256, 768
     net = class_cfg(tmp_path, size, classes)
