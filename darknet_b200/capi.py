@@ -28,7 +28,7 @@ EXPORTS = (
     "xnor_b200_pack_input_pooled", "xnor_b200_conv_forward_pooled", "xnor_b200_float_conv_small", "xnor_b200_float_conv3_io", "xnor_b200_float_conv_map_weights_bytes",
     "xnor_b200_float_conv_map_prepare", "xnor_b200_float_conv_map", "xnor_b200_float_conv_map_yolo", "xnor_b200_float_conv_1x1_tc", "xnor_b200_yolo_activate", "xnor_b200_region_activate", "xnor_b200_conv_forward_io", "xnor_b200_conv_takes_masks", "xnor_b200_tap_major_weights",
     "xnor_b200_yolo_detections", "xnor_b200_nms_sort", "xnor_b200_detection_rows", "xnor_b200_detect", "xnor_b200_rows_to_host",
-    "xnor_b200_avgpool", "xnor_b200_softmax", "xnor_b200_run_ops", "xnor_b200_float_conv3_words", "xnor_b200_float_conv_tc", "xnor_b200_float_conv_tc_prepare", "xnor_b200_float_conv_tc_weights_bytes", "xnor_b200_conv_words", "xnor_b200_conv_words_plan", "xnor_b200_conv_words_weights", "xnor_b200_conv_words_weights_bytes", "xnor_b200_sign_words", "xnor_b200_grid_block_words", "xnor_b200_grid_front",
+    "xnor_b200_avgpool", "xnor_b200_softmax", "xnor_b200_run_ops", "xnor_b200_float_conv3_words", "xnor_b200_float_conv_tc", "xnor_b200_float_conv_tc_launches", "xnor_b200_float_conv_tc_prepare", "xnor_b200_float_conv_tc_weights_bytes", "xnor_b200_conv_words", "xnor_b200_conv_words_plan", "xnor_b200_conv_words_weights", "xnor_b200_conv_words_weights_bytes", "xnor_b200_sign_words", "xnor_b200_grid_block_words", "xnor_b200_grid_front",
     "xnor_b200_measure_popc_peak", "xnor_b200_measure_bmma_peak", "xnor_b200_measure_umma_i8_peak", "xnor_b200_measure_umma_mxf4_peak",
 )
 
@@ -166,6 +166,7 @@ def lib() -> C.CDLL:
     L.xnor_b200_float_conv_tc_weights_bytes.restype = sz
     L.xnor_b200_float_conv_tc_weights_bytes.argtypes = [dp]
     L.xnor_b200_float_conv_tc_prepare.argtypes = [dp, vp, vp, vp]
+    L.xnor_b200_float_conv_tc_launches.argtypes = [dp]
     L.xnor_b200_float_conv_tc.argtypes = [dp, vp, vp, vp, vp, ci, vp]
     L.xnor_b200_float_conv3_words.argtypes = [dp, ci, vp, vp, vp, vp, ci, vp]
     L.xnor_b200_conv_takes_masks.argtypes = [dp]

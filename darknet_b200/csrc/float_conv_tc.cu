@@ -485,6 +485,22 @@ static bool ft_shape_ok(const xnor_b200_conv_desc * d)
 	return d->stride == 1 && ((d->size == 1 && d->pad == 0) || (d->size == 3 && d->pad == 1 && d->c % 32 == 0));
 }
 
+// What of the parameters follows from the shape; tiles of 128 pixels and 128 filters
+static int ft_shape(const xnor_b200_conv_desc & d, FtParams & p, long long & total, long long & tiles)
+{
+	total = (long long)d.batch * d.h * d.w;
+	if (total > 0x7fffffffLL - TC_PIX) { return XNOR_B200_ERR_TOO_LARGE; }
+	p.C = d.c; p.H = d.h; p.W = d.w; p.HW = d.h * d.w; p.N = d.n;
+	p.total = (int)total;
+	p.taps = d.size * d.size;
+	p.cblocks = (d.c + 31) / 32;
+	p.kblocks = p.taps * p.cblocks;
+	p.leaky = (d.activation == XNOR_B200_LEAKY) ? 1 : 0;
+	p.tiles_f = (d.n + FT_NF - 1) / FT_NF;
+	tiles = (long long)p.tiles_f * ((total + TC_PIX - 1) / TC_PIX);
+	return (tiles * FT_MAX_SPLIT > 0x7fffffffLL) ? XNOR_B200_ERR_TOO_LARGE : XNOR_B200_OK;
+}
+
 template <bool RAW>
 static int launch_float_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights, const float * biases, float * output,
 		int yolo_entries, cudaStream_t stream)
@@ -495,25 +511,17 @@ static int launch_float_tc(const xnor_b200_conv_desc * desc, const float * input
 	if (!ft_shape_ok(desc)) { return XNOR_B200_ERR_INVALID; }
 	if (yolo_entries < 0 || (yolo_entries > 0 && (yolo_entries < 5 || desc->n % yolo_entries != 0))) { return XNOR_B200_ERR_INVALID; }
 	if (!RAW && ((uintptr_t)weights & 15u) != 0) { return XNOR_B200_ERR_ALIGNMENT; }
-	const long long total = (long long)desc->batch * desc->h * desc->w;
-	if (total > 0x7fffffffLL - TC_PIX) { return XNOR_B200_ERR_TOO_LARGE; }
 	FtParams p;
+	long long total = 0, tiles = 0;
+	rc = ft_shape(*desc, p, total, tiles);
+	if (rc != XNOR_B200_OK) { return rc; }
 	p.x = input; p.w = weights; p.bias = biases; p.out = output;
-	p.C = desc->c; p.H = desc->h; p.W = desc->w; p.HW = desc->h * desc->w; p.N = desc->n;
-	p.total = (int)total;
-	p.taps = desc->size * desc->size;
-	p.cblocks = (desc->c + 31) / 32;
-	p.kblocks = p.taps * p.cblocks;
 	p.yolo_entries = yolo_entries;
-	p.leaky = (desc->activation == XNOR_B200_LEAKY) ? 1 : 0;
-	p.tiles_f = (desc->n + FT_NF - 1) / FT_NF;
 	TcParams tp = TcParams();
 	rc = tc_fill_launch_fields(tp);
 	if (rc != XNOR_B200_OK) { return rc; }
 	p.status = tp.status;
 	p.spin_limit = tp.spin_limit;
-	const long long tiles = (long long)p.tiles_f * ((total + TC_PIX - 1) / TC_PIX);
-	if (tiles * FT_MAX_SPLIT > 0x7fffffffLL) { return XNOR_B200_ERR_TOO_LARGE; }
 	// as many CTAs per tile as leave the grid one wave and each of them a few K blocks (about 3 us go into joining the sums)
 	p.split = 1;
 	for (int s = 2; s <= FT_MAX_SPLIT; ++s) { if (tiles * s <= sm_count() && p.kblocks >= 4 * s) { p.split = s; } }
@@ -566,6 +574,14 @@ extern "C" int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const f
 		const float * biases, float * output, int yolo_entries, void * stream)
 {
 	return launch_float_tc<false>(desc, input, tc_weights, biases, output, yolo_entries, (cudaStream_t)stream);
+}
+
+extern "C" int xnor_b200_float_conv_tc_launches(const xnor_b200_conv_desc * desc)
+{
+	FtParams p;
+	long long total = 0, tiles = 0;
+	if (desc == nullptr || validate_desc(desc) != XNOR_B200_OK || !ft_shape_ok(desc) || ft_shape(*desc, p, total, tiles) != XNOR_B200_OK) { return 0; }
+	return (total > 1024) ? float_tcp_launches(tiles, p.kblocks) : 1;
 }
 
 extern "C" int xnor_b200_float_conv_1x1_tc(const xnor_b200_conv_desc * desc, const float * input, const float * weights,

@@ -475,15 +475,25 @@ static int launch_tiles(const FtParams & p, cudaStream_t stream, bool behind = f
 }
 
 // Whole rounds of the SMs first; what is left of the tiles (all, if they are fewer than the SMs) with its K blocks dealt to as many CTAs a
-// tile as there is room for, four K blocks each at least (about 3 us go into joining the sums).
+// tile as there is room for, four K blocks each at least (about 3 us go into joining the sums).  How many CTAs that is; 1: one launch for all.
+static int rest_split(int all, int kblocks)
+{
+	const int rest = all % sm_count();
+	int split = 1;
+	for (int s = 2; s <= FT_MAX_SPLIT; ++s) { if (rest * s <= sm_count() && kblocks >= 4 * s) { split = s; } }
+	return (rest == 0 || (all > rest && kblocks < FP_REST_KBLOCKS)) ? 1 : split;
+}
+
+int float_tcp_launches(long long tiles, int kblocks)
+{
+	return (tiles >= sm_count() && rest_split((int)tiles, kblocks) > 1) ? 2 : 1;
+}
+
 int launch_float_tcp(FtParams & p, cudaStream_t stream)
 {
 	const long long tiles = (long long)p.tiles_f * ((p.total + (long long)TC_PIX - 1) / TC_PIX);
 	if (tiles * FT_MAX_SPLIT > 0x7fffffffLL || tiles / sm_count() * p.kblocks > 0x7ffffff0LL) { return XNOR_B200_ERR_TOO_LARGE; }
-	const int all = (int)tiles, rest = all % sm_count();
-	int split = 1;
-	for (int s = 2; s <= FT_MAX_SPLIT; ++s) { if (rest * s <= sm_count() && p.kblocks >= 4 * s) { split = s; } }
-	if (all > rest && p.kblocks < FP_REST_KBLOCKS) { split = 1; }
+	const int all = (int)tiles, rest = all % sm_count(), split = rest_split(all, p.kblocks);
 	p.tile0 = 0;
 	p.split = 1;
 	p.more = 0;
@@ -491,7 +501,7 @@ int launch_float_tcp(FtParams & p, cudaStream_t stream)
 	// filter tile may be narrower, and those that had no other would finish early (3x3 512 -> 144 on 128 of 13x13 252 -> 240 us, 1x1 1024 -> 425 on
 	// 256 of them 244 -> 240; narrow tiles all at the end instead: 244 and 254, a tile's pixels then come from memory twice).
 	p.turn = (sm_count() % p.tiles_f == 0) ? sm_count() : 0x7fffffff;
-	if (rest == 0 || split == 1)
+	if (split == 1)
 	{
 		p.tiles = all;
 		return launch_tiles(p, stream);

@@ -73,5 +73,7 @@ __device__ __forceinline__ float ft_activate(const FtParams & p, float sum, floa
 
 // float_conv_tcp.cu: prepared filters, any number of pixels
 int launch_float_tcp(FtParams & p, cudaStream_t stream);
+// Kernels that it launches for so many tiles
+int float_tcp_launches(long long tiles, int kblocks);
 
 }  // namespace xnor

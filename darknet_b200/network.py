@@ -731,10 +731,14 @@ def prepare_float_map_convs(net: Network) -> None:
                                                               torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_map_prepare")
 
 
+def _float_conv_tc_desc(l: Layer, batch: int) -> capi.ConvDesc:
+    return capi.ConvDesc(batch, l.c, l.h, l.w, l.n, l.size, 1, l.pad, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
+
+
 def _float_conv_tc(l: Layer, x: torch.Tensor) -> torch.Tensor:
     """1x1 or 3x3 stride-1 float convolution + bias + leaky/linear through xnor_b200_float_conv_tc."""
     import ctypes as C
-    desc = capi.ConvDesc(x.shape[0], l.c, l.h, l.w, l.n, l.size, 1, l.pad, capi.LEAKY if l.activation == "leaky" else capi.LINEAR)
+    desc = _float_conv_tc_desc(l, x.shape[0])
     out = torch.empty(x.shape[0], l.n, l.out_h, l.out_w, dtype=torch.float32, device=x.device)
     capi.check(capi.lib().xnor_b200_float_conv_tc(C.byref(desc), x.data_ptr(), l.weights_tc_gpu.data_ptr(), l.biases_gpu.data_ptr(),
                                                  out.data_ptr(), 0, torch.cuda.current_stream().cuda_stream), "xnor_b200_float_conv_tc")
@@ -1105,10 +1109,14 @@ def load_network_custom(cfg: str, weights: str, batch: int = 1, device: str = "c
 
 
 def own_launches_per_forward(net: Network) -> int:
-    """Kernels of libxnor_b200.so that one forward launches, after every fusion that load_network_custom set up (a float convolution counts
-    once, also where the last tiles of a batch are a launch of their own)."""
+    """Kernels of libxnor_b200.so that one forward launches, after every fusion that load_network_custom set up."""
+    import ctypes as C
+
+    def float_launches(desc):
+        return capi.lib().xnor_b200_float_conv_tc_launches(C.byref(desc))
     if net.plan is not None:
-        return sum(1 for op in net.plan.ops if op.kind not in (capi.OP_FORK, capi.OP_BACK, capi.OP_MARK))
+        return sum(float_launches(op.desc) if op.kind == capi.OP_FLOAT_TC else 1
+                   for op in net.plan.ops if op.kind not in (capi.OP_FORK, capi.OP_BACK, capi.OP_MARK))
     n = 0
     for l in net.layers:
         if l.type == "convolutional":
@@ -1120,7 +1128,7 @@ def own_launches_per_forward(net: Network) -> int:
             elif (l.c == 3 and l.size == 3 and l.stride == 1 and l.pad == 1) or l.c * l.size * l.size <= 128 or l.weights_blocked_gpu is not None:
                 n += 1
             elif l.weights_tc_gpu is not None:
-                n += 1                                    # tensor-core float convolution
+                n += float_launches(_float_conv_tc_desc(l, net.batch))
         elif (l.type == "yolo" and not l.yolo_done) or l.type in ("region", "avgpool", "softmax"):
             n += 1
     return n

@@ -410,6 +410,8 @@ XNOR_B200_API size_t xnor_b200_float_conv_tc_weights_bytes(const xnor_b200_conv_
 XNOR_B200_API int xnor_b200_float_conv_tc_prepare(const xnor_b200_conv_desc * desc, const float * weights, float * tc_weights, void * stream);
 XNOR_B200_API int xnor_b200_float_conv_tc(const xnor_b200_conv_desc * desc, const float * input, const float * tc_weights,
 		const float * biases, float * output, int yolo_entries, void * stream);
+/* Kernels that such a call launches on the current device (0: a shape it does not take): the last tiles of a batch may be one of their own. */
+XNOR_B200_API int xnor_b200_float_conv_tc_launches(const xnor_b200_conv_desc * desc);
 /* Same, for the convolution right in front of a [yolo] layer: yolo_entries = 4 + 1 + classes (n must be a multiple of
  * it) also applies that layer's activation step (xnor_b200_yolo_activate below) to the result; 0 = plain call. */
 XNOR_B200_API int xnor_b200_float_conv_map_yolo(const xnor_b200_conv_desc * desc, const float * input, const float * blocked_weights,

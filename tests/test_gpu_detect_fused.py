@@ -10,6 +10,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 from darknet_b200 import capi, cfgs, network  # noqa: E402
+from recorded import graph_kernels  # noqa: E402
 
 
 def iou(a, b):
@@ -226,27 +227,15 @@ def test_rows_to_host_into_either_kind_of_memory(pinned):
     assert torch.equal(host, rows[:, :33].cpu()) and torch.equal(host_count, count.cpu())
 
 
-class KernelNode(C.Structure):
-    _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("shared", C.c_uint), ("params", C.c_void_p), ("extra", C.c_void_p),
-                ("kern", C.c_void_p), ("ctx", C.c_void_p)]
-
-
 def recorded_kernels(call):
     """Kernels that `call(stream)` records into a graph, which is not run."""
-    cu, n, graph, stream = C.CDLL("libcuda.so.1"), C.c_size_t(0), C.c_void_p(), torch.cuda.Stream()
+    cu, graph, stream = C.CDLL("libcuda.so.1"), C.c_void_p(), torch.cuda.Stream()
     handle = C.c_void_p(stream.cuda_stream)
     assert cu.cuStreamBeginCapture_v2(handle, 2) == 0
     call(stream.cuda_stream)
     if cu.cuStreamEndCapture(handle, C.byref(graph)) != 0:          # what the call did cannot be recorded: no kernel, then
         return []
-    assert cu.cuGraphGetNodes(graph, None, C.byref(n)) == 0
-    nodes, kernels, kind = (C.c_void_p * n.value)(), [], C.c_int(-1)
-    assert n.value == 0 or cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0
-    for node in nodes:
-        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
-        if kind.value == 0:
-            kernels.append(KernelNode())
-            assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(kernels[-1])) == 0
+    kernels = graph_kernels(graph)
     assert cu.cuGraphDestroy(graph) == 0
     return kernels
 

@@ -10,6 +10,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 from darknet_b200 import capi, cfgs, network  # noqa: E402
+from recorded import graph_kernels  # noqa: E402
 
 YOLO = "[yolo]\nmask = 0,1,2\nanchors = 10,14, 23,27, 37,58\nclasses=3\nnum=3\n"
 HEAD = cfgs._conv(24, 1, bn=0, activation="linear")
@@ -215,3 +216,20 @@ def test_the_layer_loop_still_hands_signs_on(name, batch, tmp_path):
     net.plan = None
     for _ in range(2):
         assert_heads_close(network.forward_network_gpu(net, x), want)
+
+
+@pytest.mark.parametrize("name,batch", [("yolov3-tiny_xnor", 1), ("yolov3-tiny_xnor", 64), ("tiny-yolo_xnor", 64), ("darknet53_448_xnor", 2)])
+def test_launches_of_a_forward_are_counted(name, batch, tmp_path):
+    """Against the kernels of a captured forward; 3x3 256 -> 512 and 1x1 1024 -> 425 on 64 maps of 13x13 leave tiles for a launch of their own."""
+    cfg = tmp_path / "net.cfg"
+    size = 448 if name.startswith("darknet") else 416
+    cfg.write_text(cfgs.CFGS[name](size, size))
+    network.write_synthetic_weights(network.parse_network_cfg(str(cfg), 1, "cpu"), str(tmp_path / "w"), 1)
+    net = network.load_network_custom(str(cfg), str(tmp_path / "w"), batch)
+    x = image(batch, size, size)
+    network.forward_network_gpu(net, x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        network.forward_network_gpu(net, x)
+    assert len(graph_kernels(C.c_void_p(graph.raw_cuda_graph()))) == network.own_launches_per_forward(net)
