@@ -52,9 +52,9 @@ def test_prepared_filters_match_fp64(batch, c, h, w, n, size, leaky, entries):
     assert st.value == 0
 
 
-def prepared_conv(kind, desc, x, wt, b):
+def prepared_conv(kind, desc, x, wt, b, entries=0):
     lib, stream = capi.lib(), torch.cuda.current_stream().cuda_stream
-    call = {"tc": lambda *a: lib.xnor_b200_float_conv_tc(*a[:-1], 0, a[-1]), "map": lib.xnor_b200_float_conv_map}[kind]
+    call = {"tc": lambda *a: lib.xnor_b200_float_conv_tc(*a[:-1], entries, a[-1]), "map": lib.xnor_b200_float_conv_map}[kind]
     nbytes = getattr(lib, f"xnor_b200_float_conv_{kind}_weights_bytes")(C.byref(desc))
     assert nbytes
     prepared = torch.empty(nbytes // 4, device="cuda")
@@ -113,7 +113,8 @@ def test_error_of_batches(batch, c, h, w, n, size, bound):
     assert float((got.double() - want).norm() / want.norm()) <= bound
 
 
-@pytest.mark.parametrize("batch,c,h,w,n,size", [(2, 64, 9, 7, 140, 3), (9, 64, 13, 13, 33, 3), (2, 96, 9, 7, 140, 1), (64, 512, 13, 13, 32, 3)])
+@pytest.mark.parametrize("batch,c,h,w,n,size", [(2, 64, 9, 7, 140, 3), (9, 64, 13, 13, 33, 3), (2, 96, 9, 7, 140, 1), (64, 512, 13, 13, 32, 3),
+                                                (9, 96, 13, 13, 140, 1), (9, 300, 13, 13, 33, 1)])
 @pytest.mark.parametrize("leaky", [0, 1])
 def test_infinite_and_huge_values(batch, c, h, w, n, size, leaky):
     """Infinities and NaN come out where plain arithmetic puts them, and values next to the largest lose nothing."""
@@ -132,3 +133,22 @@ def test_infinite_and_huge_values(batch, c, h, w, n, size, leaky):
     assert torch.equal(got[got.isinf()], want32[want32.isinf()])
     fine = want32.isfinite()
     assert bool(((got[fine] - want32[fine]).abs() <= 2e-5 + 2e-5 * want32[fine].abs()).all())
+
+
+@pytest.mark.parametrize("batch,c,h,w,n,entries", [(2, 96, 9, 7, 34, 17), (9, 96, 13, 13, 34, 17), (9, 300, 13, 13, 255, 85)])
+def test_infinite_and_huge_values_behind_the_logistic(batch, c, h, w, n, entries):
+    """The [yolo] layer's step on values that are formed again: infinities become 0 and 1, but for width and height, and NaN stays."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(batch, c, h, w, generator=g, device="cuda")
+    wt = torch.randn(n, c, 1, 1, generator=g, device="cuda") * 0.05
+    b = torch.randn(n, generator=g, device="cuda")
+    x[0, 3, 1, 2], x[0, 5, 6, 6], x[1, 0, 0, 0], x[1, 7, 4, 3] = float("inf"), float("-inf"), float("nan"), 3.4e38
+    wt[2, 4], wt[3, 4], wt[5, 1] = float("inf"), float("-inf"), float("nan")
+    want = fp64(x, wt, b).float().double()                     # the sum leaves fp32 where 64 bits would hold it
+    logistic = torch.tensor([i not in (2, 3) for i in range(entries)] * (n // entries), device="cuda").view(1, n, 1, 1)
+    want = torch.where(logistic, torch.sigmoid(want), want).float()
+    got = prepared_conv("tc", capi.ConvDesc(batch, c, h, w, n, 1, 1, 0, capi.LINEAR), x, wt, b, entries)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and bool(want.isinf().any())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    assert bool(((got[fine] - want[fine]).abs() <= 2e-5 + 2e-5 * want[fine].abs()).all())
