@@ -61,16 +61,6 @@ __device__ __forceinline__ float plain_sum(const FtParams & p, int img, int pix,
 	return acc;
 }
 
-// The [yolo] layer's activation step or the convolution's own, behind the bias; entry: of the value's anchor (yolo_entries > 0)
-__device__ __forceinline__ float ft_activate(const FtParams & p, float sum, float bias, float slope, int entry)
-{
-	float v = __fadd_rn(sum, bias);
-	v = fmaxf(v, __fmul_rn(v, slope));
-	// logistic on every entry of an anchor but its width and height (head_activate.cu)
-	if (p.yolo_entries > 0 && entry != 2 && entry != 3) { v = 1.0f / (1.0f + expf(-v)); }
-	return v;
-}
-
 // float_conv_tcp.cu: prepared filters, any number of pixels
 int launch_float_tcp(FtParams & p, cudaStream_t stream);
 // Kernels that it launches for so many tiles
