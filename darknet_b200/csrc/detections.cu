@@ -135,9 +135,9 @@ __device__ __forceinline__ int score_rank(const float * s_score, int m, int c)
 	return rank;
 }
 
-// Lists of more than DET_MATRIX_MAX detections: greedy suppression of one class's m <= DET_WARP_MAX candidates by one warp.  The boxes go to shared memory in rank order, lane l
-// decides about ranks l, l + 32, ...; its verdicts stay in a register, so a step is one shuffle, one broadcast read and the
-// overlaps (reading order, score and box per step from memory took 600 cycles a candidate, this takes about 150).
+// Lists that the matrix has no room for: greedy suppression of one class's m <= DET_WARP_MAX candidates by one warp.  The boxes go to
+// shared memory in rank order, lane l decides about ranks l, l + 32, ...; its verdicts stay in a register, so a step is one shuffle, one
+// broadcast read and the overlaps (reading order, score and box per step from memory took 600 cycles a candidate, this takes about 150).
 __device__ __forceinline__ void suppress_warp(const DetectParams & p, int m, const float * s_score, const uint16_t * s_idx, uint16_t * s_order,
 		float4 * s_box, const float4 * boxes, float * probs, int k)
 {
@@ -167,8 +167,8 @@ __device__ __forceinline__ void suppress_warp(const DetectParams & p, int m, con
 	}
 }
 
-// The same for a crowded class of such a list, by the whole CTA, DET_BLOCK ranks at a time: every overlap inside the block at once as a bit
-// matrix, one warp walks the matrix in rank order (a step costs a shuffle), then the block's survivors are held against all later
+// The same for a crowded class of such a list, by the whole CTA, DET_BLOCK ranks at a time: every overlap inside the block at once as a
+// bit matrix, one warp walks the matrix in rank order (a step costs a shuffle), then the block's survivors are held against all later
 // ranks at once.  Step by step over the list, as a warp does it, 170 candidates took 45 us.
 __device__ __forceinline__ void suppress_cta(const DetectParams & p, int m, float * s_score, const uint16_t * s_idx, uint16_t * s_order,
 		const float4 * boxes, float * probs, int k)
@@ -293,7 +293,8 @@ __device__ __forceinline__ uint32_t walk_class(int m, int words, const uint16_t 
 // which of them go; s_order has the detections in rank order.
 constexpr int DET_FEW_LANE = DET_FEW / 32;
 
-__device__ __forceinline__ uint32_t suppress_few(int m, const float * s_score, const uint16_t * s_idx, uint16_t * s_order, const float4 * s_box, float thresh)
+__device__ __forceinline__ uint32_t suppress_few(int m, const float * s_score, const uint16_t * s_idx, uint16_t * s_order, const float4 * s_box,
+		float thresh)
 {
 	const int lane = threadIdx.x & 31;
 	for (int c = lane; c < m; c += 32) { s_order[score_rank(s_score, m, c)] = s_idx[c]; }
@@ -322,8 +323,9 @@ __device__ __forceinline__ uint32_t suppress_few(int m, const float * s_score, c
 // detections, so each step is a few microseconds of latency and the launches between them would cost as much again.  Work is
 // dealt to warps (a warp per detection, per class, per detection again), the scans that fix the order are short enough for every
 // CTA to do them all.  Values that another CTA of the cluster wrote are read past the L1 (__ldcg).
-// Measured at 416x416, 80 classes, one image: 237 us in four launches before (one CTA per image, a thread per detection walking the
-// classes at plane stride) at 174 detections and 843 rows, 48 us in one now; 14 us at 13 detections, 7 us at none.
+// Measured at 416x416, 80 classes, one image, in a CUDA graph, with the overlap matrix and without it (the candidates of each class held
+// against one another on the way): 174 detections and 883 rows 20.5 and 26.7 us, 13 detections and 61 rows 12.4 and 16.5, none 8.3; 300 /
+// 500 / 768 detections of five classes each 24.7 / 36.9 / 51.3 and 34.9 / 53.4 / 80.5, 174 of all 80 classes each 57 and 682.
 __global__ void __cluster_dims__(DET_CLUSTER, 1, 1) __launch_bounds__(DET_THREADS)
 detect_kernel(const __grid_constant__ DetectParams p)
 {
@@ -729,7 +731,8 @@ detect_kernel(const __grid_constant__ DetectParams p)
 constexpr size_t ROWS_KERNEL_BYTES = 256 << 10;
 
 __global__ void __launch_bounds__(256)
-rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __restrict__ row_count, int take, float * __restrict__ host_rows, int * __restrict__ host_count)
+rows_host_kernel(const float * __restrict__ rows, int max_rows, const int * __restrict__ row_count, int take, float * __restrict__ host_rows,
+		int * __restrict__ host_count)
 {
 	pdl_wait();                                                  // launched while the kernel in front of it, detect_kernel as a rule, finishes
 	const size_t b = blockIdx.y;
@@ -874,7 +877,10 @@ static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int b
 		// half an SM has, 30 / 37 / 47 so; 33 / 39 / 49 before there was a matrix)
 		const bool shared = (long long)batch * DET_CLUSTER > sm_count() && smem <= DET_SMEM_HALF;
 		const size_t room = shared ? max(smem, (size_t)DET_SMEM_SHARED) : DET_SMEM_BUDGET;
-		auto matrix_bytes = [&](int max) { return round_up((size_t)max, 4) * 4 + (size_t)max * (sizeof(float4) + DET_MATRIX_WORDS * 4 + (size_t)want * DET_LIST_BYTES); };
+		auto matrix_bytes = [&](int max)
+		{
+			return round_up((size_t)max, 4) * 4 + (size_t)max * (sizeof(float4) + DET_MATRIX_WORDS * 4 + (size_t)want * DET_LIST_BYTES);
+		};
 		p.matrix_max = min(p.max_dets, DET_MATRIX_MAX);
 		while (matrix_bytes(p.matrix_max) > room) { p.matrix_max = (p.matrix_max - 1) & ~31; }
 		if (p.matrix_max >= p.max_dets) { smem = (size_t)list_bytes; }             // no list goes without it

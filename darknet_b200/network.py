@@ -966,7 +966,7 @@ class DetectionBuffers:
         self.row_count = torch.zeros(batch, dtype=torch.int32, device=device)
         self.desc = capi.Detections(self.boxes.data_ptr(), self.objectness.data_ptr(), self.probs.data_ptr(), self.count.data_ptr(),
                                     max_dets, classes)
-        # where rows_host receives the counts and the first rows: page-locked, so that both copies are queued and waited for once
+        # where rows_host receives the counts and the first rows: page-locked, so that both are queued and waited for once
         self.host_count = torch.empty(batch, dtype=torch.int32, pin_memory=self.rows.is_cuda)
         self._take_rows(512)
 
@@ -977,8 +977,9 @@ class DetectionBuffers:
 
     def rows_host(self) -> List[np.ndarray]:
         """Per image the rows {x, y, w, h, objectness, class, probability}.  The counts and each image's first `take` rows come over
-        together (most frames have fewer: the whole list would be eight times the bytes); a longer list costs a second copy, 40 us with
-        its wait, and widens the first one for the frames to come, which show much the same scene."""
+        in one call, written by a kernel up to 256 KB and by copies beyond (most frames have fewer: the whole list would be eight times the
+        bytes); a longer list costs a copy of its own, 40 us with its wait, and widens `take` for the frames to come, which show much the
+        same scene."""
         stream = torch.cuda.current_stream(self.rows.device)
         capi.check(capi.lib().xnor_b200_rows_to_host(self.rows.data_ptr(), self.max_rows, self.row_count.data_ptr(), self.batch, self.take,
                                                     self.host_rows.data_ptr(), self.host_count.data_ptr(), stream.cuda_stream),

@@ -52,7 +52,7 @@ CASES = [
     (1, 32, 16, 16, 64, 3, 2), (2, 64, 15, 13, 128, 3, 2), (3, 128, 28, 28, 256, 3, 2), (1, 512, 28, 28, 512, 3, 2), (2, 40, 9, 8, 17, 3, 2),
     (1, 32, 8, 16, 32, 1, 1), (1, 1024, 13, 13, 256, 1, 1), (7, 64, 11, 9, 33, 1, 1), (2, 50, 20, 20, 70, 1, 1), (64, 256, 14, 14, 128, 1, 1),
     (2, 64, 9, 7, 32, 1, 2), (1, 288, 28, 28, 64, 1, 2),
-    # one or two tiles a CTA, whose filters the epilogue warps share; 16 channels and fewer, two positions a word
+    # one or two tiles a CTA, whose filters the epilogue warps share; 16 channels and fewer
     (1, 64, 26, 26, 96, 3, 1), (1, 128, 14, 14, 40, 3, 1), (1, 64, 30, 31, 72, 1, 1), (1, 32, 56, 56, 200, 3, 1), (1, 96, 120, 120, 64, 3, 1),
     (1, 16, 7, 9, 32, 3, 1), (3, 16, 208, 33, 32, 3, 1), (2, 9, 30, 62, 64, 3, 1), (1, 16, 1, 1, 160, 3, 1), (64, 15, 26, 26, 33, 3, 1), (2, 17, 20, 20, 32, 3, 1),
     # the last unit begins in the padding row, whose rows of the source lie behind its end
