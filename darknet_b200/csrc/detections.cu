@@ -874,7 +874,8 @@ static int launch_detect(DetectParams & p, const xnor_b200_detections * d, int b
 		smem = round_up((size_t)p.lists * list_bytes, 16) + (size_t)p.lists * box_bytes;
 		// The matrix takes what there is, but not the place of an SM's second CTA where the images are more than the SMs take at once and the
 		// lists leave it (64 images, lists of 768, 13 / 100 / 174 found: 49 / 62 / 78 us with a matrix for all of them, 31 / 41 / 54 with what
-		// half an SM has, 30 / 37 / 47 so; 33 / 39 / 49 before there was a matrix)
+		// half an SM has, 30 / 37 / 47 so; 33 / 39 / 49 before there was a matrix).
+		// Lists beyond it pay where nearly every detection is of nearly every class: 500 of all 80 each 3.4 ms, 0.9 with a matrix for all
 		const bool shared = (long long)batch * DET_CLUSTER > sm_count() && smem <= DET_SMEM_HALF;
 		const size_t room = shared ? max(smem, (size_t)DET_SMEM_SHARED) : DET_SMEM_BUDGET;
 		auto matrix_bytes = [&](int max)
